@@ -133,43 +133,65 @@ __global__ void __launch_bounds__(NT) k_lift(const float* __restrict__ xin, int 
 }
 
 // ------------------------------------------------------------------------------------------------ GN finalize
-__global__ void k_gn_finalize(const double* __restrict__ partials, int nparts, int C, int groups,
-                              const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
-                              float* __restrict__ coefs, double* __restrict__ gstats) {
-  __shared__ double gm[GMAX], gr[GMAX];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  // one warp per group: lane l merges partials l, l + 32, ... in order, then a fixed shuffle tree (deterministic)
-  for (int g = warp; g < groups; g += nw) {
-    GroupAcc a{0.0, 0.0, 0.0};
-    for (int p = lane; p < nparts; p += 32) {
-      const double* q = partials + ((long)p * groups + g) * 3;
-      chan_merge(a, q[0], q[1], q[2]);
-    }
+// One CTA per group, each thread a few partials: the group's mean is the weighted mean of the partials' means, and its
+// M2 the sum of the partials' M2 and of w (mean_p - mean)^2, so the loops hold no division (a serial Chan merge has two
+// dependent FP64 divisions per partial). Bound by latency: two passes over at most a few partials a thread, two
+// block-wide sums in a fixed tree (deterministic), one FP64 division. The groups take a CTA (an SM) each because the
+// FP64 rate of one SM (about two operations a cycle) would serialise eight groups of 304 partials. 304 partials,
+// 8 groups, C = 64: 22.0 us a launch with one warp per group and Chan merges -> 6.6 us (one SM: the groups' FP64 serialised; now a
+// chain of three block sums, a division and a square root).
+constexpr int FIN_NT = 128;
+
+__device__ __forceinline__ double block_sum(double v, double* red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double w = __shfl_down_sync(0xffffffffu, a.w, off);
-      const double m = __shfl_down_sync(0xffffffffu, a.mean, off);
-      const double m2 = __shfl_down_sync(0xffffffffu, a.m2, off);
-      if (lane < off) chan_merge(a, w, m, m2);
-    }
-    if (lane == 0) {
-      const double var = a.w > 0.0 ? a.m2 / a.w : 0.0;
-      const double rstd = 1.0 / sqrt(var + (double)eps);
-      gm[g] = a.mean;
-      gr[g] = rstd;
-      if (gstats) {
-        gstats[3 * g] = a.mean;
-        gstats[3 * g + 1] = rstd;
-        gstats[3 * g + 2] = a.w;
-      }
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  double s = 0.0;
+#pragma unroll
+  for (int w = 0; w < FIN_NT / 32; ++w) s += red[w];
+  return s;
+}
+
+__global__ void __launch_bounds__(FIN_NT) k_gn_finalize(const double* __restrict__ partials, int nparts, int C,
+                                                        int groups, const float* __restrict__ gamma,
+                                                        const float* __restrict__ beta, float eps,
+                                                        float* __restrict__ coefs, double* __restrict__ gstats) {
+  __shared__ double red[3][FIN_NT / 32];
+  const int g = blockIdx.x, tid = threadIdx.x;
+  double w = 0.0, wm = 0.0;
+  for (int p = tid; p < nparts; p += FIN_NT) {
+    const double* q = partials + ((long)p * groups + g) * 3;
+    if (!(q[0] <= 0.0)) {   // a NaN weight counts
+      w += q[0];
+      wm += q[0] * q[1];
     }
   }
-  __syncthreads();
+  const double wt = block_sum(w, red[0]);
+  const double ms = block_sum(wm, red[1]);
+  const double mean = wt == 0.0 ? 0.0 : ms / wt;
+  double m2 = 0.0;
+  for (int p = tid; p < nparts; p += FIN_NT) {
+    const double* q = partials + ((long)p * groups + g) * 3;
+    if (!(q[0] <= 0.0)) {
+      const double d = q[1] - mean;
+      m2 += q[2] + q[0] * d * d;
+    }
+  }
+  m2 = block_sum(m2, red[2]);
+  const double var = wt > 0.0 ? m2 / wt : 0.0;
+  const double rstd = 1.0 / sqrt(var + (double)eps);
+  if (tid == 0 && gstats) {
+    gstats[3 * g] = mean;
+    gstats[3 * g + 1] = rstd;
+    gstats[3 * g + 2] = wt;
+  }
   const int cpg = C / groups;
-  for (int c = tid; c < C; c += blockDim.x) {
-    const int g = c / cpg;
-    coefs[c] = (float)gm[g];
-    coefs[C + c] = (float)((double)gamma[c] * gr[g]);
+  for (int i = tid; i < cpg; i += FIN_NT) {
+    const int c = g * cpg + i;
+    coefs[c] = (float)mean;
+    coefs[C + c] = (float)((double)gamma[c] * rstd);
     coefs[2 * C + c] = beta[c];
   }
 }
@@ -521,7 +543,8 @@ int ffno_gn_finalize(const double* partials, int nparts, int C, int groups, cons
                      float eps, float* coefs, double* gstats, ffno_stream_t stream) {
   if (!partials || !gamma || !beta || !coefs) return FFNO_EINVAL;
   if (nparts < 1 || C < 1 || groups < 1 || groups > GMAX || C % groups) return FFNO_EINVAL;
-  k_gn_finalize<<<1, 512, 0, (cudaStream_t)stream>>>(partials, nparts, C, groups, gamma, beta, eps, coefs, gstats);
+  k_gn_finalize<<<groups, FIN_NT, 0, (cudaStream_t)stream>>>(partials, nparts, C, groups, gamma, beta, eps, coefs,
+                                                             gstats);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
