@@ -33,7 +33,6 @@ int grid_of(long V, int rows, int per_sm) {
 
 template <typename K>
 bool smem_attr(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return true;
   return ffno::smem_cap_ok(kernel, bytes);
 }
 

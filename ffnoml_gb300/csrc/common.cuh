@@ -418,7 +418,7 @@ bool smem_cap_lookup(const void* kernel, size_t* cap);
 
 template <typename K>
 inline bool smem_cap_ok(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return true;
+  if (bytes <= 40 * 1024) return true;   // 48 KB without the attribute, the kernel's static shared memory included
   size_t cap = 0;
   if (!smem_cap_lookup(reinterpret_cast<const void*>(kernel), &cap)) return false;
   return bytes <= cap;

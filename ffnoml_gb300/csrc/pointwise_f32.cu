@@ -5,6 +5,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "gemm_f32.cuh"
 
 using namespace ffno;
 
@@ -32,7 +33,6 @@ int grid_for(long V, int per_sm) {
 
 template <typename K>
 bool set_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return true;
   return ffno::smem_cap_ok(kernel, bytes);
 }
 
@@ -247,225 +247,270 @@ __global__ void k_resid_out(const float* __restrict__ x2, const float* __restric
 }
 
 // ------------------------------------------------------------------------------------------------ input gate
+// 4.2 M voxels, C = 64: 4.65 -> 2.12 ms (32 TFLOP/s), four CTAs an SM.
 template <int C>
-__global__ void __launch_bounds__(NT) k_gate(const float* __restrict__ x, long V, const float* __restrict__ w1,
-                                             const float* __restrict__ w2, const float* __restrict__ zp,
-                                             const float* __restrict__ z, float* __restrict__ out) {
-  extern __shared__ float sm[];
-  constexpr int LD = C + 1;
-  float* xs = sm;
-  float* hs = xs + BM * LD;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+__global__ void __launch_bounds__(NT, C <= 64 ? 4 : 2) k_gate(const float* __restrict__ x, long V, const float* __restrict__ w1,
+                                                const float* __restrict__ w2, const float* __restrict__ zp,
+                                                const float* __restrict__ z, float* __restrict__ out) {
+  extern __shared__ __align__(16) float sm[];
+  float* xs = sm;             // [C][64]
+  float* hs = xs + C * BM;    // [C][64]
+  g32::Ring ring(hs + C * BM, g32::KC * C);
+  using Cl = g32::Cols<C, 1>;
+  const int tx = g32::tile_tx(), ty = g32::tile_ty();
   const long nt = ntiles_of(V);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    load_rows<C>(xs, LD, x, v0, V);
-    __syncthreads();
-    float acc[4][C / 16];
-    tile_mm<C, C>(xs, LD, w1, acc);
+    ring.pre<C>(w1, C);
+    g32::load_tile<C>(xs, 0, x, v0, V);
+    float acc[C / 16][4];
+    g32::gemm<C, C>(xs, 0, w1, C, ring, acc);
+    ring.pre<C>(w2, C);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < C / 16; ++j) {
+      float h[4];
 #pragma unroll
-      for (int j = 0; j < C / 16; ++j) hs[(ty + 16 * i) * LD + tx + 16 * j] = gelu(acc[i][j]);
-    __syncthreads();
-    tile_mm<C, C>(hs, LD, w2, acc);
+      for (int e = 0; e < 4; ++e) h[e] = gelu(acc[j][e]);
+      g32::put4(hs, Cl::col(tx, j), h);
+    }
+    g32::gemm<C, C>(hs, 0, w2, C, ring, acc);
+    float zv[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty + 16 * i;
-      const long v = v0 + r;
-      if (v >= V) continue;
-      const float zv = zp ? __ldg(z + v) : 0.f;
+    for (int e = 0; e < 4; ++e) {
+      const long v = v0 + 4 * ty + e;
+      zv[e] = zp && v < V ? __ldg(z + v) : 0.f;
+    }
 #pragma unroll
-      for (int j = 0; j < C / 16; ++j) {
-        const int c = tx + 16 * j;
-        float o = xs[r * LD + c] * sigmoid(acc[i][j]);
-        if (zp) o += __ldg(zp + c) * zv;
-        out[v * C + c] = o;
+    for (int j = 0; j < C / 16; ++j) {
+      const int c = Cl::col(tx, j);
+      float xv[4];
+      g32::get4(xs, c, xv);
+      const float zc = zp ? __ldg(zp + c) : 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float o = xv[e] * sigmoid(acc[j][e]);
+        acc[j][e] = zp ? o + zc * zv[e] : o;
       }
     }
+    g32::store_rows<C>(out, nullptr, v0, V, acc);
   }
 }
 
 // ------------------------------------------------------------------------------------------------ 2-layer MLP
+// The hidden layer overwrites the input tile's region (2C channels), so a tile takes 2C x 64 floats plus the weight
+// ring: 48 KB at C = 64. Bound by instruction issue (FMAs, erff) at two CTAs an SM, the grid of the partials. 4.2 M
+// voxels, C = 64: 7.1 -> 4.35 ms (31 TFLOP/s); 296 k voxels, C = 96: 861 -> 577 us.
+template <int C>
+constexpr size_t mlp2_smem() {
+  return (2 * C * BM + 2 * g32::KC * 2 * C) * sizeof(float);
+}
+
 template <int C, int MODE>
-__global__ void __launch_bounds__(NT) k_mlp2(const float* __restrict__ in, const float* __restrict__ prev_pre,
-                                             const float* __restrict__ pc, float res, float* __restrict__ xout,
-                                             long V, const float* __restrict__ w1, const float* __restrict__ w2,
-                                             const float* __restrict__ dw, float* __restrict__ pre,
-                                             double* __restrict__ partials, int cpg, int groups) {
-  extern __shared__ float sm[];
-  constexpr int LA = C + 1, LH = 2 * C + 1;
-  float* as = sm;
-  float* hs = as + BM * LA;
-  StatsSmem<C>& st = *reinterpret_cast<StatsSmem<C>*>(hs + BM * LH);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+__global__ void __launch_bounds__(NT, 2) k_mlp2(const float* __restrict__ in, const float* __restrict__ prev_pre,
+                                                const float* __restrict__ pc, float res, float* __restrict__ xout,
+                                                long V, const float* __restrict__ w1, const float* __restrict__ w2,
+                                                const float* __restrict__ dw, float* __restrict__ pre,
+                                                double* __restrict__ partials, int cpg, int groups) {
+  extern __shared__ __align__(16) float sm[];
+  __shared__ g32::TileStats<C> st;
+  float* as = sm;   // [C][64] input, then [2C][64] hidden
+  g32::Ring ring(as + 2 * C * BM, g32::KC * 2 * C);
+  using Ch = g32::Cols<2 * C, 1>;
+  const int tx = g32::tile_tx(), ty = g32::tile_ty();
   GroupAcc acc_g{0.0, 0.0, 0.0};
   const long nt = ntiles_of(V);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    load_rows<C>(as, LA, in, v0, V);
-    if (MODE != 0) {
-      __syncthreads();
-      for (int e = threadIdx.x; e < BM * C; e += NT) {
-        const int r = e / C, c = e % C;
-        const long v = v0 + r;
-        if (v >= V) continue;
-        float y = (__ldg(prev_pre + v * C + c) - pc[c]) * pc[C + c] + pc[2 * C + c];
-        if (MODE == 1) y = gelu(y);
-        const float a = as[r * LA + c] + res * y;
-        as[r * LA + c] = a;
-        xout[v * C + c] = a;
+    ring.pre<2 * C>(w1, 2 * C);
+    g32::each_quad<C>(v0, V, [&](int r, int c, long o, bool ok) {
+      float4 a = g32::ldq(in + o, ok);
+      if (MODE != 0 && ok) {
+        float4 y = gn4(__ldg(reinterpret_cast<const float4*>(prev_pre + o)), pc, C, c);
+        if (MODE == 1) y = make_float4(gelu(y.x), gelu(y.y), gelu(y.z), gelu(y.w));
+        a = make_float4(a.x + res * y.x, a.y + res * y.y, a.z + res * y.z, a.w + res * y.w);
+        *reinterpret_cast<float4*>(xout + o) = a;
       }
-    }
-    __syncthreads();
+      g32::put_quad(as, r, c, a);
+    });
     {
-      float acc[4][2 * C / 16];
-      tile_mm<C, 2 * C>(as, LA, w1, acc);
+      float h[2 * C / 16][4];
+      g32::gemm<C, 2 * C>(as, 0, w1, 2 * C, ring, h);
+      ring.pre<C>(w2, C);
+      __syncthreads();   // every read of the input tile is done
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 2 * C / 16; ++j) {
 #pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) hs[(ty + 16 * i) * LH + tx + 16 * j] = gelu(acc[i][j]);
-    }
-    __syncthreads();
-    float acc[4][C / 16], wr[4];
-    tile_mm<2 * C, C>(hs, LH, w2, acc);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long v = v0 + ty + 16 * i;
-      wr[i] = v < V ? __ldg(dw + v) : 0.f;
-      if (v < V) {
-#pragma unroll
-        for (int j = 0; j < C / 16; ++j) pre[v * C + tx + 16 * j] = acc[i][j];
+        for (int e = 0; e < 4; ++e) h[j][e] = gelu(h[j][e]);
+        g32::put4(as, Ch::col(tx, j), h[j]);
       }
     }
-    tile_group_stats<C>(acc, wr, cpg, groups, st, acc_g);
+    float acc[C / 16][4], wr[4];
+    g32::gemm<2 * C, C>(as, 0, w2, C, ring, acc);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const long v = v0 + 4 * ty + e;
+      wr[e] = v < V ? __ldg(dw + v) : 0.f;
+    }
+    g32::store_rows<C>(pre, nullptr, v0, V, acc);
+    g32::tile_stats<C>(acc, wr, cpg, groups, st, acc_g);
   }
-  write_partial(partials, groups, acc_g);
+  g32::write_tile_partial(partials, groups, acc_g);
 }
 
 // ------------------------------------------------------------------------------------------------ gate + fuse
+// One region of 3C channels: [x | spec | vert], then the gate hidden layer over x, the gated branches in place, and the
+// fuse hidden layer over the gated branches (their residual half-sum waits in registers): 64 KB at C = 64. 4.2 M voxels,
+// C = 64: 24.1 -> 10.5 ms (36 TFLOP/s); 296 k voxels, C = 96: 3.90 -> 1.49 ms.
 template <int C>
-__global__ void __launch_bounds__(NT) k_fuse(const float* __restrict__ x, const float* __restrict__ sp,
-                                             const float* __restrict__ sc, const float* __restrict__ vp,
-                                             const float* __restrict__ vc, long V, const float* __restrict__ wg1,
-                                             const float* __restrict__ wg2, const float* __restrict__ bg2,
-                                             const float* __restrict__ wf1, const float* __restrict__ wf2,
-                                             const float* __restrict__ dw, float* __restrict__ pre,
-                                             double* __restrict__ partials, int cpg, int groups) {
-  extern __shared__ float sm[];
-  constexpr int LA = 3 * C + 1, LH = 2 * C + 1;
+constexpr size_t fuse_smem() {
+  return (3 * C * BM + 2 * g32::KC * 2 * C) * sizeof(float);
+}
+
+template <int C>
+__global__ void __launch_bounds__(NT, 2) k_fuse(const float* __restrict__ x, const float* __restrict__ sp,
+                                                const float* __restrict__ sc, const float* __restrict__ vp,
+                                                const float* __restrict__ vc, long V, const float* __restrict__ wg1,
+                                                const float* __restrict__ wg2, const float* __restrict__ bg2,
+                                                const float* __restrict__ wf1, const float* __restrict__ wf2,
+                                                const float* __restrict__ dw, float* __restrict__ pre,
+                                                double* __restrict__ partials, int cpg, int groups) {
+  extern __shared__ __align__(16) float sm[];
+  __shared__ g32::TileStats<C> st;
   float* as = sm;
-  float* hs = as + BM * LA;
-  StatsSmem<C>& st = *reinterpret_cast<StatsSmem<C>*>(hs + BM * LH);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  g32::Ring ring(as + 3 * C * BM, g32::KC * 2 * C);
+  using C1 = g32::Cols<C, 1>;
+  using C2 = g32::Cols<2 * C, 2>;   // the thread owns channel c of both branches
+  using Ch = g32::Cols<2 * C, 1>;
+  const int tx = g32::tile_tx(), ty = g32::tile_ty();
   GroupAcc acc_g{0.0, 0.0, 0.0};
   const long nt = ntiles_of(V);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    for (int e = threadIdx.x; e < BM * C; e += NT) {
-      const int r = e / C, c = e % C;
-      const long v = v0 + r;
-      float a = 0.f, s = 0.f, q = 0.f;
-      if (v < V) {
-        a = __ldg(x + v * C + c);
-        s = gelu((__ldg(sp + v * C + c) - sc[c]) * sc[C + c] + sc[2 * C + c]);
-        q = gelu((__ldg(vp + v * C + c) - vc[c]) * vc[C + c] + vc[2 * C + c]);
+    ring.pre<C>(wg1, C);
+    g32::each_quad<C>(v0, V, [&](int r, int c, long o, bool ok) {
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f), q = s;
+      if (ok) {
+        s = gn4(__ldg(reinterpret_cast<const float4*>(sp + o)), sc, C, c);
+        q = gn4(__ldg(reinterpret_cast<const float4*>(vp + o)), vc, C, c);
+        s = make_float4(gelu(s.x), gelu(s.y), gelu(s.z), gelu(s.w));
+        q = make_float4(gelu(q.x), gelu(q.y), gelu(q.z), gelu(q.w));
       }
-      as[r * LA + c] = a;
-      as[r * LA + C + c] = s;
-      as[r * LA + 2 * C + c] = q;
-    }
-    __syncthreads();
+      g32::put_quad(as, r, c, g32::ldq(x + o, ok));
+      g32::put_quad(as, r, C + c, s);
+      g32::put_quad(as, r, 2 * C + c, q);
+    });
     {
-      float acc[4][C / 16];
-      tile_mm<3 * C, C>(as, LA, wg1, acc);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < C / 16; ++j) hs[(ty + 16 * i) * LH + tx + 16 * j] = gelu(acc[i][j]);
-    }
-    __syncthreads();
-    {
-      float acc[4][2 * C / 16];
-      tile_mm<C, 2 * C>(hs, LH, wg2, acc);
-      // gates multiply spec (columns C..2C) and vert (2C..3C) in place: column n of the gates -> as[:, C + n]
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) {
-          const int n = tx + 16 * j;
-          as[(ty + 16 * i) * LA + C + n] *= sigmoid(acc[i][j] + __ldg(bg2 + n));
-        }
-    }
-    __syncthreads();
-    {
-      float acc[4][2 * C / 16];
-      tile_mm<2 * C, 2 * C>(as + C, LA, wf1, acc);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) hs[(ty + 16 * i) * LH + tx + 16 * j] = gelu(acc[i][j]);
-    }
-    __syncthreads();
-    float acc[4][C / 16], wr[4];
-    tile_mm<2 * C, C>(hs, LH, wf2, acc);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty + 16 * i;
-      const long v = v0 + r;
-      wr[i] = v < V ? __ldg(dw + v) : 0.f;
+      float h[C / 16][4];
+      g32::gemm<3 * C, C>(as, 0, wg1, C, ring, h);
+      ring.pre<2 * C>(wg2, 2 * C);
+      __syncthreads();   // every read of x is done
 #pragma unroll
       for (int j = 0; j < C / 16; ++j) {
-        const int c = tx + 16 * j;
-        acc[i][j] += 0.5f * (as[r * LA + C + c] + as[r * LA + 2 * C + c]);
-        if (v < V) pre[v * C + c] = acc[i][j];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[j][e] = gelu(h[j][e]);
+        g32::put4(as, C1::col(tx, j), h[j]);
       }
     }
-    tile_group_stats<C>(acc, wr, cpg, groups, st, acc_g);
+    float half[C / 16][4];
+    {
+      float g[2 * C / 16][4];
+      g32::gemm<C, 2 * C, 2>(as, 0, wg2, 2 * C, ring, g);
+      ring.pre<2 * C>(wf1, 2 * C);
+      // the gates multiply spec and vert in place: gate channel n belongs to region channel C + n
+#pragma unroll
+      for (int j = 0; j < 2 * C / 16; ++j) {
+        const int n = C2::col(tx, j);
+        const float b = __ldg(bg2 + n);
+        float a[4];
+        g32::get4(as, C + n, a);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g[j][e] = a[e] * sigmoid(g[j][e] + b);
+        g32::put4(as, C + n, g[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < C / 16; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) half[j][e] = 0.5f * (g[j][e] + g[j + C / 16][e]);
+    }
+    {
+      float h[2 * C / 16][4];
+      g32::gemm<2 * C, 2 * C>(as, C, wf1, 2 * C, ring, h);
+      ring.pre<C>(wf2, C);
+      __syncthreads();   // every read of the gated branches is done
+#pragma unroll
+      for (int j = 0; j < 2 * C / 16; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[j][e] = gelu(h[j][e]);
+        g32::put4(as, Ch::col(tx, j), h[j]);
+      }
+    }
+    float acc[C / 16][4], wr[4];
+    g32::gemm<2 * C, C>(as, 0, wf2, C, ring, acc);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const long v = v0 + 4 * ty + e;
+      wr[e] = v < V ? __ldg(dw + v) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < C / 16; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[j][e] += half[j][e];
+    g32::store_rows<C>(pre, nullptr, v0, V, acc);
+    g32::tile_stats<C>(acc, wr, cpg, groups, st, acc_g);
   }
-  write_partial(partials, groups, acc_g);
+  g32::write_tile_partial(partials, groups, acc_g);
 }
 
 // ------------------------------------------------------------------------------------------------ head
 
+// The chain's two GEMMs as in the MLPs, then one thread a voxel for the level-fraction head, bound by its FP64 (log-softmax
+// and LTE weights in double). 4.2 M voxels, C = 64, 12 levels: 8.5 -> 7.3 ms; 296 k voxels, C = 96: 1.11 -> 0.53 ms.
 // kLte = false: FFNO3D._run_head alone (models/ffno_model.py:790-798), the head channels into head_out, no LTE head.
 template <int C, int NHP, typename T, bool kLte = true>
-__global__ void __launch_bounds__(NT) k_head(const float* __restrict__ x, const float* __restrict__ xin, long V,
+__global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, const float* __restrict__ xin, long V,
                                              const float* __restrict__ p1, const float* __restrict__ p2,
                                              const float* __restrict__ b2, int nh,
                                              const __grid_constant__ ffno_head_params hp, float* __restrict__ out,
                                              float* __restrict__ head_out) {
-  extern __shared__ float sm[];
-  constexpr int LA = C + 1, LH = 2 * C + 1, LO = NHP + 1;
-  float* as = sm;
-  float* hs = as + BM * LA;
-  float* os = hs + BM * LH;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  extern __shared__ __align__(16) float sm[];
+  constexpr int LO = NHP + 1;
+  float* as = sm;                    // [C][64] input, then [2C][64] hidden
+  float* os = as + 2 * C * BM;       // [64][NHP + 1] head channels
+  g32::Ring ring(os + BM * LO, g32::KC * 2 * C);
+  using Ch = g32::Cols<2 * C, 1>;
+  using Co = g32::Cols<NHP, 1>;
+  const int tx = g32::tile_tx(), ty = g32::tile_ty();
   const long nt = ntiles_of(V);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    load_rows<C>(as, LA, x, v0, V);
-    __syncthreads();
+    ring.pre<2 * C>(p1, 2 * C);
+    g32::load_tile<C>(as, 0, x, v0, V);
     {
-      float acc[4][2 * C / 16];
-      tile_mm<C, 2 * C>(as, LA, p1, acc);
+      float h[2 * C / 16][4];
+      g32::gemm<C, 2 * C>(as, 0, p1, 2 * C, ring, h);
+      ring.pre<NHP>(p2, NHP);
+      __syncthreads();   // every read of the input tile is done
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 2 * C / 16; ++j) {
 #pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) hs[(ty + 16 * i) * LH + tx + 16 * j] = gelu(acc[i][j]);
+        for (int e = 0; e < 4; ++e) h[j][e] = gelu(h[j][e]);
+        g32::put4(as, Ch::col(tx, j), h[j]);
+      }
     }
-    __syncthreads();
     {
-      float acc[4][NHP / 16];
-      tile_mm<2 * C, NHP>(hs, LH, p2, acc);
+      float acc[NHP / 16][4];
+      g32::gemm<2 * C, NHP>(as, 0, p2, NHP, ring, acc);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < NHP / 16; ++j) {
+        const int n = Co::col(tx, j);
+        const float b = __ldg(b2 + n);
 #pragma unroll
-        for (int j = 0; j < NHP / 16; ++j) os[(ty + 16 * i) * LO + tx + 16 * j] = acc[i][j] + __ldg(b2 + tx + 16 * j);
+        for (int e = 0; e < 4; ++e) os[(4 * ty + e) * LO + n] = acc[j][e] + b;
+      }
     }
     __syncthreads();
     if (threadIdx.x < BM) {
@@ -582,12 +627,12 @@ int ffno_gate_fwd(const float* x, long V, int C, const float* w1, const float* w
                   float* out, ffno_stream_t stream) {
   if (!x || !w1 || !w2 || !out || !width_ok(C) || V < 1 || (zp && !z)) return FFNO_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
-  const size_t smem = 2 * BM * (C + 1) * sizeof(float);
+  const size_t smem = (2 * BM * C + 2 * g32::KC * C) * sizeof(float);
   switch (C) {
 #define L(CC)                                                                   \
   case CC:                                                                      \
     if (!set_smem(k_gate<CC>, smem)) return FFNO_ELAUNCH;                       \
-    k_gate<CC><<<grid_for(V, 2), NT, smem, s>>>(x, V, w1, w2, zp, z, out);      \
+    k_gate<CC><<<grid_for(V, CC <= 64 ? 4 : 2), NT, smem, s>>>(x, V, w1, w2, zp, z, out);      \
     break;
     L(16) L(32) L(64) L(96)
 #undef L
@@ -608,7 +653,7 @@ int ffno_mlp2_fwd(int mode, const float* in, const float* prev_pre, const float*
   switch (C) {
 #define L(CC)                                                                                          \
   case CC: {                                                                                           \
-    const size_t smem = (BM * (CC + 1) + BM * (2 * CC + 1)) * sizeof(float) + sizeof(StatsSmem<CC>);   \
+    const size_t smem = mlp2_smem<CC>();                                                               \
     if (mode == 0) {                                                                                   \
       if (!set_smem(k_mlp2<CC, 0>, smem)) return FFNO_ELAUNCH;                                         \
       k_mlp2<CC, 0><<<nparts, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,   \
@@ -645,7 +690,7 @@ int ffno_fuse_fwd(const float* x, const float* spec_pre, const float* spec_coefs
   switch (C) {
 #define L(CC)                                                                                                \
   case CC: {                                                                                                 \
-    const size_t smem = (BM * (3 * CC + 1) + BM * (2 * CC + 1)) * sizeof(float) + sizeof(StatsSmem<CC>);     \
+    const size_t smem = fuse_smem<CC>();                                                                     \
     if (!set_smem(k_fuse<CC>, smem)) return FFNO_ELAUNCH;                                                    \
     k_fuse<CC><<<nparts, NT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre, vert_coefs, V, wg1, wg2, bg2, wf1, \
                                         wf2, dw, pre, partials, cpg, groups);                                \
@@ -671,7 +716,7 @@ int ffno_head_fwd(const float* x, const float* x_in, long V, int C, const float*
   switch (C) {
 #define L(CC, NN)                                                                                       \
   if (C == CC && nhp == NN) {                                                                           \
-    const size_t smem = (BM * (CC + 1) + BM * (2 * CC + 1) + BM * (NN + 1)) * sizeof(float);            \
+    const size_t smem = (2 * CC * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);            \
     if (params->math32) {                                                                               \
       if (!set_smem(k_head<CC, NN, float>, smem)) return FFNO_ELAUNCH;                                  \
       k_head<CC, NN, float><<<grid_for(V, 2), NT, smem, s>>>(x, x_in, V, p1, p2, b2, nh, *params, out, head_out); \
@@ -697,7 +742,7 @@ int ffno_proj_fwd(const float* x, long V, int C, const float* p1, const float* p
   switch (C) {
 #define L(CC, NN)                                                                                       \
   if (C == CC && nhp == NN) {                                                                           \
-    const size_t smem = (BM * (CC + 1) + BM * (2 * CC + 1) + BM * (NN + 1)) * sizeof(float);            \
+    const size_t smem = (2 * CC * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);            \
     if (!set_smem(k_head<CC, NN, float, false>, smem)) return FFNO_ELAUNCH;                             \
     k_head<CC, NN, float, false><<<grid_for(V, 2), NT, smem, s>>>(x, nullptr, V, p1, p2, b2, nh, none,  \
                                                                   nullptr, head);                       \
