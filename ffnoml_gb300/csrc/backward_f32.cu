@@ -6,6 +6,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "gemm_f32.cuh"
 #include "tc.cuh"
 
 using namespace ffno;
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats(int mode, const float* __r
                                                       const float* __restrict__ pre, const float* __restrict__ gamma,
                                                       const float* __restrict__ beta,
                                                       const double* __restrict__ gst, long V,
-                                                      double* __restrict__ partials, int cpg, int groups) {
+                                                      double* __restrict__ partials, int nparts, int cpg, int groups) {
   using Ln = GnLanes<C, 4>;
   __shared__ GnConst k;
   __shared__ double red[8][GMAX][2];
@@ -197,6 +198,8 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats(int mode, const float* __r
     }
     partials[((long)blockIdx.x * groups + threadIdx.x) * 2] = a;
     partials[((long)blockIdx.x * groups + threadIdx.x) * 2 + 1] = b;
+    for (long p = blockIdx.x + gridDim.x; p < nparts; p += gridDim.x)   // rows past the grid: nothing to add
+      partials[(p * groups + threadIdx.x) * 2] = partials[(p * groups + threadIdx.x) * 2 + 1] = 0.0;
   }
 }
 
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats8(int mode, const float* __
                                                        const float* __restrict__ pre, const float* __restrict__ gamma,
                                                        const float* __restrict__ beta,
                                                        const double* __restrict__ gst, long V,
-                                                       double* __restrict__ partials) {
+                                                       double* __restrict__ partials, int nparts) {
   static_assert(C == 16 || C == 32 || C == 64, "eight groups of C / 8 channels");
   using Ln = GnLanes<C, 8>;
   constexpr int VW = 8, CPG = C / GMAX, NG = VW / CPG;
@@ -298,6 +301,8 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats8(int mode, const float* __
     }
     partials[((long)blockIdx.x * GMAX + threadIdx.x) * 2] = a;
     partials[((long)blockIdx.x * GMAX + threadIdx.x) * 2 + 1] = b;
+    for (long p = blockIdx.x + gridDim.x; p < nparts; p += gridDim.x)   // rows past the grid: nothing to add
+      partials[(p * GMAX + threadIdx.x) * 2] = partials[(p * GMAX + threadIdx.x) * 2 + 1] = 0.0;
   }
 }
 
@@ -381,315 +386,295 @@ __global__ void __launch_bounds__(256, 4) k_gn_bwd_apply(int mode, const float* 
 }
 
 // ------------------------------------------------------------------------------------------------ MLP backward
-// pre = gelu(a W1) W2; given pre_bar: a_bar = base + ((pre_bar W2^T) * gelu'(a W1)) W1^T.
+// pre = gelu(a W1) W2; given pre_bar: a_bar = base + ((pre_bar W2^T) * gelu'(a W1)) W1^T. The hidden gradient overwrites
+// the two input tiles (2C channels). 524 k voxels, C = 64: 1.21 -> 0.70 ms (37 TFLOP/s).
 template <int C>
-__global__ void __launch_bounds__(NT) k_mlp2_bwd(const float* __restrict__ a, const float* __restrict__ pb,
-                                                 const float* __restrict__ base, long V, const float* __restrict__ w1,
-                                                 const float* __restrict__ w2t, const float* __restrict__ w1t,
-                                                 float* __restrict__ abar) {
-  extern __shared__ float sm[];
-  constexpr int LA = C + 1, LH = 2 * C + 1;
-  float* as = sm;
-  float* ps = as + BM * LA;
-  float* hs = ps + BM * LA;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+__global__ void __launch_bounds__(NT, 2) k_mlp2_bwd(const float* __restrict__ a, const float* __restrict__ pb,
+                                                    const float* __restrict__ base, long V,
+                                                    const float* __restrict__ w1, const float* __restrict__ w2t,
+                                                    const float* __restrict__ w1t, float* __restrict__ abar, int al) {
+  extern __shared__ __align__(16) float sm[];
+  float* as = sm;   // [C][64] a, [C][64] pre_bar, then [2C][64] the hidden gradient
+  g32::Ring ring(as + 2 * C * BM, g32::KC * 2 * C, al);
+  using Ch = g32::Cols<2 * C, 1>;
+  const int tx = g32::tile_tx();
   const long nt = ntiles(V, BM);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    load_rows<C>(as, LA, a, v0, V);
-    load_rows<C>(ps, LA, pb, v0, V);
-    __syncthreads();
+    ring.pre<2 * C>(w1, 2 * C);
+    g32::load_tile<C>(as, 0, a, v0, V, al);
+    g32::load_tile<C>(as, C, pb, v0, V, al);
     {
-      float hp[4][2 * C / 16], gb[4][2 * C / 16];
-      tile_mm<C, 2 * C>(as, LA, w1, hp);
-      tile_mm<C, 2 * C>(ps, LA, w2t, gb);
+      float hp[2 * C / 16][4], gb[2 * C / 16][4];
+      g32::gemm<C, 2 * C>(as, 0, w1, 2 * C, ring, hp);
+      ring.pre<2 * C>(w2t, 2 * C);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 2 * C / 16; ++j)
 #pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) hs[(ty + 16 * i) * LH + tx + 16 * j] = gb[i][j] * gelu_grad(hp[i][j]);
-    }
-    __syncthreads();
-    float acc[4][C / 16];
-    tile_mm<2 * C, C>(hs, LH, w1t, acc);
+        for (int e = 0; e < 4; ++e) hp[j][e] = gelu_grad(hp[j][e]);
+      g32::gemm<C, 2 * C>(as, C, w2t, 2 * C, ring, gb);
+      ring.pre<C>(w1t, C);
+      __syncthreads();   // every read of the input tiles is done
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long v = v0 + ty + 16 * i;
-      if (v >= V) continue;
+      for (int j = 0; j < 2 * C / 16; ++j) {
 #pragma unroll
-      for (int j = 0; j < C / 16; ++j) {
-        const int c = tx + 16 * j;
-        abar[v * C + c] = acc[i][j] + (base ? __ldg(base + v * C + c) : 0.f);
+        for (int e = 0; e < 4; ++e) gb[j][e] *= hp[j][e];
+        g32::put4(as, Ch::col(tx, j), gb[j]);
       }
     }
+    float acc[C / 16][4];
+    g32::gemm<2 * C, C>(as, 0, w1t, C, ring, acc);
+    g32::store_rows<C>(abar, base, v0, V, acc, al);
   }
 }
 
 // ------------------------------------------------------------------------------------------------ fuse backward
 // Recomputes the gate/fuse chain of the tile and back-propagates fused_pre_bar (= pb) to x, spec and vert
-// (FFNOBlock3dBalanced._fuse_branches, models/ffno_model.py:524-534).
-template <int C, int RM>
-__global__ void __launch_bounds__(NT) k_fuse_bwd(
+// (FFNOBlock3dBalanced._fuse_branches, models/ffno_model.py:524-534). Three regions: X [C] holds x, then the gate hidden
+// layer, pb, the gate hidden gradient; SV [2C] holds spec | vert, then their gated gradients; T [2C] holds each GEMM's
+// operand in between. 80 KB and the 16 KB ring at C = 64: two CTAs an SM. 524 k voxels, C = 64: 5.51 -> 2.34 ms.
+template <int C>
+constexpr size_t fuse_bwd_smem() {
+  return (5 * C * BM + 2 * g32::KC * 2 * C) * sizeof(float);
+}
+
+template <int C>
+__global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_fuse_bwd(
     const float* __restrict__ x, const float* __restrict__ sp, const float* __restrict__ sc,
     const float* __restrict__ vp, const float* __restrict__ vc, const float* __restrict__ pb,
     const float* __restrict__ base, long V, const float* __restrict__ wg1, const float* __restrict__ wg2,
     const float* __restrict__ bg2, const float* __restrict__ wf1, const float* __restrict__ wf2t,
     const float* __restrict__ wf1t, const float* __restrict__ wg2t, const float* __restrict__ wg1t,
-    float* __restrict__ xbar, float* __restrict__ sbar, float* __restrict__ vbar) {
-  extern __shared__ float sm[];
-  constexpr int R = 16 * RM;
-  constexpr int LA = 3 * C + 1, L1 = C + 1, L2 = 2 * C + 1;
-  float* SA = sm;              // [R][3C]  x | spec | vert
-  float* SH1 = SA + R * LA;    // [R][C]   branch-gate hidden pre-activation, later its gradient
-  float* SG = SH1 + R * L1;    // [R][2C]  gates
-  float* SH2 = SG + R * L2;    // [R][2C]  fuse hidden pre-activation, later its gradient
-  float* ST = SH2 + R * L2;    // [R][2C]  GEMM operand scratch
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const long nt = ntiles(V, R);
+    float* __restrict__ xbar, float* __restrict__ sbar, float* __restrict__ vbar, int al) {
+  extern __shared__ __align__(16) float sm[];
+  float* X = sm;                 // channels 0 .. C - 1 of the region [x | spec | vert]
+  float* T = X + 3 * C * BM;
+  g32::Ring ring(T + 2 * C * BM, g32::KC * 2 * C, al);
+  constexpr int N1 = C / 16, N2 = 2 * C / 16;
+  using C1 = g32::Cols<C, 1>;
+  using C2 = g32::Cols<2 * C, 2>;   // the thread owns channel c of both branches
+  using Ch = g32::Cols<2 * C, 1>;
+  const int tx = g32::tile_tx();
+  const long nt = ntiles(V, BM);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
-    const long v0 = t * R;
+    const long v0 = t * BM;
     __syncthreads();
-    for (int e = threadIdx.x; e < R * C; e += NT) {
-      const int r = e / C, c = e % C;
-      const long v = v0 + r;
-      float a = 0.f, s = 0.f, q = 0.f, f = 0.f;
-      if (v < V) {
-        a = __ldg(x + v * C + c);
-        s = gelu((__ldg(sp + v * C + c) - sc[c]) * sc[C + c] + sc[2 * C + c]);
-        q = gelu((__ldg(vp + v * C + c) - vc[c]) * vc[C + c] + vc[2 * C + c]);
-        f = __ldg(pb + v * C + c);
+    ring.pre<C>(wg1, C);
+    g32::each_quad<C>(v0, V, [&](int r, int c, long o, bool ok) {
+      const float4 ps = g32::ldq(sp + o, ok, al), pv = g32::ldq(vp + o, ok, al);
+      const float as[4] = {ps.x, ps.y, ps.z, ps.w}, av[4] = {pv.x, pv.y, pv.z, pv.w};
+      g32::put_quad(X, r, c, g32::ldq(x + o, ok, al));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        X[g32::at(r, C + c + i)] =
+            ok ? gelu((as[i] - __ldg(sc + c + i)) * __ldg(sc + C + c + i) + __ldg(sc + 2 * C + c + i)) : 0.f;
+        X[g32::at(r, 2 * C + c + i)] =
+            ok ? gelu((av[i] - __ldg(vc + c + i)) * __ldg(vc + C + c + i) + __ldg(vc + 2 * C + c + i)) : 0.f;
       }
-      SA[r * LA + c] = a;
-      SA[r * LA + C + c] = s;
-      SA[r * LA + 2 * C + c] = q;
-      SH2[r * L2 + c] = f;  // fused_pre_bar parked in SH2 until step 4
-    }
+    });
+    // 1. branch-gate hidden layer: its gelu' stays in registers, its gelu replaces x
+    float h1[N1][4];
+    g32::gemm<3 * C, C>(X, 0, wg1, C, ring, h1);
+    ring.pre<2 * C>(wg2, 2 * C);
     __syncthreads();
-    // 1. branch-gate hidden
-    {
-      float acc[RM][C / 16];
-      tile_mm<3 * C, C, RM>(SA, LA, wg1, acc);
 #pragma unroll
-      for (int i = 0; i < RM; ++i)
+    for (int j = 0; j < N1; ++j) {
+      float h[4];
 #pragma unroll
-        for (int j = 0; j < C / 16; ++j) {
-          const int o = (ty + 16 * i);
-          SH1[o * L1 + tx + 16 * j] = acc[i][j];
-          ST[o * L2 + tx + 16 * j] = gelu(acc[i][j]);
-        }
-    }
-    __syncthreads();
-    // 2. gates
-    {
-      float acc[RM][2 * C / 16];
-      tile_mm<C, 2 * C, RM>(ST, L2, wg2, acc);
-#pragma unroll
-      for (int i = 0; i < RM; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) {
-          const int n = tx + 16 * j;
-          SG[(ty + 16 * i) * L2 + n] = sigmoid(acc[i][j] + __ldg(bg2 + n));
-        }
-    }
-    __syncthreads();
-    // 3. mixed branches B = [spec g_s, vert g_v] -> ST; fused_pre_bar moves to ST's right half is not needed:
-    //    keep F in registers of the thread that owns it below
-    float fb[RM][C / 16];
-#pragma unroll
-    for (int i = 0; i < RM; ++i)
-#pragma unroll
-      for (int j = 0; j < C / 16; ++j) fb[i][j] = SH2[(ty + 16 * i) * L2 + tx + 16 * j];
-#pragma unroll
-    for (int i = 0; i < RM; ++i)
-#pragma unroll
-      for (int j = 0; j < 2 * C / 16; ++j) {
-        const int r = ty + 16 * i, n = tx + 16 * j;
-        ST[r * L2 + n] = SA[r * LA + C + n] * SG[r * L2 + n];
+      for (int e = 0; e < 4; ++e) {
+        h[e] = gelu(h1[j][e]);
+        h1[j][e] = gelu_grad(h1[j][e]);
       }
-    __syncthreads();
-    // 4. fuse hidden pre-activation -> registers; then F (fused_pre_bar) into ST for the next GEMM
-    float hf[RM][2 * C / 16];
-    tile_mm<2 * C, 2 * C, RM>(ST, L2, wf1, hf);
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < RM; ++i)
-#pragma unroll
-      for (int j = 0; j < C / 16; ++j) ST[(ty + 16 * i) * L2 + tx + 16 * j] = fb[i][j];
-    __syncthreads();
-    // 5. fuse hidden gradient (times gelu') -> SH2
-    {
-      float acc[RM][2 * C / 16];
-      tile_mm<C, 2 * C, RM>(ST, L2, wf2t, acc);
-#pragma unroll
-      for (int i = 0; i < RM; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) SH2[(ty + 16 * i) * L2 + tx + 16 * j] = acc[i][j] * gelu_grad(hf[i][j]);
+      g32::put4(X, C1::col(tx, j), h);
     }
-    __syncthreads();
-    // 6. B_bar = SH2 Wf1^T + 0.5 [F, F]; branch grads (registers) and the gate pre-activation grad -> ST
-    float br[RM][2 * C / 16];
+    // 2. gates (registers) and the mixed branches [spec g_s, vert g_v] -> T
+    float g[N2][4];
+    g32::gemm<C, 2 * C, 2>(X, 0, wg2, 2 * C, ring, g);
+    ring.pre<2 * C>(wf1, 2 * C);
+#pragma unroll
+    for (int j = 0; j < N2; ++j) {
+      const int n = C2::col(tx, j);
+      const float b = __ldg(bg2 + n);
+      float a[4];
+      g32::get4(X, C + n, a);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        g[j][e] = sigmoid(g[j][e] + b);
+        a[e] *= g[j][e];
+      }
+      g32::put4(T, n, a);
+    }
+    // 3. fuse hidden pre-activation (registers, as gelu'); pb into X
+    float hf[N2][4];
+    g32::gemm<2 * C, 2 * C>(T, 0, wf1, 2 * C, ring, hf);
+    ring.pre<2 * C>(wf2t, 2 * C);
+    g32::load_tile<C>(X, 0, pb, v0, V, al);   // the gate GEMM's reads of X ended before the last GEMM's barriers
+#pragma unroll
+    for (int j = 0; j < N2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) hf[j][e] = gelu_grad(hf[j][e]);
+    // 4. fuse hidden gradient -> T
     {
-      float acc[RM][2 * C / 16];
-      tile_mm<2 * C, 2 * C, RM>(SH2, L2, wf1t, acc);
+      float acc[N2][4];
+      g32::gemm<C, 2 * C>(X, 0, wf2t, 2 * C, ring, acc);
+      ring.pre<2 * C>(wf1t, 2 * C);
+#pragma unroll
+      for (int j = 0; j < N2; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] *= hf[j][e];
+        g32::put4(T, Ch::col(tx, j), acc[j]);   // T's readers (step 3) passed this GEMM's barriers
+      }
+    }
+    // 5. B_bar = T Wf1^T + 0.5 [pb, pb]: the branch gradients replace spec | vert, the gate pre-activation gradient -> T
+    {
+      float acc[N2][4];
+      g32::gemm<2 * C, 2 * C, 2>(T, 0, wf1t, 2 * C, ring, acc);
+      ring.pre<C>(wg2t, C);
       __syncthreads();
 #pragma unroll
-      for (int i = 0; i < RM; ++i)
+      for (int j = 0; j < N2; ++j) {
+        const int n = C2::col(tx, j);
+        float a[4], f[4], d[4];
+        g32::get4(X, C + n, a);
+        g32::get4(X, C2::col(tx, j % N1), f);
 #pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) {
-          const int r = ty + 16 * i, n = tx + 16 * j;
-          const float bb = acc[i][j] + 0.5f * fb[i][j % (C / 16)];
-          const float g = SG[r * L2 + n];
-          br[i][j] = bb * g;                                   // d/d spec (n < C) or vert (n >= C)
-          ST[r * L2 + n] = bb * SA[r * LA + C + n] * g * (1.f - g);  // d/d gate pre-activation
+        for (int e = 0; e < 4; ++e) {
+          const float bb = acc[j][e] + 0.5f * f[e];
+          d[e] = bb * a[e] * g[j][e] * (1.f - g[j][e]);
+          a[e] = bb * g[j][e];
         }
+        g32::put4(X, C + n, a);
+        g32::put4(T, n, d);
+      }
     }
-    __syncthreads();
-    // 7. branch-gate hidden gradient (times gelu') -> SH1
+    // 6. branch-gate hidden gradient -> X
     {
-      float acc[RM][C / 16];
-      tile_mm<2 * C, C, RM>(ST, L2, wg2t, acc);
+      float acc[N1][4];
+      g32::gemm<2 * C, C>(T, 0, wg2t, C, ring, acc);
+      ring.pre<C>(wg1t, 3 * C);
 #pragma unroll
-      for (int i = 0; i < RM; ++i)
+      for (int j = 0; j < N1; ++j) {
 #pragma unroll
-        for (int j = 0; j < C / 16; ++j) {
-          const int o = (ty + 16 * i) * L1 + tx + 16 * j;
-          SH1[o] = acc[i][j] * gelu_grad(SH1[o]);
-        }
+        for (int e = 0; e < 4; ++e) acc[j][e] *= h1[j][e];
+        g32::put4(X, C1::col(tx, j), acc[j]);   // pb's readers (step 5) passed this GEMM's barriers
+      }
     }
-    __syncthreads();
-    // 8. A_bar = SH1 Wg1^T: x, spec, vert gradients
-    {
-      float acc[RM][3 * C / 16];
-      tile_mm<C, 3 * C, RM>(SH1, L1, wg1t, acc);
+    // 7. A_bar = X Wg1^T: x, spec, vert gradients
+#pragma unroll 1
+    for (int part = 0; part < 3; ++part) {
+      float acc[N1][4];
+      g32::gemm<C, C>(X, 0, wg1t + part * C, 3 * C, ring, acc);
+      if (part < 2) ring.pre<C>(wg1t + (part + 1) * C, 3 * C);
+      if (part) {
 #pragma unroll
-      for (int i = 0; i < RM; ++i) {
-        const long v = v0 + ty + 16 * i;
-        if (v >= V) continue;
+        for (int j = 0; j < N1; ++j) {
+          float b[4];
+          g32::get4(X, part * C + C1::col(tx, j), b);
 #pragma unroll
-        for (int j = 0; j < C / 16; ++j) {
-          const int c = tx + 16 * j;
-          xbar[v * C + c] = acc[i][j] + (base ? __ldg(base + v * C + c) : 0.f);
-          sbar[v * C + c] = acc[i][j + C / 16] + br[i][j];
-          vbar[v * C + c] = acc[i][j + 2 * C / 16] + br[i][j + C / 16];
+          for (int e = 0; e < 4; ++e) acc[j][e] += b[e];
         }
       }
+      g32::store_rows<C>(part == 0 ? xbar : part == 1 ? sbar : vbar, part == 0 ? base : nullptr, v0, V, acc, al);
     }
   }
 }
 
 // ------------------------------------------------------------------------------------------------ gate backward
 // x_bar = base + sum over the two branches of d/dx [x * sigmoid(gelu(x G1) G2)] applied to that branch's gradient;
-// z_bar += sum_c xv_bar * zp (the z_proj term of the vertical branch, models/ffno_model.py:265).
+// z_bar += sum_c xv_bar * zp (the z_proj term of the vertical branch, models/ffno_model.py:265). 524 k voxels, C = 64:
+// 2.86 -> 1.02 ms.
 template <int C>
-__global__ void __launch_bounds__(NT) k_gate_bwd(const float* __restrict__ x, const float* __restrict__ xsb,
+__global__ void __launch_bounds__(NT, 3) k_gate_bwd(const float* __restrict__ x, const float* __restrict__ xsb,
                                                  const float* __restrict__ xvb, const float* __restrict__ base,
                                                  long V, const float* __restrict__ s1, const float* __restrict__ s2,
                                                  const float* __restrict__ s2t, const float* __restrict__ s1t,
                                                  const float* __restrict__ v1, const float* __restrict__ v2,
                                                  const float* __restrict__ v2t, const float* __restrict__ v1t,
                                                  const float* __restrict__ zp, float* __restrict__ xbar,
-                                                 float* __restrict__ zbar) {
-  extern __shared__ float sm[];
-  constexpr int LD = C + 1;
-  float* SX = sm;
-  float* SB = SX + BM * LD;
-  float* SP = SB + BM * LD;
-  float* ST = SP + BM * LD;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+                                                 float* __restrict__ zbar, int al) {
+  extern __shared__ __align__(16) float sm[];
+  float* SX = sm;               // [C][64] x
+  float* SB = SX + C * BM;      // [C][64] the branch's gradient
+  float* ST = SB + C * BM;      // [C][64] GEMM operand
+  g32::Ring ring(ST + C * BM, g32::KC * C, al);
+  using Cl = g32::Cols<C, 1>;
+  constexpr int N = C / 16;
+  const int tx = g32::tile_tx();
   const long nt = ntiles(V, BM);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
-    float xb[4][C / 16];
+    float xb[N][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < N; ++j)
 #pragma unroll
-      for (int j = 0; j < C / 16; ++j) xb[i][j] = 0.f;
+      for (int e = 0; e < 4; ++e) xb[j][e] = 0.f;
     __syncthreads();
-    load_rows<C>(SX, LD, x, v0, V);
+    ring.pre<C>(s1, C);
+    g32::load_tile<C>(SX, 0, x, v0, V, al);
+#pragma unroll 1
     for (int br = 0; br < 2; ++br) {
       const float* gbar = br ? xvb : xsb;
       const float* g1 = br ? v1 : s1;
       const float* g2 = br ? v2 : s2;
       const float* g2t = br ? v2t : s2t;
       const float* g1t = br ? v1t : s1t;
-      __syncthreads();
-      load_rows<C>(SB, LD, gbar, v0, V);
-      __syncthreads();
-      {
-        float acc[4][C / 16];
-        tile_mm<C, C>(SX, LD, g1, acc);
+      g32::load_tile<C>(SB, 0, gbar, v0, V, al);   // its readers of the branch before passed later barriers
+      float h[N][4], acc[N][4];
+      g32::gemm<C, C>(SX, 0, g1, C, ring, h);
+      ring.pre<C>(g2, C);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < N; ++j) {
+        float a[4];
 #pragma unroll
-          for (int j = 0; j < C / 16; ++j) {
-            const int o = (ty + 16 * i) * LD + tx + 16 * j;
-            SP[o] = acc[i][j];
-            ST[o] = gelu(acc[i][j]);
-          }
-      }
-      __syncthreads();
-      {
-        float acc[4][C / 16];
-        tile_mm<C, C>(ST, LD, g2, acc);
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < C / 16; ++j) {
-            const int o = (ty + 16 * i) * LD + tx + 16 * j;
-            const float g = sigmoid(acc[i][j]);
-            const float b = SB[o];
-            xb[i][j] += b * g;
-            ST[o] = b * SX[o] * g * (1.f - g);
-          }
-      }
-      __syncthreads();
-      {
-        float acc[4][C / 16];
-        tile_mm<C, C>(ST, LD, g2t, acc);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < C / 16; ++j) {
-            const int o = (ty + 16 * i) * LD + tx + 16 * j;
-            SP[o] = acc[i][j] * gelu_grad(SP[o]);
-          }
-      }
-      __syncthreads();
-      {
-        float acc[4][C / 16];
-        tile_mm<C, C>(SP, LD, g1t, acc);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < C / 16; ++j) xb[i][j] += acc[i][j];
-      }
-      if (br == 1 && zp) {
-        // z_bar[v] += sum_c xv_bar[v][c] zp[c]; the 16 threads of one row are one half-warp
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float s = 0.f;
-#pragma unroll
-          for (int j = 0; j < C / 16; ++j) s += SB[(ty + 16 * i) * LD + tx + 16 * j] * __ldg(zp + tx + 16 * j);
-          s += __shfl_xor_sync(0xffffffffu, s, 8);
-          s += __shfl_xor_sync(0xffffffffu, s, 4);
-          s += __shfl_xor_sync(0xffffffffu, s, 2);
-          s += __shfl_xor_sync(0xffffffffu, s, 1);
-          const long v = v0 + ty + 16 * i;
-          if (tx == 0 && v < V) zbar[v] += s;
+        for (int e = 0; e < 4; ++e) {
+          a[e] = gelu(h[j][e]);
+          h[j][e] = gelu_grad(h[j][e]);
         }
+        g32::put4(ST, Cl::col(tx, j), a);   // ST's readers (the branch before) passed the last GEMM's barriers
+      }
+      g32::gemm<C, C>(ST, 0, g2, C, ring, acc);
+      ring.pre<C>(g2t, C);
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        float b[4], xv[4], d[4];
+        g32::get4(SB, Cl::col(tx, j), b);
+        g32::get4(SX, Cl::col(tx, j), xv);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float g = sigmoid(acc[j][e]);
+          xb[j][e] += b[e] * g;
+          d[e] = b[e] * xv[e] * g * (1.f - g);
+        }
+        g32::put4(ST, Cl::col(tx, j), d);
+      }
+      g32::gemm<C, C>(ST, 0, g2t, C, ring, acc);
+      ring.pre<C>(g1t, C);
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] *= h[j][e];
+        g32::put4(ST, Cl::col(tx, j), acc[j]);
+      }
+      g32::gemm<C, C>(ST, 0, g1t, C, ring, acc);
+      if (br == 0) ring.pre<C>(v1, C);
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) xb[j][e] += acc[j][e];
+      if (br == 1 && zp) {
+        // z_bar[v] += sum_c xv_bar[v][c] zp[c]: 4 lanes a voxel
+        const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
+        float a = 0.f;
+        for (int c = q; c < C; c += 4) a = fmaf(SB[g32::at(r, c)], __ldg(zp + c), a);
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+        if (q == 0 && v0 + r < V) zbar[v0 + r] += a;
       }
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long v = v0 + ty + 16 * i;
-      if (v >= V) continue;
-#pragma unroll
-      for (int j = 0; j < C / 16; ++j) {
-        const int c = tx + 16 * j;
-        xbar[v * C + c] = xb[i][j] + (base ? __ldg(base + v * C + c) : 0.f);
-      }
-    }
+    g32::store_rows<C>(xbar, base, v0, V, xb, al);
   }
 }
 
@@ -721,45 +706,52 @@ __global__ void __launch_bounds__(NT) k_lift_bwd(const float* __restrict__ pb, i
 // kLte = false: the VJP of FFNO3D._run_head alone (models/ffno_model.py:790-798); ybar is then the gradient of the
 // nh head channels [nh][V] and xin / xinbar are not used.
 template <int C, int NHP, typename T, bool kLte = true>
-__global__ void __launch_bounds__(NT) k_head_bwd(const float* __restrict__ x, const float* __restrict__ xin,
+__global__ void __launch_bounds__(NT, 2) k_head_bwd(const float* __restrict__ x, const float* __restrict__ xin,
                                                  const float* __restrict__ ybar, long V, const float* __restrict__ p1,
                                                  const float* __restrict__ p2, const float* __restrict__ b2,
                                                  const float* __restrict__ p2t, const float* __restrict__ p1t,
                                                  const __grid_constant__ ffno_head_params hp, int nh,
-                                                 float* __restrict__ xbar, float* __restrict__ xinbar) {
-  extern __shared__ float sm[];
-  constexpr int LA = C + 1, LH = 2 * C + 1, LO = NHP + 1;
-  float* SA = sm;
-  float* SP = SA + BM * LA;   // hidden pre-activation
-  float* SG = SP + BM * LH;   // gelu(hidden), later the hidden gradient
-  float* SO = SG + BM * LH;   // head channels, later their gradient
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+                                                 float* __restrict__ xbar, float* __restrict__ xinbar, int al) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int LO = NHP + 1, N2 = 2 * C / 16;
+  float* SA = sm;                    // [C][64] input, then [2C][64] hidden, then its gradient
+  float* SG = SA + 2 * C * BM;       // [NHP][64] gradient of the head channels
+  float* SO = SG + NHP * BM;         // [64][NHP + 1] head channels, then their gradient
+  g32::Ring ring(SO + BM * LO, g32::KC * 2 * C, al);
+  using Ch = g32::Cols<2 * C, 1>;
+  using Co = g32::Cols<NHP, 1>;
+  const int tx = g32::tile_tx(), ty = g32::tile_ty();
   const long nt = ntiles(V, BM);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    load_rows<C>(SA, LA, x, v0, V);
+    ring.pre<2 * C>(p1, 2 * C);
+    g32::load_tile<C>(SA, 0, x, v0, V, al);
+    float h[N2][4];   // gelu' of the hidden pre-activation
+    g32::gemm<C, 2 * C>(SA, 0, p1, 2 * C, ring, h);
+    ring.pre<NHP>(p2, NHP);
     __syncthreads();
-    {
-      float acc[4][2 * C / 16];
-      tile_mm<C, 2 * C>(SA, LA, p1, acc);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < N2; ++j) {
+      float a[4];
 #pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) {
-          const int o = (ty + 16 * i) * LH + tx + 16 * j;
-          SP[o] = acc[i][j];
-          SG[o] = gelu(acc[i][j]);
-        }
+      for (int e = 0; e < 4; ++e) {
+        a[e] = gelu(h[j][e]);
+        h[j][e] = gelu_grad(h[j][e]);
+      }
+      g32::put4(SA, Ch::col(tx, j), a);
     }
-    __syncthreads();
     {
-      float acc[4][NHP / 16];
-      tile_mm<2 * C, NHP>(SG, LH, p2, acc);
+      float acc[NHP / 16][4];
+      g32::gemm<2 * C, NHP>(SA, 0, p2, NHP, ring, acc);
+      ring.pre<2 * C>(p2t, 2 * C);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < NHP / 16; ++j) {
+        const int n = Co::col(tx, j);
+        const float b = __ldg(b2 + n);
 #pragma unroll
-        for (int j = 0; j < NHP / 16; ++j) SO[(ty + 16 * i) * LO + tx + 16 * j] = acc[i][j] + __ldg(b2 + tx + 16 * j);
+        for (int e = 0; e < 4; ++e) SO[(4 * ty + e) * LO + n] = acc[j][e] + b;
+      }
     }
     __syncthreads();
     if (threadIdx.x < BM) {
@@ -772,33 +764,24 @@ __global__ void __launch_bounds__(NT) k_head_bwd(const float* __restrict__ x, co
         } else {
           for (int c = 0; c < NHP; ++c) o[c] = c < nh ? __ldg(ybar + (long)c * V + v) : 0.f;
         }
-      } else {
-        for (int c = 0; c < NHP; ++c) o[c] = 0.f;
+      }
+      for (int c = 0; c < NHP; ++c) SG[g32::at(r, c)] = v < V ? o[c] : 0.f;
+    }
+    {
+      float acc[N2][4];
+      g32::gemm<NHP, 2 * C>(SG, 0, p2t, 2 * C, ring, acc);
+      ring.pre<C>(p1t, C);
+#pragma unroll
+      for (int j = 0; j < N2; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] *= h[j][e];
+        g32::put4(SA, Ch::col(tx, j), acc[j]);   // the hidden layer's readers passed later barriers
       }
     }
-    __syncthreads();
     {
-      float acc[4][2 * C / 16];
-      tile_mm<NHP, 2 * C>(SO, LO, p2t, acc);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) {
-          const int o = (ty + 16 * i) * LH + tx + 16 * j;
-          SG[o] = acc[i][j] * gelu_grad(SP[o]);
-        }
-    }
-    __syncthreads();
-    {
-      float acc[4][C / 16];
-      tile_mm<2 * C, C>(SG, LH, p1t, acc);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const long v = v0 + ty + 16 * i;
-        if (v >= V) continue;
-#pragma unroll
-        for (int j = 0; j < C / 16; ++j) xbar[v * C + tx + 16 * j] = acc[i][j];
-      }
+      float acc[C / 16][4];
+      g32::gemm<2 * C, C>(SA, 0, p1t, C, ring, acc);
+      g32::store_rows<C>(xbar, nullptr, v0, V, acc, al);
     }
   }
 }
@@ -955,10 +938,11 @@ int ffno_gn_bwd_stats(int mode, const float* u, float r, const float* pre, const
   if (!width_ok(C) || V < 1 || groups < 1 || groups > GMAX || C % groups || nparts < 1) return FFNO_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   const int cpg = C / groups;
+  const int grid = nparts < 2 * sms() ? nparts : 2 * sms();   // the CTAs an SM holds (97-124 registers a thread)
   if (groups == GMAX && C <= 64 &&
       (reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(pre)) % 32 == 0) {   // 32-byte lanes
     switch (C) {
-#define L(CC) case CC: k_gn_bwd_stats8<CC><<<nparts, 256, 0, s>>>(mode, u, r, pre, gamma, beta, gstats, V, partials); break;
+#define L(CC) case CC: k_gn_bwd_stats8<CC><<<grid, 256, 0, s>>>(mode, u, r, pre, gamma, beta, gstats, V, partials, nparts); break;
       L(16) L(32) L(64)
 #undef L
     }
@@ -966,7 +950,7 @@ int ffno_gn_bwd_stats(int mode, const float* u, float r, const float* pre, const
     return FFNO_OK;
   }
   switch (C) {
-#define L(CC) case CC: k_gn_bwd_stats<CC><<<nparts, 256, 0, s>>>(mode, u, r, pre, gamma, beta, gstats, V, partials, cpg, groups); break;
+#define L(CC) case CC: k_gn_bwd_stats<CC><<<grid, 256, 0, s>>>(mode, u, r, pre, gamma, beta, gstats, V, partials, nparts, cpg, groups); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -1006,13 +990,14 @@ int ffno_gn_bwd_apply(int mode, const float* u, float r, const float* pre, const
 int ffno_mlp2_bwd(const float* a, const float* pre_bar, const float* base, long V, int C, const float* w1,
                   const float* w2t, const float* w1t, float* a_bar, ffno_stream_t stream) {
   if (!a || !pre_bar || !w1 || !w2t || !w1t || !a_bar || !width_ok(C) || V < 1) return FFNO_EINVAL;
+  const int al = g32::aligned(a, pre_bar, base, w1, w2t, w1t, a_bar);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
 #define L(CC)                                                                                   \
   case CC: {                                                                                    \
-    const size_t smem = (2 * BM * (CC + 1) + BM * (2 * CC + 1)) * sizeof(float);                \
+    const size_t smem = (2 * CC * BM + 2 * g32::KC * 2 * CC) * sizeof(float);                   \
     if (!smem_attr(k_mlp2_bwd<CC>, smem)) return FFNO_ELAUNCH;                                  \
-    k_mlp2_bwd<CC><<<grid_of(V, BM, 2), NT, smem, s>>>(a, pre_bar, base, V, w1, w2t, w1t, a_bar); \
+    k_mlp2_bwd<CC><<<grid_of(V, BM, 2), NT, smem, s>>>(a, pre_bar, base, V, w1, w2t, w1t, a_bar, al); \
     break;                                                                                      \
   }
     L(16) L(32) L(64) L(96)
@@ -1031,19 +1016,21 @@ int ffno_fuse_bwd(const float* x, const float* spec_pre, const float* spec_coefs
       !wf2t || !wf1t || !wg2t || !wg1t || !x_bar || !spec_bar || !vert_bar)
     return FFNO_EINVAL;
   if (!width_ok(C) || V < 1) return FFNO_EINVAL;
+  const int al = g32::aligned(x, spec_pre, vert_pre, fused_pre_bar, base, wg1, wg2, wf1, wf2t, wf1t, wg2t, wg1t, x_bar,
+                              spec_bar, vert_bar);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
-#define L(CC, RMV)                                                                                          \
+#define L(CC)                                                                                               \
   case CC: {                                                                                                \
-    constexpr int R = 16 * RMV;                                                                             \
-    const size_t smem = (size_t)R * ((3 * CC + 1) + (CC + 1) + 3 * (2 * CC + 1)) * sizeof(float);          \
-    if (!smem_attr(k_fuse_bwd<CC, RMV>, smem)) return FFNO_ELAUNCH;                                         \
-    k_fuse_bwd<CC, RMV><<<grid_of(V, R, 2), NT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre, vert_coefs,     \
-                                                           fused_pre_bar, base, V, wg1, wg2, bg2, wf1, wf2t,  \
-                                                           wf1t, wg2t, wg1t, x_bar, spec_bar, vert_bar);      \
+    const size_t smem = fuse_bwd_smem<CC>();                                                                \
+    if (!smem_attr(k_fuse_bwd<CC>, smem)) return FFNO_ELAUNCH;                                              \
+    k_fuse_bwd<CC><<<grid_of(V, BM, CC <= 64 ? 2 : 1), NT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre,     \
+                                                                      vert_coefs, fused_pre_bar, base, V,   \
+                                                                      wg1, wg2, bg2, wf1, wf2t, wf1t, wg2t, \
+                                                                      wg1t, x_bar, spec_bar, vert_bar, al); \
     break;                                                                                                  \
   }
-    L(16, 4) L(32, 4) L(64, 4) L(96, 2)
+    L(16) L(32) L(64) L(96)
 #undef L
   }
   FFNO_CHECK_LAUNCH();
@@ -1057,14 +1044,15 @@ int ffno_gate_bwd(const float* x, const float* xs_bar, const float* xv_bar, cons
   if (!x || !xs_bar || !xv_bar || !s_w1 || !s_w2 || !s_w2t || !s_w1t || !v_w1 || !v_w2 || !v_w2t || !v_w1t || !x_bar)
     return FFNO_EINVAL;
   if (!width_ok(C) || V < 1 || (zp && !z_bar)) return FFNO_EINVAL;
+  const int al = g32::aligned(x, xs_bar, xv_bar, base, s_w1, s_w2, s_w2t, s_w1t, v_w1, v_w2, v_w2t, v_w1t, x_bar);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
 #define L(CC)                                                                                              \
   case CC: {                                                                                               \
-    const size_t smem = 4 * BM * (CC + 1) * sizeof(float);                                                  \
+    const size_t smem = (3 * CC * BM + 2 * g32::KC * CC) * sizeof(float);                                  \
     if (!smem_attr(k_gate_bwd<CC>, smem)) return FFNO_ELAUNCH;                                             \
-    k_gate_bwd<CC><<<grid_of(V, BM, 2), NT, smem, s>>>(x, xs_bar, xv_bar, base, V, s_w1, s_w2, s_w2t, s_w1t, \
-                                                       v_w1, v_w2, v_w2t, v_w1t, zp, x_bar, z_bar);          \
+    k_gate_bwd<CC><<<grid_of(V, BM, 3), NT, smem, s>>>(x, xs_bar, xv_bar, base, V, s_w1, s_w2, s_w2t, s_w1t, \
+                                                       v_w1, v_w2, v_w2t, v_w1t, zp, x_bar, z_bar, al);     \
     break;                                                                                                 \
   }
     L(16) L(32) L(64) L(96)
@@ -1093,19 +1081,20 @@ int ffno_head_bwd(const float* x, const float* x_in, const float* y_bar, long V,
   if (!x || !x_in || !y_bar || !p1 || !p2 || !b2 || !p2t || !p1t || !x_bar || !x_in_bar) return FFNO_EINVAL;
   if (!width_ok(C) || V < 1 || !params || (nhp != 16 && nhp != 32)) return FFNO_EINVAL;
   if (params->nspecies < 1 || params->nspecies > FFNO_MAX_SPECIES || params->in_channels > 8) return FFNO_EINVAL;
+  const int al = g32::aligned(x, p1, p2, p2t, p1t, x_bar);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
 #define L(CC, NN)                                                                                        \
   if (C == CC && nhp == NN) {                                                                            \
-    const size_t smem = (BM * (CC + 1) + 2 * BM * (2 * CC + 1) + BM * (NN + 1)) * sizeof(float);         \
+    const size_t smem = (2 * CC * BM + NN * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);  \
     if (params->math32) {                                                                               \
       if (!smem_attr(k_head_bwd<CC, NN, float>, smem)) return FFNO_ELAUNCH;                             \
       k_head_bwd<CC, NN, float><<<grid_of(V, BM, 2), NT, smem, s>>>(x, x_in, y_bar, V, p1, p2, b2, p2t, p1t, \
-                                                                    *params, NN, x_bar, x_in_bar);          \
+                                                                    *params, NN, x_bar, x_in_bar, al);      \
     } else {                                                                                            \
       if (!smem_attr(k_head_bwd<CC, NN, double>, smem)) return FFNO_ELAUNCH;                            \
       k_head_bwd<CC, NN, double><<<grid_of(V, BM, 2), NT, smem, s>>>(x, x_in, y_bar, V, p1, p2, b2, p2t, p1t, \
-                                                                     *params, NN, x_bar, x_in_bar);         \
+                                                                     *params, NN, x_bar, x_in_bar, al);     \
     }                                                                                                   \
   }
     default:
@@ -1207,15 +1196,16 @@ int ffno_proj_bwd(const float* x, const float* head_bar, long V, int C, const fl
                   ffno_stream_t stream) {
   if (!x || !head_bar || !p1 || !p2 || !b2 || !p2t || !p1t || !x_bar) return FFNO_EINVAL;
   if (!width_ok(C) || V < 1 || (nhp != 16 && nhp != 32) || nh < 1 || nh > nhp) return FFNO_EINVAL;
+  const int al = g32::aligned(x, p1, p2, p2t, p1t, x_bar);
   cudaStream_t s = (cudaStream_t)stream;
   ffno_head_params none{};
   switch (C) {
 #define L(CC, NN)                                                                                        \
   if (C == CC && nhp == NN) {                                                                            \
-    const size_t smem = (BM * (CC + 1) + 2 * BM * (2 * CC + 1) + BM * (NN + 1)) * sizeof(float);         \
+    const size_t smem = (2 * CC * BM + NN * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);  \
     if (!smem_attr(k_head_bwd<CC, NN, float, false>, smem)) return FFNO_ELAUNCH;                         \
     k_head_bwd<CC, NN, float, false><<<grid_of(V, BM, 2), NT, smem, s>>>(x, nullptr, head_bar, V, p1, p2, b2, \
-                                                                         p2t, p1t, none, nh, x_bar, nullptr); \
+                                                                         p2t, p1t, none, nh, x_bar, nullptr, al); \
   }
     default:
       L(16, 16) L(16, 32) L(32, 16) L(32, 32) L(64, 16) L(64, 32) L(96, 16) L(96, 32)

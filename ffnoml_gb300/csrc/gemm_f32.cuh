@@ -46,16 +46,25 @@ struct Cols {
 struct Ring {
   float* buf;
   int floats, st;   // floats per stage; the stage the next chunk goes to
-  __device__ __forceinline__ Ring(float* b, int f) : buf(b), floats(f), st(0) {}
+  int al;           // the weights start on 16 bytes (else 4-byte copies)
+  __device__ __forceinline__ Ring(float* b, int f, int a) : buf(b), floats(f), st(0), al(a) {}
   template <int N>
   __device__ __forceinline__ void issue(const float* __restrict__ w, int ldw) {
     constexpr int Q = N / 4;
-    float* dst = buf + st * floats;
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(buf + st * floats));
+    if (al) {
 #pragma unroll
-    for (int u = threadIdx.x; u < KC * Q; u += NT) {
-      const int k = u / Q, q = u % Q;
-      const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst + k * N + 4 * q));
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(w + (long)k * ldw + 4 * q) : "memory");
+      for (int u = threadIdx.x; u < KC * Q; u += NT) {
+        const int k = u / Q, q = u % Q;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4 * (k * N + 4 * q)),
+                     "l"(w + (long)k * ldw + 4 * q)
+                     : "memory");
+      }
+    } else {
+#pragma unroll 1
+      for (int u = threadIdx.x; u < KC * N; u += NT)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4 * u), "l"(w + (long)(u / N) * ldw + u % N)
+                     : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -148,8 +157,23 @@ __device__ __forceinline__ void each_quad(long v0, long V, F f) {
   }
 }
 
-__device__ __forceinline__ float4 ldq(const float* p, bool ok) {
-  return ok ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+// Whether every pointer starts on 16 bytes: the kernels' `al` argument, which picks 16-byte or 4-byte accesses.
+template <typename... P>
+inline int aligned(const P*... p) {
+  return ((... | reinterpret_cast<uintptr_t>(p)) % 16) == 0;
+}
+
+__device__ __forceinline__ float4 ldq(const float* p, bool ok, int al) {
+  if (!ok) return make_float4(0.f, 0.f, 0.f, 0.f);
+  if (al) return __ldg(reinterpret_cast<const float4*>(p));
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+__device__ __forceinline__ void stq(float* p, float4 v, int al) {
+  if (al) {
+    *reinterpret_cast<float4*>(p) = v;
+  } else {
+    p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
+  }
 }
 __device__ __forceinline__ void put_quad(float* s, int r, int c, float4 v) {
   s[at(r, c)] = v.x;
@@ -160,38 +184,40 @@ __device__ __forceinline__ void put_quad(float* s, int r, int c, float4 v) {
 
 // Rows v0 .. v0 + 63 of g [V][C] into channels k0 .. k0 + C - 1 of a region; rows at or past V are zero.
 template <int C>
-__device__ __forceinline__ void load_tile(float* s, int k0, const float* __restrict__ g, long v0, long V) {
-  each_quad<C>(v0, V, [&](int r, int c, long o, bool ok) { put_quad(s, r, k0 + c, ldq(g + o, ok)); });
+__device__ __forceinline__ void load_tile(float* s, int k0, const float* __restrict__ g, long v0, long V, int al) {
+  each_quad<C>(v0, V, [&](int r, int c, long o, bool ok) { put_quad(s, r, k0 + c, ldq(g + o, ok, al)); });
 }
 
 // Store the thread's CV consecutive channels of one voxel (v: the values of channels j .. j + CV - 1).
 template <int CV>
-__device__ __forceinline__ void st_run(float* p, const float* v) {
-  if constexpr (CV == 4)
+__device__ __forceinline__ void st_run(float* p, const float* v, int al) {
+  if (CV == 1 || !al) {
+#pragma unroll
+    for (int i = 0; i < CV; ++i) p[i] = v[i];
+  } else if constexpr (CV == 4) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-  else if constexpr (CV == 2)
+  } else if constexpr (CV == 2) {
     *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-  else
-    *p = v[0];
+  }
 }
 template <int CV>
-__device__ __forceinline__ void ld_run(const float* p, float* v) {
-  if constexpr (CV == 4) {
+__device__ __forceinline__ void ld_run(const float* p, float* v, int al) {
+  if (CV == 1 || !al) {
+#pragma unroll
+    for (int i = 0; i < CV; ++i) v[i] = __ldg(p + i);
+  } else if constexpr (CV == 4) {
     const float4 q = __ldg(reinterpret_cast<const float4*>(p));
     v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
   } else if constexpr (CV == 2) {
     const float2 q = __ldg(reinterpret_cast<const float2*>(p));
     v[0] = q.x, v[1] = q.y;
-  } else {
-    v[0] = __ldg(p);
   }
 }
 
-// out[v][c] = val (+ base[v][c]) for the thread's voxels and channels of a C-channel output (base may be null); j0: the
-// first accumulator column of this output.
+// out[v][c] = val (+ base[v][c]) for the thread's voxels and channels of a C-channel output (base may be null).
 template <int C, int NACC>
 __device__ __forceinline__ void store_rows(float* __restrict__ out, const float* __restrict__ base, long v0, long V,
-                                           const float (&acc)[NACC][4], int j0 = 0) {
+                                           const float (&acc)[NACC][4], int al) {
   using Cl = Cols<C, 1>;
   const int tx = tile_tx(), ty = tile_ty();
 #pragma unroll
@@ -203,14 +229,14 @@ __device__ __forceinline__ void store_rows(float* __restrict__ out, const float*
       const long o = v * C + Cl::col(tx, j);
       float t[Cl::CV];
 #pragma unroll
-      for (int i = 0; i < Cl::CV; ++i) t[i] = acc[j0 + j + i][e];
+      for (int i = 0; i < Cl::CV; ++i) t[i] = acc[j + i][e];
       if (base) {
         float b[Cl::CV];
-        ld_run<Cl::CV>(base + o, b);
+        ld_run<Cl::CV>(base + o, b, al);
 #pragma unroll
         for (int i = 0; i < Cl::CV; ++i) t[i] += b[i];
       }
-      st_run<Cl::CV>(out + o, t);
+      st_run<Cl::CV>(out + o, t, al);
     }
   }
 }
@@ -274,14 +300,19 @@ __device__ __forceinline__ void tile_stats(const float (&acc)[C / 16][4], const 
   __syncthreads();
 }
 
-// Partials row of this CTA, from thread 32 g's accumulators of group g.
-__device__ __forceinline__ void write_tile_partial(double* partials, int groups, const GroupAcc& a) {
+// Partials row of this CTA, from thread 32 g's accumulators of group g; the rows past the grid (nparts is the most CTAs
+// any of these kernels runs) hold no weight.
+__device__ __forceinline__ void write_tile_partial(double* partials, int nparts, int groups, const GroupAcc& a) {
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   if (lane == 0 && g < groups) {
     double* p = partials + ((long)blockIdx.x * groups + g) * 3;
     p[0] = a.w;
     p[1] = a.mean;
     p[2] = a.m2;
+    for (long r = blockIdx.x + gridDim.x; r < nparts; r += gridDim.x) {
+      p = partials + (r * groups + g) * 3;
+      p[0] = p[1] = p[2] = 0.0;
+    }
   }
 }
 

@@ -7,6 +7,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "gemm_f32.cuh"
 
 using namespace ffno;
 
@@ -167,198 +168,202 @@ __global__ void k_gn_jvp_apply(const float* __restrict__ pre, const float* __res
 }
 
 // ------------------------------------------------------------------------------------------------ chains
-// Tiles of BM voxels, thread (ty, tx) owns rows ty + 16 i and columns tx + 16 j of every tile GEMM (tile_mm).
+// Tiles of BM voxels on the tile GEMM of gemm_f32.cuh; the primal and its tangent share each weight chunk (NA = 2).
 
 // Input gate: out = x sigmoid(g), g = gelu(x G1) G2 (+ zp z, constant in x): out' = x' s + x s (1 - s) g',
-// g' = (gelu'(x G1) x' G1) G2.
+// g' = (gelu'(x G1) x' G1) G2. 147 k voxels, C = 64: 269 -> 136 us.
 template <int C>
-__global__ void __launch_bounds__(NT) k_gate_jvp(const float* __restrict__ x, const float* __restrict__ xd, long V,
-                                                 const float* __restrict__ w1, const float* __restrict__ w2,
-                                                 float* __restrict__ outd) {
-  extern __shared__ float sm[];
-  constexpr int L = C + 1;
-  float* xs = sm;
-  float* xds = xs + BM * L;
-  float* hs = xds + BM * L;
-  float* hds = hs + BM * L;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+__global__ void __launch_bounds__(NT, C <= 64 ? 3 : 2) k_gate_jvp(const float* __restrict__ x, const float* __restrict__ xd, long V,
+                                                    const float* __restrict__ w1, const float* __restrict__ w2,
+                                                    float* __restrict__ outd, int al) {
+  extern __shared__ __align__(16) float sm[];
+  float* xs = sm;               // [2C][64]: x, x'
+  float* hs = xs + 2 * C * BM;  // [2C][64]: the hidden layer and its tangent
+  g32::Ring ring(hs + 2 * C * BM, g32::KC * C, al);
+  using Cl = g32::Cols<C, 1>;
+  const int tx = g32::tile_tx();
   const long nt = (V + BM - 1) / BM;
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    load_rows<C>(xs, L, x, v0, V);
-    load_rows<C>(xds, L, xd, v0, V);
-    __syncthreads();
-    {
-      float a[4][C / 16], b[4][C / 16];
-      tile_mm<C, C>(xs, L, w1, a);
-      tile_mm<C, C>(xds, L, w1, b);
+    ring.pre<C>(w1, C);
+    g32::load_tile<C>(xs, 0, x, v0, V, al);
+    g32::load_tile<C>(xs + C * BM, 0, xd, v0, V, al);
+    float a[2][C / 16][4];
+    g32::gemm_n<C, C, 1, 2>(xs, C * BM, 0, w1, C, ring, a);
+    ring.pre<C>(w2, C);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < C / 16; ++j) {
+      const int c = Cl::col(tx, j);
 #pragma unroll
-        for (int j = 0; j < C / 16; ++j) {
-          const int r = ty + 16 * i, c = tx + 16 * j;
-          hs[r * L + c] = gelu(a[i][j]);
-          hds[r * L + c] = gelu_grad(a[i][j]) * b[i][j];
-        }
+      for (int e = 0; e < 4; ++e) {
+        a[1][j][e] *= gelu_grad(a[0][j][e]);
+        a[0][j][e] = gelu(a[0][j][e]);
+      }
+      g32::put4(hs, c, a[0][j]);
+      g32::put4(hs + C * BM, c, a[1][j]);
     }
-    __syncthreads();
-    float a[4][C / 16], b[4][C / 16];
-    tile_mm<C, C>(hs, L, w2, a);
-    tile_mm<C, C>(hds, L, w2, b);
+    g32::gemm_n<C, C, 1, 2>(hs, C * BM, 0, w2, C, ring, a);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty + 16 * i;
-      const long v = v0 + r;
-      if (v >= V) continue;
+    for (int j = 0; j < C / 16; ++j) {
+      const int c = Cl::col(tx, j);
+      float xv[4], xt[4];
+      g32::get4(xs, c, xv);
+      g32::get4(xs + C * BM, c, xt);
 #pragma unroll
-      for (int j = 0; j < C / 16; ++j) {
-        const int c = tx + 16 * j;
-        const float s = sigmoid(a[i][j]);
-        outd[v * C + c] = xds[r * L + c] * s + xs[r * L + c] * s * (1.f - s) * b[i][j];
+      for (int e = 0; e < 4; ++e) {
+        const float s = sigmoid(a[0][j][e]);
+        a[0][j][e] = xt[e] * s + xv[e] * s * (1.f - s) * a[1][j][e];
       }
     }
+    g32::store_rows<C>(outd, nullptr, v0, V, a[0], al);
   }
 }
 
-// Two-layer MLP C -> 2C -> C: pre' = (gelu'(a W1) a' W1) W2.
+// Two-layer MLP C -> 2C -> C: pre' = (gelu'(a W1) a' W1) W2. 147 k voxels, C = 64: 305 -> 190 us.
 template <int C>
-__global__ void __launch_bounds__(NT) k_mlp2_jvp(const float* __restrict__ a, const float* __restrict__ ad, long V,
-                                                 const float* __restrict__ w1, const float* __restrict__ w2,
-                                                 float* __restrict__ outd) {
-  extern __shared__ float sm[];
-  constexpr int LA = C + 1, LH = 2 * C + 1;
-  float* as = sm;
-  float* ads = as + BM * LA;
-  float* hds = ads + BM * LA;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+__global__ void __launch_bounds__(NT, 2) k_mlp2_jvp(const float* __restrict__ a, const float* __restrict__ ad, long V,
+                                                    const float* __restrict__ w1, const float* __restrict__ w2,
+                                                    float* __restrict__ outd, int al) {
+  extern __shared__ __align__(16) float sm[];
+  float* as = sm;   // [C][64] a, [C][64] a', then [2C][64] the hidden tangent
+  g32::Ring ring(as + 2 * C * BM, g32::KC * 2 * C, al);
+  using Ch = g32::Cols<2 * C, 1>;
+  const int tx = g32::tile_tx();
   const long nt = (V + BM - 1) / BM;
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    load_rows<C>(as, LA, a, v0, V);
-    load_rows<C>(ads, LA, ad, v0, V);
-    __syncthreads();
+    ring.pre<2 * C>(w1, 2 * C);
+    g32::load_tile<C>(as, 0, a, v0, V, al);
+    g32::load_tile<C>(as + C * BM, 0, ad, v0, V, al);
     {
-      float h[4][2 * C / 16], hd[4][2 * C / 16];
-      tile_mm<C, 2 * C>(as, LA, w1, h);
-      tile_mm<C, 2 * C>(ads, LA, w1, hd);
+      float h[2][2 * C / 16][4];
+      g32::gemm_n<C, 2 * C, 1, 2>(as, C * BM, 0, w1, 2 * C, ring, h);
+      ring.pre<C>(w2, C);
+      __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 2 * C / 16; ++j) {
 #pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) hds[(ty + 16 * i) * LH + tx + 16 * j] = gelu_grad(h[i][j]) * hd[i][j];
+        for (int e = 0; e < 4; ++e) h[1][j][e] *= gelu_grad(h[0][j][e]);
+        g32::put4(as, Ch::col(tx, j), h[1][j]);
+      }
     }
-    __syncthreads();
-    float o[4][C / 16];
-    tile_mm<2 * C, C>(hds, LH, w2, o);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long v = v0 + ty + 16 * i;
-      if (v >= V) continue;
-#pragma unroll
-      for (int j = 0; j < C / 16; ++j) outd[v * C + tx + 16 * j] = o[i][j];
-    }
+    float o[C / 16][4];
+    g32::gemm<2 * C, C>(as, 0, w2, C, ring, o);
+    g32::store_rows<C>(outd, nullptr, v0, V, o, al);
   }
 }
 
 // Gate + fuse (_fuse_branches): A = [x, s, v] with s = gelu(GN(spec_pre)), v likewise (sd, vd: their tangents);
-// gates = sigmoid(gelu(A Wg1) Wg2 + b); B = [s gs, v gv]; fused = gelu(B Wf1) Wf2 + (B_s + B_v) / 2 -> fused'.
-template <int C, int RM>
-__global__ void __launch_bounds__(NT) k_fuse_jvp(const float* __restrict__ x, const float* __restrict__ xd,
-                                                 const float* __restrict__ sp, const float* __restrict__ sc,
-                                                 const float* __restrict__ vp, const float* __restrict__ vc,
-                                                 const float* __restrict__ sd, const float* __restrict__ vd, long V,
-                                                 const float* __restrict__ wg1, const float* __restrict__ wg2,
-                                                 const float* __restrict__ bg2, const float* __restrict__ wf1,
-                                                 const float* __restrict__ wf2, float* __restrict__ outd) {
-  extern __shared__ float sm[];
-  constexpr int TB = 16 * RM;                     // voxels per tile
-  constexpr int LA = 3 * C + 1, LH = C + 1, LB = 2 * C + 1;
+// gates = sigmoid(gelu(A Wg1) Wg2 + b); B = [s gs, v gv]; fused = gelu(B Wf1) Wf2 + (B_s + B_v) / 2 -> fused'. One
+// region [A | A'] of 6C channels that each stage overwrites: the gate hidden layer over x, B over [s, v], the fuse hidden
+// tangent over B. 147 k voxels, C = 64: 1587 -> 618 us.
+template <int C>
+constexpr size_t fuse_jvp_smem() {
+  return (6 * C * BM + 2 * g32::KC * 2 * C) * sizeof(float);
+}
+
+template <int C>
+__global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_fuse_jvp(const float* __restrict__ x, const float* __restrict__ xd,
+                                                    const float* __restrict__ sp, const float* __restrict__ sc,
+                                                    const float* __restrict__ vp, const float* __restrict__ vc,
+                                                    const float* __restrict__ sd, const float* __restrict__ vd, long V,
+                                                    const float* __restrict__ wg1, const float* __restrict__ wg2,
+                                                    const float* __restrict__ bg2, const float* __restrict__ wf1,
+                                                    const float* __restrict__ wf2, float* __restrict__ outd, int al) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int TAN = 3 * C * BM, N1 = C / 16, N2 = 2 * C / 16;   // TAN: offset of the tangent's region
   float* A = sm;
-  float* Ad = A + TB * LA;
-  float* H = Ad + TB * LA;
-  float* Hd = H + TB * LH;
-  float* Bm = Hd + TB * LH;
-  float* Bd = Bm + TB * LB;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const long nt = (V + TB - 1) / TB;
+  float* Ad = sm + TAN;
+  g32::Ring ring(sm + 2 * TAN, g32::KC * 2 * C, al);
+  using C1 = g32::Cols<C, 1>;
+  using C2 = g32::Cols<2 * C, 2>;
+  using Ch = g32::Cols<2 * C, 1>;
+  const int tx = g32::tile_tx();
+  const long nt = (V + BM - 1) / BM;
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
-    const long v0 = t * TB;
+    const long v0 = t * BM;
     __syncthreads();
-    for (int e = threadIdx.x; e < TB * C; e += NT) {
-      const int r = e / C, c = e % C;
-      const long v = v0 + r;
-      float a = 0.f, s = 0.f, q = 0.f, ad = 0.f, s_d = 0.f, q_d = 0.f;
-      if (v < V) {
-        a = __ldg(x + v * C + c);
-        s = gelu((__ldg(sp + v * C + c) - __ldg(sc + c)) * __ldg(sc + C + c) + __ldg(sc + 2 * C + c));
-        q = gelu((__ldg(vp + v * C + c) - __ldg(vc + c)) * __ldg(vc + C + c) + __ldg(vc + 2 * C + c));
-        ad = __ldg(xd + v * C + c);
-        s_d = __ldg(sd + v * C + c);
-        q_d = __ldg(vd + v * C + c);
+    ring.pre<C>(wg1, C);
+    g32::each_quad<C>(v0, V, [&](int r, int c, long o, bool ok) {
+      const float4 ps = g32::ldq(sp + o, ok, al), pv = g32::ldq(vp + o, ok, al);
+      const float as[4] = {ps.x, ps.y, ps.z, ps.w}, av[4] = {pv.x, pv.y, pv.z, pv.w};
+      g32::put_quad(A, r, c, g32::ldq(x + o, ok, al));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        A[g32::at(r, C + c + i)] =
+            ok ? gelu((as[i] - __ldg(sc + c + i)) * __ldg(sc + C + c + i) + __ldg(sc + 2 * C + c + i)) : 0.f;
+        A[g32::at(r, 2 * C + c + i)] =
+            ok ? gelu((av[i] - __ldg(vc + c + i)) * __ldg(vc + C + c + i) + __ldg(vc + 2 * C + c + i)) : 0.f;
       }
-      A[r * LA + c] = a;
-      A[r * LA + C + c] = s;
-      A[r * LA + 2 * C + c] = q;
-      Ad[r * LA + c] = ad;
-      Ad[r * LA + C + c] = s_d;
-      Ad[r * LA + 2 * C + c] = q_d;
-    }
-    __syncthreads();
+      g32::put_quad(Ad, r, c, g32::ldq(xd + o, ok, al));
+      g32::put_quad(Ad, r, C + c, g32::ldq(sd + o, ok, al));
+      g32::put_quad(Ad, r, 2 * C + c, g32::ldq(vd + o, ok, al));
+    });
     {
-      float h[RM][C / 16], hd[RM][C / 16];
-      tile_mm<3 * C, C, RM>(A, LA, wg1, h);
-      tile_mm<3 * C, C, RM>(Ad, LA, wg1, hd);
+      float h[2][N1][4];
+      g32::gemm_n<3 * C, C, 1, 2>(A, TAN, 0, wg1, C, ring, h);
+      ring.pre<2 * C>(wg2, 2 * C);
+      __syncthreads();
 #pragma unroll
-      for (int i = 0; i < RM; ++i)
+      for (int j = 0; j < N1; ++j) {
+        const int c = C1::col(tx, j);
 #pragma unroll
-        for (int j = 0; j < C / 16; ++j) {
-          const int r = ty + 16 * i, c = tx + 16 * j;
-          H[r * LH + c] = gelu(h[i][j]);
-          Hd[r * LH + c] = gelu_grad(h[i][j]) * hd[i][j];
+        for (int e = 0; e < 4; ++e) {
+          h[1][j][e] *= gelu_grad(h[0][j][e]);
+          h[0][j][e] = gelu(h[0][j][e]);
         }
-    }
-    __syncthreads();
-    {
-      float q[RM][2 * C / 16], qd[RM][2 * C / 16];
-      tile_mm<C, 2 * C, RM>(H, LH, wg2, q);
-      tile_mm<C, 2 * C, RM>(Hd, LH, wg2, qd);
-#pragma unroll
-      for (int i = 0; i < RM; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) {
-          const int r = ty + 16 * i, n = tx + 16 * j;
-          const float g = sigmoid(q[i][j] + __ldg(bg2 + n));
-          const float gd = g * (1.f - g) * qd[i][j];
-          const float s = A[r * LA + C + n], s_d = Ad[r * LA + C + n];
-          Bm[r * LB + n] = s * g;
-          Bd[r * LB + n] = s_d * g + s * gd;
-        }
-    }
-    __syncthreads();
-    {
-      float h[RM][2 * C / 16], hd[RM][2 * C / 16];
-      tile_mm<2 * C, 2 * C, RM>(Bm, LB, wf1, h);
-      tile_mm<2 * C, 2 * C, RM>(Bd, LB, wf1, hd);
-#pragma unroll
-      for (int i = 0; i < RM; ++i)
-#pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) A[(ty + 16 * i) * LA + tx + 16 * j] = gelu_grad(h[i][j]) * hd[i][j];
-    }
-    __syncthreads();
-    float o[RM][C / 16];
-    tile_mm<2 * C, C, RM>(A, LA, wf2, o);
-#pragma unroll
-    for (int i = 0; i < RM; ++i) {
-      const int r = ty + 16 * i;
-      const long v = v0 + r;
-      if (v >= V) continue;
-#pragma unroll
-      for (int j = 0; j < C / 16; ++j) {
-        const int c = tx + 16 * j;
-        outd[v * C + c] = o[i][j] + 0.5f * (Bd[r * LB + c] + Bd[r * LB + C + c]);
+        g32::put4(A, c, h[0][j]);
+        g32::put4(Ad, c, h[1][j]);
       }
     }
+    float half[N1][4];
+    {
+      float q[2][N2][4];
+      g32::gemm_n<C, 2 * C, 2, 2>(A, TAN, 0, wg2, 2 * C, ring, q);
+      ring.pre<2 * C>(wf1, 2 * C);
+#pragma unroll
+      for (int j = 0; j < N2; ++j) {
+        const int n = C2::col(tx, j);
+        const float b = __ldg(bg2 + n);
+        float s[4], st[4];
+        g32::get4(A, C + n, s);
+        g32::get4(Ad, C + n, st);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float g = sigmoid(q[0][j][e] + b);
+          const float gd = g * (1.f - g) * q[1][j][e];
+          q[1][j][e] = st[e] * g + s[e] * gd;
+          q[0][j][e] = s[e] * g;
+        }
+        g32::put4(A, C + n, q[0][j]);
+        g32::put4(Ad, C + n, q[1][j]);
+      }
+#pragma unroll
+      for (int j = 0; j < N1; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) half[j][e] = 0.5f * (q[1][j][e] + q[1][j + N1][e]);
+    }
+    {
+      float h[2][N2][4];
+      g32::gemm_n<2 * C, 2 * C, 1, 2>(A, TAN, C, wf1, 2 * C, ring, h);
+      ring.pre<C>(wf2, C);
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < N2; ++j) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) h[1][j][e] *= gelu_grad(h[0][j][e]);
+        g32::put4(A, Ch::col(tx, j), h[1][j]);
+      }
+    }
+    float o[N1][4];
+    g32::gemm<2 * C, C>(A, 0, wf2, C, ring, o);
+#pragma unroll
+    for (int j = 0; j < N1; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[j][e] += half[j][e];
+    g32::store_rows<C>(outd, nullptr, v0, V, o, al);
   }
 }
 
@@ -368,54 +373,58 @@ __global__ void __launch_bounds__(NT) k_fuse_jvp(const float* __restrict__ x, co
 // + (l_i' - sum_j p_j l_j') / ln 10 with l = h + lte (p = softmax(l)); lte' follows MULTI3D's LTE weights through
 // log10 T and log10 ne (models/ffno_model.py:131-141).
 template <int C, int NHP>
-__global__ void __launch_bounds__(NT) k_head_jvp(const float* __restrict__ x, const float* __restrict__ xd,
+__global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* __restrict__ x, const float* __restrict__ xd,
                                                  const float* __restrict__ xin, const float* __restrict__ xind, long V,
                                                  const float* __restrict__ p1, const float* __restrict__ p2,
                                                  const float* __restrict__ b2, ffno_head_params hp,
-                                                 float* __restrict__ outd) {
-  extern __shared__ float sm[];
-  constexpr int LA = C + 1, LH = 2 * C + 1, LO = NHP + 1;
-  float* as = sm;
-  float* ads = as + BM * LA;
-  float* hs = ads + BM * LA;
-  float* hds = hs + BM * LH;
-  float* os = hds + BM * LH;
+                                                 float* __restrict__ outd, int al) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int LO = NHP + 1, TAN = 2 * C * BM;
+  float* as = sm;                 // [C][64] input, then [2C][64] hidden; their tangents TAN floats on
+  float* os = as + 2 * TAN;       // [64][NHP + 1] head channels, then their tangents
   float* ods = os + BM * LO;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  g32::Ring ring(ods + BM * LO, g32::KC * 2 * C, al);
+  using Ch = g32::Cols<2 * C, 1>;
+  using Co = g32::Cols<NHP, 1>;
+  const int tx = g32::tile_tx(), ty = g32::tile_ty();
   const double lnc = kLN_CCON;
   const long nt = (V + BM - 1) / BM;
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
     __syncthreads();
-    load_rows<C>(as, LA, x, v0, V);
-    load_rows<C>(ads, LA, xd, v0, V);
-    __syncthreads();
+    ring.pre<2 * C>(p1, 2 * C);
+    g32::load_tile<C>(as, 0, x, v0, V, al);
+    g32::load_tile<C>(as + TAN, 0, xd, v0, V, al);
     {
-      float h[4][2 * C / 16], hd[4][2 * C / 16];
-      tile_mm<C, 2 * C>(as, LA, p1, h);
-      tile_mm<C, 2 * C>(ads, LA, p1, hd);
+      float h[2][2 * C / 16][4];
+      g32::gemm_n<C, 2 * C, 1, 2>(as, TAN, 0, p1, 2 * C, ring, h);
+      ring.pre<NHP>(p2, NHP);
+      __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 2 * C / 16; ++j) {
+        const int c = Ch::col(tx, j);
 #pragma unroll
-        for (int j = 0; j < 2 * C / 16; ++j) {
-          const int r = ty + 16 * i, c = tx + 16 * j;
-          hs[r * LH + c] = gelu(h[i][j]);
-          hds[r * LH + c] = gelu_grad(h[i][j]) * hd[i][j];
+        for (int e = 0; e < 4; ++e) {
+          h[1][j][e] *= gelu_grad(h[0][j][e]);
+          h[0][j][e] = gelu(h[0][j][e]);
         }
+        g32::put4(as, c, h[0][j]);
+        g32::put4(as + TAN, c, h[1][j]);
+      }
     }
-    __syncthreads();
     {
-      float o[4][NHP / 16], od[4][NHP / 16];
-      tile_mm<2 * C, NHP>(hs, LH, p2, o);
-      tile_mm<2 * C, NHP>(hds, LH, p2, od);
+      float o[2][NHP / 16][4];
+      g32::gemm_n<2 * C, NHP, 1, 2>(as, TAN, 0, p2, NHP, ring, o);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < NHP / 16; ++j) {
+        const int n = Co::col(tx, j);
+        const float b = __ldg(b2 + n);
 #pragma unroll
-        for (int j = 0; j < NHP / 16; ++j) {
-          const int r = ty + 16 * i, n = tx + 16 * j;
-          os[r * LO + n] = o[i][j] + __ldg(b2 + n);
-          ods[r * LO + n] = od[i][j];
+        for (int e = 0; e < 4; ++e) {
+          os[(4 * ty + e) * LO + n] = o[0][j][e] + b;
+          ods[(4 * ty + e) * LO + n] = o[1][j][e];
         }
+      }
     }
     __syncthreads();
     if (threadIdx.x < BM) {
@@ -550,13 +559,14 @@ int ffno_gn_jvp_apply(const float* pre, const float* pre_dot, const float* gamma
 int ffno_gate_jvp(const float* x, const float* x_dot, long V, int C, const float* w1, const float* w2, float* out_dot,
                   ffno_stream_t stream) {
   if (!x || !x_dot || !w1 || !w2 || !out_dot || !width_ok(C) || V < 1) return FFNO_EINVAL;
+  const int al = g32::aligned(x, x_dot, w1, w2, out_dot);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
 #define L(CC)                                                                                 \
   case CC: {                                                                                  \
-    const size_t smem = 4 * BM * (CC + 1) * sizeof(float);                                    \
+    const size_t smem = (4 * CC * BM + 2 * g32::KC * CC) * sizeof(float);                     \
     if (!smem_attr(k_gate_jvp<CC>, smem)) return FFNO_ELAUNCH;                                \
-    k_gate_jvp<CC><<<grid_rows(V, BM, 2), NT, smem, s>>>(x, x_dot, V, w1, w2, out_dot);        \
+    k_gate_jvp<CC><<<grid_rows(V, BM, CC <= 64 ? 3 : 2), NT, smem, s>>>(x, x_dot, V, w1, w2, out_dot, al); \
     break;                                                                                    \
   }
     L(16) L(32) L(64) L(96)
@@ -569,13 +579,14 @@ int ffno_gate_jvp(const float* x, const float* x_dot, long V, int C, const float
 int ffno_mlp2_jvp(const float* a, const float* a_dot, long V, int C, const float* w1, const float* w2, float* out_dot,
                   ffno_stream_t stream) {
   if (!a || !a_dot || !w1 || !w2 || !out_dot || !width_ok(C) || V < 1) return FFNO_EINVAL;
+  const int al = g32::aligned(a, a_dot, w1, w2, out_dot);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
 #define L(CC)                                                                                   \
   case CC: {                                                                                    \
-    const size_t smem = (2 * BM * (CC + 1) + BM * (2 * CC + 1)) * sizeof(float);                \
+    const size_t smem = (2 * CC * BM + 2 * g32::KC * 2 * CC) * sizeof(float);                   \
     if (!smem_attr(k_mlp2_jvp<CC>, smem)) return FFNO_ELAUNCH;                                  \
-    k_mlp2_jvp<CC><<<grid_rows(V, BM, 2), NT, smem, s>>>(a, a_dot, V, w1, w2, out_dot);          \
+    k_mlp2_jvp<CC><<<grid_rows(V, BM, 2), NT, smem, s>>>(a, a_dot, V, w1, w2, out_dot, al);      \
     break;                                                                                      \
   }
     L(16) L(32) L(64) L(96)
@@ -592,18 +603,20 @@ int ffno_fuse_jvp(const float* x, const float* x_dot, const float* spec_pre, con
   if (!x || !x_dot || !spec_pre || !spec_coefs || !vert_pre || !vert_coefs || !spec_dot || !vert_dot || !wg1 ||
       !wg2 || !bg2 || !wf1 || !wf2 || !fused_dot || !width_ok(C) || V < 1)
     return FFNO_EINVAL;
+  const int al = g32::aligned(x, x_dot, spec_pre, vert_pre, spec_dot, vert_dot, wg1, wg2, wf1, wf2, fused_dot);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
-#define L(CC, RM)                                                                                             \
+#define L(CC)                                                                                                 \
   case CC: {                                                                                                  \
-    const size_t smem = (size_t)16 * RM * (12 * CC + 6) * sizeof(float);                                      \
-    if (!smem_attr(k_fuse_jvp<CC, RM>, smem)) return FFNO_ELAUNCH;                                           \
-    k_fuse_jvp<CC, RM><<<grid_rows(V, 16 * RM, 1), NT, smem, s>>>(x, x_dot, spec_pre, spec_coefs, vert_pre,    \
-                                                                  vert_coefs, spec_dot, vert_dot, V, wg1, wg2, \
-                                                                  bg2, wf1, wf2, fused_dot);                   \
+    const size_t smem = fuse_jvp_smem<CC>();                                                                  \
+    if (!smem_attr(k_fuse_jvp<CC>, smem)) return FFNO_ELAUNCH;                                                \
+    k_fuse_jvp<CC><<<grid_rows(V, BM, CC <= 64 ? 2 : 1), NT, smem, s>>>(x, x_dot, spec_pre, spec_coefs,        \
+                                                                        vert_pre, vert_coefs, spec_dot,       \
+                                                                        vert_dot, V, wg1, wg2, bg2, wf1, wf2, \
+                                                                        fused_dot, al);                       \
     break;                                                                                                    \
   }
-    L(16, 4) L(32, 4) L(64, 4) L(96, 2)
+    L(16) L(32) L(64) L(96)
 #undef L
   }
   FFNO_CHECK_LAUNCH();
@@ -615,13 +628,15 @@ int ffno_head_jvp(const float* x, const float* x_dot, const float* x_in, const f
                   float* out_dot, ffno_stream_t stream) {
   if (!x || !x_dot || !x_in || !x_in_dot || !p1 || !p2 || !b2 || !params || !out_dot || !width_ok(C) || V < 1)
     return FFNO_EINVAL;
+  const int al = g32::aligned(x, x_dot, p1, p2);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C * 1000 + nhp) {
 #define L(CC, NN)                                                                                                  \
   case CC * 1000 + NN: {                                                                                           \
-    const size_t smem = (2 * BM * (CC + 1) + 2 * BM * (2 * CC + 1) + 2 * BM * (NN + 1)) * sizeof(float);           \
+    const size_t smem = (4 * CC * BM + 2 * BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);                  \
     if (!smem_attr(k_head_jvp<CC, NN>, smem)) return FFNO_ELAUNCH;                                                \
-    k_head_jvp<CC, NN><<<grid_rows(V, BM, 2), NT, smem, s>>>(x, x_dot, x_in, x_in_dot, V, p1, p2, b2, *params, out_dot); \
+    k_head_jvp<CC, NN><<<grid_rows(V, BM, CC <= 64 ? 2 : 1), NT, smem, s>>>(x, x_dot, x_in, x_in_dot, V, p1, p2, b2,    \
+                                                                            *params, out_dot, al);                     \
     break;                                                                                                         \
   }
     L(16, 16) L(16, 32) L(32, 16) L(32, 32) L(64, 16) L(64, 32) L(96, 16) L(96, 32)

@@ -31,6 +31,10 @@ int grid_for(long V, int per_sm) {
   return (int)(t < g ? (t > 0 ? t : 1) : g);
 }
 
+// CTAs an SM of the statistics chains (k_mlp2, k_fuse): three of 80 registers a thread, two where the accumulators of a
+// 2C = 192 column GEMM need up to 128.
+__host__ __device__ constexpr int tile_ctas(int C) { return C <= 64 ? 3 : 2; }
+
 template <typename K>
 bool set_smem(K kernel, size_t bytes) {
   return ffno::smem_cap_ok(kernel, bytes);
@@ -199,10 +203,10 @@ __global__ void __launch_bounds__(FIN_NT) k_gn_finalize(const double* __restrict
 // ------------------------------------------------------------------------------------------------ elementwise
 // y = GN(pre) from the finalized coefficients, 4 channels a thread (float4), two float4 in flight per round; the
 // channel index from a 32-bit modulo (n / 4 < 2^31 is checked by the launchers).
-__device__ __forceinline__ float4 gn4(float4 p, const float* __restrict__ cf, int C, int c) {
-  const float4 m = __ldg(reinterpret_cast<const float4*>(cf + c));
-  const float4 sc = __ldg(reinterpret_cast<const float4*>(cf + C + c));
-  const float4 b = __ldg(reinterpret_cast<const float4*>(cf + 2 * C + c));
+__device__ __forceinline__ float4 gn4(float4 p, const float* __restrict__ cf, int C, int c, int al = 1) {
+  const float4 m = g32::ldq(cf + c, true, al);
+  const float4 sc = g32::ldq(cf + C + c, true, al);
+  const float4 b = g32::ldq(cf + 2 * C + c, true, al);
   return make_float4((p.x - m.x) * sc.x + b.x, (p.y - m.y) * sc.y + b.y, (p.z - m.z) * sc.z + b.z,
                      (p.w - m.w) * sc.w + b.w);
 }
@@ -251,11 +255,11 @@ __global__ void k_resid_out(const float* __restrict__ x2, const float* __restric
 template <int C>
 __global__ void __launch_bounds__(NT, C <= 64 ? 4 : 2) k_gate(const float* __restrict__ x, long V, const float* __restrict__ w1,
                                                 const float* __restrict__ w2, const float* __restrict__ zp,
-                                                const float* __restrict__ z, float* __restrict__ out) {
+                                                const float* __restrict__ z, float* __restrict__ out, int al) {
   extern __shared__ __align__(16) float sm[];
   float* xs = sm;             // [C][64]
   float* hs = xs + C * BM;    // [C][64]
-  g32::Ring ring(hs + C * BM, g32::KC * C);
+  g32::Ring ring(hs + C * BM, g32::KC * C, al);
   using Cl = g32::Cols<C, 1>;
   const int tx = g32::tile_tx(), ty = g32::tile_ty();
   const long nt = ntiles_of(V);
@@ -263,7 +267,7 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 4 : 2) k_gate(const float* __res
     const long v0 = t * BM;
     __syncthreads();
     ring.pre<C>(w1, C);
-    g32::load_tile<C>(xs, 0, x, v0, V);
+    g32::load_tile<C>(xs, 0, x, v0, V, al);
     float acc[C / 16][4];
     g32::gemm<C, C>(xs, 0, w1, C, ring, acc);
     ring.pre<C>(w2, C);
@@ -293,29 +297,29 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 4 : 2) k_gate(const float* __res
         acc[j][e] = zp ? o + zc * zv[e] : o;
       }
     }
-    g32::store_rows<C>(out, nullptr, v0, V, acc);
+    g32::store_rows<C>(out, nullptr, v0, V, acc, al);
   }
 }
 
 // ------------------------------------------------------------------------------------------------ 2-layer MLP
 // The hidden layer overwrites the input tile's region (2C channels), so a tile takes 2C x 64 floats plus the weight
-// ring: 48 KB at C = 64. Bound by instruction issue (FMAs, erff) at two CTAs an SM, the grid of the partials. 4.2 M
-// voxels, C = 64: 7.1 -> 4.35 ms (31 TFLOP/s); 296 k voxels, C = 96: 861 -> 577 us.
+// ring: 48 KB at C = 64. Bound by the operand reads from shared memory (4 x 8 outputs a thread). 4.2 M
+// voxels, C = 64: 7.1 -> 4.0 ms (34 TFLOP/s); 296 k voxels, C = 96: 861 -> 577 us.
 template <int C>
 constexpr size_t mlp2_smem() {
   return (2 * C * BM + 2 * g32::KC * 2 * C) * sizeof(float);
 }
 
 template <int C, int MODE>
-__global__ void __launch_bounds__(NT, 2) k_mlp2(const float* __restrict__ in, const float* __restrict__ prev_pre,
+__global__ void __launch_bounds__(NT, tile_ctas(C)) k_mlp2(const float* __restrict__ in, const float* __restrict__ prev_pre,
                                                 const float* __restrict__ pc, float res, float* __restrict__ xout,
                                                 long V, const float* __restrict__ w1, const float* __restrict__ w2,
                                                 const float* __restrict__ dw, float* __restrict__ pre,
-                                                double* __restrict__ partials, int cpg, int groups) {
+                                                double* __restrict__ partials, int nparts, int cpg, int groups, int al) {
   extern __shared__ __align__(16) float sm[];
   __shared__ g32::TileStats<C> st;
   float* as = sm;   // [C][64] input, then [2C][64] hidden
-  g32::Ring ring(as + 2 * C * BM, g32::KC * 2 * C);
+  g32::Ring ring(as + 2 * C * BM, g32::KC * 2 * C, al);
   using Ch = g32::Cols<2 * C, 1>;
   const int tx = g32::tile_tx(), ty = g32::tile_ty();
   GroupAcc acc_g{0.0, 0.0, 0.0};
@@ -325,12 +329,12 @@ __global__ void __launch_bounds__(NT, 2) k_mlp2(const float* __restrict__ in, co
     __syncthreads();
     ring.pre<2 * C>(w1, 2 * C);
     g32::each_quad<C>(v0, V, [&](int r, int c, long o, bool ok) {
-      float4 a = g32::ldq(in + o, ok);
+      float4 a = g32::ldq(in + o, ok, al);
       if (MODE != 0 && ok) {
-        float4 y = gn4(__ldg(reinterpret_cast<const float4*>(prev_pre + o)), pc, C, c);
+        float4 y = gn4(g32::ldq(prev_pre + o, ok, al), pc, C, c, al);
         if (MODE == 1) y = make_float4(gelu(y.x), gelu(y.y), gelu(y.z), gelu(y.w));
         a = make_float4(a.x + res * y.x, a.y + res * y.y, a.z + res * y.z, a.w + res * y.w);
-        *reinterpret_cast<float4*>(xout + o) = a;
+        g32::stq(xout + o, a, al);
       }
       g32::put_quad(as, r, c, a);
     });
@@ -353,10 +357,10 @@ __global__ void __launch_bounds__(NT, 2) k_mlp2(const float* __restrict__ in, co
       const long v = v0 + 4 * ty + e;
       wr[e] = v < V ? __ldg(dw + v) : 0.f;
     }
-    g32::store_rows<C>(pre, nullptr, v0, V, acc);
+    g32::store_rows<C>(pre, nullptr, v0, V, acc, al);
     g32::tile_stats<C>(acc, wr, cpg, groups, st, acc_g);
   }
-  g32::write_tile_partial(partials, groups, acc_g);
+  g32::write_tile_partial(partials, nparts, groups, acc_g);
 }
 
 // ------------------------------------------------------------------------------------------------ gate + fuse
@@ -369,17 +373,17 @@ constexpr size_t fuse_smem() {
 }
 
 template <int C>
-__global__ void __launch_bounds__(NT, 2) k_fuse(const float* __restrict__ x, const float* __restrict__ sp,
+__global__ void __launch_bounds__(NT, tile_ctas(C)) k_fuse(const float* __restrict__ x, const float* __restrict__ sp,
                                                 const float* __restrict__ sc, const float* __restrict__ vp,
                                                 const float* __restrict__ vc, long V, const float* __restrict__ wg1,
                                                 const float* __restrict__ wg2, const float* __restrict__ bg2,
                                                 const float* __restrict__ wf1, const float* __restrict__ wf2,
                                                 const float* __restrict__ dw, float* __restrict__ pre,
-                                                double* __restrict__ partials, int cpg, int groups) {
+                                                double* __restrict__ partials, int nparts, int cpg, int groups, int al) {
   extern __shared__ __align__(16) float sm[];
   __shared__ g32::TileStats<C> st;
   float* as = sm;
-  g32::Ring ring(as + 3 * C * BM, g32::KC * 2 * C);
+  g32::Ring ring(as + 3 * C * BM, g32::KC * 2 * C, al);
   using C1 = g32::Cols<C, 1>;
   using C2 = g32::Cols<2 * C, 2>;   // the thread owns channel c of both branches
   using Ch = g32::Cols<2 * C, 1>;
@@ -393,12 +397,12 @@ __global__ void __launch_bounds__(NT, 2) k_fuse(const float* __restrict__ x, con
     g32::each_quad<C>(v0, V, [&](int r, int c, long o, bool ok) {
       float4 s = make_float4(0.f, 0.f, 0.f, 0.f), q = s;
       if (ok) {
-        s = gn4(__ldg(reinterpret_cast<const float4*>(sp + o)), sc, C, c);
-        q = gn4(__ldg(reinterpret_cast<const float4*>(vp + o)), vc, C, c);
+        s = gn4(g32::ldq(sp + o, ok, al), sc, C, c, al);
+        q = gn4(g32::ldq(vp + o, ok, al), vc, C, c, al);
         s = make_float4(gelu(s.x), gelu(s.y), gelu(s.z), gelu(s.w));
         q = make_float4(gelu(q.x), gelu(q.y), gelu(q.z), gelu(q.w));
       }
-      g32::put_quad(as, r, c, g32::ldq(x + o, ok));
+      g32::put_quad(as, r, c, g32::ldq(x + o, ok, al));
       g32::put_quad(as, r, C + c, s);
       g32::put_quad(as, r, 2 * C + c, q);
     });
@@ -458,10 +462,10 @@ __global__ void __launch_bounds__(NT, 2) k_fuse(const float* __restrict__ x, con
     for (int j = 0; j < C / 16; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[j][e] += half[j][e];
-    g32::store_rows<C>(pre, nullptr, v0, V, acc);
+    g32::store_rows<C>(pre, nullptr, v0, V, acc, al);
     g32::tile_stats<C>(acc, wr, cpg, groups, st, acc_g);
   }
-  g32::write_tile_partial(partials, groups, acc_g);
+  g32::write_tile_partial(partials, nparts, groups, acc_g);
 }
 
 // ------------------------------------------------------------------------------------------------ head
@@ -474,12 +478,12 @@ __global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, con
                                              const float* __restrict__ p1, const float* __restrict__ p2,
                                              const float* __restrict__ b2, int nh,
                                              const __grid_constant__ ffno_head_params hp, float* __restrict__ out,
-                                             float* __restrict__ head_out) {
+                                             float* __restrict__ head_out, int al) {
   extern __shared__ __align__(16) float sm[];
   constexpr int LO = NHP + 1;
   float* as = sm;                    // [C][64] input, then [2C][64] hidden
   float* os = as + 2 * C * BM;       // [64][NHP + 1] head channels
-  g32::Ring ring(os + BM * LO, g32::KC * 2 * C);
+  g32::Ring ring(os + BM * LO, g32::KC * 2 * C, al);
   using Ch = g32::Cols<2 * C, 1>;
   using Co = g32::Cols<NHP, 1>;
   const int tx = g32::tile_tx(), ty = g32::tile_ty();
@@ -488,7 +492,7 @@ __global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, con
     const long v0 = t * BM;
     __syncthreads();
     ring.pre<2 * C>(p1, 2 * C);
-    g32::load_tile<C>(as, 0, x, v0, V);
+    g32::load_tile<C>(as, 0, x, v0, V, al);
     {
       float h[2 * C / 16][4];
       g32::gemm<C, 2 * C>(as, 0, p1, 2 * C, ring, h);
@@ -549,7 +553,7 @@ extern "C" {
 
 const char* ffno_version(void) { return "ffnoml_gb300 0.1 (sm_103a)"; }
 
-int ffno_stats_parts(long V) { return grid_for(V, 2); }
+int ffno_stats_parts(long V) { return grid_for(V, 3); }
 
 int ffno_depth_weights(const float* z, int D, long HW, float* w, ffno_stream_t stream) {
   if (!z || !w || D < 1 || HW < 1) return FFNO_EINVAL;
@@ -628,11 +632,12 @@ int ffno_gate_fwd(const float* x, long V, int C, const float* w1, const float* w
   if (!x || !w1 || !w2 || !out || !width_ok(C) || V < 1 || (zp && !z)) return FFNO_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   const size_t smem = (2 * BM * C + 2 * g32::KC * C) * sizeof(float);
+  const int al = g32::aligned(x, w1, w2, out);
   switch (C) {
 #define L(CC)                                                                   \
   case CC:                                                                      \
     if (!set_smem(k_gate<CC>, smem)) return FFNO_ELAUNCH;                       \
-    k_gate<CC><<<grid_for(V, CC <= 64 ? 4 : 2), NT, smem, s>>>(x, V, w1, w2, zp, z, out);      \
+    k_gate<CC><<<grid_for(V, CC <= 64 ? 4 : 2), NT, smem, s>>>(x, V, w1, w2, zp, z, out, al); \
     break;
     L(16) L(32) L(64) L(96)
 #undef L
@@ -648,24 +653,26 @@ int ffno_mlp2_fwd(int mode, const float* in, const float* prev_pre, const float*
   if (!width_ok(C) || V < 1 || mode < 0 || mode > 2 || groups < 1 || groups > GMAX || C % groups) return FFNO_EINVAL;
   if (mode && (!prev_pre || !prev_coefs || !xout)) return FFNO_EINVAL;
   if (nparts != ffno_stats_parts(V)) return FFNO_EINVAL;
+  const int al = g32::aligned(in, w1, w2, pre) && (!mode || g32::aligned(prev_pre, prev_coefs, xout));
   cudaStream_t s = (cudaStream_t)stream;
   const int cpg = C / groups;
   switch (C) {
 #define L(CC)                                                                                          \
   case CC: {                                                                                           \
     const size_t smem = mlp2_smem<CC>();                                                               \
+    const int grid = grid_for(V, tile_ctas(CC));                                                       \
     if (mode == 0) {                                                                                   \
       if (!set_smem(k_mlp2<CC, 0>, smem)) return FFNO_ELAUNCH;                                         \
-      k_mlp2<CC, 0><<<nparts, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,   \
-                                             partials, cpg, groups);                                   \
+      k_mlp2<CC, 0><<<grid, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
+                                            partials, nparts, cpg, groups, al);                       \
     } else if (mode == 1) {                                                                            \
       if (!set_smem(k_mlp2<CC, 1>, smem)) return FFNO_ELAUNCH;                                         \
-      k_mlp2<CC, 1><<<nparts, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,   \
-                                             partials, cpg, groups);                                   \
+      k_mlp2<CC, 1><<<grid, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
+                                            partials, nparts, cpg, groups, al);                       \
     } else {                                                                                           \
       if (!set_smem(k_mlp2<CC, 2>, smem)) return FFNO_ELAUNCH;                                         \
-      k_mlp2<CC, 2><<<nparts, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,   \
-                                             partials, cpg, groups);                                   \
+      k_mlp2<CC, 2><<<grid, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
+                                            partials, nparts, cpg, groups, al);                       \
     }                                                                                                  \
     break;                                                                                             \
   }
@@ -685,15 +692,17 @@ int ffno_fuse_fwd(const float* x, const float* spec_pre, const float* spec_coefs
     return FFNO_EINVAL;
   if (!width_ok(C) || V < 1 || groups < 1 || groups > GMAX || C % groups) return FFNO_EINVAL;
   if (nparts != ffno_stats_parts(V)) return FFNO_EINVAL;
+  const int al = g32::aligned(x, spec_pre, spec_coefs, vert_pre, vert_coefs, wg1, wg2, wf1, wf2, pre);
   cudaStream_t s = (cudaStream_t)stream;
   const int cpg = C / groups;
   switch (C) {
 #define L(CC)                                                                                                \
   case CC: {                                                                                                 \
     const size_t smem = fuse_smem<CC>();                                                                     \
+    const int grid = grid_for(V, tile_ctas(CC));                                                             \
     if (!set_smem(k_fuse<CC>, smem)) return FFNO_ELAUNCH;                                                    \
-    k_fuse<CC><<<nparts, NT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre, vert_coefs, V, wg1, wg2, bg2, wf1, \
-                                        wf2, dw, pre, partials, cpg, groups);                                \
+    k_fuse<CC><<<grid, NT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre, vert_coefs, V, wg1, wg2, bg2, wf1,   \
+                                      wf2, dw, pre, partials, nparts, cpg, groups, al);                      \
     break;                                                                                                   \
   }
     L(16) L(32) L(64) L(96)
@@ -712,6 +721,7 @@ int ffno_head_fwd(const float* x, const float* x_in, long V, int C, const float*
   int tot = 0;
   for (int s = 0; s < params->nspecies; ++s) tot += params->levels[s] + 1;
   if (tot != nh) return FFNO_EINVAL;
+  const int al = g32::aligned(x, p1, p2);
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
 #define L(CC, NN)                                                                                       \
@@ -719,10 +729,10 @@ int ffno_head_fwd(const float* x, const float* x_in, long V, int C, const float*
     const size_t smem = (2 * CC * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);            \
     if (params->math32) {                                                                               \
       if (!set_smem(k_head<CC, NN, float>, smem)) return FFNO_ELAUNCH;                                  \
-      k_head<CC, NN, float><<<grid_for(V, 2), NT, smem, s>>>(x, x_in, V, p1, p2, b2, nh, *params, out, head_out); \
+      k_head<CC, NN, float><<<grid_for(V, 2), NT, smem, s>>>(x, x_in, V, p1, p2, b2, nh, *params, out, head_out, al); \
     } else {                                                                                            \
       if (!set_smem(k_head<CC, NN, double>, smem)) return FFNO_ELAUNCH;                                 \
-      k_head<CC, NN, double><<<grid_for(V, 2), NT, smem, s>>>(x, x_in, V, p1, p2, b2, nh, *params, out, head_out); \
+      k_head<CC, NN, double><<<grid_for(V, 2), NT, smem, s>>>(x, x_in, V, p1, p2, b2, nh, *params, out, head_out, al); \
     }                                                                                                   \
   }
     default:
@@ -737,6 +747,7 @@ int ffno_proj_fwd(const float* x, long V, int C, const float* p1, const float* p
                   float* head, ffno_stream_t stream) {
   if (!x || !p1 || !p2 || !b2 || !head) return FFNO_EINVAL;
   if (!width_ok(C) || V < 1 || (nhp != 16 && nhp != 32) || nh < 1 || nh > nhp) return FFNO_EINVAL;
+  const int al = g32::aligned(x, p1, p2);
   cudaStream_t s = (cudaStream_t)stream;
   ffno_head_params none{};
   switch (C) {
@@ -745,7 +756,7 @@ int ffno_proj_fwd(const float* x, long V, int C, const float* p1, const float* p
     const size_t smem = (2 * CC * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);            \
     if (!set_smem(k_head<CC, NN, float, false>, smem)) return FFNO_ELAUNCH;                             \
     k_head<CC, NN, float, false><<<grid_for(V, 2), NT, smem, s>>>(x, nullptr, V, p1, p2, b2, nh, none,  \
-                                                                  nullptr, head);                       \
+                                                                  nullptr, head, al);                       \
   }
     default:
       L(16, 16) L(16, 32) L(32, 16) L(32, 32) L(64, 16) L(64, 32) L(96, 16) L(96, 32)
