@@ -409,6 +409,50 @@ __device__ __forceinline__ void write_partial(double* partials, int groups, cons
   }
 }
 
+// Partials row [groups][2] of this CTA (8 warps) from every lane's VW channel sums (channels VW q ..): over the lanes that
+// hold the same channels by shuffles, over the warps per channel, then over each group's channels, in a fixed order. The
+// FP64 pipe is narrow (about two lanes a cycle and SM), so each value is added a few times only: eight groups by a
+// full-warp double reduction each were 80 double additions a lane, 25 us a launch. Rows past the grid hold zeros.
+template <int C, int VW>
+__device__ __forceinline__ void stats_partial_rows(double (&d1)[VW], double (&d2)[VW], bool active, int q, int cpg,
+                                                   int groups, int nparts, double* __restrict__ partials) {
+  constexpr int LPV = C / VW;
+  constexpr bool POW2 = LPV <= 32 && (LPV & (LPV - 1)) == 0;
+  __shared__ double ch[2][8][C];
+  __shared__ double sum[2][C];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int j = 0; j < VW; ++j) {
+    if constexpr (POW2) {
+#pragma unroll
+      for (int o = 16; o >= LPV; o >>= 1) {
+        d1[j] += __shfl_xor_sync(0xffffffffu, d1[j], o);
+        d2[j] += __shfl_xor_sync(0xffffffffu, d2[j], o);
+      }
+    }
+    if (active && lane < LPV) {
+      ch[0][warp][VW * q + j] = d1[j];
+      ch[1][warp][VW * q + j] = d2[j];
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 2 * C; e += blockDim.x) {
+    const int i = e / C, c = e % C;
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += ch[i][w][c];
+    sum[i][c] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * groups) {
+    const int g = threadIdx.x >> 1, i = threadIdx.x & 1;
+    double s = 0.0;
+    for (int c = g * cpg; c < (g + 1) * cpg; ++c) s += sum[i][c];
+    partials[((long)blockIdx.x * groups + g) * 2 + i] = s;
+    for (long p = blockIdx.x + gridDim.x; p < nparts; p += gridDim.x) partials[(p * groups + g) * 2 + i] = 0.0;
+  }
+}
+
 // The dynamic shared memory a kernel may take is a process-wide attribute of that kernel. The service launches the
 // same kernels from several host threads with different sizes (one request per thread), and a thread that lowered the
 // attribute to its own size between another thread's setting and that thread's launch made the launch fail. So the

@@ -329,17 +329,27 @@ __global__ void __launch_bounds__(CT1) k_column_finish(const double* __restrict_
       for (int m = 0; m < live; ++m) g += terms[n + (long)m * D + j - 1];
     gz[j] = g;
   }
-  // d L / d f_m per mode, weighted by d f_m / d dz, summed over the modes in order by one warp
-  if (threadIdx.x < 32) {
+  // d L / d f_m per mode (a warp a mode, its lanes over the nodes), weighted by d f_m / d dz; the warps' sums in order.
+  // One warp with a mode a lane read a whole row of terms per lane: 0.30 ms of latency at 340 modes x 256 nodes
+  {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double t = 0.0;
-    for (int m = threadIdx.x; m < live; m += 32) {
+    for (int m = warp; m < live; m += CT1 / 32) {
       double dl = 0.0;
-      for (int j = 0; j < D; ++j) dl += terms[2 * n + (long)m * D + j];
+#pragma unroll 4
+      for (int j = lane; j < D; j += 32) dl += terms[2 * n + (long)m * D + j];
       t += dl * df[m];
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (threadIdx.x == 0) gtap = t;
+    __shared__ double wt[CT1 / 32];
+    if (lane == 0) wt[warp] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double a = 0.0;
+      for (int w = 0; w < CT1 / 32; ++w) a += wt[w];
+      gtap = a;
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {

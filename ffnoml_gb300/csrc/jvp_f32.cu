@@ -48,7 +48,6 @@ __global__ void __launch_bounds__(256) k_gn_jvp_stats(const float* __restrict__ 
   constexpr int LPV = C / 4;                       // lanes per voxel (float4 each)
   constexpr int VPW = LPV <= 32 ? 32 / LPV : 1;    // voxels per warp step
   __shared__ float mean[GMAX], rstd[GMAX];
-  __shared__ double red[8][GMAX][2];
   if (threadIdx.x < groups) {
     mean[threadIdx.x] = (float)gst[3 * threadIdx.x];
     rstd[threadIdx.x] = (float)gst[3 * threadIdx.x + 1];
@@ -92,34 +91,7 @@ __global__ void __launch_bounds__(256) k_gn_jvp_stats(const float* __restrict__ 
     d1[j] += f1[j];
     d2[j] += f2[j];
   }
-  for (int g = 0; g < groups; ++g) {
-    double a = 0.0, b = 0.0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (active && grp[j] == g) {
-        a += d1[j];
-        b += d2[j];
-      }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if (lane == 0) {
-      red[warp][g][0] = a;
-      red[warp][g][1] = b;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < groups) {
-    double a = 0.0, b = 0.0;
-    for (int w = 0; w < 8; ++w) {
-      a += red[w][threadIdx.x][0];
-      b += red[w][threadIdx.x][1];
-    }
-    partials[((long)blockIdx.x * groups + threadIdx.x) * 2] = a;
-    partials[((long)blockIdx.x * groups + threadIdx.x) * 2 + 1] = b;
-  }
+  stats_partial_rows<C, 4>(d1, d2, active, q, cpg, groups, gridDim.x, partials);
 }
 
 // out = base + res * y' (base may be null; act 1: y' times gelu'(y), a GELU after the GroupNorm)

@@ -41,30 +41,42 @@ bool set_smem(K kernel, size_t bytes) {
 }
 
 // ------------------------------------------------------------------------------------------------ depth weights
-__global__ void k_depth_weights(const float* __restrict__ z, int D, long HW, float* __restrict__ w) {
-  const long col = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (col >= HW) return;
+// A CTA holds DW_COLS neighbouring columns (coalesced rows), DW_SEGS threads share each column's levels, and the column
+// sum is the fixed-order sum of the segments' sums. Bound by latency: with one thread a column, each of its D levels waited for
+// memory twice. 101 x 45 x 75: 37 -> 5 us.
+constexpr int DW_COLS = 32, DW_SEGS = 16;
+
+__global__ void __launch_bounds__(DW_COLS* DW_SEGS) k_depth_weights(const float* __restrict__ z, int D, long HW,
+                                                                    float* __restrict__ w) {
+  __shared__ float part[DW_SEGS][DW_COLS];
+  const int tx = threadIdx.x % DW_COLS, sg = threadIdx.x / DW_COLS;
+  const long col = (long)blockIdx.x * DW_COLS + tx;
+  const bool ok = col < HW;
   if (D == 1) {
-    w[col] = 1.f;
+    if (ok && sg == 0) w[col] = 1.f;
     return;
   }
-  float sum = 0.f;
-  float prev = z[col];
-  float half_prev = 0.f;
-  for (int d = 0; d < D; ++d) {
-    float half_next = 0.f;
-    if (d + 1 < D) {
-      const float nx = z[(long)(d + 1) * HW + col];
-      half_next = 0.5f * fabsf(nx - prev);
-      prev = nx;
-    }
-    const float t = half_prev + half_next;
-    w[(long)d * HW + col] = t;
-    sum += t;
-    half_prev = half_next;
+  // share of level d: half the distances to its neighbours
+  auto share = [&](int d) {
+    const float zd = __ldg(z + (long)d * HW + col);
+    const float lo = d > 0 ? 0.5f * fabsf(zd - __ldg(z + (long)(d - 1) * HW + col)) : 0.f;
+    const float hi = d + 1 < D ? 0.5f * fabsf(__ldg(z + (long)(d + 1) * HW + col) - zd) : 0.f;
+    return lo + hi;
+  };
+  float s = 0.f;
+  if (ok) {
+#pragma unroll 4
+    for (int d = sg; d < D; d += DW_SEGS) s += share(d);
   }
-  const float mean = fmaxf(sum / (float)D, 1e-12f);
-  for (int d = 0; d < D; ++d) w[(long)d * HW + col] /= mean;
+  part[sg][tx] = s;
+  __syncthreads();
+  if (!ok) return;
+  s = 0.f;
+#pragma unroll
+  for (int i = 0; i < DW_SEGS; ++i) s += part[i][tx];
+  const float mean = fmaxf(s / (float)D, 1e-12f);
+#pragma unroll 4
+  for (int d = sg; d < D; d += DW_SEGS) w[(long)d * HW + col] = share(d) / mean;
 }
 
 // ------------------------------------------------------------------------------------------------ column info
@@ -98,42 +110,67 @@ __global__ void k_column_info_final(unsigned int* flags) {
 }
 
 // ------------------------------------------------------------------------------------------------ lift
+// x_in arrives channels-first: a tile's rows of each input channel are 64 consecutive floats. The thread mapping is the tile
+// GEMM's (4 voxels x C / 16 channels, 16-byte stores, 4-barrier statistics); bound by the store of pre. 4.2 M voxels,
+// C = 64: 1.34 -> 0.98 ms.
 template <int C>
-__global__ void __launch_bounds__(NT) k_lift(const float* __restrict__ xin, int cin, long V,
-                                             const float* __restrict__ wl, const float* __restrict__ dw,
-                                             float* __restrict__ pre, double* __restrict__ partials, int cpg,
-                                             int groups) {
-  __shared__ float xs[8][BM];
-  __shared__ StatsSmem<C> st;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  GroupAcc acc{0.0, 0.0, 0.0};
+__global__ void __launch_bounds__(NT, 3) k_lift(const float* __restrict__ xin, int cin, long V,
+                                                const float* __restrict__ wl, const float* __restrict__ dw,
+                                                float* __restrict__ pre, double* __restrict__ partials, int cpg,
+                                                int groups, int al) {
+  __shared__ __align__(16) float xs[2][8][BM];
+  __shared__ __align__(16) float ws[8][C];
+  __shared__ g32::TileStats<C> st;
+  using Cl = g32::Cols<C, 1>;
+  const int tx = g32::tile_tx(), ty = g32::tile_ty();
+  GroupAcc acc_g{0.0, 0.0, 0.0};
   const long nt = ntiles_of(V);
-  for (long t = blockIdx.x; t < nt; t += gridDim.x) {
+  for (int e = threadIdx.x; e < cin * C; e += NT) ws[e / C][e % C] = __ldg(wl + e);
+  // the next tile's inputs wait in registers (at most 2 of the 8 x 64 values a thread) while this one is processed
+  float nx[2];
+  auto fetch = [&](long t) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int e = threadIdx.x + i * NT, k = e / BM, r = e % BM;
+      const long v = t * BM + r;
+      nx[i] = k < cin && t < nt && v < V ? __ldg(xin + (long)k * V + v) : 0.f;
+    }
+  };
+  fetch(blockIdx.x);
+  int buf = 0;
+  for (long t = blockIdx.x; t < nt; t += gridDim.x, buf ^= 1) {
     const long v0 = t * BM;
-    __syncthreads();
-    for (int e = threadIdx.x; e < cin * BM; e += NT) {
-      const int k = e / BM, r = e % BM;
-      xs[k][r] = (v0 + r < V) ? __ldg(xin + (long)k * V + v0 + r) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int e = threadIdx.x + i * NT;
+      xs[buf][e / BM][e % BM] = nx[i];
     }
     __syncthreads();
-    float val[4][C / 16], wr[4];
+    fetch(t + gridDim.x);
+    float acc[C / 16][4], wr[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = ty + 16 * i;
-      const long v = v0 + r;
-      wr[i] = v < V ? __ldg(dw + v) : 0.f;
+    for (int j = 0; j < C / 16; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+    for (int k = 0; k < cin; ++k) {
+      const float4 q = *reinterpret_cast<const float4*>(&xs[buf][k][4 * ty]);
+      const float x[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int j = 0; j < C / 16; ++j) {
-        const int c = tx + 16 * j;
-        float s = 0.f;
-        for (int k = 0; k < cin; ++k) s = fmaf(xs[k][r], __ldg(wl + k * C + c), s);
-        val[i][j] = s;
-        if (v < V) pre[v * C + c] = s;
+        const float w = ws[k][Cl::col(tx, j)];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = fmaf(x[e], w, acc[j][e]);
       }
     }
-    tile_group_stats<C>(val, wr, cpg, groups, st, acc);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const long v = v0 + 4 * ty + e;
+      wr[e] = v < V ? __ldg(dw + v) : 0.f;
+    }
+    g32::store_rows<C>(pre, nullptr, v0, V, acc, al);
+    g32::tile_stats<C>(acc, wr, cpg, groups, st, acc_g);
   }
-  write_partial(partials, groups, acc);
+  g32::write_tile_partial(partials, gridDim.x, groups, acc_g);
 }
 
 // ------------------------------------------------------------------------------------------------ GN finalize
@@ -557,7 +594,7 @@ int ffno_stats_parts(long V) { return grid_for(V, 3); }
 
 int ffno_depth_weights(const float* z, int D, long HW, float* w, ffno_stream_t stream) {
   if (!z || !w || D < 1 || HW < 1) return FFNO_EINVAL;
-  k_depth_weights<<<(unsigned)((HW + 255) / 256), 256, 0, (cudaStream_t)stream>>>(z, D, HW, w);
+  k_depth_weights<<<(unsigned)((HW + DW_COLS - 1) / DW_COLS), DW_COLS * DW_SEGS, 0, (cudaStream_t)stream>>>(z, D, HW, w);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -577,10 +614,11 @@ int ffno_lift_fwd(const float* x_in, int cin, long V, int C, const float* w_lift
   if (!x_in || !w_lift || !dw || !pre || !partials) return FFNO_EINVAL;
   if (!width_ok(C) || cin < 1 || cin > 8 || V < 1 || groups < 1 || groups > GMAX || C % groups) return FFNO_EINVAL;
   if (nparts != ffno_stats_parts(V)) return FFNO_EINVAL;
+  const int al = g32::aligned(pre);
   cudaStream_t s = (cudaStream_t)stream;
   const int cpg = C / groups;
   switch (C) {
-#define L(CC) case CC: k_lift<CC><<<nparts, NT, 0, s>>>(x_in, cin, V, w_lift, dw, pre, partials, cpg, groups); break;
+#define L(CC) case CC: k_lift<CC><<<nparts, NT, 0, s>>>(x_in, cin, V, w_lift, dw, pre, partials, cpg, groups, al); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }

@@ -816,14 +816,27 @@ __global__ void __launch_bounds__(OT, 1) k_outer_tc(const float* __restrict__ A,
   if (warp == 0) tc::tmem_free(tmem, ncol);
 }
 
-// part [nsplit][rows][cols] -> out rows of stride ldo (ldo = cols: out is the contiguous [rows][cols] product)
-__global__ void k_outer_tc_reduce(const float* __restrict__ part, long nsplit, long n, long cols, long ldo,
-                                  double* __restrict__ out, int accumulate) {
-  const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (e >= n) return;
+// part [nsplit][rows][cols] -> out rows of stride ldo (ldo = cols: out is the contiguous [rows][cols] product). RD_SEGS
+// threads an element, each every RD_SEGS-th split, summed in FP64 in a fixed order (one thread an element is bound by
+// the latency of its walk over the splits: 33 us at 152 splits of 6666 elements -> 12 us).
+constexpr int RD_EL = 32, RD_SEGS = 8;
+
+__global__ void __launch_bounds__(RD_EL* RD_SEGS) k_outer_tc_reduce(const float* __restrict__ part, long nsplit, long n,
+                                                                    long cols, long ldo, double* __restrict__ out,
+                                                                    int accumulate) {
+  __shared__ double red[RD_SEGS][RD_EL];
+  const int tx = threadIdx.x % RD_EL, sg = threadIdx.x / RD_EL;
+  const long e = (long)blockIdx.x * RD_EL + tx;
   double s = 0.0;
-#pragma unroll 8
-  for (long p = 0; p < nsplit; ++p) s += (double)part[p * n + e];   // loads issued ahead, sums in order
+  if (e < n) {
+#pragma unroll 4
+    for (long p = sg; p < nsplit; p += RD_SEGS) s += (double)__ldg(part + p * n + e);
+  }
+  red[sg][tx] = s;
+  __syncthreads();
+  if (sg || e >= n) return;
+#pragma unroll
+  for (int i = 1; i < RD_SEGS; ++i) s += red[i][tx];
   double* o = out + (e / cols) * ldo + e % cols;
   *o = accumulate ? *o + s : s;
 }
@@ -1002,7 +1015,7 @@ int ffno_outer_tc_ld(const float* A, long lda, int Ma, const float* B, long ldb,
     k_outer_tc<<<nsplit, OT, smem, s>>>(B, ldb, Mb, A, lda, Ma, N, TI, NB, NS, cps, part, n, 1, Mb, err);
   else
     k_outer_tc<<<nsplit, OT, smem, s>>>(A, lda, Ma, B, ldb, Mb, N, TI, NB, NS, cps, part, n, Mb, 1, err);
-  k_outer_tc_reduce<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(part, nsplit, n, Mb, ldo, out, accumulate);
+  k_outer_tc_reduce<<<(unsigned)((n + RD_EL - 1) / RD_EL), RD_EL * RD_SEGS, 0, s>>>(part, nsplit, n, Mb, ldo, out, accumulate);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
