@@ -273,6 +273,83 @@ __device__ __forceinline__ void chan_merge(GroupAcc& a, double wt, double mt, do
   a.w = wn;
 }
 
+// The same running statistics without a division per merge: sums of w, w (mean - ref) and m2 + w (mean - ref)^2 about
+// the first merged mean, in FP64. A Chan merge has two dependent FP64 divisions, microseconds of a serial chain on this
+// chip's FP64 pipe, where a tile's whole budget is three; this is five FP64 multiply-adds whose results nothing waits
+// for. get(): the (w, mean, m2) that the Chan merges would have given, to FP64 rounding about ref.
+struct ShiftAcc {
+  double w = 0.0, s1 = 0.0, s2 = 0.0, ref = 0.0;
+  __device__ __forceinline__ void add(float wt, float mean, float m2) {
+    if (wt <= 0.f) return;   // a NaN weight counts
+    if (w == 0.0) ref = (double)mean;
+    const double d = (double)mean - ref, wd = (double)wt * d;
+    w += (double)wt;
+    s1 += wd;
+    s2 += (double)m2 + wd * d;
+  }
+  __device__ __forceinline__ GroupAcc get() const {
+    if (w == 0.0) return GroupAcc{0.0, 0.0, 0.0};
+    const double m = s1 / w;
+    const double m2 = s2 - s1 * m;
+    return GroupAcc{w, ref + m, m2 < 0.0 ? 0.0 : m2};
+  }
+};
+
+// Sum of s[g] over the warp's lanes, for the group g = lane / 4: a butterfly that halves the groups a lane carries at
+// each step (9 shuffles for the eight sums; 40 when every lane reduces all of them).
+__device__ __forceinline__ float warp_group_sum(const float (&s)[GMAX]) {
+  static_assert(GMAX == 8, "three halving steps");
+  const int lane = threadIdx.x & 31;
+  float a[4], b[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float keep = (lane & 16) ? s[4 + i] : s[i], send = (lane & 16) ? s[i] : s[4 + i];
+    a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float keep = (lane & 8) ? a[2 + i] : a[i], send = (lane & 8) ? a[i] : a[2 + i];
+    b[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  float r = ((lane & 4) ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, (lane & 4) ? b[0] : b[1], 4);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  r += __shfl_xor_sync(0xffffffffu, r, 1);
+  return r;
+}
+
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The partials row of a CTA from NW warps' statistics acc[warp][group] (shared memory, written before a barrier), merged
+// in warp order by thread g.
+template <int NW>
+__device__ __forceinline__ void write_warp_partials(double* partials, const double (&acc)[NW][GMAX][3]) {
+  if (threadIdx.x < GMAX) {
+    const int g = threadIdx.x;
+    GroupAcc a{0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int w = 0; w < NW; ++w) chan_merge(a, acc[w][g][0], acc[w][g][1], acc[w][g][2]);
+    double* o = partials + ((long)blockIdx.x * GMAX + g) * 3;
+    o[0] = a.w;
+    o[1] = a.mean;
+    o[2] = a.m2;
+  }
+}
+
+// Lane 4 g's running statistics of group g into the warp's row of acc.
+__device__ __forceinline__ void put_warp_stats(double (*acc)[3], const ShiftAcc& st) {
+  const int lane = threadIdx.x & 31;
+  if ((lane & 3) == 0) {
+    const GroupAcc a = st.get();
+    acc[lane >> 2][0] = a.w;
+    acc[lane >> 2][1] = a.mean;
+    acc[lane >> 2][2] = a.m2;
+  }
+}
+
 // Scratch (shared memory) for tile_group_stats: colsum [16][N], col [N], gmean [GMAX], gw (1)
 template <int N>
 struct StatsSmem {

@@ -254,7 +254,7 @@ struct TileStats {
 // order; 4 barriers.
 template <int C>
 __device__ __forceinline__ void tile_stats(const float (&acc)[C / 16][4], const float (&wr)[4], int cpg, int groups,
-                                           TileStats<C>& st, GroupAcc& acc_g) {
+                                           TileStats<C>& st, ShiftAcc& acc_g) {
   using Cl = Cols<C, 1>;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = tile_tx();
   auto columns = [&](auto value) {
@@ -295,16 +295,17 @@ __device__ __forceinline__ void tile_stats(const float (&acc)[C / 16][4], const 
   __syncthreads();
   if (warp < groups) {
     const float s = group_sum();
-    if (lane == 0) chan_merge(acc_g, (double)wsum * cpg, (double)st.gmean[warp], (double)s);
+    if (lane == 0) acc_g.add(wt, st.gmean[warp], s);
   }
   __syncthreads();
 }
 
 // Partials row of this CTA, from thread 32 g's accumulators of group g; the rows past the grid (nparts is the most CTAs
 // any of these kernels runs) hold no weight.
-__device__ __forceinline__ void write_tile_partial(double* partials, int nparts, int groups, const GroupAcc& a) {
+__device__ __forceinline__ void write_tile_partial(double* partials, int nparts, int groups, const ShiftAcc& acc_g) {
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   if (lane == 0 && g < groups) {
+    const GroupAcc a = acc_g.get();
     double* p = partials + ((long)blockIdx.x * groups + g) * 3;
     p[0] = a.w;
     p[1] = a.mean;

@@ -112,7 +112,7 @@ __global__ void k_column_info_final(unsigned int* flags) {
 // ------------------------------------------------------------------------------------------------ lift
 // x_in arrives channels-first: a tile's rows of each input channel are 64 consecutive floats. The thread mapping is the tile
 // GEMM's (4 voxels x C / 16 channels, 16-byte stores, 4-barrier statistics); bound by the store of pre. 4.2 M voxels,
-// C = 64: 1.34 -> 0.98 ms.
+// C = 64: 1.34 -> 0.53 ms.
 template <int C>
 __global__ void __launch_bounds__(NT, 3) k_lift(const float* __restrict__ xin, int cin, long V,
                                                 const float* __restrict__ wl, const float* __restrict__ dw,
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(NT, 3) k_lift(const float* __restrict__ xin, i
   __shared__ g32::TileStats<C> st;
   using Cl = g32::Cols<C, 1>;
   const int tx = g32::tile_tx(), ty = g32::tile_ty();
-  GroupAcc acc_g{0.0, 0.0, 0.0};
+  ShiftAcc acc_g;
   const long nt = ntiles_of(V);
   for (int e = threadIdx.x; e < cin * C; e += NT) ws[e / C][e % C] = __ldg(wl + e);
   // the next tile's inputs wait in registers (at most 2 of the 8 x 64 values a thread) while this one is processed
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(NT, tile_ctas(C)) k_mlp2(const float* __restri
   g32::Ring ring(as + 2 * C * BM, g32::KC * 2 * C, al);
   using Ch = g32::Cols<2 * C, 1>;
   const int tx = g32::tile_tx(), ty = g32::tile_ty();
-  GroupAcc acc_g{0.0, 0.0, 0.0};
+  ShiftAcc acc_g;
   const long nt = ntiles_of(V);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(NT, tile_ctas(C)) k_fuse(const float* __restri
   using C2 = g32::Cols<2 * C, 2>;   // the thread owns channel c of both branches
   using Ch = g32::Cols<2 * C, 1>;
   const int tx = g32::tile_tx(), ty = g32::tile_ty();
-  GroupAcc acc_g{0.0, 0.0, 0.0};
+  ShiftAcc acc_g;
   const long nt = ntiles_of(V);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;

@@ -424,53 +424,32 @@ __device__ __forceinline__ void put16(Split t, int r, int c0, int K, const float
   *reinterpret_cast<uint4*>(t.lo() + o1) = make_uint4(l[4], l[5], l[6], l[7]);
 }
 
-// Depth-weighted statistics of a row-oriented tile: every thread holds, in v[C], the chunks of its row it owns and
-// the row's weight w (0 past the cube). Merged with Chan's update into acc[g] by thread g < GMAX; fixed order.
-// red: [8][GMAX + 1] of this pipeline.
+// Depth-weighted statistics of a row-oriented tile: every thread holds, in v[C], the chunks of its row it owns and the
+// row's weight w (0 past the cube). Each warp takes its own 32 rows and its half of the chunks through two passes and adds
+// them to its running statistics (lanes 4 g .. 4 g + 3: group g), so no barrier and no division chain stands between
+// two tiles.
 template <int C>
-__device__ __forceinline__ void row_stats(const Pipe& p, const float (&v)[C], float w, float* red, float* gm,
-                                          float* wsum, double* acc) {
-  constexpr int CPG = C / GMAX, NW = PT / 32;
-  const int lane = p.lane, wl = p.ptid >> 5;
-  float ws = p.half == 0 ? w : 0.f;
+__device__ __forceinline__ void row_stats(const Pipe& p, const float (&v)[C], float w, ShiftAcc& st) {
+  constexpr int CPG = C / GMAX;
+  const int gl = p.lane >> 2;
+  int n = 0;   // channels of this lane's group in the warp's chunks
 #pragma unroll
-  for (int o = 16; o; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
-  float s[GMAX];
+  for (int i = 0; i < CPG; ++i) n += owns((gl * CPG + i) / 16, p.half) ? 1 : 0;
+  const float wt = warp_sum(w) * (float)n;
+  float s[GMAX], gm[GMAX];
 #pragma unroll
   for (int g = 0; g < GMAX; ++g) s[g] = 0.f;
 #pragma unroll
   for (int c = 0; c < C; ++c)
     if (owns(c / 16, p.half)) s[c / CPG] += v[c];
 #pragma unroll
+  for (int g = 0; g < GMAX; ++g) s[g] *= w;
+  const float tot = warp_group_sum(s), mean = wt > 0.f ? tot / wt : 0.f;
+#pragma unroll
   for (int g = 0; g < GMAX; ++g) {
-    float x = w * s[g];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    s[g] = x;
+    gm[g] = __shfl_sync(0xffffffffu, mean, 4 * g);
+    s[g] = 0.f;
   }
-  if (lane == 0) {
-    red[wl * (GMAX + 1) + GMAX] = ws;
-#pragma unroll
-    for (int g = 0; g < GMAX; ++g) red[wl * (GMAX + 1) + g] = s[g];
-  }
-  pipe_sync(p.id);
-  if (p.ptid == 0) {
-    float t = 0.f;
-    for (int q = 0; q < NW; ++q) t += red[q * (GMAX + 1) + GMAX];
-    *wsum = t;
-  }
-  if (p.ptid < GMAX) {
-    float t = 0.f, wt = 0.f;
-    for (int q = 0; q < NW; ++q) {
-      t += red[q * (GMAX + 1) + p.ptid];
-      wt += red[q * (GMAX + 1) + GMAX];
-    }
-    wt *= CPG;
-    gm[p.ptid] = wt > 0.f ? t / wt : 0.f;
-  }
-  pipe_sync(p.id);
-#pragma unroll
-  for (int g = 0; g < GMAX; ++g) s[g] = 0.f;
 #pragma unroll
   for (int c = 0; c < C; ++c)
     if (owns(c / 16, p.half)) {
@@ -478,27 +457,8 @@ __device__ __forceinline__ void row_stats(const Pipe& p, const float (&v)[C], fl
       s[c / CPG] += d * d;
     }
 #pragma unroll
-  for (int g = 0; g < GMAX; ++g) {
-    float x = w * s[g];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    s[g] = x;
-  }
-  if (lane == 0)
-#pragma unroll
-    for (int g = 0; g < GMAX; ++g) red[wl * (GMAX + 1) + g] = s[g];
-  pipe_sync(p.id);
-  if (p.ptid < GMAX) {
-    float t = 0.f;
-    for (int q = 0; q < NW; ++q) t += red[q * (GMAX + 1) + p.ptid];
-    double* a = acc + 3 * p.ptid;
-    GroupAcc ga{a[0], a[1], a[2]};
-    chan_merge(ga, (double)*wsum * CPG, (double)gm[p.ptid], (double)t);
-    a[0] = ga.w;
-    a[1] = ga.mean;
-    a[2] = ga.m2;
-  }
-  pipe_sync(p.id);
+  for (int g = 0; g < GMAX; ++g) s[g] *= w;
+  st.add(wt, mean, warp_group_sum(s));
 }
 
 // The CTA's GroupNorm partial: pipeline 1's statistics merged into pipeline 0's (fixed order). All threads call it.
@@ -1414,11 +1374,10 @@ __global__ void __launch_bounds__(PT, 1) k_mlp2_tc96(const float* __restrict__ i
   constexpr int C = C96;
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(C, 2 * C);
-  __shared__ float red[(PT / 32) * (GMAX + 1)], gm[GMAX], wsum;
-  __shared__ double acc[GMAX * 3];
+  __shared__ double acc[PT / 32][GMAX][3];   // the warps' statistics
+  ShiftAcc stat;
   PIPE_PROLOGUE(3 * C, 1)
   const Split T = split_at(smem + B1 + B2, TM, C);   // the input tile, then each K-half of the hidden layer
-  if (tid < GMAX * 3) acc[tid] = 0.0;
   P.ok = load_weights(smem, wpack, B1 + B2, wcx, err);
   const Op w1 = wop(smem, 2 * C, C);
   const int row = P.feat();
@@ -1472,15 +1431,11 @@ __global__ void __launch_bounds__(PT, 1) k_mlp2_tc96(const float* __restrict__ i
         st8(pre + v * C + 16 * j + 8, r + 8);
       }
     }
-    row_stats<C>(P, vals, w, red, gm, &wsum, acc);
+    row_stats<C>(P, vals, w, stat);
   }
+  put_warp_stats(acc[tid >> 5], stat);
   __syncthreads();
-  if (tid < GMAX) {
-    double* o = partials + ((long)blockIdx.x * GMAX + tid) * 3;
-    o[0] = acc[3 * tid];
-    o[1] = acc[3 * tid + 1];
-    o[2] = acc[3 * tid + 2];
-  }
+  write_warp_partials<PT / 32>(partials, acc);
   pipe_finish(P, tslot, NCOL);
 }
 
@@ -1694,11 +1649,10 @@ __global__ void __launch_bounds__(PT, 1) k_fuse_out_tc96(const float* __restrict
   constexpr int C = C96;
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr uint32_t B1 = mat_bytes(C, 2 * C);
-  __shared__ float red[(PT / 32) * (GMAX + 1)], gm[GMAX], wsum;
-  __shared__ double acc[GMAX * 3];
+  __shared__ double acc[PT / 32][GMAX][3];   // the warps' statistics
+  ShiftAcc stat;
   PIPE_PROLOGUE(C, 1)
   const Split T = split_at(smem + B1, TM, KS);
-  if (tid < GMAX * 3) acc[tid] = 0.0;
   P.ok = load_weights(smem, wpack, B1, wcx, err);
   const int row = P.feat();
   for (long t = t0; P.ok && t < nt; t += tstep) {
@@ -1746,15 +1700,11 @@ __global__ void __launch_bounds__(PT, 1) k_fuse_out_tc96(const float* __restrict
 #pragma unroll
       for (int i = 0; i < 16; ++i) vals[16 * j + i] = r[i];
     }
-    row_stats<C>(P, vals, w, red, gm, &wsum, acc);
+    row_stats<C>(P, vals, w, stat);
   }
+  put_warp_stats(acc[tid >> 5], stat);
   __syncthreads();
-  if (tid < GMAX) {
-    double* o = partials + ((long)blockIdx.x * GMAX + tid) * 3;
-    o[0] = acc[3 * tid];
-    o[1] = acc[3 * tid + 1];
-    o[2] = acc[3 * tid + 2];
-  }
+  write_warp_partials<PT / 32>(partials, acc);
   pipe_finish(P, tslot, NCOL);
 }
 

@@ -63,20 +63,6 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
 
-// barrier of the four epilogue-2 warps (named barrier 1)
-__device__ __forceinline__ void e2_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
-
-// The same barrier returning whether p holds in all four warps, so that they leave their tile loop together.
-__device__ __forceinline__ bool e2_sync_and(bool p) {
-  uint32_t r;
-  asm volatile(
-      "{\n .reg .pred pi, po;\n setp.ne.u32 pi, %1, 0;\n bar.red.and.pred po, 1, 128, pi;\n selp.u32 %0, 1, 0, po;\n}"
-      : "=r"(r)
-      : "r"((uint32_t)p)
-      : "memory");
-  return r != 0;
-}
-
 template <int C>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_mlp2_bwd_ws(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_pb,
@@ -318,8 +304,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   __shared__ uint64_t stg_full[2], stg_empty[2], a_full[NA], a_empty[NA], d2_full[NA], d1_full[2], h_full[2], wbar;
   __shared__ uint32_t tslot;
   __shared__ float cf[3 * C];                 // GroupNorm coefficients of prev: mean, gamma rstd, beta
-  __shared__ float red[4][GMAX + 1], gmean[GMAX], wsum;
-  __shared__ double acc[GMAX * 3];
+  __shared__ double acc[4][GMAX][3];          // the epilogue-2 warps' statistics
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) tc::tmem_alloc(&tslot, 512);
   if (threadIdx.x == 0) {
@@ -339,7 +324,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
   if (MODE != 0)
     for (int e = threadIdx.x; e < 3 * C; e += NTHREADS) cf[e] = pc[e];
-  if (threadIdx.x < GMAX * 3) acc[threadIdx.x] = 0.0;
+  if (threadIdx.x < 4 * GMAX * 3) (&acc[0][0][0])[threadIdx.x] = 0.0;
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
@@ -508,15 +493,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   } else if (ok && warp >= W_E2) {
     const int q = warp & 3, r = 32 * q + lane, wl = warp - W_E2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
+    ShiftAcc stat;
     for (int i = 0; i < niter; ++i) {
       const int sa = i % NA;
       const long v = tile_of(i) * TM + r;
       const bool live = v < V;
       const float w = live ? __ldg(dw + v) : 0.f;
-      if (!e2_sync_and(tc::mbar_wait_for(&d2_full[sa], (uint32_t)(i / NA) & 1u, WAIT_NS))) {
-        if (lane == 0) atomicExch(err, 10);
-        break;
-      }
+      if (!warp_wait(&d2_full[sa], (uint32_t)(i / NA) & 1u, err, 10)) break;
       tc::tc_after_sync();
       // pass 1: pre to HBM and the weighted group sums (CPG = C / 8 channels per group; a 16-column chunk holds
       // 16 / CPG groups)
@@ -541,25 +524,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           gs[g] += __uint_as_float(d[e]);
         }
       }
-      float ws = w;
+      // the warp's own 32 voxels: weight and mean of each group (lanes 4 g .. 4 g + 3 hold group g), no barrier
+      const float wt = warp_sum(w) * CPG;
 #pragma unroll
-      for (int m = 16; m; m >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, m);
+      for (int g = 0; g < GMAX; ++g) gs[g] *= w;
+      const float tot = warp_group_sum(gs), mean = wt > 0.f ? tot / wt : 0.f;
+      float gm[GMAX];
 #pragma unroll
-      for (int g = 0; g < GMAX; ++g) {
-        float t = w * gs[g];
-#pragma unroll
-        for (int m = 16; m; m >>= 1) t += __shfl_xor_sync(0xffffffffu, t, m);
-        if (lane == 0) red[wl][g] = t;
-      }
-      if (lane == 0) red[wl][GMAX] = ws;
-      e2_sync();
-      if (threadIdx.x - 32 * W_E2 < GMAX) {
-        const int g = threadIdx.x - 32 * W_E2;
-        const float wt = ((red[0][GMAX] + red[1][GMAX]) + (red[2][GMAX] + red[3][GMAX])) * CPG;
-        gmean[g] = wt > 0.f ? ((red[0][g] + red[1][g]) + (red[2][g] + red[3][g])) / wt : 0.f;
-        if (g == 0) wsum = wt;
-      }
-      e2_sync();
+      for (int g = 0; g < GMAX; ++g) gm[g] = __shfl_sync(0xffffffffu, mean, 4 * g);
       // pass 2 (D2 read again from tensor memory): centred sums of squares
 #pragma unroll
       for (int k = 0; k < C / 16; ++k) {
@@ -570,40 +542,22 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         for (int e = 0; e < 16; ++e) {
           const int g = (16 * k + e) / CPG;
           if (e % CPG == 0) gs[g] = 0.f;
-          const float x = __uint_as_float(d[e]) - gmean[g];
+          const float x = __uint_as_float(d[e]) - gm[g];
           gs[g] = fmaf(x, x, gs[g]);
         }
       }
       tc::tc_before_sync();
       tc::mbar_arrive(&a_empty[sa]);   // D2 has been read: the stage may take a new tile
 #pragma unroll
-      for (int g = 0; g < GMAX; ++g) {
-        float t = w * gs[g];
-#pragma unroll
-        for (int m = 16; m; m >>= 1) t += __shfl_xor_sync(0xffffffffu, t, m);
-        if (lane == 0) red[wl][g] = t;
-      }
-      e2_sync();
-      if (threadIdx.x - 32 * W_E2 < GMAX) {
-        const int g = threadIdx.x - 32 * W_E2;
-        GroupAcc a{acc[3 * g], acc[3 * g + 1], acc[3 * g + 2]};
-        chan_merge(a, (double)wsum, (double)gmean[g], (double)((red[0][g] + red[1][g]) + (red[2][g] + red[3][g])));
-        acc[3 * g] = a.w;
-        acc[3 * g + 1] = a.mean;
-        acc[3 * g + 2] = a.m2;
-      }
-      e2_sync();
+      for (int g = 0; g < GMAX; ++g) gs[g] *= w;
+      stat.add(wt, mean, warp_group_sum(gs));
     }
+    put_warp_stats(acc[wl], stat);
   }
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
-  if (threadIdx.x < GMAX) {
-    double* o = partials + ((long)blockIdx.x * GMAX + threadIdx.x) * 3;
-    o[0] = acc[3 * threadIdx.x];
-    o[1] = acc[3 * threadIdx.x + 1];
-    o[2] = acc[3 * threadIdx.x + 2];
-  }
+  write_warp_partials<4>(partials, acc);
   if (warp == 0) tc::tmem_free(tmem, 512);
 }
 
@@ -1107,8 +1061,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       wbar;
   __shared__ uint32_t tslot;
   __shared__ float cf[2][3 * C];              // GroupNorm coefficients of spec and vert: mean, gamma rstd, beta
-  __shared__ float red[4][GMAX + 1], gmean[GMAX], wsum;
-  __shared__ double acc[GMAX * 3];
+  __shared__ double acc[4][GMAX][3];          // the epilogue-2 warps' statistics
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) tc::tmem_alloc(&tslot, 512);
   if (threadIdx.x == 0) {
@@ -1131,7 +1084,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     cf[0][e] = sc[e];
     cf[1][e] = vc[e];
   }
-  if (threadIdx.x < GMAX * 3) acc[threadIdx.x] = 0.0;
+  if (threadIdx.x < 4 * GMAX * 3) (&acc[0][0][0])[threadIdx.x] = 0.0;
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
@@ -1303,15 +1256,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   } else if (ok && warp >= W_E2) {
     const int q = warp & 3, r = 32 * q + lane, wl = warp - W_E2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
+    ShiftAcc stat;
     for (int i = 0; i < niter; ++i) {
       const int s = i & 1;
       const long v = tile_of(i) * TM + r;
       const bool live = v < V;
       const float w = live ? __ldg(dw + v) : 0.f;
-      if (!e2_sync_and(tc::mbar_wait_for(&d2_full[s], ((uint32_t)i >> 1) & 1u, WAIT_NS))) {
-        if (lane == 0) atomicExch(err, 10);
-        break;
-      }
+      if (!warp_wait(&d2_full[s], ((uint32_t)i >> 1) & 1u, err, 10)) break;
       tc::tc_after_sync();
       const uint32_t D = tmem + lq + TD2 + (uint32_t)(C * s);
       float gs[GMAX];
@@ -1334,25 +1285,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           gs[g] += __uint_as_float(d[e]);
         }
       }
-      float ws = w;
+      // the warp's own 32 voxels: weight and mean of each group (lanes 4 g .. 4 g + 3 hold group g), no barrier
+      const float wt = warp_sum(w) * CPG;
 #pragma unroll
-      for (int m = 16; m; m >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, m);
+      for (int g = 0; g < GMAX; ++g) gs[g] *= w;
+      const float tot = warp_group_sum(gs), mean = wt > 0.f ? tot / wt : 0.f;
+      float gm[GMAX];
 #pragma unroll
-      for (int g = 0; g < GMAX; ++g) {
-        float t = w * gs[g];
-#pragma unroll
-        for (int m = 16; m; m >>= 1) t += __shfl_xor_sync(0xffffffffu, t, m);
-        if (lane == 0) red[wl][g] = t;
-      }
-      if (lane == 0) red[wl][GMAX] = ws;
-      e2_sync();
-      if (threadIdx.x - 32 * W_E2 < GMAX) {
-        const int g = threadIdx.x - 32 * W_E2;
-        const float wt = ((red[0][GMAX] + red[1][GMAX]) + (red[2][GMAX] + red[3][GMAX])) * CPG;
-        gmean[g] = wt > 0.f ? ((red[0][g] + red[1][g]) + (red[2][g] + red[3][g])) / wt : 0.f;
-        if (g == 0) wsum = wt;
-      }
-      e2_sync();
+      for (int g = 0; g < GMAX; ++g) gm[g] = __shfl_sync(0xffffffffu, mean, 4 * g);
 #pragma unroll
       for (int k = 0; k < C / 16; ++k) {
         uint32_t d[16];
@@ -1362,40 +1302,22 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         for (int e = 0; e < 16; ++e) {
           const int g = (16 * k + e) / CPG;
           if (e % CPG == 0) gs[g] = 0.f;
-          const float x = __uint_as_float(d[e]) - gmean[g];
+          const float x = __uint_as_float(d[e]) - gm[g];
           gs[g] = fmaf(x, x, gs[g]);
         }
       }
       tc::tc_before_sync();
       tc::mbar_arrive(&d2_free[s]);   // D2[s] has been read: conversion may write the residual of tile i + 2
 #pragma unroll
-      for (int g = 0; g < GMAX; ++g) {
-        float t = w * gs[g];
-#pragma unroll
-        for (int m = 16; m; m >>= 1) t += __shfl_xor_sync(0xffffffffu, t, m);
-        if (lane == 0) red[wl][g] = t;
-      }
-      e2_sync();
-      if (threadIdx.x - 32 * W_E2 < GMAX) {
-        const int g = threadIdx.x - 32 * W_E2;
-        GroupAcc a{acc[3 * g], acc[3 * g + 1], acc[3 * g + 2]};
-        chan_merge(a, (double)wsum, (double)gmean[g], (double)((red[0][g] + red[1][g]) + (red[2][g] + red[3][g])));
-        acc[3 * g] = a.w;
-        acc[3 * g + 1] = a.mean;
-        acc[3 * g + 2] = a.m2;
-      }
-      e2_sync();
+      for (int g = 0; g < GMAX; ++g) gs[g] *= w;
+      stat.add(wt, mean, warp_group_sum(gs));
     }
+    put_warp_stats(acc[wl], stat);
   }
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
-  if (threadIdx.x < GMAX) {
-    double* o = partials + ((long)blockIdx.x * GMAX + threadIdx.x) * 3;
-    o[0] = acc[3 * threadIdx.x];
-    o[1] = acc[3 * threadIdx.x + 1];
-    o[2] = acc[3 * threadIdx.x + 2];
-  }
+  write_warp_partials<4>(partials, acc);
   if (warp == 0) tc::tmem_free(tmem, 512);
 }
 
