@@ -27,6 +27,11 @@ constexpr int TM = 128;
 constexpr int NWARPS = 18;
 constexpr int NTHREADS = NWARPS * 32;
 constexpr int W_TMA = 0, W_MMA = 1, W_CVT = 2, W_E1 = 6, W_E2 = 14;
+// The kernels whose conversion applies GroupNorms and GELUs (forward MLP, both halves of the fusion) run two groups of
+// four conversion warps, which share out a tile's channels: one group's arithmetic (about 30 instructions a channel and
+// voxel, one warp per SM sub-partition) took longer than the tile's MMAs and HBM traffic. 22 warps, at most 88 registers
+// a thread.
+constexpr int F_NTHREADS = 22 * 32, F_E1 = 10, F_E2 = 18;
 constexpr uint32_t BOX_BYTES = TM * 32 * 4;   // one [128][32] FP32 box
 constexpr uint32_t D1 = 256, D2 = 384;        // accumulator columns
 
@@ -286,7 +291,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // Tensor memory: four A stages of C columns from column 0 ([x hi | x lo], D2 of the stage's tile over them: a stage is
 // held from conversion to epilogue 2), D1 buffers at 256 and 384.
 template <int C, int MODE>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(F_NTHREADS, 1)
     k_mlp2_fwd_ws(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_prev,
                   const float* __restrict__ pc, float res, float* __restrict__ xout, long V,
                   const uint8_t* __restrict__ wpack, const float* __restrict__ dw, float* __restrict__ pre,
@@ -310,12 +315,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
       tc::mbar_init(&stg_full[s], 1);
-      tc::mbar_init(&stg_empty[s], 128);
+      tc::mbar_init(&stg_empty[s], 256);
       tc::mbar_init(&d1_full[s], 1);
       tc::mbar_init(&h_full[s], 256);
     }
     for (int s = 0; s < NA; ++s) {
-      tc::mbar_init(&a_full[s], 128);
+      tc::mbar_init(&a_full[s], 256);
       tc::mbar_init(&a_empty[s], 128);
       tc::mbar_init(&d2_full[s], 1);
     }
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     tc::mbar_init_fence();
   }
   if (MODE != 0)
-    for (int e = threadIdx.x; e < 3 * C; e += NTHREADS) cf[e] = pc[e];
+    for (int e = threadIdx.x; e < 3 * C; e += F_NTHREADS) cf[e] = pc[e];
   if (threadIdx.x < 4 * GMAX * 3) (&acc[0][0][0])[threadIdx.x] = 0.0;
   tc::tc_before_sync();
   __syncthreads();
@@ -410,8 +415,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
     }
     if (last) tc::mbar_wait_for(last, last_par, WAIT_NS);   // no MMA in flight when tensor memory is freed
-  } else if (ok && warp >= W_CVT && warp < W_E1) {
-    const int q = warp & 3, r = 32 * q + lane;
+  } else if (ok && warp >= W_CVT && warp < F_E1) {
+    const int q = warp & 3, r = 32 * q + lane, grp = (warp - W_CVT) >> 2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     for (int i = 0; i < niter; ++i) {
       const int s = i & 1;
@@ -424,7 +429,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const uint32_t A = tmem + lq + (uint32_t)(C * sa);
       const long v = tile_of(i) * TM + r;
 #pragma unroll 1
-      for (int bh = 0; bh < 2 * NB; ++bh) {   // half boxes: 16 channels, 8 hi and 8 lo columns
+      for (int bh = NB * grp; bh < NB * (grp + 1); ++bh) {   // half boxes: 16 channels, 8 hi and 8 lo columns
         const int b = bh >> 1;
         const uint8_t* rin = st + b * BOX_BYTES + r * 128;
         uint32_t hi[8], lo[8];
@@ -465,8 +470,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       tc::tc_before_sync();
       tc::mbar_arrive(&a_full[sa]);
     }
-  } else if (ok && warp >= W_E1 && warp < W_E2) {
-    const int q = warp & 3, hf = (warp - W_E1) >> 2;
+  } else if (ok && warp >= F_E1 && warp < F_E2) {
+    const int q = warp & 3, hf = (warp - F_E1) >> 2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     for (int i = 0; i < niter; ++i) {
       const int s = i & 1;
@@ -490,8 +495,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       tc::tc_before_sync();
       tc::mbar_arrive(&h_full[s]);
     }
-  } else if (ok && warp >= W_E2) {
-    const int q = warp & 3, r = 32 * q + lane, wl = warp - W_E2;
+  } else if (ok && warp >= F_E2) {
+    const int q = warp & 3, r = 32 * q + lane, wl = warp - F_E2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     ShiftAcc stat;
     for (int i = 0; i < niter; ++i) {
@@ -795,7 +800,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // conversion; warps 6-13 epilogue 1: hg to HBM, H = gelu(D1) split over D1; warps 14-17 epilogue 2: the gates.
 // Tensor memory: A stages of 3C columns at 0 and 3C, D1 buffers at 6C and 7C.
 template <int C>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(F_NTHREADS, 1)
     k_fuse1_ws(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_sp,
                const __grid_constant__ CUtensorMap map_vp, const float* __restrict__ sc, const float* __restrict__ vc,
                long V, const uint8_t* __restrict__ wpack, const float* __restrict__ bias, float* __restrict__ gates,
@@ -821,7 +826,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       tc::mbar_init(&stg_empty[s], 128);
     }
     for (int s = 0; s < 2; ++s) {
-      tc::mbar_init(&a_full[s], 128);
+      tc::mbar_init(&a_full[s], 256);
       tc::mbar_init(&a_empty[s], 128);
       tc::mbar_init(&d1_full[s], 1);
       tc::mbar_init(&h_full[s], 256);
@@ -830,11 +835,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     tc::mbar_init(&wbar, 1);
     tc::mbar_init_fence();
   }
-  for (int e = threadIdx.x; e < 3 * C; e += NTHREADS) {
+  for (int e = threadIdx.x; e < 3 * C; e += F_NTHREADS) {
     cf[0][e] = sc[e];
     cf[1][e] = vc[e];
   }
-  for (int e = threadIdx.x; e < 2 * C; e += NTHREADS) bs[e] = bias[e];
+  for (int e = threadIdx.x; e < 2 * C; e += F_NTHREADS) bs[e] = bias[e];
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
@@ -923,8 +928,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
     }
     if (last) tc::mbar_wait_for(last, last_par, WAIT_NS);   // no MMA in flight when tensor memory is freed
-  } else if (ok && warp >= W_CVT && warp < W_E1) {
-    const int q = warp & 3, r = 32 * q + lane;
+  } else if (ok && warp >= W_CVT && warp < F_E1) {
+    const int q = warp & 3, r = 32 * q + lane, grp = (warp - W_CVT) >> 2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     bool alive = true;
     for (int i = 0; i < niter && alive; ++i) {
@@ -934,6 +939,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const uint32_t A = tmem + lq + (uint32_t)(3 * C * s);
       for (int ph = 0; ph < NPH; ++ph) {
         const int u = i * NPH + ph, st = u % NS;
+        if ((u & 1) != grp) continue;   // the groups take alternate phases
         if (!warp_wait(&stg_full[st], (uint32_t)(u / NS) & 1u, err, 8)) {
           alive = false;
           break;
@@ -966,8 +972,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       tc::tc_before_sync();
       tc::mbar_arrive(&a_full[s]);
     }
-  } else if (ok && warp >= W_E1 && warp < W_E2) {
-    const int q = warp & 3, hf = (warp - W_E1) >> 2, r = 32 * q + lane;
+  } else if (ok && warp >= F_E1 && warp < F_E2) {
+    const int q = warp & 3, hf = (warp - F_E1) >> 2, r = 32 * q + lane;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     for (int i = 0; i < niter; ++i) {
       const int s = i & 1;
@@ -998,7 +1004,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       tc::tc_before_sync();
       tc::mbar_arrive(&h_full[s]);
     }
-  } else if (ok && warp >= W_E2) {
+  } else if (ok && warp >= F_E2) {
     const int q = warp & 3, r = 32 * q + lane;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     for (int i = 0; i < niter; ++i) {
@@ -1042,7 +1048,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // split over D1; warps 14-17 epilogue 2: pre and its statistics, as in the forward MLP. Tensor memory (8C columns):
 // A stages at 0 and 2C, D1 at 4C, D2 buffers at 6C and 7C.
 template <int C>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(F_NTHREADS, 1)
     k_fuse2_ws(const __grid_constant__ CUtensorMap map_sp, const __grid_constant__ CUtensorMap map_vp,
                const __grid_constant__ CUtensorMap map_g, const float* __restrict__ sc, const float* __restrict__ vc,
                long V, const uint8_t* __restrict__ wpack, const float* __restrict__ dw, float* __restrict__ pre,
@@ -1070,7 +1076,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       tc::mbar_init(&stg_empty[s], 128);
     }
     for (int s = 0; s < 2; ++s) {
-      tc::mbar_init(&a_full[s], 128);
+      tc::mbar_init(&a_full[s], NB == 1 ? 128 : 256);
       tc::mbar_init(&a_empty[s], 1);
       tc::mbar_init(&d2_free[s], 128);
       tc::mbar_init(&d2_full[s], 1);
@@ -1080,7 +1086,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     tc::mbar_init(&wbar, 1);
     tc::mbar_init_fence();
   }
-  for (int e = threadIdx.x; e < 3 * C; e += NTHREADS) {
+  for (int e = threadIdx.x; e < 3 * C; e += F_NTHREADS) {
     cf[0][e] = sc[e];
     cf[1][e] = vc[e];
   }
@@ -1171,11 +1177,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
     }
     if (last) tc::mbar_wait_for(last, last_par, WAIT_NS);   // no MMA in flight when tensor memory is freed
-  } else if (ok && warp >= W_CVT && warp < W_E1) {
-    const int q = warp & 3, r = 32 * q + lane;
+  } else if (ok && warp >= W_CVT && warp < F_E1) {
+    const int q = warp & 3, r = 32 * q + lane, grp = (warp - W_CVT) >> 2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     bool alive = true;
     for (int i = 0; i < niter && alive; ++i) {
+      // the groups take alternate channel phases (both branches of a channel, whose residual meets in D2), or, with
+      // one phase a branch (C = 32), alternate tiles
+      if (NB == 1 && (i & 1) != grp) continue;
       const int s = i & 1;
       const uint32_t n2 = ((uint32_t)i >> 1) & 1u;
       if (!warp_wait(&a_empty[s], n2 ^ 1u, err, 7)) break;    // GEMM1 of tile i-2 has read the A stage
@@ -1184,6 +1193,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const uint32_t A = tmem + lq + TA + (uint32_t)(2 * C * s), D2 = tmem + lq + TD2 + (uint32_t)(C * s);
       for (int ph = 0; ph < NPH; ++ph) {
         const int u = i * NPH + ph, st = u % NS;
+        if (NB > 1 && (ph & 1) != grp) continue;
         if (!warp_wait(&stg_full[st], (uint32_t)(u / NS) & 1u, err, 12)) {
           alive = false;
           break;
@@ -1230,8 +1240,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       tc::tc_before_sync();
       tc::mbar_arrive(&a_full[s]);
     }
-  } else if (ok && warp >= W_E1 && warp < W_E2) {
-    const int q = warp & 3, hf = (warp - W_E1) >> 2;
+  } else if (ok && warp >= F_E1 && warp < F_E2) {
+    const int q = warp & 3, hf = (warp - F_E1) >> 2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     for (int i = 0; i < niter; ++i) {
       if (!warp_wait(&d1_full, (uint32_t)i & 1u, err, 9)) break;
@@ -1253,8 +1263,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       tc::tc_before_sync();
       tc::mbar_arrive(&h_full);
     }
-  } else if (ok && warp >= W_E2) {
-    const int q = warp & 3, r = 32 * q + lane, wl = warp - W_E2;
+  } else if (ok && warp >= F_E2) {
+    const int q = warp & 3, r = 32 * q + lane, wl = warp - F_E2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     ShiftAcc stat;
     for (int i = 0; i < niter; ++i) {
@@ -1674,7 +1684,7 @@ int launch_mlp2_fwd(const float* in, const float* prev, const float* pc, float r
   if (MODE != 0 ? !row_map(&mp, prev, V, C) : !row_map(&mp, in, V, C)) return FFNO_EINVAL;
   const size_t smem = 1024 + 2 * (size_t)mat_bytes(2 * C, C) + 2 * (size_t)((MODE == 0 ? 1 : 2) * (C / 32) * BOX_BYTES);
   if (!ffno::smem_cap_ok(k_mlp2_fwd_ws<C, MODE>, smem)) return FFNO_ELAUNCH;
-  k_mlp2_fwd_ws<C, MODE><<<nparts, NTHREADS, smem, s>>>(mi, mp, pc, res, xout, V, static_cast<const uint8_t*>(wpack),
+  k_mlp2_fwd_ws<C, MODE><<<nparts, F_NTHREADS, smem, s>>>(mi, mp, pc, res, xout, V, static_cast<const uint8_t*>(wpack),
                                                          dw, pre, partials, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
@@ -1716,7 +1726,7 @@ int launch_fuse2(const float* sp, const float* sc, const float* vp, const float*
   const size_t smem = 1024 + (size_t)mat_bytes(2 * C, 2 * C) + mat_bytes(C, 2 * C) + 3 * (size_t)(2 * BOX_BYTES);
   if (!ffno::smem_cap_ok(k_fuse2_ws<C>, smem))
     return FFNO_ELAUNCH;
-  k_fuse2_ws<C><<<nparts, NTHREADS, smem, s>>>(ms, mv, mg, sc, vc, V, static_cast<const uint8_t*>(wpack), dw, pre,
+  k_fuse2_ws<C><<<nparts, F_NTHREADS, smem, s>>>(ms, mv, mg, sc, vc, V, static_cast<const uint8_t*>(wpack), dw, pre,
                                                 partials, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
@@ -1731,7 +1741,7 @@ int launch_fuse1(const float* x, const float* sp, const float* sc, const float* 
     return FFNO_ELAUNCH;
   const long nt = (V + TM - 1) / TM;
   const int grid = (int)(nt < sms() ? nt : sms());
-  k_fuse1_ws<C><<<grid, NTHREADS, smem, s>>>(mx, ms, mv, sc, vc, V, static_cast<const uint8_t*>(wpack), bias, gates,
+  k_fuse1_ws<C><<<grid, F_NTHREADS, smem, s>>>(mx, ms, mv, sc, vc, V, static_cast<const uint8_t*>(wpack), bias, gates,
                                               hg, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
