@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
   static_assert(C == 32 || C == 64, "widths 32 and 64");
   constexpr uint32_t B1 = mat_bytes(C, 3 * C), B2 = mat_bytes(2 * C, C);
   constexpr uint32_t WB = B1 + B2;
-  constexpr int NB = C / 32, NPH = 3 * NB, NS = 4;
+  constexpr int NB = C / 32, NPH = 3 * NB, NS = 4;   // NS even: see the conversion
   constexpr uint32_t SB = BOX_BYTES;             // one ring stage: one box
   constexpr uint32_t TD1 = 6 * C;
   static_assert(WB % 1024 == 0, "the ring must stay 1024-byte aligned (128-byte swizzle)");
@@ -939,7 +939,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
       const uint32_t A = tmem + lq + (uint32_t)(3 * C * s);
       for (int ph = 0; ph < NPH; ++ph) {
         const int u = i * NPH + ph, st = u % NS;
-        if ((u & 1) != grp) continue;   // the groups take alternate phases
+        if ((u & 1) != grp) continue;   // alternate phases; four stages, so a stage's uses all go to one group
         if (!warp_wait(&stg_full[st], (uint32_t)(u / NS) & 1u, err, 8)) {
           alive = false;
           break;
@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < NS; ++s) {
       tc::mbar_init(&stg_full[s], 1);
-      tc::mbar_init(&stg_empty[s], 128);
+      tc::mbar_init(&stg_empty[s], 256);
     }
     for (int s = 0; s < 2; ++s) {
       tc::mbar_init(&a_full[s], NB == 1 ? 128 : 256);
@@ -1182,21 +1182,27 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     bool alive = true;
     for (int i = 0; i < niter && alive; ++i) {
-      // the groups take alternate channel phases (both branches of a channel, whose residual meets in D2), or, with
-      // one phase a branch (C = 32), alternate tiles
-      if (NB == 1 && (i & 1) != grp) continue;
       const int s = i & 1;
       const uint32_t n2 = ((uint32_t)i >> 1) & 1u;
-      if (!warp_wait(&a_empty[s], n2 ^ 1u, err, 7)) break;    // GEMM1 of tile i-2 has read the A stage
-      if (!warp_wait(&d2_free[s], n2 ^ 1u, err, 8)) break;    // epilogue 2 of tile i-2 has read D2[s]
+      // the groups take alternate channel phases (both branches of a channel, whose residual meets in D2), or, with
+      // one phase a branch (C = 32), alternate tiles. Three stages for two groups: consecutive uses of a stage go to
+      // different groups, so each group waits for every use of every stage and releases it too. A group that waited
+      // for its own uses only could take an earlier use's phase for its own (the parities repeat every two uses) when
+      // the copies of two stages land out of order.
+      const bool mine = NB > 1 || (i & 1) == grp;
+      if (mine && !warp_wait(&a_empty[s], n2 ^ 1u, err, 7)) break;    // GEMM1 of tile i-2 has read the A stage
+      if (mine && !warp_wait(&d2_free[s], n2 ^ 1u, err, 8)) break;    // epilogue 2 of tile i-2 has read D2[s]
       tc::tc_after_sync();
       const uint32_t A = tmem + lq + TA + (uint32_t)(2 * C * s), D2 = tmem + lq + TD2 + (uint32_t)(C * s);
       for (int ph = 0; ph < NPH; ++ph) {
         const int u = i * NPH + ph, st = u % NS;
-        if (NB > 1 && (ph & 1) != grp) continue;
         if (!warp_wait(&stg_full[st], (uint32_t)(u / NS) & 1u, err, 12)) {
           alive = false;
           break;
+        }
+        if (!mine || (NB > 1 && (ph & 1) != grp)) {
+          tc::mbar_arrive(&stg_empty[st]);
+          continue;
         }
         const int br = ph / NB, c0 = 32 * (ph % NB);   // branch (0 spec, 1 vert) and its first channel
         const float* k = cf[br];
@@ -1236,6 +1242,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
         }
       }
       if (!alive) break;
+      if (!mine) continue;
       tc::tmem_wait_st();
       tc::tc_before_sync();
       tc::mbar_arrive(&a_full[s]);
