@@ -51,6 +51,58 @@ __device__ __forceinline__ float gelu_grad_tc(float x) {
   const Cdf c = cdf_tc(x);
   return fmaf(x, c.pdf, c.cdf);
 }
+// Two FP32 lanes in one 64-bit register (fma.rn.f32x2 and its relatives: two IEEE operations per issued instruction).
+__device__ __forceinline__ uint64_t pk2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void upk2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// cdf_tc of two values at once, the same operations: the epilogues and conversions of the
+// tensor-core kernels are bound by issue slots, and the packed polynomial takes half of them.
+struct Cdf2 {
+  uint64_t cdf, e;   // Phi(x) and exp(-x^2 / 2), two lanes each
+};
+__device__ __forceinline__ Cdf2 cdf_tc2(float x0, float x1) {
+  const uint64_t x = pk2(x0, x1);
+  const uint64_t u = mul2(pk2(fabsf(x0), fabsf(x1)), pk2(0.70710678118654752440f, 0.70710678118654752440f));
+  float d0, d1, q0, q1;
+  upk2(fma2(pk2(0.3275911f, 0.3275911f), u, pk2(1.f, 1.f)), d0, d1);
+  upk2(mul2(mul2(pk2(-0.5f, -0.5f), x), x), q0, q1);
+  const uint64_t t = pk2(__fdividef(1.f, d0), __fdividef(1.f, d1));
+  const uint64_t e = pk2(__expf(q0), __expf(q1));
+  uint64_t p = fma2(t, pk2(1.061405429f, 1.061405429f), pk2(-1.453152027f, -1.453152027f));
+  p = fma2(t, p, pk2(1.421413741f, 1.421413741f));
+  p = fma2(t, p, pk2(-0.284496736f, -0.284496736f));
+  p = fma2(t, p, pk2(0.254829592f, 0.254829592f));
+  const uint64_t h = mul2(mul2(pk2(0.5f, 0.5f), mul2(p, t)), e);   // (1 - erf(u)) / 2
+  float h0, h1, g0, g1;
+  upk2(h, h0, h1);
+  upk2(fma2(h, pk2(-1.f, -1.f), pk2(1.f, 1.f)), g0, g1);
+  return Cdf2{pk2(x0 < 0.f ? h0 : g0, x1 < 0.f ? h1 : g1), e};
+}
+__device__ __forceinline__ void gelu_tc2(float& x0, float& x1) {
+  upk2(mul2(pk2(x0, x1), cdf_tc2(x0, x1).cdf), x0, x1);
+}
+// y *= gelu'(x)
+__device__ __forceinline__ void mul_gelu_grad_tc2(float x0, float x1, float& y0, float& y1) {
+  const Cdf2 c = cdf_tc2(x0, x1);
+  const uint64_t pdf = mul2(pk2(0.39894228040143267794f, 0.39894228040143267794f), c.e);
+  upk2(mul2(pk2(y0, y1), fma2(pk2(x0, x1), pdf, c.cdf)), y0, y1);
+}
 __device__ __forceinline__ float sigmoid_tc(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
 // Math of the level-fraction head in the scalar type of the caller: FP64 (the reference's arithmetic) or FP32.

@@ -102,7 +102,10 @@ template <bool GELU>
 __device__ __forceinline__ float4 gn_apply(float4 p, const Gn4& g) {
   float4 y = make_float4((p.x - g.m.x) * g.s.x + g.b.x, (p.y - g.m.y) * g.s.y + g.b.y, (p.z - g.m.z) * g.s.z + g.b.z,
                          (p.w - g.m.w) * g.s.w + g.b.w);
-  if (GELU) y = make_float4(gelu_tc(y.x), gelu_tc(y.y), gelu_tc(y.z), gelu_tc(y.w));
+  if (GELU) {
+    gelu_tc2(y.x, y.y);
+    gelu_tc2(y.z, y.w);
+  }
   return y;
 }
 
@@ -558,7 +561,7 @@ __global__ void __launch_bounds__(CT, 1) k_mlp2_tc(const float* __restrict__ in,
       float v[16];
       tld(P, 0, c, v);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = gelu_tc(v[i]);
+      for (int i = 0; i < 16; i += 2) gelu_tc2(v[i], v[i + 1]);
       if (f < 2 * C) put_mn(H, f, 64 * P.half + 16 * c, v);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem, w2, mop(H), 2 * C, false})) break;
@@ -610,7 +613,7 @@ __global__ void __launch_bounds__(CT, 1) k_gate_tc(const float* __restrict__ x, 
       float v[16];
       rld(P, 0, j, v);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = gelu_tc(v[i]);
+      for (int i = 0; i < 16; i += 2) gelu_tc2(v[i], v[i + 1]);
       put16(X, row, 16 * j, C, v);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem, kop(X, C), g2, C, false, C})) break;
@@ -698,7 +701,7 @@ __global__ void __launch_bounds__(CT, 1) k_fuse1_tc(const float* __restrict__ x,
         for (int i = 0; i < 16; i += 4)
           *reinterpret_cast<float4*>(hg + v * C + c0 + i) = make_float4(h[i], h[i + 1], h[i + 2], h[i + 3]);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) h[i] = gelu_tc(h[i]);
+      for (int i = 0; i < 16; i += 2) gelu_tc2(h[i], h[i + 1]);
       put16(A, f, c0, C, h);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem, wg2, kop(A, C), C, false})) break;
@@ -795,7 +798,7 @@ __global__ void __launch_bounds__(CT, 1) k_fuse2_tc(const float* __restrict__ sp
       float h[16];
       tld(P, 0, c, h);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) h[i] = gelu_tc(h[i]);
+      for (int i = 0; i < 16; i += 2) gelu_tc2(h[i], h[i + 1]);
       if (f < 2 * C) put_mn(A, f, 64 * P.half + 16 * c, h);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem + TM, wf2, mop(A), 2 * C, true})) break;
@@ -857,7 +860,7 @@ __global__ void __launch_bounds__(CT, 1) k_mlp2_bwd_tc(const float* __restrict__
       tld(P, 0, c, hp);
       tld(P, TM, c, gb);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) gb[i] *= gelu_grad_tc(hp[i]);
+      for (int i = 0; i < 16; i += 2) mul_gelu_grad_tc2(hp[i], hp[i + 1], gb[i], gb[i + 1]);
       if (f < 2 * C) put_mn(H, f, 64 * P.half + 16 * c, gb);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem, mop(H), w1t, 2 * C, false, C})) break;
@@ -929,7 +932,7 @@ __global__ void __launch_bounds__(NP * PT, 1) k_gate_bwd_tc(const float* __restr
       float h[16];
       rld(P, D1, j, h);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) h[i] = gelu_tc(h[i]);
+      for (int i = 0; i < 16; i += 2) gelu_tc2(h[i], h[i + 1]);
       put16(T, row, 16 * j, C, h);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem + D2, kop(T, C), g2, C, false, C})) break;
@@ -974,7 +977,7 @@ __global__ void __launch_bounds__(NP * PT, 1) k_gate_bwd_tc(const float* __restr
       rld(P, D3, j, hb);
       rld(P, D1, j, hp);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) hb[i] *= gelu_grad_tc(hp[i]);
+      for (int i = 0; i < 16; i += 2) mul_gelu_grad_tc2(hp[i], hp[i + 1], hb[i], hb[i + 1]);
       put16(T, row, 16 * j, C, hb);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem + D4, kop(T, C), g1t, C, true, C})) break;
@@ -1160,7 +1163,7 @@ __global__ void __launch_bounds__(CT, 1) k_fuse_bwd_b_tc(const float* __restrict
         for (int i = 0; i < 16; ++i) h8[i] = 0.f;
       }
 #pragma unroll
-      for (int i = 0; i < 16; ++i) hb[i] *= gelu_grad_tc(h8[i]);
+      for (int i = 0; i < 16; i += 2) mul_gelu_grad_tc2(h8[i], h8[i + 1], hb[i], hb[i + 1]);
       put16(T, row, c0, C, hb);
     }
     // GEMM3: the branch rows of Wg1 accumulate onto the direct gradients (columns 0 .. 2C), the x rows go to the
@@ -1240,7 +1243,7 @@ __global__ void __launch_bounds__(CT, 1) k_head_tc(const float* __restrict__ x, 
       float v[16];
       tld(P, 0, c, v);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = gelu_tc(v[i]);
+      for (int i = 0; i < 16; i += 2) gelu_tc2(v[i], v[i + 1]);
       if (f < 2 * C) put_mn(H, f, 64 * P.half + 16 * c, v);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem, mop(H), w2, 2 * C, false, NHP})) break;
@@ -1301,7 +1304,7 @@ __global__ void __launch_bounds__(CT, 1) k_head_bwd_tc(const float* __restrict__
       float v[16];
       tld(P, 0, c, v);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = gelu_tc(v[i]);
+      for (int i = 0; i < 16; i += 2) gelu_tc2(v[i], v[i + 1]);
       if (f < 2 * C) put_mn(H, f, 64 * P.half + 16 * c, v);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem + TM, mop(H), w2, 2 * C, false, NHP})) break;
@@ -1337,7 +1340,7 @@ __global__ void __launch_bounds__(CT, 1) k_head_bwd_tc(const float* __restrict__
       tld(P, 0, c, hp_);
       tld(P, TM, c, gb);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) gb[i] *= gelu_grad_tc(hp_[i]);
+      for (int i = 0; i < 16; i += 2) mul_gelu_grad_tc2(hp_[i], hp_[i + 1], gb[i], gb[i + 1]);
       if (f < 2 * C) put_mn(H, f, 64 * P.half + 16 * c, gb);
     }
     if (!pipe_gemms(P, err, Gemm{P.tmem, mop(H), w1t, 2 * C, false, C})) break;
@@ -1409,7 +1412,7 @@ __global__ void __launch_bounds__(PT, 1) k_mlp2_tc96(const float* __restrict__ i
         float v[16];
         rld(P, 0, j, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] = gelu_tc(v[i]);
+        for (int i = 0; i < 16; i += 2) gelu_tc2(v[i], v[i + 1]);
         put16(T, row, 16 * j - C * h, C, v);
       }
       if (!pipe_gemms(P, err, Gemm{P.tmem + 2 * C, kop(T, C), wop(smem + B1, C, 2 * C, 0, C * h), C, h > 0, C}))
@@ -1474,7 +1477,7 @@ __global__ void __launch_bounds__(PT, 1) k_mlp2_bwd_tc96(const float* __restrict
         rld(P, 0, j, hp);
         rld(P, 2 * C, j, gb);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) gb[i] *= gelu_grad_tc(hp[i]);
+        for (int i = 0; i < 16; i += 2) mul_gelu_grad_tc2(hp[i], hp[i + 1], gb[i], gb[i + 1]);
         put16(T, row, 16 * j - C * h, C, gb);
       }
       if (!pipe_gemms(P, err, Gemm{P.tmem + 4 * C, kop(T, C), wop_t(smem, 2 * C, C, C * h), C, h > 0, C})) break;
@@ -1566,7 +1569,7 @@ __global__ void __launch_bounds__(PT, 1) k_fuse1_tc96(const float* __restrict__ 
           st8(hg + v * C + 16 * j + 8, hv + 8);
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) hv[i] = gelu_tc(hv[i]);
+        for (int i = 0; i < 16; i += 2) gelu_tc2(hv[i], hv[i + 1]);
         put16(T, row, 16 * j - KS * h, KS, hv);
       }
       if (!pipe_gemms(P, err, Gemm{P.tmem + C, kop(T, KS), wop(smem + B1, 2 * C, C, 0, KS * h), KS, h > 0, 2 * C}))
@@ -1668,7 +1671,7 @@ __global__ void __launch_bounds__(PT, 1) k_fuse_out_tc96(const float* __restrict
       fill_oct<KS>(T, v0, V, P.ptid, [&](long v, int k, float (&o)[8]) {
         ld8(hf + v * 2 * C + sl * KS + k, o);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = gelu_tc(o[i]);
+        for (int i = 0; i < 8; i += 2) gelu_tc2(o[i], o[i + 1]);
       });
       if (!pipe_gemms(P, err, Gemm{P.tmem, kop(T, KS), wop(smem, C, 2 * C, 0, sl * KS), KS, sl > 0, C})) break;
     }
@@ -1741,7 +1744,7 @@ __global__ void __launch_bounds__(PT, 1) k_fuse_bwd_h_tc96(const float* __restri
         ld8(hf + v * 2 * C + 16 * j, *reinterpret_cast<float(*)[8]>(h));
         ld8(hf + v * 2 * C + 16 * j + 8, *reinterpret_cast<float(*)[8]>(h + 8));
 #pragma unroll
-        for (int i = 0; i < 16; ++i) r[i] *= gelu_grad_tc(h[i]);
+        for (int i = 0; i < 16; i += 2) mul_gelu_grad_tc2(h[i], h[i + 1], r[i], r[i + 1]);
         st8(hfb + v * 2 * C + 16 * j, r);
         st8(hfb + v * 2 * C + 16 * j + 8, r + 8);
       }
@@ -1847,7 +1850,7 @@ __global__ void __launch_bounds__(PT, 1) k_fuse_bwd_x_tc96(const float* __restri
           ld8(hg + v * C + 16 * j, *reinterpret_cast<float(*)[8]>(hv));
           ld8(hg + v * C + 16 * j + 8, *reinterpret_cast<float(*)[8]>(hv + 8));
 #pragma unroll
-          for (int i = 0; i < 16; ++i) d[i] *= gelu_grad_tc(hv[i]);
+          for (int i = 0; i < 16; i += 2) mul_gelu_grad_tc2(hv[i], hv[i + 1], d[i], d[i + 1]);
         } else {
 #pragma unroll
           for (int i = 0; i < 16; ++i) d[i] = 0.f;
@@ -2038,7 +2041,7 @@ __global__ void __launch_bounds__(PT, 1) k_head_tc96(const float* __restrict__ x
         float h[16];
         rld(P, 0, j, h);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) h[i] = gelu_tc(h[i]);
+        for (int i = 0; i < 16; i += 2) gelu_tc2(h[i], h[i + 1]);
         put16(T_, row, 16 * j - KS * sl, KS, h);
       }
       if (!pipe_gemms(P, err, Gemm{P.tmem + 2 * C, kop(T_, KS), wop(smem + B1, NHP, 2 * C, 0, sl * KS), KS, sl > 0,
@@ -2105,7 +2108,7 @@ __global__ void __launch_bounds__(PT, 1) k_head_bwd_tc96(const float* __restrict
         float h[16];
         rld(P, 0, j, h);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) h[i] = gelu_tc(h[i]);
+        for (int i = 0; i < 16; i += 2) gelu_tc2(h[i], h[i + 1]);
         put16(T_, row, 16 * j - KS * sl, KS, h);
       }
       if (!pipe_gemms(P, err, Gemm{P.tmem + DO, kop(T_, KS), wop(smem + B1, NHP, 2 * C, 0, sl * KS), KS, sl > 0,
@@ -2146,7 +2149,7 @@ __global__ void __launch_bounds__(PT, 1) k_head_bwd_tc96(const float* __restrict
         rld(P, 0, j, hp_);
         rld(P, D3, j, gb);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) gb[i] *= gelu_grad_tc(hp_[i]);
+        for (int i = 0; i < 16; i += 2) mul_gelu_grad_tc2(hp_[i], hp_[i + 1], gb[i], gb[i + 1]);
         put16(T_, row, 16 * j - KS * sl, KS, gb);
       }
       if (!pipe_gemms(P, err, Gemm{P.tmem + D4, kop(T_, KS), wop_t(smem, 2 * C, C, sl * KS), KS, sl > 0, C})) break;

@@ -225,8 +225,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         uint32_t hi[8], lo[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const float g0 = __uint_as_float(gb[2 * e]) * gelu_grad_tc(__uint_as_float(h[2 * e]));
-          const float g1 = __uint_as_float(gb[2 * e + 1]) * gelu_grad_tc(__uint_as_float(h[2 * e + 1]));
+          float g0 = __uint_as_float(gb[2 * e]), g1 = __uint_as_float(gb[2 * e + 1]);
+          mul_gelu_grad_tc2(__uint_as_float(h[2 * e]), __uint_as_float(h[2 * e + 1]), g0, g1);
           tc::split_pack(g0, g1, hi[e], lo[e]);
         }
         tc::tmem_st8u(tmem + lq + D1 + 16u * j, hi);
@@ -446,7 +446,10 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               y[e] = (y[e] - cf[k + e]) * cf[C + k + e] + cf[2 * C + k + e];
-              if (MODE == 1) y[e] = gelu_tc(y[e]);
+            }
+            if (MODE == 1) {
+              gelu_tc2(y[0], y[1]);
+              gelu_tc2(y[2], y[3]);
             }
             x = make_float4(fmaf(res, y[0], x.x), fmaf(res, y[1], x.y), fmaf(res, y[2], x.z), fmaf(res, y[3], x.w));
             xs[4 * cc] = x.x;
@@ -486,8 +489,11 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
         tc::tmem_wait_ld();
         uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          tc::split_pack(gelu_tc(__uint_as_float(h[2 * e])), gelu_tc(__uint_as_float(h[2 * e + 1])), hi[e], lo[e]);
+        for (int e = 0; e < 8; ++e) {
+          float g0 = __uint_as_float(h[2 * e]), g1 = __uint_as_float(h[2 * e + 1]);
+          gelu_tc2(g0, g1);
+          tc::split_pack(g0, g1, hi[e], lo[e]);
+        }
         tc::tmem_st8u(D + 16u * j, hi);
         tc::tmem_st8u(D + 16u * j + 8u, lo);
       }
@@ -735,8 +741,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         tc::tmem_wait_ld();
         uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          tc::split_pack(gelu_tc(__uint_as_float(h[2 * e])), gelu_tc(__uint_as_float(h[2 * e + 1])), hi[e], lo[e]);
+        for (int e = 0; e < 8; ++e) {
+          float g0 = __uint_as_float(h[2 * e]), g1 = __uint_as_float(h[2 * e + 1]);
+          gelu_tc2(g0, g1);
+          tc::split_pack(g0, g1, hi[e], lo[e]);
+        }
         tc::tmem_st8u(D + 16u * j, hi);
         tc::tmem_st8u(D + 16u * j + 8u, lo);
       }
@@ -956,8 +965,10 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int c = c0 + 4 * cc + e;
-              y[e] = gelu_tc((y[e] - k[c]) * k[C + c] + k[2 * C + c]);
+              y[e] = (y[e] - k[c]) * k[C + c] + k[2 * C + c];
             }
+            gelu_tc2(y[0], y[1]);
+            gelu_tc2(y[2], y[3]);
           }
           tc::split_pack(y[0], y[1], hi[2 * cc], lo[2 * cc]);
           tc::split_pack(y[2], y[3], hi[2 * cc + 1], lo[2 * cc + 1]);
@@ -995,8 +1006,11 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
         }
         uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          tc::split_pack(gelu_tc(__uint_as_float(h[2 * e])), gelu_tc(__uint_as_float(h[2 * e + 1])), hi[e], lo[e]);
+        for (int e = 0; e < 8; ++e) {
+          float g0 = __uint_as_float(h[2 * e]), g1 = __uint_as_float(h[2 * e + 1]);
+          gelu_tc2(g0, g1);
+          tc::split_pack(g0, g1, hi[e], lo[e]);
+        }
         tc::tmem_st8u(D + 16u * j, hi);
         tc::tmem_st8u(D + 16u * j + 8u, lo);
       }
@@ -1217,8 +1231,12 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int c = c0 + 4 * cc + e;
-            b[4 * cc + e] = gelu_tc((pp[e] - k[c]) * k[C + c] + k[2 * C + c]) * gg[e];
+            b[4 * cc + e] = (pp[e] - k[c]) * k[C + c] + k[2 * C + c];
           }
+          gelu_tc2(b[4 * cc], b[4 * cc + 1]);
+          gelu_tc2(b[4 * cc + 2], b[4 * cc + 3]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) b[4 * cc + e] *= gg[e];
         }
         tc::mbar_arrive(&stg_empty[st]);
         uint32_t hi[16], lo[16];
@@ -1261,8 +1279,11 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
         tc::tmem_wait_ld();
         uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          tc::split_pack(gelu_tc(__uint_as_float(h[2 * e])), gelu_tc(__uint_as_float(h[2 * e + 1])), hi[e], lo[e]);
+        for (int e = 0; e < 8; ++e) {
+          float g0 = __uint_as_float(h[2 * e]), g1 = __uint_as_float(h[2 * e + 1]);
+          gelu_tc2(g0, g1);
+          tc::split_pack(g0, g1, hi[e], lo[e]);
+        }
         tc::tmem_st8u(D + 16u * j, hi);
         tc::tmem_st8u(D + 16u * j + 8u, lo);
       }
@@ -1521,8 +1542,11 @@ __global__ void __launch_bounds__(448, 1)
           tc::tmem_wait_ld();
           uint32_t hi[8], lo[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            tc::split_pack(gelu_tc(__uint_as_float(h[2 * e])), gelu_tc(__uint_as_float(h[2 * e + 1])), hi[e], lo[e]);
+          for (int e = 0; e < 8; ++e) {
+            float g0 = __uint_as_float(h[2 * e]), g1 = __uint_as_float(h[2 * e + 1]);
+            gelu_tc2(g0, g1);
+            tc::split_pack(g0, g1, hi[e], lo[e]);
+          }
           tc::tmem_st8u(RH(t) + lq + 16u * k, hi);
           tc::tmem_st8u(RH(t) + lq + 16u * k + 8u, lo);
         }
@@ -1541,9 +1565,11 @@ __global__ void __launch_bounds__(448, 1)
           tc::tmem_wait_ld();
           uint32_t hi[8], lo[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            tc::split_pack(__uint_as_float(tv[2 * e]) * gelu_grad_tc(__uint_as_float(h[2 * e])),
-                           __uint_as_float(tv[2 * e + 1]) * gelu_grad_tc(__uint_as_float(h[2 * e + 1])), hi[e], lo[e]);
+          for (int e = 0; e < 8; ++e) {
+            float t0 = __uint_as_float(tv[2 * e]), t1 = __uint_as_float(tv[2 * e + 1]);
+            mul_gelu_grad_tc2(__uint_as_float(h[2 * e]), __uint_as_float(h[2 * e + 1]), t0, t1);
+            tc::split_pack(t0, t1, hi[e], lo[e]);
+          }
           tc::tmem_st8u(RH(t) + lq + 16u * k, hi);
           tc::tmem_st8u(RH(t) + lq + 16u * k + 8u, lo);
         }
