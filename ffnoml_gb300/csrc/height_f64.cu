@@ -20,7 +20,6 @@
 namespace {
 
 constexpr int HT = 128;    // threads per column
-constexpr int HCH = 32;    // intervals per reduction chunk of the gradient
 
 // Lower-end (a) and upper-end (b) Filon terms of interval (za, zb) at wavenumber k (tables.filon, one interval).
 struct FilonTerms {
@@ -30,6 +29,7 @@ struct FilonTerms {
 // r = int_0^1 u e^{-i th u} du, l = int_0^1 (1 - u) e^{-i th u} du and their derivatives in th
 struct RL {
   double r_re, r_im, l_re, l_im, dr_re, dr_im, dl_re, dl_im;
+  double s, c;   // sin th, cos th (|th| >= 1e-2)
 };
 
 __device__ __forceinline__ RL filon_rl(double th, bool deriv) {
@@ -50,17 +50,25 @@ __device__ __forceinline__ RL filon_rl(double th, bool deriv) {
     const double t = th, t2 = t * t;
     double s, c;
     sincos(t, &s, &c);
-    o.r_re = (c + t * s - 1) / t2;
-    o.r_im = (t * c - s) / t2;
-    o.l_re = s / t - o.r_re;
-    o.l_im = (c - 1) / t - o.r_im;
-    if (deriv) {
-      const double t3 = t2 * t;
-      o.dr_re = (t2 * c - 2 * (c + t * s - 1)) / t3;
-      o.dr_im = (-t2 * s - 2 * (t * c - s)) / t3;
-      o.dl_re = (c * t - s) / t2 - o.dr_re;
-      o.dl_im = (-s * t - (c - 1)) / t2 - o.dr_im;
+    if (deriv) {   // one division: the eight quotients by powers of t are products with its reciprocal
+      const double i1 = 1.0 / t, i2 = i1 * i1, i3 = i2 * i1;
+      const double a = c + t * s - 1, b = t * c - s;
+      o.r_re = a * i2;
+      o.r_im = b * i2;
+      o.l_re = s * i1 - o.r_re;
+      o.l_im = (c - 1) * i1 - o.r_im;
+      o.dr_re = (t2 * c - 2 * a) * i3;
+      o.dr_im = (-t2 * s - 2 * b) * i3;
+      o.dl_re = b * i2 - o.dr_re;
+      o.dl_im = (-s * t - (c - 1)) * i2 - o.dr_im;
+    } else {
+      o.r_re = (c + t * s - 1) / t2;
+      o.r_im = (t * c - s) / t2;
+      o.l_re = s / t - o.r_re;
+      o.l_im = (c - 1) / t - o.r_im;
     }
+    o.s = s;
+    o.c = c;
   }
   return o;
 }
@@ -77,16 +85,30 @@ __device__ __forceinline__ FilonTerms filon_terms(double za, double zb, double k
   return FilonTerms{hi_re, hi_im, lo_re, lo_im};
 }
 
-// d L / d za and d L / d zb of L = ga_re a_re + ga_im a_im + gb_re b_re + gb_im b_im for interval (za, zb).
+// d L / d za and d L / d zb of L = ga_re a_re + ga_im a_im + gb_re b_re + gb_im b_im for interval (za, zb), and sin and
+// cos of za k: the lower end's, or, when za is the upper end, the lower end's turned by the interval's angle.
 __device__ __forceinline__ void filon_terms_vjp(double za, double zb, double k, double ga_re, double ga_im,
-                                                double gb_re, double gb_im, double& dza, double& dzb) {
+                                                double gb_re, double gb_im, double& dza, double& dzb, double& sna,
+                                                double& csa) {
   dza = dzb = 0.0;
-  if (za == zb) return;   // a zero-length interval: its terms are 0 and so is their gradient (|zb - za|' = 0 there)
+  if (za == zb) {   // a zero-length interval: its terms are 0 and so is their gradient (|zb - za|' = 0 there)
+    sincos(za * k, &sna, &csa);
+    return;
+  }
   const bool up = za < zb;
   const double lo = up ? za : zb, h = up ? zb - za : za - zb;
   const RL w = filon_rl(h * k, true);
   double sp, cp;
   sincos(lo * k, &sp, &cp);
+  if (up) {
+    sna = sp;
+    csa = cp;
+  } else if (fabs(h * k) < 1e-2) {
+    sincos(za * k, &sna, &csa);
+  } else {
+    sna = sp * w.c + cp * w.s;
+    csa = cp * w.c - sp * w.s;
+  }
   const double e_re = h * cp, e_im = -h * sp;
   // the l terms go to the interval's lower end, the r terms to its upper end
   const double wl_re = up ? ga_re : gb_re, wl_im = up ? ga_im : gb_im;
@@ -168,8 +190,15 @@ __global__ void __launch_bounds__(HT) k_percol_tables(const double* __restrict__
   }
 }
 
-// z_bar[j * ncol + c] += d/dz_raw[c][j] of sum(tzf_bar * tzf) + sum(tzi_bar * tzi) for every column c.
-__global__ void __launch_bounds__(HT) k_percol_tables_vjp(const double* __restrict__ z_raw, int D, long ncol,
+// z_bar[j * ncol + c] += d/dz_raw[c][j] of sum(tzf_bar * tzf) + sum(tzi_bar * tzi) for every column c, one CTA a column. A
+// thread owns a node j (lanes: consecutive nodes, so the table gradients of a mode are read coalesced) and every P-th
+// mode; its sums into nodes j and j + 1 and into the median spacing stay in registers until the modes are done. Bound by
+// the FP64 pipe: about 130 operations a (mode, node) pair, two sine-cosine pairs and one division among them. (A thread
+// per mode left 95 of 128 threads idle at 33 modes and took three sine-cosine pairs and eight divisions.) 1920 columns
+// of 128 nodes, 33 modes: 8.5 -> 1.97 ms.
+constexpr int VT = 256;
+
+__global__ void __launch_bounds__(VT) k_percol_tables_vjp(const double* __restrict__ z_raw, int D, long ncol,
                                                           const double* __restrict__ k, int live,
                                                           const double* __restrict__ f,
                                                           const double* __restrict__ df, const int* __restrict__ med,
@@ -177,92 +206,103 @@ __global__ void __launch_bounds__(HT) k_percol_tables_vjp(const double* __restri
                                                           const double* __restrict__ tzi_bar,
                                                           float* __restrict__ z_bar) {
   extern __shared__ double sh[];
-  double* zs = sh;                     // [D] shifted heights
-  double* gz = zs + D;                 // [D] gradient w.r.t. the shifted heights
-  double* dldf = gz + D;               // [live] d L / d f_m
-  double* bufa = dldf + live;          // [HT][HCH + 1] per-thread sums into node j0 + jj (lower ends, tzi)
-  double* bufb = bufa + HT * (HCH + 1);   // [HT][HCH + 1] per-thread sums into node j0 + jj + 1 (upper ends)
-  __shared__ double red[HT / 32];
+  double* zs = sh;        // [D] shifted heights
+  double* gz = zs + D;    // [D] gradient w.r.t. the shifted heights
+  __shared__ double red[VT / 32], bufa[VT], bufb[VT], carry;
   const long c = blockIdx.x;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double* zr = z_raw + c * D;
   const double zmin = shift_column(zr, D, zs, red);
-  for (int j = tid; j < D; j += HT) gz[j] = 0.0;
-  for (int m = tid; m < live; m += HT) dldf[m] = 0.0;
   const long M2 = 2L * live;
   const double* Fb = tzf_bar + c * M2 * D;   // [2M'][D]
   const double* Ib = tzi_bar + c * D * M2;   // [D][2M']
-  __syncthreads();
-  double* sa = bufa + tid * (HCH + 1);   // this thread's row: its modes' sums, in mode order
-  double* sb = bufb + tid * (HCH + 1);
-  for (int j0 = 0; j0 < D; j0 += HCH) {
-    const int nj = D - j0 < HCH ? D - j0 : HCH;
-    for (int jj = 0; jj < HCH; ++jj) sa[jj] = sb[jj] = 0.0;
-    for (int m = tid; m < live; m += HT) {
-      const double km = k[m], fm = f[c * live + m];
-      double dlf = 0.0;
+  int jt = 32;                               // nodes of a pass: a power of two up to VT
+  while (jt < D && jt < VT) jt <<= 1;
+  const int parts = VT / jt, tj = tid % jt, part = tid / jt;
+  double gt = 0.0;                           // d L / d (median spacing)
+  if (tid == 0) carry = 0.0;
+  for (int j0 = 0; j0 < D; j0 += jt) {
+    const int j = j0 + tj;
+    double sa = 0.0, sb = 0.0;
+    if (j < D) {
 #pragma unroll 1
-      for (int jj = 0; jj < nj; ++jj) {
-        const int j = j0 + jj;
-        // node j's inverse-table entries
+      for (int m = part; m < live; m += parts) {
+        const double km = k[m];
         double sn, cs;
-        sincos(zs[j] * km, &sn, &cs);
-        const double gc = Ib[(long)j * M2 + m], gs = Ib[(long)j * M2 + live + m];
-        sa[jj] += fm * km * (-gc * sn - gs * cs);
-        dlf += gc * cs - gs * sn;
-        // interval (j, j + 1): its lower-end terms sit in node j's table entries, its upper-end terms in node j + 1's
         if (j + 1 < D) {
           double dza, dzb;
           filon_terms_vjp(zs[j], zs[j + 1], km, Fb[(long)m * D + j], Fb[(long)(live + m) * D + j],
-                          Fb[(long)m * D + j + 1], Fb[(long)(live + m) * D + j + 1], dza, dzb);
-          sa[jj] += dza;
-          sb[jj] += dzb;
+                          Fb[(long)m * D + j + 1], Fb[(long)(live + m) * D + j + 1], dza, dzb, sn, cs);
+          sa += dza;
+          sb += dzb;
+        } else {
+          sincos(zs[j] * km, &sn, &cs);
         }
+        // node j's inverse-table entries
+        const double gc = Ib[(long)j * M2 + m], gs = Ib[(long)j * M2 + live + m];
+        sa += f[c * live + m] * km * (-gc * sn - gs * cs);
+        gt += df[c * live + m] * (gc * cs - gs * sn);
       }
-      dldf[m] += dlf;
     }
-    // fixed-order sums over the threads: node j0 + jj gets the lower-end sums, then node j0 + jj + 1 the upper-end
+    bufa[tid] = sa;
+    bufb[tid] = sb;
     __syncthreads();
-    if (tid < nj) {
-      double s = 0.0;
-      for (int t = 0; t < HT; ++t) s += bufa[t * (HCH + 1) + tid];
-      gz[j0 + tid] += s;
+    // fixed-order sums over the parts: node j takes its own lower-end sums and node j - 1's upper-end sums
+    if (part == 0) {
+      double a = tj ? 0.0 : carry;
+      for (int q = 0; q < parts; ++q) {
+        a += bufa[q * jt + tj];
+        if (tj) a += bufb[q * jt + tj - 1];
+      }
+      if (j < D) gz[j] = a;
     }
     __syncthreads();
-    if (tid < nj && j0 + tid + 1 < D) {
-      double s = 0.0;
-      for (int t = 0; t < HT; ++t) s += bufb[t * (HCH + 1) + tid];
-      gz[j0 + tid + 1] += s;
+    if (tid == 0) {
+      double a = 0.0;
+      for (int q = 0; q < parts; ++q) a += bufb[q * jt + jt - 1];
+      carry = a;
     }
     __syncthreads();
   }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) gt += __shfl_xor_sync(0xffffffffu, gt, o);
+  if (lane == 0) red[warp] = gt;
+  __syncthreads();
   if (tid == 0) {
     // the taper through the median spacing |z_p+1 - z_p|
     double g = 0.0;
-    for (int m = 0; m < live; ++m) g += dldf[m] * df[c * live + m];
+    for (int w = 0; w < VT / 32; ++w) g += red[w];
     const int p = med[c];
     const double d = zs[p + 1] - zs[p];
     const double sg = d > 0 ? 1.0 : (d < 0 ? -1.0 : 0.0);
     gz[p + 1] += g * sg;
     gz[p] -= g * sg;
-    // the shift by the minimum: its gradient (minus the sum) shared evenly by the tied minima
+  }
+  __syncthreads();
+  // the shift by the minimum: its gradient (minus the sum) shared evenly by the tied minima
+  if (warp == 0) {
     double tot = 0.0;
     int nt = 0;
-    for (int j = 0; j < D; ++j) {
+    for (int j = lane; j < D; j += 32) {
       tot += gz[j];
       nt += zr[j] == zmin;
     }
-    red[0] = tot / nt;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      tot += __shfl_xor_sync(0xffffffffu, tot, o);
+      nt += __shfl_xor_sync(0xffffffffu, nt, o);
+    }
+    if (lane == 0) red[0] = tot / nt;
   }
   __syncthreads();
   const double share = red[0];
-  for (int j = tid; j < D; j += HT) {
+  for (int j = tid; j < D; j += VT) {
     const double g = gz[j] - (zr[j] == zmin ? share : 0.0);
     z_bar[(long)j * ncol + c] += (float)g;
   }
 }
 
-size_t vjp_smem(int D, int live) { return (size_t)(2 * D + live + 2 * HT * (HCH + 1)) * sizeof(double); }
+size_t vjp_smem(int D) { return (size_t)2 * D * sizeof(double); }
 
 // ---------------------------------------------------------------------------------------- one column, many CTAs
 // The same gradient for one column (a shared height grid), spread over the (mode, node) pairs: k_column_terms writes
@@ -296,17 +336,14 @@ __global__ void __launch_bounds__(CT1) k_column_terms(const double* __restrict__
   const long M2 = 2L * live;
   const double km = k[m], fm = f[m];
   const double zj = zr[j] - zmin;
-  double sn, cs;
-  sincos(zj * km, &sn, &cs);
-  const double gc = tzi_bar[(long)j * M2 + m], gs = tzi_bar[(long)j * M2 + live + m];
-  double lo = fm * km * (-gc * sn - gs * cs), up = 0.0;
-  if (j + 1 < D) {
-    double dza, dzb;
+  double sn, cs, dza = 0.0, up = 0.0;
+  if (j + 1 < D)
     filon_terms_vjp(zj, zr[j + 1] - zmin, km, tzf_bar[(long)m * D + j], tzf_bar[(long)(live + m) * D + j],
-                    tzf_bar[(long)m * D + j + 1], tzf_bar[(long)(live + m) * D + j + 1], dza, dzb);
-    lo += dza;
-    up = dzb;
-  }
+                    tzf_bar[(long)m * D + j + 1], tzf_bar[(long)(live + m) * D + j + 1], dza, up, sn, cs);
+  else
+    sincos(zj * km, &sn, &cs);
+  const double gc = tzi_bar[(long)j * M2 + m], gs = tzi_bar[(long)j * M2 + live + m];
+  const double lo = fm * km * (-gc * sn - gs * cs) + dza;
   const long n = (long)live * D;
   terms[e] = lo;
   terms[n + e] = up;
@@ -410,9 +447,9 @@ int ffno_percol_tables_vjp(const double* z_raw, int D, long ncol, const double* 
   if (!z_raw || !k || !f || !df || !med || !tzf_bar || !tzi_bar || !z_bar || D < 2 || ncol < 1 || live < 1)
     return FFNO_EINVAL;
   if (D > FFNO_PERCOL_MAX_D || live > FFNO_PERCOL_MAX_LIVE || ncol > 2147483647L) return FFNO_EINVAL;
-  const size_t smem = vjp_smem(D, live);
+  const size_t smem = vjp_smem(D);
   if (!ffno::smem_cap_ok(k_percol_tables_vjp, smem)) return FFNO_ELAUNCH;
-  k_percol_tables_vjp<<<(unsigned)ncol, HT, smem, (cudaStream_t)stream>>>(z_raw, D, ncol, k, live, f, df, med,
+  k_percol_tables_vjp<<<(unsigned)ncol, VT, smem, (cudaStream_t)stream>>>(z_raw, D, ncol, k, live, f, df, med,
                                                                          tzf_bar, tzi_bar, z_bar);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
