@@ -1008,9 +1008,11 @@ class Executor:
         self._gn_jvp(ws, tw, ws.mlp_pre, tw.mlp, bp["mlp_g"], bp["mlp_b"], "mlp", 0, tw.x2, r_mlp, tw.x)
 
     # -------------------------------------------------------------------------------------------- VJP
-    def backward(self, state, ybar, errs=None):
+    def backward(self, state, ybar, errs=None, heights=True):
         """Input VJP: ybar [B, L, D, H, W] -> (x_bar [B, Cin, D, H, W], z_bar [B, D, H, W]). errs: as in forward
-        (the backward's flag and that of the forward that made the state)."""
+        (the backward's flag and that of the forward that made the state). heights False: the caller takes no
+        gradient in the heights; z_bar is None and what only it needs (the height tables' gradient products and
+        their walk back to the columns, the z_proj and depth-weight terms) does not run."""
         m = self.model
         x, z_scale, dx, dy = state["x"], state["z"], state["dx"], state["dy"]
         pk, geo, hgt, pln, pfr = self._setup(x, z_scale, dx, dy, state.get("geo"))
@@ -1020,10 +1022,11 @@ class Executor:
         s = _stream()
         ybar = ybar.contiguous()
         xbar_in = torch.zeros_like(x)
-        zbar = torch.zeros_like(z_scale)
+        zbar = torch.zeros_like(z_scale) if heights else None
         tc = self._tc()
         ws = gb = None
-        if geo.shared:
+        tzf_bar = tzi_bar = None
+        if geo.shared and heights:
             live = hgt["live"]
             tzf_bar = torch.zeros(2 * live, D, dtype=torch.float64, device=dev)
             tzi_bar = torch.zeros(D, 2 * live, dtype=torch.float64, device=dev)
@@ -1033,7 +1036,7 @@ class Executor:
             if ws is None or ws.live != live:
                 ws = Workspace(D, H, W, C, live, pk.groups, dev)
                 gb = _GradBuffers(D, H, W, C, live, pk.groups, ws.nparts, dev)
-            if not geo.shared:
+            if not geo.shared and heights:
                 # this sample's per-column table gradients: [HW][2M'][D] and [HW][D][2M']
                 tzf_bar = torch.zeros(HW, 2 * live, D, dtype=torch.float64, device=dev)
                 tzi_bar = torch.zeros(HW, D, 2 * live, dtype=torch.float64, device=dev)
@@ -1060,18 +1063,20 @@ class Executor:
                 else:
                     wb = ws
                     self._block(pk, ws, i, z, D, H, W, hgt_b, pln, pfr[i], x_in=inputs[i])
-                self._block_bwd(pk, wb, gb, i, inputs[i], z, zbar[b], D, H, W, hgt_b, pln, pfr[i], tzf_bar, tzi_bar)
+                self._block_bwd(pk, wb, gb, i, inputs[i], z, zbar[b] if heights else None, D, H, W, hgt_b, pln,
+                                pfr[i], tzf_bar, tzi_bar)
             # lift: x0 = gelu(GN(pre0))
             self._lift(pk, ws, xin)
             self._gn_bwd(ws, gb, 1, gb.xbar, 1.0, ws.pre, pk.lift_g, pk.lift_b, "lift", gb.pbar)
             nat.call("ffno_lift_bwd", gb.pbar.data_ptr(), Cin, V, C, pk.lift_w.data_ptr(), xbar_in[b].data_ptr(), s)
-            nat.call("ffno_depth_weights_bwd", z.data_ptr(), gb.wbar.data_ptr(), D, HW, zbar[b].data_ptr(), s)
-            if not geo.shared:
+            if heights:
+                nat.call("ffno_depth_weights_bwd", z.data_ptr(), gb.wbar.data_ptr(), D, HW, zbar[b].data_ptr(), s)
+            if not geo.shared and heights:
                 # every column's own tables depend on that column's heights (ffno_percol_tables_vjp, FP64)
                 nat.call("ffno_percol_tables_vjp", hgt_b["z"].data_ptr(), D, HW, hgt_b["k"].data_ptr(), live,
                          hgt_b["f"].data_ptr(), hgt_b["df"].data_ptr(), hgt_b["med"].data_ptr(), tzf_bar.data_ptr(),
                          tzi_bar.data_ptr(), zbar[b].data_ptr(), s)
-        if geo.shared:
+        if geo.shared and heights:
             # the height tables depend on the shared column (sample 0, column (0, 0)): their gradient goes there, on
             # the device in FP64, spread over the column's (mode, node) pairs
             self._column_tables_vjp(hgt, D, tzf_bar, tzi_bar, zbar[0], H * W)
@@ -1105,7 +1110,8 @@ class Executor:
 
     def _block_bwd(self, pk, ws, gb, i, x, z, zbar, D, H, W, hgt, pln, fq, tzf_bar, tzi_bar):
         """gb.xbar (gradient of the block output) -> gb.xbar (gradient of the block input x); accumulates the
-        depth-weight gradient in gb.wbar, the z_proj gradient in zbar and the height-table gradients."""
+        depth-weight gradient in gb.wbar, the z_proj gradient in zbar and the height-table gradients (zbar None: no
+        gradient in the heights is taken, tzf_bar and tzi_bar are not used)."""
         m = self.model
         C, V, HW, Wf = m.width, ws.V, H * W, W // 2 + 1
         s = _stream()
@@ -1185,32 +1191,37 @@ class Executor:
         hq = hgt["freq"][i]
         N = HW * C
         if hgt.get("percol"):
-            nat.call("ffno_col_outer", gb.yvb.data_ptr(), D, ws.vb.data_ptr(), 2 * live, HW, C, N,
-                     tzi_bar.data_ptr(), 1, s)
+            if zbar is not None:
+                nat.call("ffno_col_outer", gb.yvb.data_ptr(), D, ws.vb.data_ptr(), 2 * live, HW, C, N,
+                         tzi_bar.data_ptr(), 1, s)
             nat.call("ffno_xform_pt", hgt["tzi_t"].data_ptr(), 2 * live * D, gb.yvb.data_ptr(), ws.va.data_ptr(),
                      d["pcf"], 0, s)
             self._mix(ws, "v", bp, hq, ws.va, ws.vb, live, HW, HW * C, C, live * HW * C, True)
-            nat.call("ffno_col_outer", ws.vb.data_ptr(), 2 * live, ws.xv.data_ptr(), D, HW, C, N,
-                     tzf_bar.data_ptr(), 1, s)
+            if zbar is not None:
+                nat.call("ffno_col_outer", ws.vb.data_ptr(), 2 * live, ws.xv.data_ptr(), D, HW, C, N,
+                         tzf_bar.data_ptr(), 1, s)
             nat.call("ffno_xform_pt", hgt["tzf_t"].data_ptr(), 2 * live * D, ws.vb.data_ptr(), gb.xvb.data_ptr(),
                      d["pci"], 0, s)
         else:
-            self._outer(ws, gb.yvb, D, ws.vb, 2 * live, N, gb.opart, gb.osplit_i, tzi_bar)
+            if zbar is not None:
+                self._outer(ws, gb.yvb, D, ws.vb, 2 * live, N, gb.opart, gb.osplit_i, tzi_bar)
             self._xf(hgt, "tzi_t", gb.yvb, ws.va, d["zf"], ws)
             self._mix(ws, "v", bp, hq, ws.va, ws.vb, live, HW, HW * C, C, live * HW * C, True)
-            self._outer(ws, ws.vb, 2 * live, ws.xv, D, N, gb.opart, gb.osplit_f, tzf_bar)
+            if zbar is not None:
+                self._outer(ws, ws.vb, 2 * live, ws.xv, D, N, gb.opart, gb.osplit_f, tzf_bar)
             self._xf(hgt, "tzf_t", ws.vb, gb.xvb, d["zi"], ws)
         # input gates (and z_proj)
+        zp = None if zbar is None else bp["v_zp"].data_ptr()
         if tc_chan:
             nat.call("ffno_gate_bwd_tc", x.data_ptr(), gb.xsb.data_ptr(), gb.xacc.data_ptr(), V, C,
                      bp["tcb_s_gate"].data_ptr(), None, gb.xbar.data_ptr(), None, err, s)
             nat.call("ffno_gate_bwd_tc", x.data_ptr(), gb.xvb.data_ptr(), gb.xbar.data_ptr(), V, C,
-                     bp["tcb_v_gate"].data_ptr(), bp["v_zp"].data_ptr(), gb.xbar.data_ptr(), zbar.data_ptr(), err, s)
+                     bp["tcb_v_gate"].data_ptr(), zp, gb.xbar.data_ptr(), _ptr(zbar), err, s)
         else:
             nat.call("ffno_gate_bwd", x.data_ptr(), gb.xsb.data_ptr(), gb.xvb.data_ptr(), gb.xacc.data_ptr(), V, C,
                      bp["s_g1"].data_ptr(), bp["s_g2"].data_ptr(), bp["s_g2t"].data_ptr(), bp["s_g1t"].data_ptr(),
                      bp["v_g1"].data_ptr(), bp["v_g2"].data_ptr(), bp["v_g2t"].data_ptr(), bp["v_g1t"].data_ptr(),
-                     bp["v_zp"].data_ptr(), gb.xbar.data_ptr(), zbar.data_ptr(), s)
+                     zp, gb.xbar.data_ptr(), _ptr(zbar), s)
 
 
 class _GradBuffers:
@@ -1327,7 +1338,7 @@ class _FFNOFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, ybar):
-        xbar, zbar = ctx.executor.backward(ctx.state, ybar)
+        xbar, zbar = ctx.executor.backward(ctx.state, ybar, heights=ctx.needs_input_grad[1])
         ctx.state = None
         return xbar, zbar, None, None, None
 
