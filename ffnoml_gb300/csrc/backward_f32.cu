@@ -674,7 +674,9 @@ __global__ void __launch_bounds__(NT, 2) k_head_bwd(const float* __restrict__ x,
                                                  const __grid_constant__ ffno_head_params hp, int nh,
                                                  float* __restrict__ xbar, float* __restrict__ xinbar, int al) {
   extern __shared__ __align__(16) float sm[];
+  __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1, N2 = 2 * C / 16;
+  if (kLte) fill_exp_table(etab);
   float* SA = sm;                    // [C][64] input, then [2C][64] hidden, then its gradient
   float* SG = SA + 2 * C * BM;       // [NHP][64] gradient of the head channels
   float* SO = SG + NHP * BM;         // [64][NHP + 1] head channels, then their gradient
@@ -721,7 +723,7 @@ __global__ void __launch_bounds__(NT, 2) k_head_bwd(const float* __restrict__ x,
       float* o = SO + r * LO;
       if (v < V) {
         if constexpr (kLte) {
-          head_voxel_bwd<T>(hp, o, NHP, head_inputs(hp, xin, V, v), ybar, V, v, xinbar);
+          head_voxel_bwd<T>(hp, o, NHP, head_inputs(hp, xin, V, v), ybar, V, v, xinbar, etab);
         } else {
           for (int c = 0; c < NHP; ++c) o[c] = c < nh ? __ldg(ybar + (long)c * V + v) : 0.f;
         }
@@ -754,10 +756,13 @@ __global__ void __launch_bounds__(256) k_head_output_bwd(const float* __restrict
                                                          const float* __restrict__ ybar, long V, int nh,
                                                          const __grid_constant__ ffno_head_params hp,
                                                          float* __restrict__ hbar, float* __restrict__ xinbar) {
+  __shared__ double etab[EXP_TAB];
+  fill_exp_table(etab);
+  __syncthreads();
   float o[FFNO_MAX_LEVELS + FFNO_MAX_SPECIES];
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < V; v += (long)gridDim.x * blockDim.x) {
     for (int c = 0; c < nh; ++c) o[c] = __ldg(head + (long)c * V + v);
-    head_voxel_bwd<T>(hp, o, nh, head_inputs(hp, xin, V, v), ybar, V, v, xinbar);
+    head_voxel_bwd<T>(hp, o, nh, head_inputs(hp, xin, V, v), ybar, V, v, xinbar, etab);
     for (int c = 0; c < nh; ++c) hbar[(long)c * V + v] = o[c];
   }
 }

@@ -108,14 +108,8 @@ __device__ __forceinline__ float sigmoid_tc(float x) { return __fdividef(1.f, 1.
 // Math of the level-fraction head in the scalar type of the caller: FP64 (the reference's arithmetic) or FP32.
 __device__ __forceinline__ double mexp10(double x) { return exp10(x); }
 __device__ __forceinline__ float mexp10(float x) { return exp10f(x); }
-__device__ __forceinline__ double mexp(double x) { return exp(x); }
-__device__ __forceinline__ float mexp(float x) { return expf(x); }
-__device__ __forceinline__ double mlog(double x) { return log(x); }
-__device__ __forceinline__ float mlog(float x) { return logf(x); }
 __device__ __forceinline__ double msqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float msqrt(float x) { return sqrtf(x); }
-__device__ __forceinline__ double mtanh(double x) { return tanh(x); }
-__device__ __forceinline__ float mtanh(float x) { return tanhf(x); }
 
 // MULTI3D constants, cgs (models/ffno_model.py:111-112)
 constexpr double kEE = 1.602189e-12, kBK = 1.380662e-16;
@@ -145,17 +139,122 @@ __device__ __forceinline__ HeadInputs head_inputs(const ffno_head_params& hp, co
   return HeadInputs{__ldg(xin + (long)tc * V + v), __ldg(xin + (long)ec * V + v), __ldg(xin + (long)rc * V + v)};
 }
 
+// FP64 elementary functions of the head. The FP64 pipe of this chip takes about two lanes a cycle and SM, so the head is
+// bound by the number of its FP64 operations: about 1100 a voxel of two six-level species with CUDA's exp, log, exp10,
+// tanh, division and square root, about 370 with these. Each is the textbook method, full double precision (a few
+// 2^-53) on the range that the caller checks; outside it the head takes CUDA's functions.
+//   exp(x) = 2^(n / 128) e^r, n = round(128 x / ln 2), |r| <= ln 2 / 256: a table of 2^(i / 128) (filled once per CTA with
+//     exp2) and the Taylor polynomial of e^r - 1 to r^5 (remainder 5e-19);
+//   10^x the same with n = round(128 x log2 10);
+//   log(s), s near 1 .. 32: one Newton step y + e - e^2 / 2, e = s exp(-y) - 1, from FP32's y (e < 1e-6);
+//   tanh(x) = sign(x) (1 - q) / (1 + q), q = exp(-2 |x|);
+//   1 / x: two Newton-Raphson steps from the hardware's 20-bit reciprocal.
+constexpr int EXP_TAB = 128;
+// ln 2 / 128 and log10(2) / 128 in two parts, the first with 32 trailing zero bits (its products with n are exact)
+constexpr double LN2HI = 0.005415208637714386, LN2LO = 3.710410186743494e-09;
+constexpr double LG2HI = 0.002351796254515648, LG2LO = 5.866092051994237e-10;
+
+__device__ __forceinline__ void fill_exp_table(double* tab) {
+  for (int i = threadIdx.x; i < EXP_TAB; i += blockDim.x) tab[i] = exp2((double)i / EXP_TAB);
+}
+
+__device__ __forceinline__ double rcp64(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// 2^(n / 128) e^r for |r| <= 0.003, n in a double's exponent range; t = n + 1.5 2^52 carries n in its low word
+__device__ __forceinline__ double exp_parts(const double* tab, double t, double r) {
+  const int n = __double2loint(t);
+  double c = fma(r, 1.0 / 120, 1.0 / 24);
+  c = fma(r, c, 1.0 / 6);
+  c = fma(r, c, 0.5);
+  const double p = fma(r * r, c, r);
+  const double b = tab[n & (EXP_TAB - 1)];
+  const double v = fma(b, p, b);
+  return __hiloint2double(__double2hiint(v) + ((n >> 7) << 20), __double2loint(v));
+}
+constexpr double kRoundMagic = 6755399441055744.0;   // 1.5 2^52
+
+// exp(x), x finite and below 700; 0 below -700 (a level's share there is under 1e-304)
+__device__ __forceinline__ double exp_tab(const double* tab, double x) {
+  const double t = fma(x, 184.6649652337873, kRoundMagic);
+  const double n = t - kRoundMagic;
+  const double r = fma(n, -LN2LO, fma(n, -LN2HI, x));
+  const double v = exp_parts(tab, t, r);
+  return (unsigned)__double2hiint(x) > 0xc085e000u ? 0.0 : v;
+}
+// 10^x, |x| < 300
+__device__ __forceinline__ double exp10_tab(const double* tab, double x) {
+  const double t = fma(x, 425.20679614558236, kRoundMagic);
+  const double n = t - kRoundMagic;
+  return exp_parts(tab, t, fma(n, -LG2LO, fma(n, -LG2HI, x)) * kLN10);
+}
+__device__ __forceinline__ double log_tab(const double* tab, double s) {
+  const double y = (double)logf((float)s);
+  const double e = fma(s, exp_tab(tab, -y), -1.0);
+  return y + fma(-0.5 * e, e, e);
+}
+__device__ __forceinline__ double tanh_tab(const double* tab, double x) {
+  const double q = exp_tab(tab, -2.0 * fabs(x));
+  return copysign((1.0 - q) * rcp64(1.0 + q), x);
+}
+
+// The head's functions in T: FP64 by table where `fast`, else CUDA's.
+template <typename T>
+struct HeadMath;
+template <>
+struct HeadMath<double> {
+  const double* tab;
+  bool fast;   // every head channel below 1e6 in size, 0.5 < log10 T < 15, |log10 ne| < 40
+  __device__ __forceinline__ double exp_(double x) const { return fast ? exp_tab(tab, x) : exp(x); }
+  __device__ __forceinline__ double log_(double x) const { return fast ? log_tab(tab, x) : log(x); }
+  __device__ __forceinline__ double tanh_(double x) const { return fast ? tanh_tab(tab, x) : tanh(x); }
+  __device__ __forceinline__ double inv_(double x) const { return fast ? rcp64(x) : 1.0 / x; }
+};
+template <>
+struct HeadMath<float> {
+  const double* tab;
+  bool fast;
+  __device__ __forceinline__ float exp_(float x) const { return expf(x); }
+  __device__ __forceinline__ float log_(float x) const { return logf(x); }
+  __device__ __forceinline__ float tanh_(float x) const { return tanhf(x); }
+  __device__ __forceinline__ float inv_(float x) const { return 1.f / x; }
+};
+
+__device__ __forceinline__ bool head_fast(const ffno_head_params& hp, const float* o, int nh, const HeadInputs& in) {
+  const float lt = fmaf(in.lt, hp.std_x[hp.temperature_channel], hp.mean_x[hp.temperature_channel]);
+  const float ln = fmaf(in.lne, hp.std_x[hp.ne_channel], hp.mean_x[hp.ne_channel]);
+  bool ok = lt > 0.5f && lt < 15.f && fabsf(ln) < 40.f;
+  for (int c = 0; c < nh; ++c) ok = ok && fabsf(o[c]) < 1e6f;
+  return ok;
+}
+__device__ __forceinline__ int head_channels(const ffno_head_params& hp) {
+  int n = 0;
+  for (int s = 0; s < hp.nspecies; ++s) n += hp.levels[s] + 1;
+  return n;
+}
+
 template <typename T>
 struct Lte {
   T lt, lne, conl, dxi, ek_t;
-  __device__ __forceinline__ Lte(const ffno_head_params& hp, const HeadInputs& in) {
+  __device__ __forceinline__ Lte(const ffno_head_params& hp, const HeadInputs& in, const HeadMath<T>& hm) {
     const int tc = hp.temperature_channel, ec = hp.ne_channel;
     const T LN10 = (T)kLN10;
     lt = (T)in.lt * (T)hp.std_x[tc] + (T)hp.mean_x[tc];
     lne = (T)in.lne * (T)hp.std_x[ec] + (T)hp.mean_x[ec];
+    conl = (T)kLN_CCON + (lne - (T)6) * LN10 - (T)1.5 * lt * LN10;
+    if constexpr (sizeof(T) == 8) {
+      if (hm.fast) {   // 4.98e-4 5040 sqrt(BK) sqrt(ne / T), ne in cm^-3; E / (k T)
+        dxi = 2.9491955176246003e-08 * exp10_tab(hm.tab, 0.5 * (lne - 6.0 - lt));
+        ek_t = (kEE / kBK) * exp10_tab(hm.tab, -lt);
+        return;
+      }
+    }
     const T tk = mexp10(lt);
     const T ne = mexp10(lne - (T)6);  // cm^-3
-    conl = (T)kLN_CCON + (lne - (T)6) * LN10 - (T)1.5 * lt * LN10;
     dxi = (T)(4.98e-4 * 5040.0) / tk * msqrt(ne * (T)kBK * tk);
     ek_t = (T)(kEE / kBK) / tk;
   }
@@ -169,14 +268,12 @@ struct Lte {
 // improved Kahan-Babuska summation (A. Neumaier, "Rundungsfehleranalyse einiger Verfahren zur Summation endlicher
 // Summen", ZAMM 54 (1974) 39-51): the rounding error of every addition is carried in c and added once at the end,
 // so the result is the exactly rounded sum of the rounded terms up to O(L u^2).
-template <typename T>
-__device__ __forceinline__ T shifted_exp_sum(const T* logit, int L, T mx) {
-  T s = 0;
-  for (int i = 0; i < L; ++i) s += mexp(logit[i] - mx);
+__device__ __forceinline__ double shifted_exp_sum(const HeadMath<double>& hm, const double* logit, int L, double mx) {
+  double s = 0;
+  for (int i = 0; i < L; ++i) s += hm.exp_(logit[i] - mx);
   return s;
 }
-template <>
-__device__ __forceinline__ float shifted_exp_sum<float>(const float* logit, int L, float mx) {
+__device__ __forceinline__ float shifted_exp_sum(const HeadMath<float>&, const float* logit, int L, float mx) {
   float s = 0.f, c = 0.f;
   for (int i = 0; i < L; ++i) {
     const float t = expf(logit[i] - mx);
@@ -187,14 +284,49 @@ __device__ __forceinline__ float shifted_exp_sum<float>(const float* logit, int 
   return s + c;
 }
 
-// Forward: out[g * V + v] = the normalised log10 population of level g.
+// log10 n - mean_y of one level from base (log10 n of the whole species), the level's shifted logit d and the log-sum lse:
+// base + (d - lse) / ln 10 - mean, the large terms cancelling. FP64: in FP64.
+struct HeadBase64 {
+  double base;
+  __device__ __forceinline__ explicit HeadBase64(double b) : base(b) {}
+  __device__ __forceinline__ float level(double d, double lse, float mean) const {
+    return (float)(base + (d - lse) * kINV_LN10 - (double)mean);
+  }
+};
+// FP32 (the split-BF16 path): in pairs of floats (value and rounding error, 48 bits), by the error-free sum of Knuth and
+// the error-free product by fused multiply-add: 20 FP32 operations where the FP64 form has 6 at 1 / 64 of the rate.
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+  return s;
+}
+struct HeadBase32 {
+  float hi, lo;
+  __device__ __forceinline__ explicit HeadBase32(double b) : hi((float)b) { lo = (float)(b - (double)hi); }
+  __device__ __forceinline__ float level(float d, float lse, float mean) const {
+    constexpr float IH = 0.4342944920063019f, IL = -1.0103050052231683e-08f;   // 1 / ln 10 in two floats
+    float de, me, se;
+    const float dd = two_sum(d, -lse, de);
+    const float p = __fmul_rn(dd, IH);
+    const float pe = fmaf(dd, IL, fmaf(de, IH, fmaf(dd, IH, -p)));
+    const float m = two_sum(hi, -mean, me);
+    const float r = two_sum(m, p, se);
+    return __fadd_rn(r, __fadd_rn(se, __fadd_rn(__fadd_rn(me, lo), pe)));
+  }
+};
+__device__ __forceinline__ HeadBase64 head_base(double b, double) { return HeadBase64(b); }
+__device__ __forceinline__ HeadBase32 head_base(double b, float) { return HeadBase32(b); }
+
+// Forward: out[g * V + v] = the normalised log10 population of level g. tab: fill_exp_table's.
 template <typename T>
 __device__ __forceinline__ void head_voxel_fwd(const ffno_head_params& hp, const float* o, const HeadInputs& in,
-                                               float* __restrict__ out, long V, long v) {
-  const Lte<T> e(hp, in);
-  // the total term and the assembly of log10 n (log10 rho - log10 m + s ~ 20, minus mean_Y) stay in FP64 for both
+                                               float* __restrict__ out, long V, long v, const double* tab) {
+  HeadMath<T> hm{tab, false};
+  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, o, head_channels(hp), in);
+  const Lte<T> e(hp, in, hm);
+  // the total term and the assembly of log10 n (log10 rho - log10 m + s ~ 20, minus mean_Y) stay beyond FP32 for both
   // T: in FP32 their rounding (~1e-6 dex at that magnitude, and a few ulp of b for tanh) would move every level of
-  // the voxel against its total, past the 1e-6 bar on the level shares' sum; they are a handful of FP64 operations
+  // the voxel against its total, past the 1e-6 bar on the level shares' sum
   const double lrho = (double)in.lrho * (double)hp.std_x[hp.rho_channel] + (double)hp.mean_x[hp.rho_channel];
   int hc = 0, lvl = 0;
   for (int s = 0; s < hp.nspecies; ++s) {
@@ -205,14 +337,15 @@ __device__ __forceinline__ void head_voxel_fwd(const ffno_head_params& hp, const
       logit[i] = (T)o[hc + i] + e.weight(hp, lvl + i);
       mx = fmax(mx, logit[i]);
     }
-    const T lse = mlog(shifted_exp_sum<T>(logit, L, mx));
+    const T lse = hm.log_(shifted_exp_sum(hm, logit, L, mx));
     const double tb = (double)hp.total_bound;
-    const double base = lrho - (double)hp.log10_particle_mass[s] + tb * tanh((double)o[hc + L] / tb);
+    const float u = o[hc + L];
+    const double th = fabsf(u) < 1e6f ? tanh_tab(tab, (double)u * rcp64(tb)) : tanh((double)u / tb);
+    const auto base = head_base(lrho - (double)hp.log10_particle_mass[s] + tb * th, T(0));
     for (int i = 0; i < L; ++i) {
       const int g = lvl + i;
-      const double l10 = base + ((double)(logit[i] - mx) - (double)lse) * kINV_LN10;
-      // the large terms cancel in FP64; the difference (a few units) is normalised in FP32
-      out[(long)g * V + v] = (float)(l10 - (double)hp.mean_y[g]) / hp.std_y[g];
+      // the large terms cancel before the difference (a few units) is normalised in FP32
+      out[(long)g * V + v] = base.level(logit[i] - mx, lse, hp.mean_y[g]) / hp.std_y[g];
     }
     hc += L + 1;
     lvl += L;
@@ -224,9 +357,10 @@ __device__ __forceinline__ void head_voxel_fwd(const ffno_head_params& hp, const
 template <typename T>
 __device__ __forceinline__ void head_voxel_bwd(const ffno_head_params& hp, float* o, int nhp, const HeadInputs& in,
                                                const float* __restrict__ ybar, long V, long v,
-                                               float* __restrict__ xinbar) {
-  const Lte<T> e(hp, in);
-  const T LN10 = (T)kLN10;
+                                               float* __restrict__ xinbar, const double* tab) {
+  HeadMath<T> hm{tab, false};
+  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, o, head_channels(hp), in);
+  const Lte<T> e(hp, in, hm);
   T gsum = 0, ltb = 0, lneb = 0;
   int hc = 0, lvl = 0;
   for (int s = 0; s < hp.nspecies; ++s) {
@@ -237,23 +371,25 @@ __device__ __forceinline__ void head_voxel_bwd(const ffno_head_params& hp, float
       logit[i] = (T)o[hc + i] + e.weight(hp, lvl + i);
       mx = fmax(mx, logit[i]);
     }
-    const T se = shifted_exp_sum<T>(logit, L, mx);
+    const T se = shifted_exp_sum(hm, logit, L, mx), ise = hm.inv_(se);
     T G = 0;
     for (int i = 0; i < L; ++i) {
-      gl[i] = (T)__ldg(ybar + (long)(lvl + i) * V + v) / (T)hp.std_y[lvl + i];
+      gl[i] = (T)__ldg(ybar + (long)(lvl + i) * V + v);
+      gl[i] = sizeof(T) == 8 ? gl[i] * hm.inv_((T)hp.std_y[lvl + i]) : gl[i] / (T)hp.std_y[lvl + i];
       G += gl[i];
     }
     gsum += G;
     const T tb = (T)hp.total_bound;
-    const T th = mtanh((T)o[hc + L] / tb);
+    const T th = hm.tanh_(sizeof(T) == 8 ? (T)o[hc + L] * hm.inv_(tb) : (T)o[hc + L] / tb);
     const float ubar = (float)(G * ((T)1 - th * th));
     for (int i = 0; i < L; ++i) {
       const int g = lvl + i;
-      const T p = mexp(logit[i] - mx) / se;
-      const T lb = (gl[i] - p * G) / LN10;
+      const T ex = hm.exp_(logit[i] - mx), p = sizeof(T) == 8 ? ex * ise : ex / se;
+      const T d = gl[i] - p * G;                    // the logit's gradient times ln 10
+      const T lb = d * (T)kINV_LN10;
       o[hc + i] = (float)lb;
-      ltb += lb * LN10 * (e.ek_t * ((T)hp.ev[g] - (T)1.5 * e.dxi * (T)hp.ndxi[g]) + (T)1.5 * (T)hp.dion[g]);
-      lneb += lb * LN10 * ((T)0.5 * e.ek_t * e.dxi * (T)hp.ndxi[g] - (T)hp.dion[g]);
+      ltb += d * (e.ek_t * ((T)hp.ev[g] - (T)1.5 * e.dxi * (T)hp.ndxi[g]) + (T)1.5 * (T)hp.dion[g]);
+      lneb += d * ((T)0.5 * e.ek_t * e.dxi * (T)hp.ndxi[g] - (T)hp.dion[g]);
     }
     o[hc + L] = ubar;
     hc += L + 1;

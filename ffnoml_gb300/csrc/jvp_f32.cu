@@ -351,7 +351,9 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* _
                                                  const float* __restrict__ b2, ffno_head_params hp,
                                                  float* __restrict__ outd, int al) {
   extern __shared__ __align__(16) float sm[];
+  __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1, TAN = 2 * C * BM;
+  fill_exp_table(etab);
   float* as = sm;                 // [C][64] input, then [2C][64] hidden; their tangents TAN floats on
   float* os = as + 2 * TAN;       // [64][NHP + 1] head channels, then their tangents
   float* ods = os + BM * LO;
@@ -359,7 +361,6 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* _
   using Ch = g32::Cols<2 * C, 1>;
   using Co = g32::Cols<NHP, 1>;
   const int tx = g32::tile_tx(), ty = g32::tile_ty();
-  const double lnc = kLN_CCON;
   const long nt = (V + BM - 1) / BM;
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
     const long v0 = t * BM;
@@ -406,16 +407,12 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* _
         const float* o = os + r * LO;
         const float* od = ods + r * LO;
         const int tc = hp.temperature_channel, ec = hp.ne_channel, rc = hp.rho_channel;
-        const double lt = (double)__ldg(xin + (long)tc * V + v) * (double)hp.std_x[tc] + (double)hp.mean_x[tc];
-        const double lne = (double)__ldg(xin + (long)ec * V + v) * (double)hp.std_x[ec] + (double)hp.mean_x[ec];
+        const HeadInputs in = head_inputs(hp, xin, V, v);
+        const HeadMath<double> hm{etab, head_fast(hp, o, head_channels(hp), in)};
+        const Lte<double> le(hp, in, hm);
         const double dlt = (double)__ldg(xind + (long)tc * V + v) * (double)hp.std_x[tc];
         const double dlne = (double)__ldg(xind + (long)ec * V + v) * (double)hp.std_x[ec];
         const double dlrho = (double)__ldg(xind + (long)rc * V + v) * (double)hp.std_x[rc];
-        const double tk = exp10(lt);
-        const double ne = exp10(lne - 6.0);  // cm^-3
-        const double conl = lnc + (lne - 6.0) * kLN10 - 1.5 * lt * kLN10;
-        const double dxi = 4.98e-4 * 5040.0 / tk * sqrt(ne * kBK * tk);
-        const double ek_t = (kEE / kBK) / tk;
         int hc = 0, lvl = 0;
         for (int s = 0; s < hp.nspecies; ++s) {
           const int L = hp.levels[s];
@@ -423,25 +420,27 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* _
           double mx = -1e300;
           for (int i = 0; i < L; ++i) {
             const int g = lvl + i;
-            const double lte = hp.log_g[g] - ek_t * (hp.ev[g] - dxi * hp.ndxi[g]) - hp.dion[g] * conl;
+            const double lte = le.weight(hp, g);
             // d lte / d log10 T and d lte / d log10 ne (through t, the Debye term dxi ~ sqrt(ne / t) and conl)
-            const double dT = kLN10 * (ek_t * (hp.ev[g] - 1.5 * dxi * hp.ndxi[g]) + 1.5 * hp.dion[g]);
-            const double dN = kLN10 * (0.5 * ek_t * hp.ndxi[g] * dxi - hp.dion[g]);
+            const double dT = kLN10 * (le.ek_t * (hp.ev[g] - 1.5 * le.dxi * hp.ndxi[g]) + 1.5 * hp.dion[g]);
+            const double dN = kLN10 * (0.5 * le.ek_t * hp.ndxi[g] * le.dxi - hp.dion[g]);
             logit[i] = (double)o[hc + i] + lte;
             dl[i] = (double)od[hc + i] + dT * dlt + dN * dlne;
             mx = fmax(mx, logit[i]);
           }
-          double se = 0.0;
-          for (int i = 0; i < L; ++i) se += exp(logit[i] - mx);
-          double md = 0.0;
-          for (int i = 0; i < L; ++i) md += exp(logit[i] - mx) / se * dl[i];
-          const double tb = (double)hp.total_bound;
-          const double th = tanh((double)o[hc + L] / tb);
+          double se = 0.0, md = 0.0;
+          for (int i = 0; i < L; ++i) {
+            const double ex = hm.exp_(logit[i] - mx);
+            se += ex;
+            md += ex * dl[i];
+          }
+          md *= hm.inv_(se);
+          const double th = hm.tanh_((double)o[hc + L] * hm.inv_((double)hp.total_bound));
           const double dtot = (1.0 - th * th) * (double)od[hc + L];
           for (int i = 0; i < L; ++i) {
             const int g = lvl + i;
-            const double d = dlrho + dtot + (dl[i] - md) / kLN10;
-            outd[(long)g * V + v] = (float)(d / (double)hp.std_y[g]);
+            const double d = dlrho + dtot + (dl[i] - md) * kINV_LN10;
+            outd[(long)g * V + v] = (float)(d * hm.inv_((double)hp.std_y[g]));
           }
           hc += L + 1;
           lvl += L;

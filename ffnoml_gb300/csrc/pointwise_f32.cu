@@ -517,7 +517,9 @@ __global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, con
                                              const __grid_constant__ ffno_head_params hp, float* __restrict__ out,
                                              float* __restrict__ head_out, int al) {
   extern __shared__ __align__(16) float sm[];
+  __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1;
+  if (kLte) fill_exp_table(etab);
   float* as = sm;                    // [C][64] input, then [2C][64] hidden
   float* os = as + 2 * C * BM;       // [64][NHP + 1] head channels
   g32::Ring ring(os + BM * LO, g32::KC * 2 * C, al);
@@ -561,7 +563,7 @@ __global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, con
         const float* o = os + r * LO;
         if (head_out)
           for (int c = 0; c < nh; ++c) head_out[(long)c * V + v] = o[c];
-        if constexpr (kLte) head_voxel_fwd<T>(hp, o, head_inputs(hp, xin, V, v), out, V, v);
+        if constexpr (kLte) head_voxel_fwd<T>(hp, o, head_inputs(hp, xin, V, v), out, V, v, etab);
       }
     }
   }
@@ -574,10 +576,13 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_head_output(const float* __restrict__ head, const float* __restrict__ xin,
                                                      long V, int nh, const __grid_constant__ ffno_head_params hp,
                                                      float* __restrict__ out) {
+  __shared__ double etab[EXP_TAB];
+  fill_exp_table(etab);
+  __syncthreads();
   float o[FFNO_MAX_LEVELS + FFNO_MAX_SPECIES];
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < V; v += (long)gridDim.x * blockDim.x) {
     for (int c = 0; c < nh; ++c) o[c] = __ldg(head + (long)c * V + v);
-    head_voxel_fwd<T>(hp, o, head_inputs(hp, xin, V, v), out, V, v);
+    head_voxel_fwd<T>(hp, o, head_inputs(hp, xin, V, v), out, V, v, etab);
   }
 }
 

@@ -1222,6 +1222,9 @@ __global__ void __launch_bounds__(CT, 1) k_head_tc(const float* __restrict__ x, 
                                                    float* __restrict__ out, float* __restrict__ head_out,
                                                    int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ double etab[EXP_TAB];
+  fill_exp_table(etab);
+  __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C), RB = head_region(C, NHP, false);
   constexpr int LO = NHP + 1;
   PIPE_PROLOGUE(TM, 2)
@@ -1261,7 +1264,7 @@ __global__ void __launch_bounds__(CT, 1) k_head_tc(const float* __restrict__ x, 
       const float* o = os + f * LO;
       if (head_out)
         for (int c = 0; c < nh; ++c) head_out[(long)c * V + v] = o[c];
-      head_voxel_fwd<T>(hp, o, head_inputs(hp, xin, V, v), out, V, v);
+      head_voxel_fwd<T>(hp, o, head_inputs(hp, xin, V, v), out, V, v, etab);
     }
     pipe_sync(P.id);   // the rows are read before the next tile's fill overwrites them
   }
@@ -1281,6 +1284,9 @@ __global__ void __launch_bounds__(CT, 1) k_head_bwd_tc(const float* __restrict__
                                                        float* __restrict__ xbar, float* __restrict__ xinbar,
                                                        int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ double etab[EXP_TAB];
+  if (sizeof(T) == 8) fill_exp_table(etab);
+  __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C), RB = head_region(C, NHP, true);
   constexpr int LO = NHP + 1;
   PIPE_PROLOGUE(2 * TM, 2)
@@ -1321,7 +1327,7 @@ __global__ void __launch_bounds__(CT, 1) k_head_bwd_tc(const float* __restrict__
       const long v = v0 + f;
       float* o = os + f * LO;
       if (v < V) {
-        head_voxel_bwd<T>(hp, o, NHP, head_inputs(hp, xin, V, v), ybar, V, v, xinbar);
+        head_voxel_bwd<T>(hp, o, NHP, head_inputs(hp, xin, V, v), ybar, V, v, xinbar, etab);
       } else {
         for (int c = 0; c < NHP; ++c) o[c] = 0.f;
       }
@@ -2018,6 +2024,9 @@ __global__ void __launch_bounds__(PT, 1) k_head_tc96(const float* __restrict__ x
                                                      int* __restrict__ err) {
   constexpr int C = C96;
   extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ double etab[EXP_TAB];
+  fill_exp_table(etab);
+  __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C);
   PIPE_PROLOGUE(2 * C + NHP, 1)
   const Split T_ = split_at(smem + B1 + B2, TM, KS);
@@ -2062,7 +2071,7 @@ __global__ void __launch_bounds__(PT, 1) k_head_tc96(const float* __restrict__ x
       if (v < V) {
         if (head_out)
           for (int c = 0; c < nh; ++c) head_out[(long)c * V + v] = o[c];
-        head_voxel_fwd<T>(hp, o, head_inputs(hp, xin, V, v), out, V, v);
+        head_voxel_fwd<T>(hp, o, head_inputs(hp, xin, V, v), out, V, v, etab);
       }
     }
   }
@@ -2083,6 +2092,9 @@ __global__ void __launch_bounds__(PT, 1) k_head_bwd_tc96(const float* __restrict
                                                          int* __restrict__ err) {
   constexpr int C = C96;
   extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ double etab[EXP_TAB];
+  if (sizeof(T) == 8) fill_exp_table(etab);
+  __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C);
   constexpr uint32_t DO = 2 * C, D3 = 2 * C + NHP, D4 = 4 * C + NHP;
   static_assert(D4 + C <= 512, "tensor memory");
@@ -2127,7 +2139,7 @@ __global__ void __launch_bounds__(PT, 1) k_head_bwd_tc96(const float* __restrict
         for (int i = 0; i < 16; ++i) o[16 * j + i] = r[i] + __ldg(b2 + 16 * j + i);
       }
       if (v < V) {
-        head_voxel_bwd<T>(hp, o, NHP, head_inputs(hp, xin, V, v), ybar, V, v, xinbar);
+        head_voxel_bwd<T>(hp, o, NHP, head_inputs(hp, xin, V, v), ybar, V, v, xinbar, etab);
       } else {
 #pragma unroll
         for (int c = 0; c < NHP; ++c) o[c] = 0.f;
