@@ -95,12 +95,21 @@ __device__ __forceinline__ void gemm_n(const float* __restrict__ as, int stride_
   using Cl = Cols<N, G>;
   static_assert(K % KC == 0, "whole chunks");
   const int tx = tile_tx(), ty = tile_ty();
+  // two neighbouring channels of a run per FMA where the run has two (f32x2: half the issue slots, the same products and
+  // sums): NP accumulators of PW channels
+  constexpr int PW = Cl::CV > 1 ? 2 : 1, NP = Cl::NC / PW;
+  uint64_t acc2[PW == 2 ? NA : 1][PW == 2 ? NP : 1][4];
 #pragma unroll
   for (int a = 0; a < NA; ++a)
 #pragma unroll
-    for (int j = 0; j < Cl::NC; ++j)
+    for (int j = 0; j < NP; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[a][j][e] = 0.f;
+      for (int e = 0; e < 4; ++e) {
+        if constexpr (PW == 2)
+          acc2[a][j][e] = 0;
+        else
+          acc[a][j][e] = 0.f;
+      }
 #pragma unroll 1
   for (int c = 0; c < K / KC; ++c) {
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -120,12 +129,32 @@ __device__ __forceinline__ void gemm_n(const float* __restrict__ as, int stride_
       for (int a = 0; a < NA; ++a) {
         const float4 v = *reinterpret_cast<const float4*>(ab + a * stride_a + k * BM + ((ty ^ sw ^ (k >> 2)) << 2));
         const float x[4] = {v.x, v.y, v.z, v.w};
+        if constexpr (PW == 2) {
+          uint64_t xx[4];
 #pragma unroll
-        for (int j = 0; j < Cl::NC; ++j)
+          for (int e = 0; e < 4; ++e) xx[e] = pk2(x[e], x[e]);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) acc[a][j][e] = fmaf(x[e], b[j], acc[a][j][e]);
+          for (int j = 0; j < NP; ++j) {
+            const uint64_t bb = pk2(b[2 * j], b[2 * j + 1]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc2[a][j][e] = fma2(xx[e], bb, acc2[a][j][e]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < Cl::NC; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[a][j][e] = fmaf(x[e], b[j], acc[a][j][e]);
+        }
       }
     }
+  }
+  if constexpr (PW == 2) {
+#pragma unroll
+    for (int a = 0; a < NA; ++a)
+#pragma unroll
+      for (int j = 0; j < NP; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) upk2(acc2[a][j][e], acc[a][2 * j][e], acc[a][2 * j + 1][e]);
   }
 }
 

