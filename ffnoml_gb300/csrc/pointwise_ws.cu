@@ -819,12 +819,15 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
   constexpr uint32_t WB = B1 + B2;
   constexpr int NB = C / 32, NPH = 3 * NB, NS = 4;   // NS even: see the conversion
   constexpr uint32_t SB = BOX_BYTES;             // one ring stage: one box
-  constexpr uint32_t TD1 = 6 * C;
+  constexpr int NSL = 4;                         // A slots of one phase (even: a slot's uses all go to one group)
+  constexpr uint32_t TD1 = 32 * NSL, TD2 = TD1 + 2 * C;
+  static_assert(TD2 + 4 * C <= 512, "tensor memory");
   static_assert(WB % 1024 == 0, "the ring must stay 1024-byte aligned (128-byte swizzle)");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* ring = smem + WB;
-  __shared__ uint64_t stg_full[NS], stg_empty[NS], a_full[2], a_empty[2], d1_full[2], h_full[2], d2_full[2], wbar;
+  __shared__ uint64_t stg_full[NS], stg_empty[NS], sl_full[NSL], sl_empty[NSL], d1_full[2], h_full[2], d2_full[2],
+      d2_free[2], wbar;
   __shared__ uint32_t tslot;
   __shared__ float cf[2][3 * C], bs[2 * C];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -834,9 +837,12 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
       tc::mbar_init(&stg_full[s], 1);
       tc::mbar_init(&stg_empty[s], 128);
     }
+    for (int s = 0; s < NSL; ++s) {
+      tc::mbar_init(&sl_full[s], 128);
+      tc::mbar_init(&sl_empty[s], 1);
+    }
     for (int s = 0; s < 2; ++s) {
-      tc::mbar_init(&a_full[s], 256);
-      tc::mbar_init(&a_empty[s], 128);
+      tc::mbar_init(&d2_free[s], 128);
       tc::mbar_init(&d1_full[s], 1);
       tc::mbar_init(&h_full[s], 256);
       tc::mbar_init(&d2_full[s], 1);
@@ -892,49 +898,51 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
     uint64_t* last = nullptr;
     uint32_t last_par = 0;
     bool alive = true;
-    auto gemm2 = [&](int j) {   // D2 (over A stage j % 2) = H(j) Wg2^T, H in D1[j % 2] as [hi 8 | lo 8], K = C
+    auto commit = [&](uint64_t* bar, uint32_t par) {
+      tc::mma_commit(bar);
+      last = bar;
+      last_par = par;
+    };
+    auto gemm2 = [&](int j) {   // D2[j % 2] = H(j) Wg2^T, H in D1[j % 2] as [hi 8 | lo 8], K = C
+      // epilogue 2 of tile j - 2 has read D2[j % 2]
+      if (j >= 2 && !wait_or_flag(&d2_free[j & 1], ((uint32_t)(j - 2) >> 1) & 1u, err, 13)) return false;
+      if (!wait_or_flag(&h_full[j & 1], ((uint32_t)j >> 1) & 1u, err, 5)) return false;
+      tc::tc_after_sync();
       const uint32_t h = tmem + TD1 + (uint32_t)(C * (j & 1));
 #pragma unroll 1
       for (int k = 0; k < C / 16; ++k)
-        mma3_ta(tmem + (uint32_t)(3 * C * (j & 1)), h + 16u * k, h + 16u * k + 8u,
+        mma3_ta(tmem + TD2 + (uint32_t)(2 * C * (j & 1)), h + 16u * k, h + 16u * k + 8u,
                 tc::kmajor_desc(w2 + 256u * k, 128u, C * 16u), tc::kmajor_desc(w2 + B2 / 2 + 256u * k, 128u, C * 16u),
                 i2, k > 0);
-      tc::mma_commit(&d2_full[j & 1]);
-      last = &d2_full[j & 1];
-      last_par = ((uint32_t)j >> 1) & 1u;
+      commit(&d2_full[j & 1], ((uint32_t)j >> 1) & 1u);
+      return true;
     };
     for (int i = 0; i < niter && alive; ++i) {
       const int s = i & 1;
-      const uint32_t n = (uint32_t)i >> 1;
-      if (!wait_or_flag(&a_full[s], n & 1u, err, 4)) {
-        alive = false;
-        break;
-      }
-      if (i >= 2 && !wait_or_flag(&d2_full[s], ((uint32_t)(i - 2) >> 1) & 1u, err, 11)) {
-        alive = false;   // GEMM2 of tile i-2, the last reader of D1[s], has completed
-        break;
-      }
-      tc::tc_after_sync();
-      const uint32_t A = tmem + (uint32_t)(3 * C * s), D = tmem + TD1 + (uint32_t)(C * s);
-#pragma unroll 1
-      for (int k = 0; k < 3 * C / 16; ++k)
-        mma3_ta(D, A + 8u * k, A + 3 * C / 2 + 8u * k, tc::kmajor_desc(w1 + 256u * k, 128u, 3 * C * 16u),
-                tc::kmajor_desc(w1 + B1 / 2 + 256u * k, 128u, 3 * C * 16u), i1, k > 0);
-      tc::mma_commit(&d1_full[s]);
-      last = &d1_full[s];
-      last_par = n & 1u;
-      if (i >= 1) {
-        if (!wait_or_flag(&h_full[(i - 1) & 1], ((uint32_t)(i - 1) >> 1) & 1u, err, 5)) { alive = false; break; }
+      if (i >= 2 && !wait_or_flag(&d2_full[s], ((uint32_t)(i - 2) >> 1) & 1u, err, 11)) break;
+      // GEMM2 of tile i - 2, the last reader of D1[s], has completed
+      const uint32_t D = tmem + TD1 + (uint32_t)(C * s);
+      for (int ph = 0; ph < NPH; ++ph) {   // GEMM1, phase by phase as the slots fill
+        const int u = i * NPH + ph, sl = u % NSL;
+        const uint32_t n = (uint32_t)(u / NSL) & 1u;
+        if (!wait_or_flag(&sl_full[sl], n, err, 4)) {
+          alive = false;
+          break;
+        }
         tc::tc_after_sync();
-        gemm2(i - 1);
+        const uint32_t A = tmem + 32u * sl;
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          const uint32_t k = (uint32_t)(2 * ph + kk);
+          mma3_ta(D, A + 8u * kk, A + 16u + 8u * kk, tc::kmajor_desc(w1 + 256u * k, 128u, 3 * C * 16u),
+                  tc::kmajor_desc(w1 + B1 / 2 + 256u * k, 128u, 3 * C * 16u), i1, k > 0);
+        }
+        commit(&sl_empty[sl], n);
       }
-    }
-    if (alive && niter >= 1) {
-      const int j = niter - 1;
-      if (wait_or_flag(&h_full[j & 1], ((uint32_t)j >> 1) & 1u, err, 6)) {
-        tc::tc_after_sync();
-        gemm2(j);
-      }
+      if (!alive) break;
+      commit(&d1_full[s], ((uint32_t)i >> 1) & 1u);
+      if (i >= 1 && !gemm2(i - 1)) alive = false;
+      if (i == niter - 1 && alive) gemm2(i);
     }
     if (last) tc::mbar_wait_for(last, last_par, WAIT_NS);   // no MMA in flight when tensor memory is freed
   } else if (ok && warp >= W_CVT && warp < F_E1) {
@@ -942,17 +950,16 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     bool alive = true;
     for (int i = 0; i < niter && alive; ++i) {
-      const int s = i & 1;
-      if (!warp_wait(&a_empty[s], (((uint32_t)i >> 1) & 1u) ^ 1u, err, 7)) break;   // D2 of tile i-2 read
-      tc::tc_after_sync();
-      const uint32_t A = tmem + lq + (uint32_t)(3 * C * s);
       for (int ph = 0; ph < NPH; ++ph) {
         const int u = i * NPH + ph, st = u % NS;
         if ((u & 1) != grp) continue;   // alternate phases; four stages, so a stage's uses all go to one group
-        if (!warp_wait(&stg_full[st], (uint32_t)(u / NS) & 1u, err, 8)) {
+        const int sl = u % NSL;
+        if (!warp_wait(&sl_empty[sl], ((uint32_t)(u / NSL) & 1u) ^ 1u, err, 7) ||   // GEMM1 has read the slot
+            !warp_wait(&stg_full[st], (uint32_t)(u / NS) & 1u, err, 8)) {
           alive = false;
           break;
         }
+        tc::tc_after_sync();
         const int t = ph / NB, c0 = 32 * (ph % NB);
         const uint8_t* rp = ring + st * SB + r * 128;
         uint32_t hi[16], lo[16];
@@ -974,14 +981,13 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
           tc::split_pack(y[2], y[3], hi[2 * cc + 1], lo[2 * cc + 1]);
         }
         tc::mbar_arrive(&stg_empty[st]);
-        const uint32_t kc = (uint32_t)((t * C + c0) / 2);
-        tc::tmem_st16u(A + kc, hi);
-        tc::tmem_st16u(A + (uint32_t)(3 * C / 2) + kc, lo);
+        const uint32_t A = tmem + lq + 32u * sl;
+        tc::tmem_st16u(A, hi);
+        tc::tmem_st16u(A + 16u, lo);
+        tc::tmem_wait_st();
+        tc::tc_before_sync();
+        tc::mbar_arrive(&sl_full[sl]);
       }
-      if (!alive) break;
-      tc::tmem_wait_st();
-      tc::tc_before_sync();
-      tc::mbar_arrive(&a_full[s]);
     }
   } else if (ok && warp >= F_E1 && warp < F_E2) {
     const int q = warp & 3, hf = (warp - F_E1) >> 2, r = 32 * q + lane;
@@ -1026,15 +1032,15 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
       const long v = tile_of(i) * TM + r;
       if (!warp_wait(&d2_full[s], ((uint32_t)i >> 1) & 1u, err, 10)) break;
       tc::tc_after_sync();
-      const uint32_t D = tmem + lq + (uint32_t)(3 * C * s);
+      const uint32_t D = tmem + lq + TD2 + (uint32_t)(2 * C * s);
 #pragma unroll
       for (int k = 0; k < 2 * C / 16; ++k) {
         uint32_t d[16];
         tc::tmem_ld16u(D + 16u * k, d);
         tc::tmem_wait_ld();
-        if (k == 2 * C / 16 - 1) {   // the A stage is free once D2 is in registers
+        if (k == 2 * C / 16 - 1) {   // D2[s] is free once its last columns are in registers
           tc::tc_before_sync();
-          tc::mbar_arrive(&a_empty[s]);
+          tc::mbar_arrive(&d2_free[s]);
         }
         if (v < V) {
           float o[16];
@@ -1072,13 +1078,15 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
   constexpr uint32_t WB = B1 + B2;
   constexpr int NB = C / 32, NPH = 2 * NB, NS = 3, CPG = C / GMAX;
   constexpr uint32_t SB = 2 * BOX_BYTES;         // one ring stage: a pre box and its gates box
-  constexpr uint32_t TA = 0, TD1 = 4 * C, TD2 = 6 * C;
+  constexpr int NSL = 4;                         // A slots of one phase (a slot's uses all go to one group)
+  constexpr uint32_t TD1 = 32 * NSL, TD2 = TD1 + 4 * C;
+  static_assert(TD2 + 2 * C <= 512, "tensor memory");
   static_assert(WB % 1024 == 0, "the ring must stay 1024-byte aligned (128-byte swizzle)");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* ring = smem + WB;
-  __shared__ uint64_t stg_full[NS], stg_empty[NS], a_full[2], a_empty[2], d2_free[2], d2_full[2], d1_full, h_full,
-      wbar;
+  __shared__ uint64_t stg_full[NS], stg_empty[NS], sl_full[NSL], sl_empty[NSL], d2_free[2], d2_full[2], d1_full[2],
+      h_full[2], wbar;
   __shared__ uint32_t tslot;
   __shared__ float cf[2][3 * C];              // GroupNorm coefficients of spec and vert: mean, gamma rstd, beta
   __shared__ double acc[4][GMAX][3];          // the epilogue-2 warps' statistics
@@ -1090,13 +1098,15 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
       tc::mbar_init(&stg_empty[s], 256);
     }
     for (int s = 0; s < 2; ++s) {
-      tc::mbar_init(&a_full[s], NB == 1 ? 128 : 256);
-      tc::mbar_init(&a_empty[s], 1);
       tc::mbar_init(&d2_free[s], 128);
       tc::mbar_init(&d2_full[s], 1);
+      tc::mbar_init(&d1_full[s], 1);
+      tc::mbar_init(&h_full[s], 256);
     }
-    tc::mbar_init(&d1_full, 1);
-    tc::mbar_init(&h_full, 256);
+    for (int s = 0; s < NSL; ++s) {
+      tc::mbar_init(&sl_full[s], 128);
+      tc::mbar_init(&sl_empty[s], 1);
+    }
     tc::mbar_init(&wbar, 1);
     tc::mbar_init_fence();
   }
@@ -1148,47 +1158,49 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
     uint64_t* last = nullptr;
     uint32_t last_par = 0;
     bool alive = true;
-    auto gemm2 = [&](int j) {   // D2[j % 2] += H(j) Wf2^T, H in D1 as [hi 8 | lo 8] per 16-wide k chunk, K = 2C
+    auto commit = [&](uint64_t* bar, uint32_t par) {
+      tc::mma_commit(bar);
+      last = bar;
+      last_par = par;
+    };
+    auto gemm2 = [&](int j) {   // D2[j % 2] += H(j) Wf2^T, H in D1[j % 2] as [hi 8 | lo 8] per 16-wide k chunk, K = 2C
+      if (!wait_or_flag(&h_full[j & 1], ((uint32_t)j >> 1) & 1u, err, 5)) return false;
+      tc::tc_after_sync();
+      const uint32_t h = tmem + TD1 + (uint32_t)(2 * C * (j & 1));
 #pragma unroll 1
       for (int k = 0; k < 2 * C / 16; ++k)
-        mma3_ta(tmem + TD2 + (uint32_t)(C * (j & 1)), tmem + TD1 + 16u * k, tmem + TD1 + 16u * k + 8u,
+        mma3_ta(tmem + TD2 + (uint32_t)(C * (j & 1)), h + 16u * k, h + 16u * k + 8u,
                 tc::kmajor_desc(w2 + 256u * k, 128u, 2 * C * 16u),
                 tc::kmajor_desc(w2 + B2 / 2 + 256u * k, 128u, 2 * C * 16u), i2, true);
-      tc::mma_commit(&d2_full[j & 1]);
-      last = &d2_full[j & 1];
-      last_par = ((uint32_t)j >> 1) & 1u;
+      commit(&d2_full[j & 1], ((uint32_t)j >> 1) & 1u);
+      return true;
     };
     for (int i = 0; i < niter && alive; ++i) {
       const int s = i & 1;
-      if (!wait_or_flag(&a_full[s], ((uint32_t)i >> 1) & 1u, err, 4)) {
-        alive = false;
-        break;
-      }
-      if (i >= 1) {   // GEMM2 of the previous tile reads D1 before GEMM1 of this one overwrites it
-        if (!wait_or_flag(&h_full, (uint32_t)(i - 1) & 1u, err, 5)) {
+      if (i >= 2 && !wait_or_flag(&d2_full[s], ((uint32_t)(i - 2) >> 1) & 1u, err, 11)) break;
+      // GEMM2 of tile i - 2, the last reader of D1[s], has completed
+      const uint32_t D = tmem + TD1 + (uint32_t)(2 * C * s);
+      for (int ph = 0; ph < NPH; ++ph) {   // GEMM1, phase by phase as the slots fill
+        const int u = i * NPH + ph, sl = u % NSL;
+        const uint32_t n = (uint32_t)(u / NSL) & 1u;
+        if (!wait_or_flag(&sl_full[sl], n, err, 4)) {
           alive = false;
           break;
         }
         tc::tc_after_sync();
-        gemm2(i - 1);
+        const uint32_t A = tmem + 32u * sl;
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          const uint32_t k = (uint32_t)(2 * ph + kk);
+          mma3_ta(D, A + 8u * kk, A + 16u + 8u * kk, tc::kmajor_desc(w1 + 256u * k, 128u, 2 * C * 16u),
+                  tc::kmajor_desc(w1 + B1 / 2 + 256u * k, 128u, 2 * C * 16u), i1, k > 0);
+        }
+        commit(&sl_empty[sl], n);
       }
-      tc::tc_after_sync();
-      const uint32_t A = tmem + TA + (uint32_t)(2 * C * s);
-#pragma unroll 1
-      for (int k = 0; k < 2 * C / 16; ++k)
-        mma3_ta(tmem + TD1, A + 8u * k, A + C + 8u * k, tc::kmajor_desc(w1 + 256u * k, 128u, 2 * C * 16u),
-                tc::kmajor_desc(w1 + B1 / 2 + 256u * k, 128u, 2 * C * 16u), i1, k > 0);
-      tc::mma_commit(&d1_full);
-      tc::mma_commit(&a_empty[s]);
-      last = &a_empty[s];
-      last_par = ((uint32_t)i >> 1) & 1u;
-    }
-    if (alive && niter >= 1) {
-      const int j = niter - 1;
-      if (wait_or_flag(&h_full, (uint32_t)j & 1u, err, 6)) {
-        tc::tc_after_sync();
-        gemm2(j);
-      }
+      if (!alive) break;
+      commit(&d1_full[s], ((uint32_t)i >> 1) & 1u);
+      if (i >= 1 && !gemm2(i - 1)) alive = false;
+      if (i == niter - 1 && alive) gemm2(i);
     }
     if (last) tc::mbar_wait_for(last, last_par, WAIT_NS);   // no MMA in flight when tensor memory is freed
   } else if (ok && warp >= W_CVT && warp < F_E1) {
@@ -1204,10 +1216,9 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
       // for its own uses only could take an earlier use's phase for its own (the parities repeat every two uses) when
       // the copies of two stages land out of order.
       const bool mine = NB > 1 || (i & 1) == grp;
-      if (mine && !warp_wait(&a_empty[s], n2 ^ 1u, err, 7)) break;    // GEMM1 of tile i-2 has read the A stage
       if (mine && !warp_wait(&d2_free[s], n2 ^ 1u, err, 8)) break;    // epilogue 2 of tile i-2 has read D2[s]
       tc::tc_after_sync();
-      const uint32_t A = tmem + lq + TA + (uint32_t)(2 * C * s), D2 = tmem + lq + TD2 + (uint32_t)(C * s);
+      const uint32_t D2 = tmem + lq + TD2 + (uint32_t)(C * s);
       for (int ph = 0; ph < NPH; ++ph) {
         const int u = i * NPH + ph, st = u % NS;
         if (!warp_wait(&stg_full[st], (uint32_t)(u / NS) & 1u, err, 12)) {
@@ -1218,6 +1229,12 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
           tc::mbar_arrive(&stg_empty[st]);
           continue;
         }
+        const int sl = u % NSL;
+        if (!warp_wait(&sl_empty[sl], ((uint32_t)(u / NSL) & 1u) ^ 1u, err, 7)) {   // GEMM1 has read the slot
+          alive = false;
+          break;
+        }
+        tc::tc_after_sync();
         const int br = ph / NB, c0 = 32 * (ph % NB);   // branch (0 spec, 1 vert) and its first channel
         const float* k = cf[br];
         const uint8_t* rp = ring + st * SB + r * 128;
@@ -1242,9 +1259,8 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) tc::split_pack(b[2 * e], b[2 * e + 1], hi[e], lo[e]);
-        const uint32_t kc = (uint32_t)((br * C + c0) / 2);   // first column of this phase's channel pairs
-        tc::tmem_st16u(A + kc, hi);
-        tc::tmem_st16u(A + (uint32_t)C + kc, lo);
+        tc::tmem_st16u(tmem + lq + 32u * sl, hi);
+        tc::tmem_st16u(tmem + lq + 32u * sl + 16u, lo);
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {   // residual (B[c] + B[C + c]) / 2 in D2
           float rr[16];
@@ -1258,20 +1274,19 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
           }
           tc::tmem_st16(D2 + (uint32_t)(c0 + 16 * hh), rr);
         }
+        tc::tmem_wait_st();
+        tc::tc_before_sync();
+        tc::mbar_arrive(&sl_full[sl]);
       }
-      if (!alive) break;
-      if (!mine) continue;
-      tc::tmem_wait_st();
-      tc::tc_before_sync();
-      tc::mbar_arrive(&a_full[s]);
     }
   } else if (ok && warp >= F_E1 && warp < F_E2) {
     const int q = warp & 3, hf = (warp - F_E1) >> 2;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     for (int i = 0; i < niter; ++i) {
-      if (!warp_wait(&d1_full, (uint32_t)i & 1u, err, 9)) break;
+      const int s = i & 1;
+      if (!warp_wait(&d1_full[s], ((uint32_t)i >> 1) & 1u, err, 9)) break;
       tc::tc_after_sync();
-      const uint32_t D = tmem + lq + TD1;
+      const uint32_t D = tmem + lq + TD1 + (uint32_t)(2 * C * s);
 #pragma unroll 1
       for (int j = hf; j < 2 * C / 16; j += 2) {
         uint32_t h[16];
@@ -1289,7 +1304,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
       }
       tc::tmem_wait_st();
       tc::tc_before_sync();
-      tc::mbar_arrive(&h_full);
+      tc::mbar_arrive(&h_full[s]);
     }
   } else if (ok && warp >= F_E2) {
     const int q = warp & 3, r = 32 * q + lane, wl = warp - F_E2;
