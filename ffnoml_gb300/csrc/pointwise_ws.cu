@@ -807,7 +807,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // 3 NB phases of 32 channels per tile (x, spec_pre, vert_pre boxes) through a four-stage ring; warp 1 MMA: GEMM1
 // D1[t % 2] = A Wg1^T (N = C), and GEMM2 D2 = H Wg2^T (N = 2C) one tile behind, over the tile's A stage; warps 2-5
 // conversion; warps 6-13 epilogue 1: hg to HBM, H = gelu(D1) split over D1; warps 14-17 epilogue 2: the gates.
-// Tensor memory: A stages of 3C columns at 0 and 3C, D1 buffers at 6C and 7C.
+// Tensor memory: four A slots of one phase (16 columns hi, 16 lo) at 0, two D1 buffers (C) behind them, two D2 buffers
+// (2C). GEMM1 takes each phase as its slot fills, so conversion, GEMM1, epilogue 1, GEMM2 and epilogue 2 of neighbouring
+// tiles overlap. 4.2 M voxels, C = 64: 1.34 ms (2.22 with a whole tile's operand per stage and one conversion group).
 template <int C>
 __global__ void __launch_bounds__(F_NTHREADS, 1)
     k_fuse1_ws(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_sp,
@@ -1065,8 +1067,10 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
 // matching gates box, through a three-stage ring; warp 1 MMA: GEMM1 D1 = B Wf1^T (N = K = 2C) and, one tile behind,
 // GEMM2 D2 += H Wf2^T (N = C); warps 2-5 conversion: B split into the tile's A stage and the FP32 residual
 // (B[:, c] + B[:, C + c]) / 2 into its D2 buffer (GEMM2 accumulates onto it); warps 6-13 epilogue 1: H = gelu(D1),
-// split over D1; warps 14-17 epilogue 2: pre and its statistics, as in the forward MLP. Tensor memory (8C columns):
-// A stages at 0 and 2C, D1 at 4C, D2 buffers at 6C and 7C.
+// split over D1; warps 14-17 epilogue 2: pre and its statistics, as in the forward MLP. Tensor memory: A slots
+// of one phase (32 columns each), two D1 buffers (2C), three D2 buffers (C). GEMM1 takes each phase as its slot fills; a
+// tile's residual needs its D2 buffer free, so with three of them conversion runs up to two tiles ahead of epilogue 2.
+// 4.2 M voxels, C = 64: 1.42 ms (1.95 with a whole tile's operand per stage, one D1 and one conversion group).
 template <int C>
 __global__ void __launch_bounds__(F_NTHREADS, 1)
     k_fuse2_ws(const __grid_constant__ CUtensorMap map_sp, const __grid_constant__ CUtensorMap map_vp,
@@ -1078,14 +1082,15 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
   constexpr uint32_t WB = B1 + B2;
   constexpr int NB = C / 32, NPH = 2 * NB, NS = 3, CPG = C / GMAX;
   constexpr uint32_t SB = 2 * BOX_BYTES;         // one ring stage: a pre box and its gates box
-  constexpr int NSL = 4;                         // A slots of one phase (a slot's uses all go to one group)
+  constexpr int NSL = NB == 1 ? 4 : 2;           // A slots of one phase (a slot's uses all go to one group)
+  constexpr int ND2 = 3;                         // D2 buffers: conversion of a tile writes its residual three ahead
   constexpr uint32_t TD1 = 32 * NSL, TD2 = TD1 + 4 * C;
-  static_assert(TD2 + 2 * C <= 512, "tensor memory");
+  static_assert(TD2 + ND2 * C <= 512, "tensor memory");
   static_assert(WB % 1024 == 0, "the ring must stay 1024-byte aligned (128-byte swizzle)");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* ring = smem + WB;
-  __shared__ uint64_t stg_full[NS], stg_empty[NS], sl_full[NSL], sl_empty[NSL], d2_free[2], d2_full[2], d1_full[2],
+  __shared__ uint64_t stg_full[NS], stg_empty[NS], sl_full[NSL], sl_empty[NSL], d2_free[ND2], d2_full[ND2], d1_full[2],
       h_full[2], wbar;
   __shared__ uint32_t tslot;
   __shared__ float cf[2][3 * C];              // GroupNorm coefficients of spec and vert: mean, gamma rstd, beta
@@ -1098,10 +1103,12 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
       tc::mbar_init(&stg_empty[s], 256);
     }
     for (int s = 0; s < 2; ++s) {
-      tc::mbar_init(&d2_free[s], 128);
-      tc::mbar_init(&d2_full[s], 1);
       tc::mbar_init(&d1_full[s], 1);
       tc::mbar_init(&h_full[s], 256);
+    }
+    for (int s = 0; s < ND2; ++s) {
+      tc::mbar_init(&d2_free[s], 128);
+      tc::mbar_init(&d2_full[s], 1);
     }
     for (int s = 0; s < NSL; ++s) {
       tc::mbar_init(&sl_full[s], 128);
@@ -1163,21 +1170,21 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
       last = bar;
       last_par = par;
     };
-    auto gemm2 = [&](int j) {   // D2[j % 2] += H(j) Wf2^T, H in D1[j % 2] as [hi 8 | lo 8] per 16-wide k chunk, K = 2C
+    auto gemm2 = [&](int j) {   // D2[j % ND2] += H(j) Wf2^T, H in D1[j % 2] as [hi 8 | lo 8] per 16-wide k chunk, K = 2C
       if (!wait_or_flag(&h_full[j & 1], ((uint32_t)j >> 1) & 1u, err, 5)) return false;
       tc::tc_after_sync();
       const uint32_t h = tmem + TD1 + (uint32_t)(2 * C * (j & 1));
 #pragma unroll 1
       for (int k = 0; k < 2 * C / 16; ++k)
-        mma3_ta(tmem + TD2 + (uint32_t)(C * (j & 1)), h + 16u * k, h + 16u * k + 8u,
+        mma3_ta(tmem + TD2 + (uint32_t)(C * (j % ND2)), h + 16u * k, h + 16u * k + 8u,
                 tc::kmajor_desc(w2 + 256u * k, 128u, 2 * C * 16u),
                 tc::kmajor_desc(w2 + B2 / 2 + 256u * k, 128u, 2 * C * 16u), i2, true);
-      commit(&d2_full[j & 1], ((uint32_t)j >> 1) & 1u);
+      commit(&d2_full[j % ND2], (uint32_t)(j / ND2) & 1u);
       return true;
     };
     for (int i = 0; i < niter && alive; ++i) {
       const int s = i & 1;
-      if (i >= 2 && !wait_or_flag(&d2_full[s], ((uint32_t)(i - 2) >> 1) & 1u, err, 11)) break;
+      if (i >= 2 && !wait_or_flag(&d2_full[(i - 2) % ND2], (uint32_t)((i - 2) / ND2) & 1u, err, 11)) break;
       // GEMM2 of tile i - 2, the last reader of D1[s], has completed
       const uint32_t D = tmem + TD1 + (uint32_t)(2 * C * s);
       for (int ph = 0; ph < NPH; ++ph) {   // GEMM1, phase by phase as the slots fill
@@ -1208,15 +1215,15 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     bool alive = true;
     for (int i = 0; i < niter && alive; ++i) {
-      const int s = i & 1;
-      const uint32_t n2 = ((uint32_t)i >> 1) & 1u;
+      const int s = i % ND2;
+      const uint32_t n2 = (uint32_t)(i / ND2) & 1u;
       // the groups take alternate channel phases (both branches of a channel, whose residual meets in D2), or, with
       // one phase a branch (C = 32), alternate tiles. Three stages for two groups: consecutive uses of a stage go to
       // different groups, so each group waits for every use of every stage and releases it too. A group that waited
       // for its own uses only could take an earlier use's phase for its own (the parities repeat every two uses) when
       // the copies of two stages land out of order.
       const bool mine = NB > 1 || (i & 1) == grp;
-      if (mine && !warp_wait(&d2_free[s], n2 ^ 1u, err, 8)) break;    // epilogue 2 of tile i-2 has read D2[s]
+      if (mine && !warp_wait(&d2_free[s], n2 ^ 1u, err, 8)) break;    // epilogue 2 of tile i - ND2 has read D2[s]
       tc::tc_after_sync();
       const uint32_t D2 = tmem + lq + TD2 + (uint32_t)(C * s);
       for (int ph = 0; ph < NPH; ++ph) {
@@ -1311,11 +1318,11 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     ShiftAcc stat;
     for (int i = 0; i < niter; ++i) {
-      const int s = i & 1;
+      const int s = i % ND2;
       const long v = tile_of(i) * TM + r;
       const bool live = v < V;
       const float w = live ? __ldg(dw + v) : 0.f;
-      if (!warp_wait(&d2_full[s], ((uint32_t)i >> 1) & 1u, err, 10)) break;
+      if (!warp_wait(&d2_full[s], (uint32_t)(i / ND2) & 1u, err, 10)) break;
       tc::tc_after_sync();
       const uint32_t D = tmem + lq + TD2 + (uint32_t)(C * s);
       float gs[GMAX];
@@ -1360,7 +1367,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
         }
       }
       tc::tc_before_sync();
-      tc::mbar_arrive(&d2_free[s]);   // D2[s] has been read: conversion may write the residual of tile i + 2
+      tc::mbar_arrive(&d2_free[s]);   // D2[s] has been read: conversion may write the residual of tile i + ND2
 #pragma unroll
       for (int g = 0; g < GMAX; ++g) gs[g] *= w;
       stat.add(wt, mean, warp_group_sum(gs));
