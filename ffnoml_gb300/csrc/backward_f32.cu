@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats(int mode, const float* __r
                                                       const float* __restrict__ beta,
                                                       const double* __restrict__ gst, long V,
                                                       double* __restrict__ partials, int nparts, int cpg, int groups) {
+  griddep_sync();
   using Ln = GnLanes<C, 4>;
   __shared__ GnConst k;
   load_gn_const(k, gst, nullptr, groups, 0.f);
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats8(int mode, const float* __
                                                        const float* __restrict__ beta,
                                                        const double* __restrict__ gst, long V,
                                                        double* __restrict__ partials, int nparts) {
+  griddep_sync();
   static_assert(C == 16 || C == 32 || C == 64, "eight groups of C / 8 channels");
   using Ln = GnLanes<C, 8>;
   constexpr int VW = 8, CPG = C / GMAX, NG = VW / CPG;
@@ -268,6 +270,7 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats8(int mode, const float* __
 }
 
 __global__ void k_gn_bwd_final(const double* __restrict__ partials, int nparts, int groups, double* __restrict__ sums) {
+  griddep_sync();
   // one warp per group: strided partial sums per lane, then a fixed shuffle tree (deterministic)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int g = warp; g < groups; g += nw) {
@@ -297,6 +300,7 @@ __global__ void __launch_bounds__(256, 4) k_gn_bwd_apply(int mode, const float* 
                                                       const float* __restrict__ dw, long V,
                                                       float* __restrict__ pre_bar, float* __restrict__ w_bar, int cpg,
                                                       int groups, float eps) {
+  griddep_sync();
   using Ln = GnLanes<C, 8>;
   __shared__ GnConst k;
   load_gn_const(k, gst, sums, groups, eps);
@@ -354,6 +358,7 @@ __global__ void __launch_bounds__(NT, 2) k_mlp2_bwd(const float* __restrict__ a,
                                                     const float* __restrict__ base, long V,
                                                     const float* __restrict__ w1, const float* __restrict__ w2t,
                                                     const float* __restrict__ w1t, float* __restrict__ abar, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   float* as = sm;   // [C][64] a, [C][64] pre_bar, then [2C][64] the hidden gradient
   g32::Ring ring(as + 2 * C * BM, g32::KC * 2 * C, al);
@@ -408,6 +413,7 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_fuse_bwd(
     const float* __restrict__ bg2, const float* __restrict__ wf1, const float* __restrict__ wf2t,
     const float* __restrict__ wf1t, const float* __restrict__ wg2t, const float* __restrict__ wg1t,
     float* __restrict__ xbar, float* __restrict__ sbar, float* __restrict__ vbar, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   float* X = sm;                 // channels 0 .. C - 1 of the region [x | spec | vert]
   float* T = X + 3 * C * BM;
@@ -554,6 +560,7 @@ __global__ void __launch_bounds__(NT, 3) k_gate_bwd(const float* __restrict__ x,
                                                  const float* __restrict__ v2t, const float* __restrict__ v1t,
                                                  const float* __restrict__ zp, float* __restrict__ xbar,
                                                  float* __restrict__ zbar, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   float* SX = sm;               // [C][64] x
   float* SB = SX + C * BM;      // [C][64] the branch's gradient
@@ -644,6 +651,7 @@ __global__ void __launch_bounds__(NT, 3) k_gate_bwd(const float* __restrict__ x,
 template <int C>
 __global__ void __launch_bounds__(NT) k_lift_bwd(const float* __restrict__ pb, int cin, long V,
                                                  const float* __restrict__ wl, float* __restrict__ xib) {
+  griddep_sync();
   __shared__ float ps[BM][C + 1];
   const long nt = ntiles(V, BM);
   for (long t = blockIdx.x; t < nt; t += gridDim.x) {
@@ -673,6 +681,7 @@ __global__ void __launch_bounds__(NT, 2) k_head_bwd(const float* __restrict__ x,
                                                  const float* __restrict__ p2t, const float* __restrict__ p1t,
                                                  const __grid_constant__ ffno_head_params hp, int nh,
                                                  float* __restrict__ xbar, float* __restrict__ xinbar, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1, N2 = 2 * C / 16;
@@ -756,6 +765,7 @@ __global__ void __launch_bounds__(256) k_head_output_bwd(const float* __restrict
                                                          const float* __restrict__ ybar, long V, int nh,
                                                          const __grid_constant__ ffno_head_params hp,
                                                          float* __restrict__ hbar, float* __restrict__ xinbar) {
+  griddep_sync();
   __shared__ double etab[EXP_TAB];
   fill_exp_table(etab);
   __syncthreads();
@@ -777,6 +787,7 @@ constexpr int DB_COLS = 32, DB_SEGS = 16;
 __global__ void __launch_bounds__(DB_COLS* DB_SEGS) k_depth_weights_bwd(const float* __restrict__ z,
                                                                         const float* __restrict__ wb, int D, long HW,
                                                                         float* __restrict__ zb) {
+  griddep_sync();
   __shared__ float part[2][DB_SEGS][DB_COLS];
   const int tx = threadIdx.x % DB_COLS, sg = threadIdx.x / DB_COLS;
   const long col = (long)blockIdx.x * DB_COLS + tx;
@@ -835,6 +846,7 @@ __global__ void __launch_bounds__(DB_COLS* DB_SEGS) k_depth_weights_bwd(const fl
 __global__ void __launch_bounds__(NT) k_outer(const float* __restrict__ A, long lda, int Ma,
                                               const float* __restrict__ B, long ldb, int Mb, long N, long chunk,
                                               int ti, int tj, float* __restrict__ part) {
+  griddep_sync();
   // 64 x 64 output tile, k in chunks of 64 read as float4 (16 threads per row: 256 contiguous bytes)
   __shared__ float as[64][65];
   __shared__ float bs[64][65];
@@ -915,6 +927,7 @@ constexpr int OR_EL = 32, OR_SEGS = 8;
 
 __global__ void __launch_bounds__(OR_EL* OR_SEGS) k_outer_reduce(const float* __restrict__ part, long nsplit, long n,
                                                                  double* __restrict__ out, int accumulate) {
+  griddep_sync();
   __shared__ double red[OR_SEGS][OR_EL];
   const int tx = threadIdx.x % OR_EL, sg = threadIdx.x / OR_EL;
   const long e = (long)blockIdx.x * OR_EL + tx;
@@ -948,7 +961,7 @@ int ffno_gn_bwd_stats(int mode, const float* u, float r, const float* pre, const
   if (groups == GMAX && C <= 64 &&
       (reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(pre)) % 32 == 0) {   // 32-byte lanes
     switch (C) {
-#define L(CC) case CC: k_gn_bwd_stats8<CC><<<grid, 256, 0, s>>>(mode, u, r, pre, gamma, beta, gstats, V, partials, nparts); break;
+#define L(CC) case CC: ffno::launch(k_gn_bwd_stats8<CC>, grid, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, V, partials, nparts); break;
       L(16) L(32) L(64)
 #undef L
     }
@@ -956,7 +969,7 @@ int ffno_gn_bwd_stats(int mode, const float* u, float r, const float* pre, const
     return FFNO_OK;
   }
   switch (C) {
-#define L(CC) case CC: k_gn_bwd_stats<CC><<<grid, 256, 0, s>>>(mode, u, r, pre, gamma, beta, gstats, V, partials, nparts, cpg, groups); break;
+#define L(CC) case CC: ffno::launch(k_gn_bwd_stats<CC>, grid, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, V, partials, nparts, cpg, groups); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -966,7 +979,7 @@ int ffno_gn_bwd_stats(int mode, const float* u, float r, const float* pre, const
 
 int ffno_gn_bwd_final(const double* partials, int nparts, int groups, double* sums, ffno_stream_t stream) {
   if (!partials || !sums || nparts < 1 || groups < 1 || groups > GMAX) return FFNO_EINVAL;
-  k_gn_bwd_final<<<1, 512, 0, (cudaStream_t)stream>>>(partials, nparts, groups, sums);
+  ffno::launch(k_gn_bwd_final, 1, 512, 0, (cudaStream_t)stream, partials, nparts, groups, sums);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -985,7 +998,7 @@ int ffno_gn_bwd_apply(int mode, const float* u, float r, const float* pre, const
   const int cpg = C / groups;
   const int blocks = grid_of(V, 8 * 8, 4);
   switch (C) {
-#define L(CC) case CC: k_gn_bwd_apply<CC><<<blocks, 256, 0, s>>>(mode, u, r, pre, gamma, beta, gstats, sums, dw, V, pre_bar, w_bar, cpg, groups, eps); break;
+#define L(CC) case CC: ffno::launch(k_gn_bwd_apply<CC>, blocks, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, sums, dw, V, pre_bar, w_bar, cpg, groups, eps); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -1003,7 +1016,7 @@ int ffno_mlp2_bwd(const float* a, const float* pre_bar, const float* base, long 
   case CC: {                                                                                    \
     const size_t smem = (2 * CC * BM + 2 * g32::KC * 2 * CC) * sizeof(float);                   \
     if (!smem_attr(k_mlp2_bwd<CC>, smem)) return FFNO_ELAUNCH;                                  \
-    k_mlp2_bwd<CC><<<grid_of(V, BM, 2), NT, smem, s>>>(a, pre_bar, base, V, w1, w2t, w1t, a_bar, al); \
+    ffno::launch(k_mlp2_bwd<CC>, grid_of(V, BM, 2), NT, smem, s, a, pre_bar, base, V, w1, w2t, w1t, a_bar, al); \
     break;                                                                                      \
   }
     L(16) L(32) L(64) L(96)
@@ -1030,7 +1043,7 @@ int ffno_fuse_bwd(const float* x, const float* spec_pre, const float* spec_coefs
   case CC: {                                                                                                \
     const size_t smem = fuse_bwd_smem<CC>();                                                                \
     if (!smem_attr(k_fuse_bwd<CC>, smem)) return FFNO_ELAUNCH;                                              \
-    k_fuse_bwd<CC><<<grid_of(V, BM, CC <= 64 ? 2 : 1), NT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre,     \
+    ffno::launch(k_fuse_bwd<CC>, grid_of(V, BM, CC <= 64 ? 2 : 1), NT, smem, s, x, spec_pre, spec_coefs, vert_pre,     \
                                                                       vert_coefs, fused_pre_bar, base, V,   \
                                                                       wg1, wg2, bg2, wf1, wf2t, wf1t, wg2t, \
                                                                       wg1t, x_bar, spec_bar, vert_bar, al); \
@@ -1057,7 +1070,7 @@ int ffno_gate_bwd(const float* x, const float* xs_bar, const float* xv_bar, cons
   case CC: {                                                                                               \
     const size_t smem = (3 * CC * BM + 2 * g32::KC * CC) * sizeof(float);                                  \
     if (!smem_attr(k_gate_bwd<CC>, smem)) return FFNO_ELAUNCH;                                             \
-    k_gate_bwd<CC><<<grid_of(V, BM, 3), NT, smem, s>>>(x, xs_bar, xv_bar, base, V, s_w1, s_w2, s_w2t, s_w1t, \
+    ffno::launch(k_gate_bwd<CC>, grid_of(V, BM, 3), NT, smem, s, x, xs_bar, xv_bar, base, V, s_w1, s_w2, s_w2t, s_w1t, \
                                                        v_w1, v_w2, v_w2t, v_w1t, zp, x_bar, z_bar, al);     \
     break;                                                                                                 \
   }
@@ -1073,7 +1086,7 @@ int ffno_lift_bwd(const float* pre_bar, int cin, long V, int C, const float* w_l
   if (!pre_bar || !w_lift || !x_in_bar || !width_ok(C) || V < 1 || cin < 1 || cin > 8) return FFNO_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
-#define L(CC) case CC: k_lift_bwd<CC><<<grid_of(V, BM, 4), NT, 0, s>>>(pre_bar, cin, V, w_lift, x_in_bar); break;
+#define L(CC) case CC: ffno::launch(k_lift_bwd<CC>, grid_of(V, BM, 4), NT, 0, s, pre_bar, cin, V, w_lift, x_in_bar); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -1095,11 +1108,11 @@ int ffno_head_bwd(const float* x, const float* x_in, const float* y_bar, long V,
     const size_t smem = (2 * CC * BM + NN * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);  \
     if (params->math32) {                                                                               \
       if (!smem_attr(k_head_bwd<CC, NN, float>, smem)) return FFNO_ELAUNCH;                             \
-      k_head_bwd<CC, NN, float><<<grid_of(V, BM, 2), NT, smem, s>>>(x, x_in, y_bar, V, p1, p2, b2, p2t, p1t, \
+      ffno::launch(k_head_bwd<CC, NN, float>, grid_of(V, BM, 2), NT, smem, s, x, x_in, y_bar, V, p1, p2, b2, p2t, p1t, \
                                                                     *params, NN, x_bar, x_in_bar, al);      \
     } else {                                                                                            \
       if (!smem_attr(k_head_bwd<CC, NN, double>, smem)) return FFNO_ELAUNCH;                            \
-      k_head_bwd<CC, NN, double><<<grid_of(V, BM, 2), NT, smem, s>>>(x, x_in, y_bar, V, p1, p2, b2, p2t, p1t, \
+      ffno::launch(k_head_bwd<CC, NN, double>, grid_of(V, BM, 2), NT, smem, s, x, x_in, y_bar, V, p1, p2, b2, p2t, p1t, \
                                                                      *params, NN, x_bar, x_in_bar, al);     \
     }                                                                                                   \
   }
@@ -1113,7 +1126,7 @@ int ffno_head_bwd(const float* x, const float* x_in, const float* y_bar, long V,
 
 int ffno_depth_weights_bwd(const float* z, const float* w_bar, int D, long HW, float* z_bar, ffno_stream_t stream) {
   if (!z || !w_bar || !z_bar || D < 1 || HW < 1) return FFNO_EINVAL;
-  k_depth_weights_bwd<<<(unsigned)((HW + DB_COLS - 1) / DB_COLS), DB_COLS * DB_SEGS, 0, (cudaStream_t)stream>>>(
+  ffno::launch(k_depth_weights_bwd, (unsigned)((HW + DB_COLS - 1) / DB_COLS), DB_COLS * DB_SEGS, 0, (cudaStream_t)stream, 
       z, w_bar, D, HW, z_bar);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -1137,9 +1150,9 @@ int ffno_outer(const float* A, long lda, int Ma, const float* B, long ldb, int M
   long chunk = (N + nsplit - 1) / nsplit;
   chunk = (chunk + 63) / 64 * 64;
   cudaStream_t s = (cudaStream_t)stream;
-  k_outer<<<(unsigned)((long)ti * tj * nsplit), NT, 0, s>>>(A, lda, Ma, B, ldb, Mb, N, chunk, ti, tj, part);
+  ffno::launch(k_outer, (unsigned)((long)ti * tj * nsplit), NT, 0, s, A, lda, Ma, B, ldb, Mb, N, chunk, ti, tj, part);
   const long n = (long)Ma * Mb;
-  k_outer_reduce<<<(unsigned)((n + OR_EL - 1) / OR_EL), OR_EL * OR_SEGS, 0, s>>>(part, nsplit, n, out, accumulate);
+  ffno::launch(k_outer_reduce, (unsigned)((n + OR_EL - 1) / OR_EL), OR_EL * OR_SEGS, 0, s, part, nsplit, n, out, accumulate);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -1192,8 +1205,8 @@ int ffno_outer_noalloc(const float* A, long lda, int Ma, const float* B, long ld
   chunk = (chunk + 63) / 64 * 64;
   cudaStream_t s = (cudaStream_t)stream;
   // every partial sum the reduction reads is written first by k_outer: nothing in the scratch has to start at zero
-  k_outer<<<(unsigned)((long)ti * tj * nsplit), NT, 0, s>>>(A, lda, Ma, B, ldb, Mb, N, chunk, ti, tj, scratch);
-  k_outer_reduce<<<(unsigned)((n + OR_EL - 1) / OR_EL), OR_EL * OR_SEGS, 0, s>>>(scratch, nsplit, n, out, accumulate);
+  ffno::launch(k_outer, (unsigned)((long)ti * tj * nsplit), NT, 0, s, A, lda, Ma, B, ldb, Mb, N, chunk, ti, tj, scratch);
+  ffno::launch(k_outer_reduce, (unsigned)((n + OR_EL - 1) / OR_EL), OR_EL * OR_SEGS, 0, s, scratch, nsplit, n, out, accumulate);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -1211,7 +1224,7 @@ int ffno_proj_bwd(const float* x, const float* head_bar, long V, int C, const fl
   if (C == CC && nhp == NN) {                                                                            \
     const size_t smem = (2 * CC * BM + NN * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);  \
     if (!smem_attr(k_head_bwd<CC, NN, float, false>, smem)) return FFNO_ELAUNCH;                         \
-    k_head_bwd<CC, NN, float, false><<<grid_of(V, BM, 2), NT, smem, s>>>(x, nullptr, head_bar, V, p1, p2, b2, \
+    ffno::launch(k_head_bwd<CC, NN, float, false>, grid_of(V, BM, 2), NT, smem, s, x, nullptr, head_bar, V, p1, p2, b2, \
                                                                          p2t, p1t, none, nh, x_bar, nullptr, al); \
   }
     default:
@@ -1238,9 +1251,9 @@ int ffno_head_output_bwd(const float* head, const float* x_in, const float* y_ba
   const long want = (V + 255) / 256, cap = 8L * sms();   // 8 CTAs of 256 threads per SM, grid-stride
   const long blocks = want < cap ? want : cap;
   if (params->math32)
-    k_head_output_bwd<float><<<(unsigned)blocks, 256, 0, s>>>(head, x_in, y_bar, V, nh, *params, head_bar, x_in_bar);
+    ffno::launch(k_head_output_bwd<float>, (unsigned)blocks, 256, 0, s, head, x_in, y_bar, V, nh, *params, head_bar, x_in_bar);
   else
-    k_head_output_bwd<double><<<(unsigned)blocks, 256, 0, s>>>(head, x_in, y_bar, V, nh, *params, head_bar,
+    ffno::launch(k_head_output_bwd<double>, (unsigned)blocks, 256, 0, s, head, x_in, y_bar, V, nh, *params, head_bar,
                                                                x_in_bar);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;

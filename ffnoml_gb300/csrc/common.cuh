@@ -733,6 +733,35 @@ inline bool smem_cap_ok(K kernel, size_t bytes) {
   return bytes <= cap;
 }
 
+// Programmatic dependent launch. The model kernels are launched with it allowed (launch below): the next kernel
+// of the stream is set up and its CTAs placed while this one drains, which takes the 2-3 us between two dependent
+// kernels (half of a small cube's kernels last 5-25 us) down to about 1. A kernel touches global memory only after
+// griddep_wait, which returns once the kernel before it in the stream has completed with its writes visible; it lets
+// its own successor be placed only after that (and, where it owns tensor memory, after it has allocated it: a placed
+// successor never holds what its predecessor still needs). With every kernel waiting for its predecessor, completion
+// stays in stream order. Kernels of other libraries before or after see ordinary stream order.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_sync() {
+  griddep_wait();
+  griddep_launch();
+}
+
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // its error is read by FFNO_CHECK_LAUNCH
+}
+
 }  // namespace ffno
 
 #define FFNO_CHECK_LAUNCH()                                   \

@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(HT) k_percol_tables(const double* __restrict__
                                                       const double* __restrict__ f, float* __restrict__ tzf,
                                                       float* __restrict__ tzi, float* __restrict__ tzf_t,
                                                       float* __restrict__ tzi_t) {
+  ffno::griddep_sync();
   extern __shared__ double zs[];   // [D]
   __shared__ double red[HT / 32];
   const long c = blockIdx.x;
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(VT) k_percol_tables_vjp(const double* __restri
                                                           const double* __restrict__ tzf_bar,
                                                           const double* __restrict__ tzi_bar,
                                                           float* __restrict__ z_bar) {
+  ffno::griddep_sync();
   extern __shared__ double sh[];
   double* zs = sh;        // [D] shifted heights
   double* gz = zs + D;    // [D] gradient w.r.t. the shifted heights
@@ -328,6 +330,7 @@ __global__ void __launch_bounds__(CT1) k_column_terms(const double* __restrict__
                                                       const double* __restrict__ f,
                                                       const double* __restrict__ tzf_bar,
                                                       const double* __restrict__ tzi_bar, double* __restrict__ terms) {
+  ffno::griddep_sync();
   __shared__ double red[CT1 / 32];
   const double zmin = column_min(zr, D, red);
   const long e = (long)blockIdx.x * CT1 + threadIdx.x;
@@ -354,6 +357,7 @@ __global__ void __launch_bounds__(CT1) k_column_finish(const double* __restrict_
                                                        const double* __restrict__ df, int med,
                                                        const double* __restrict__ terms, float* __restrict__ z_bar,
                                                        long z_stride) {
+  ffno::griddep_sync();
   extern __shared__ double gz[];   // [D]
   __shared__ double red[CT1 / 32];
   __shared__ double share, gtap;
@@ -421,7 +425,7 @@ int ffno_percol_tables(const double* z_raw, int D, long ncol, const double* k, i
   if (D > FFNO_PERCOL_MAX_D || live > FFNO_PERCOL_MAX_LIVE || ncol > 2147483647L) return FFNO_EINVAL;
   const size_t smem = (size_t)D * sizeof(double);
   if (!ffno::smem_cap_ok(k_percol_tables, smem)) return FFNO_ELAUNCH;
-  k_percol_tables<<<(unsigned)ncol, HT, smem, (cudaStream_t)stream>>>(z_raw, D, ncol, k, live, f, tzf, tzi, tzf_t,
+  ffno::launch(k_percol_tables, (unsigned)ncol, HT, smem, (cudaStream_t)stream, z_raw, D, ncol, k, live, f, tzf, tzi, tzf_t,
                                                                      tzi_t);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -435,8 +439,8 @@ int ffno_column_tables_vjp(const double* z_raw, int D, const double* k, int live
   if (D > FFNO_PERCOL_MAX_D || live > FFNO_PERCOL_MAX_LIVE || med < 0 || med > D - 2) return FFNO_EINVAL;
   const long n = (long)live * D;
   cudaStream_t s = (cudaStream_t)stream;
-  k_column_terms<<<(unsigned)((n + CT1 - 1) / CT1), CT1, 0, s>>>(z_raw, D, k, live, f, tzf_bar, tzi_bar, scratch);
-  k_column_finish<<<1, CT1, (size_t)D * sizeof(double), s>>>(z_raw, D, live, df, med, scratch, z_bar, z_stride);
+  ffno::launch(k_column_terms, (unsigned)((n + CT1 - 1) / CT1), CT1, 0, s, z_raw, D, k, live, f, tzf_bar, tzi_bar, scratch);
+  ffno::launch(k_column_finish, 1, CT1, (size_t)D * sizeof(double), s, z_raw, D, live, df, med, scratch, z_bar, z_stride);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -449,7 +453,7 @@ int ffno_percol_tables_vjp(const double* z_raw, int D, long ncol, const double* 
   if (D > FFNO_PERCOL_MAX_D || live > FFNO_PERCOL_MAX_LIVE || ncol > 2147483647L) return FFNO_EINVAL;
   const size_t smem = vjp_smem(D);
   if (!ffno::smem_cap_ok(k_percol_tables_vjp, smem)) return FFNO_ELAUNCH;
-  k_percol_tables_vjp<<<(unsigned)ncol, VT, smem, (cudaStream_t)stream>>>(z_raw, D, ncol, k, live, f, df, med,
+  ffno::launch(k_percol_tables_vjp, (unsigned)ncol, VT, smem, (cudaStream_t)stream, z_raw, D, ncol, k, live, f, df, med,
                                                                          tzf_bar, tzi_bar, z_bar);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;

@@ -45,6 +45,7 @@ template <int C>
 __global__ void __launch_bounds__(256) k_gn_jvp_stats(const float* __restrict__ pre, const float* __restrict__ ud,
                                                       const double* __restrict__ gst, const float* __restrict__ dw,
                                                       long V, double* __restrict__ partials, int cpg, int groups) {
+  griddep_sync();
   constexpr int LPV = C / 4;                       // lanes per voxel (float4 each)
   constexpr int VPW = LPV <= 32 ? 32 / LPV : 1;    // voxels per warp step
   __shared__ float mean[GMAX], rstd[GMAX];
@@ -101,6 +102,7 @@ __global__ void k_gn_jvp_apply(const float* __restrict__ pre, const float* __res
                                const double* __restrict__ gst, const double* __restrict__ sums, int act,
                                const float* __restrict__ base, float res, long V, float* __restrict__ out, int cpg,
                                int groups) {
+  griddep_sync();
   __shared__ float mean[GMAX], rstd[GMAX], s1[GMAX], s2[GMAX];
   if (threadIdx.x < groups) {
     const int g = threadIdx.x;
@@ -148,6 +150,7 @@ template <int C>
 __global__ void __launch_bounds__(NT, C <= 64 ? 3 : 2) k_gate_jvp(const float* __restrict__ x, const float* __restrict__ xd, long V,
                                                     const float* __restrict__ w1, const float* __restrict__ w2,
                                                     float* __restrict__ outd, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   float* xs = sm;               // [2C][64]: x, x'
   float* hs = xs + 2 * C * BM;  // [2C][64]: the hidden layer and its tangent
@@ -197,6 +200,7 @@ template <int C>
 __global__ void __launch_bounds__(NT, 2) k_mlp2_jvp(const float* __restrict__ a, const float* __restrict__ ad, long V,
                                                     const float* __restrict__ w1, const float* __restrict__ w2,
                                                     float* __restrict__ outd, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   float* as = sm;   // [C][64] a, [C][64] a', then [2C][64] the hidden tangent
   g32::Ring ring(as + 2 * C * BM, g32::KC * 2 * C, al);
@@ -244,6 +248,7 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_fuse_jvp(const float* _
                                                     const float* __restrict__ wg1, const float* __restrict__ wg2,
                                                     const float* __restrict__ bg2, const float* __restrict__ wf1,
                                                     const float* __restrict__ wf2, float* __restrict__ outd, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   constexpr int TAN = 3 * C * BM, N1 = C / 16, N2 = 2 * C / 16;   // TAN: offset of the tangent's region
   float* A = sm;
@@ -350,6 +355,7 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* _
                                                  const float* __restrict__ p1, const float* __restrict__ p2,
                                                  const float* __restrict__ b2, ffno_head_params hp,
                                                  float* __restrict__ outd, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1, TAN = 2 * C * BM;
@@ -455,6 +461,7 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* _
 // inputs (log10 T, v / 1e3, ..., then (x - mean) / std; ffno_fsdp_runtime.py:48-58, 274-280). flags |= 1 on NaN/Inf.
 __global__ void k_si_input_tangent(const float* __restrict__ feat, const float* __restrict__ td, long V,
                                    const float* __restrict__ std_x, float* __restrict__ xd, int* __restrict__ flags) {
+  griddep_sync();
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < 6 * V; e += (long)gridDim.x * blockDim.x) {
     const int c = (int)(e / V);
     const float t = td[e];
@@ -476,6 +483,7 @@ __global__ void k_si_input_tangent(const float* __restrict__ feat, const float* 
 __global__ void k_si_population_tangent(const float* __restrict__ y, const float* __restrict__ yd, long V, int L,
                                         const float* __restrict__ mean_y, const float* __restrict__ std_y,
                                         float* __restrict__ out, int* __restrict__ flags) {
+  griddep_sync();
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < (long)L * V; e += (long)gridDim.x * blockDim.x) {
     const long v = e / L;
     const int l = (int)(e % L);
@@ -500,7 +508,7 @@ int ffno_gn_jvp_stats(const float* pre, const float* pre_dot, const double* gsta
   cudaStream_t s = (cudaStream_t)stream;
   const int cpg = C / groups;
   switch (C) {
-#define L(CC) case CC: k_gn_jvp_stats<CC><<<nparts, 256, 0, s>>>(pre, pre_dot, gstats, dw, V, partials, cpg, groups); break;
+#define L(CC) case CC: ffno::launch(k_gn_jvp_stats<CC>, nparts, 256, 0, s, pre, pre_dot, gstats, dw, V, partials, cpg, groups); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -519,7 +527,7 @@ int ffno_gn_jvp_apply(const float* pre, const float* pre_dot, const float* gamma
   const long n4 = V * (C / 4);
   const int blocks = (int)((n4 + 255) / 256 < 8L * sms() ? (n4 + 255) / 256 : 8L * sms());
   switch (C) {
-#define L(CC) case CC: k_gn_jvp_apply<CC><<<blocks, 256, 0, s>>>(pre, pre_dot, gamma, beta, gstats, sums, act, base, res, V, out, cpg, groups); break;
+#define L(CC) case CC: ffno::launch(k_gn_jvp_apply<CC>, blocks, 256, 0, s, pre, pre_dot, gamma, beta, gstats, sums, act, base, res, V, out, cpg, groups); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -537,7 +545,7 @@ int ffno_gate_jvp(const float* x, const float* x_dot, long V, int C, const float
   case CC: {                                                                                  \
     const size_t smem = (4 * CC * BM + 2 * g32::KC * CC) * sizeof(float);                     \
     if (!smem_attr(k_gate_jvp<CC>, smem)) return FFNO_ELAUNCH;                                \
-    k_gate_jvp<CC><<<grid_rows(V, BM, CC <= 64 ? 3 : 2), NT, smem, s>>>(x, x_dot, V, w1, w2, out_dot, al); \
+    ffno::launch(k_gate_jvp<CC>, grid_rows(V, BM, CC <= 64 ? 3 : 2), NT, smem, s, x, x_dot, V, w1, w2, out_dot, al); \
     break;                                                                                    \
   }
     L(16) L(32) L(64) L(96)
@@ -557,7 +565,7 @@ int ffno_mlp2_jvp(const float* a, const float* a_dot, long V, int C, const float
   case CC: {                                                                                    \
     const size_t smem = (2 * CC * BM + 2 * g32::KC * 2 * CC) * sizeof(float);                   \
     if (!smem_attr(k_mlp2_jvp<CC>, smem)) return FFNO_ELAUNCH;                                  \
-    k_mlp2_jvp<CC><<<grid_rows(V, BM, 2), NT, smem, s>>>(a, a_dot, V, w1, w2, out_dot, al);      \
+    ffno::launch(k_mlp2_jvp<CC>, grid_rows(V, BM, 2), NT, smem, s, a, a_dot, V, w1, w2, out_dot, al);      \
     break;                                                                                      \
   }
     L(16) L(32) L(64) L(96)
@@ -581,7 +589,7 @@ int ffno_fuse_jvp(const float* x, const float* x_dot, const float* spec_pre, con
   case CC: {                                                                                                  \
     const size_t smem = fuse_jvp_smem<CC>();                                                                  \
     if (!smem_attr(k_fuse_jvp<CC>, smem)) return FFNO_ELAUNCH;                                                \
-    k_fuse_jvp<CC><<<grid_rows(V, BM, CC <= 64 ? 2 : 1), NT, smem, s>>>(x, x_dot, spec_pre, spec_coefs,        \
+    ffno::launch(k_fuse_jvp<CC>, grid_rows(V, BM, CC <= 64 ? 2 : 1), NT, smem, s, x, x_dot, spec_pre, spec_coefs,        \
                                                                         vert_pre, vert_coefs, spec_dot,       \
                                                                         vert_dot, V, wg1, wg2, bg2, wf1, wf2, \
                                                                         fused_dot, al);                       \
@@ -606,7 +614,7 @@ int ffno_head_jvp(const float* x, const float* x_dot, const float* x_in, const f
   case CC * 1000 + NN: {                                                                                           \
     const size_t smem = (4 * CC * BM + 2 * BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);                  \
     if (!smem_attr(k_head_jvp<CC, NN>, smem)) return FFNO_ELAUNCH;                                                \
-    k_head_jvp<CC, NN><<<grid_rows(V, BM, CC <= 64 ? 2 : 1), NT, smem, s>>>(x, x_dot, x_in, x_in_dot, V, p1, p2, b2,    \
+    ffno::launch(k_head_jvp<CC, NN>, grid_rows(V, BM, CC <= 64 ? 2 : 1), NT, smem, s, x, x_dot, x_in, x_in_dot, V, p1, p2, b2,    \
                                                                             *params, out_dot, al);                     \
     break;                                                                                                         \
   }
@@ -624,7 +632,7 @@ int ffno_si_input_tangent(const float* features, const float* tangent, long V, c
   if (!features || !tangent || !std_x || !x_dot || !flags || V < 1) return FFNO_EINVAL;
   const long n = 6 * V;
   const int blocks = (int)((n + 255) / 256 < 8L * sms() ? (n + 255) / 256 : 8L * sms());
-  k_si_input_tangent<<<blocks, 256, 0, (cudaStream_t)stream>>>(features, tangent, V, std_x, x_dot, flags);
+  ffno::launch(k_si_input_tangent, blocks, 256, 0, (cudaStream_t)stream, features, tangent, V, std_x, x_dot, flags);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -634,7 +642,7 @@ int ffno_si_population_tangent(const float* y, const float* y_dot, long V, int L
   if (!y || !y_dot || !mean_y || !std_y || !out || !flags || V < 1 || L < 1) return FFNO_EINVAL;
   const long n = (long)L * V;
   const int blocks = (int)((n + 255) / 256 < 8L * sms() ? (n + 255) / 256 : 8L * sms());
-  k_si_population_tangent<<<blocks, 256, 0, (cudaStream_t)stream>>>(y, y_dot, V, L, mean_y, std_y, out, flags);
+  ffno::launch(k_si_population_tangent, blocks, 256, 0, (cudaStream_t)stream, y, y_dot, V, L, mean_y, std_y, out, flags);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }

@@ -48,6 +48,7 @@ constexpr int DW_COLS = 32, DW_SEGS = 16;
 
 __global__ void __launch_bounds__(DW_COLS* DW_SEGS) k_depth_weights(const float* __restrict__ z, int D, long HW,
                                                                     float* __restrict__ w) {
+  griddep_sync();
   __shared__ float part[DW_SEGS][DW_COLS];
   const int tx = threadIdx.x % DW_COLS, sg = threadIdx.x / DW_COLS;
   const long col = (long)blockIdx.x * DW_COLS + tx;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(DW_COLS* DW_SEGS) k_depth_weights(const float*
 
 // ------------------------------------------------------------------------------------------------ column info
 __global__ void k_column_info(const float* __restrict__ z, int D, long HW, unsigned int* __restrict__ flags) {
+  griddep_sync();
   // flags[0]: 1 while every column equals column 0 (each shifted by its own minimum); flags[1]: float bits of the
   // largest span (non-negative floats order as unsigned ints)
   const long col = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -99,11 +101,13 @@ __global__ void k_column_info(const float* __restrict__ z, int D, long HW, unsig
 }
 
 __global__ void k_column_info_init(unsigned int* flags) {
+  griddep_sync();
   flags[0] = 1u;
   flags[1] = 0u;
 }
 
 __global__ void k_column_info_final(unsigned int* flags) {
+  griddep_sync();
   float* out = reinterpret_cast<float*>(flags);
   const unsigned int s = flags[0];
   out[0] = s ? 1.f : 0.f;  // flags[1] already holds the span's float bits
@@ -118,6 +122,7 @@ __global__ void __launch_bounds__(NT, 3) k_lift(const float* __restrict__ xin, i
                                                 const float* __restrict__ wl, const float* __restrict__ dw,
                                                 float* __restrict__ pre, double* __restrict__ partials, int cpg,
                                                 int groups, int al) {
+  griddep_sync();
   __shared__ __align__(16) float xs[2][8][BM];
   __shared__ __align__(16) float ws[8][C];
   __shared__ g32::TileStats<C> st;
@@ -199,6 +204,7 @@ __global__ void __launch_bounds__(FIN_NT) k_gn_finalize(const double* __restrict
                                                         int groups, const float* __restrict__ gamma,
                                                         const float* __restrict__ beta, float eps,
                                                         float* __restrict__ coefs, double* __restrict__ gstats) {
+  griddep_sync();
   __shared__ double red[3][FIN_NT / 32];
   const int g = blockIdx.x, tid = threadIdx.x;
   double w = 0.0, wm = 0.0;
@@ -250,6 +256,7 @@ __device__ __forceinline__ float4 gn4(float4 p, const float* __restrict__ cf, in
 
 __global__ void k_gn_act(const float* __restrict__ pre, const float* __restrict__ coefs, unsigned n4, int C, int act,
                          float* __restrict__ out) {
+  griddep_sync();
   const unsigned C4 = (unsigned)C / 4, stride = gridDim.x * blockDim.x;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += 2 * stride) {
     const unsigned i2 = i + stride;
@@ -268,6 +275,7 @@ __global__ void k_gn_act(const float* __restrict__ pre, const float* __restrict_
 
 __global__ void k_resid_out(const float* __restrict__ x2, const float* __restrict__ pre,
                             const float* __restrict__ coefs, float res, unsigned n4, int C, float* __restrict__ out) {
+  griddep_sync();
   const unsigned C4 = (unsigned)C / 4, stride = gridDim.x * blockDim.x;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += 2 * stride) {
     const unsigned i2 = i + stride;
@@ -293,6 +301,7 @@ template <int C>
 __global__ void __launch_bounds__(NT, C <= 64 ? 4 : 2) k_gate(const float* __restrict__ x, long V, const float* __restrict__ w1,
                                                 const float* __restrict__ w2, const float* __restrict__ zp,
                                                 const float* __restrict__ z, float* __restrict__ out, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   float* xs = sm;             // [C][64]
   float* hs = xs + C * BM;    // [C][64]
@@ -353,6 +362,7 @@ __global__ void __launch_bounds__(NT, tile_ctas(C)) k_mlp2(const float* __restri
                                                 long V, const float* __restrict__ w1, const float* __restrict__ w2,
                                                 const float* __restrict__ dw, float* __restrict__ pre,
                                                 double* __restrict__ partials, int nparts, int cpg, int groups, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   __shared__ g32::TileStats<C> st;
   float* as = sm;   // [C][64] input, then [2C][64] hidden
@@ -417,6 +427,7 @@ __global__ void __launch_bounds__(NT, tile_ctas(C)) k_fuse(const float* __restri
                                                 const float* __restrict__ wf1, const float* __restrict__ wf2,
                                                 const float* __restrict__ dw, float* __restrict__ pre,
                                                 double* __restrict__ partials, int nparts, int cpg, int groups, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   __shared__ g32::TileStats<C> st;
   float* as = sm;
@@ -516,6 +527,7 @@ __global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, con
                                              const float* __restrict__ b2, int nh,
                                              const __grid_constant__ ffno_head_params hp, float* __restrict__ out,
                                              float* __restrict__ head_out, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1;
@@ -576,6 +588,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_head_output(const float* __restrict__ head, const float* __restrict__ xin,
                                                      long V, int nh, const __grid_constant__ ffno_head_params hp,
                                                      float* __restrict__ out) {
+  griddep_sync();
   __shared__ double etab[EXP_TAB];
   fill_exp_table(etab);
   __syncthreads();
@@ -599,7 +612,7 @@ int ffno_stats_parts(long V) { return grid_for(V, 3); }
 
 int ffno_depth_weights(const float* z, int D, long HW, float* w, ffno_stream_t stream) {
   if (!z || !w || D < 1 || HW < 1) return FFNO_EINVAL;
-  k_depth_weights<<<(unsigned)((HW + DW_COLS - 1) / DW_COLS), DW_COLS * DW_SEGS, 0, (cudaStream_t)stream>>>(z, D, HW, w);
+  ffno::launch(k_depth_weights, (unsigned)((HW + DW_COLS - 1) / DW_COLS), DW_COLS * DW_SEGS, 0, (cudaStream_t)stream, z, D, HW, w);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -607,9 +620,9 @@ int ffno_depth_weights(const float* z, int D, long HW, float* w, ffno_stream_t s
 int ffno_column_info(const float* z, int D, long HW, float* out, ffno_stream_t stream) {
   if (!z || !out || D < 1 || HW < 1) return FFNO_EINVAL;
   unsigned int* flags = reinterpret_cast<unsigned int*>(out);
-  k_column_info_init<<<1, 1, 0, (cudaStream_t)stream>>>(flags);
-  k_column_info<<<(unsigned)((HW + 255) / 256), 256, 0, (cudaStream_t)stream>>>(z, D, HW, flags);
-  k_column_info_final<<<1, 1, 0, (cudaStream_t)stream>>>(flags);
+  ffno::launch(k_column_info_init, 1, 1, 0, (cudaStream_t)stream, flags);
+  ffno::launch(k_column_info, (unsigned)((HW + 255) / 256), 256, 0, (cudaStream_t)stream, z, D, HW, flags);
+  ffno::launch(k_column_info_final, 1, 1, 0, (cudaStream_t)stream, flags);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -623,7 +636,7 @@ int ffno_lift_fwd(const float* x_in, int cin, long V, int C, const float* w_lift
   cudaStream_t s = (cudaStream_t)stream;
   const int cpg = C / groups;
   switch (C) {
-#define L(CC) case CC: k_lift<CC><<<nparts, NT, 0, s>>>(x_in, cin, V, w_lift, dw, pre, partials, cpg, groups, al); break;
+#define L(CC) case CC: ffno::launch(k_lift<CC>, nparts, NT, 0, s, x_in, cin, V, w_lift, dw, pre, partials, cpg, groups, al); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -635,7 +648,7 @@ int ffno_gn_finalize(const double* partials, int nparts, int C, int groups, cons
                      float eps, float* coefs, double* gstats, ffno_stream_t stream) {
   if (!partials || !gamma || !beta || !coefs) return FFNO_EINVAL;
   if (nparts < 1 || C < 1 || groups < 1 || groups > GMAX || C % groups) return FFNO_EINVAL;
-  k_gn_finalize<<<groups, FIN_NT, 0, (cudaStream_t)stream>>>(partials, nparts, C, groups, gamma, beta, eps, coefs,
+  ffno::launch(k_gn_finalize, groups, FIN_NT, 0, (cudaStream_t)stream, partials, nparts, C, groups, gamma, beta, eps, coefs,
                                                              gstats);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -654,7 +667,7 @@ int elementwise_blocks(long n4) {
 int ffno_gn_act(const float* pre, const float* coefs, long V, int C, int act, float* out, ffno_stream_t stream) {
   if (!pre || !coefs || !out || !elementwise_ok(V, C, pre, coefs, out)) return FFNO_EINVAL;
   const long n4 = V * C / 4;
-  k_gn_act<<<elementwise_blocks(n4), 256, 0, (cudaStream_t)stream>>>(pre, coefs, (unsigned)n4, C, act, out);
+  ffno::launch(k_gn_act, elementwise_blocks(n4), 256, 0, (cudaStream_t)stream, pre, coefs, (unsigned)n4, C, act, out);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -665,7 +678,7 @@ int ffno_resid_out(const float* x2, const float* pre, const float* coefs, float 
       reinterpret_cast<uintptr_t>(coefs) % 16)
     return FFNO_EINVAL;
   const long n4 = V * C / 4;
-  k_resid_out<<<elementwise_blocks(n4), 256, 0, (cudaStream_t)stream>>>(x2, pre, coefs, res, (unsigned)n4, C, out);
+  ffno::launch(k_resid_out, elementwise_blocks(n4), 256, 0, (cudaStream_t)stream, x2, pre, coefs, res, (unsigned)n4, C, out);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -680,7 +693,7 @@ int ffno_gate_fwd(const float* x, long V, int C, const float* w1, const float* w
 #define L(CC)                                                                   \
   case CC:                                                                      \
     if (!set_smem(k_gate<CC>, smem)) return FFNO_ELAUNCH;                       \
-    k_gate<CC><<<grid_for(V, CC <= 64 ? 4 : 2), NT, smem, s>>>(x, V, w1, w2, zp, z, out, al); \
+    ffno::launch(k_gate<CC>, grid_for(V, CC <= 64 ? 4 : 2), NT, smem, s, x, V, w1, w2, zp, z, out, al); \
     break;
     L(16) L(32) L(64) L(96)
 #undef L
@@ -706,15 +719,15 @@ int ffno_mlp2_fwd(int mode, const float* in, const float* prev_pre, const float*
     const int grid = grid_for(V, tile_ctas(CC));                                                       \
     if (mode == 0) {                                                                                   \
       if (!set_smem(k_mlp2<CC, 0>, smem)) return FFNO_ELAUNCH;                                         \
-      k_mlp2<CC, 0><<<grid, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
+      ffno::launch(k_mlp2<CC, 0>, grid, NT, smem, s, in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
                                             partials, nparts, cpg, groups, al);                       \
     } else if (mode == 1) {                                                                            \
       if (!set_smem(k_mlp2<CC, 1>, smem)) return FFNO_ELAUNCH;                                         \
-      k_mlp2<CC, 1><<<grid, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
+      ffno::launch(k_mlp2<CC, 1>, grid, NT, smem, s, in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
                                             partials, nparts, cpg, groups, al);                       \
     } else {                                                                                           \
       if (!set_smem(k_mlp2<CC, 2>, smem)) return FFNO_ELAUNCH;                                         \
-      k_mlp2<CC, 2><<<grid, NT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
+      ffno::launch(k_mlp2<CC, 2>, grid, NT, smem, s, in, prev_pre, prev_coefs, res, xout, V, w1, w2, dw, pre,    \
                                             partials, nparts, cpg, groups, al);                       \
     }                                                                                                  \
     break;                                                                                             \
@@ -744,7 +757,7 @@ int ffno_fuse_fwd(const float* x, const float* spec_pre, const float* spec_coefs
     const size_t smem = fuse_smem<CC>();                                                                     \
     const int grid = grid_for(V, tile_ctas(CC));                                                             \
     if (!set_smem(k_fuse<CC>, smem)) return FFNO_ELAUNCH;                                                    \
-    k_fuse<CC><<<grid, NT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre, vert_coefs, V, wg1, wg2, bg2, wf1,   \
+    ffno::launch(k_fuse<CC>, grid, NT, smem, s, x, spec_pre, spec_coefs, vert_pre, vert_coefs, V, wg1, wg2, bg2, wf1,   \
                                       wf2, dw, pre, partials, nparts, cpg, groups, al);                      \
     break;                                                                                                   \
   }
@@ -772,10 +785,10 @@ int ffno_head_fwd(const float* x, const float* x_in, long V, int C, const float*
     const size_t smem = (2 * CC * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);            \
     if (params->math32) {                                                                               \
       if (!set_smem(k_head<CC, NN, float>, smem)) return FFNO_ELAUNCH;                                  \
-      k_head<CC, NN, float><<<grid_for(V, 2), NT, smem, s>>>(x, x_in, V, p1, p2, b2, nh, *params, out, head_out, al); \
+      ffno::launch(k_head<CC, NN, float>, grid_for(V, 2), NT, smem, s, x, x_in, V, p1, p2, b2, nh, *params, out, head_out, al); \
     } else {                                                                                            \
       if (!set_smem(k_head<CC, NN, double>, smem)) return FFNO_ELAUNCH;                                 \
-      k_head<CC, NN, double><<<grid_for(V, 2), NT, smem, s>>>(x, x_in, V, p1, p2, b2, nh, *params, out, head_out, al); \
+      ffno::launch(k_head<CC, NN, double>, grid_for(V, 2), NT, smem, s, x, x_in, V, p1, p2, b2, nh, *params, out, head_out, al); \
     }                                                                                                   \
   }
     default:
@@ -798,7 +811,7 @@ int ffno_proj_fwd(const float* x, long V, int C, const float* p1, const float* p
   if (C == CC && nhp == NN) {                                                                           \
     const size_t smem = (2 * CC * BM + BM * (NN + 1) + 2 * g32::KC * 2 * CC) * sizeof(float);            \
     if (!set_smem(k_head<CC, NN, float, false>, smem)) return FFNO_ELAUNCH;                             \
-    k_head<CC, NN, float, false><<<grid_for(V, 2), NT, smem, s>>>(x, nullptr, V, p1, p2, b2, nh, none,  \
+    ffno::launch(k_head<CC, NN, float, false>, grid_for(V, 2), NT, smem, s, x, nullptr, V, p1, p2, b2, nh, none,  \
                                                                   nullptr, head, al);                       \
   }
     default:
@@ -825,9 +838,9 @@ int ffno_head_output(const float* head, const float* x_in, long V, int nh, const
   const long want = (V + 255) / 256, cap = 8L * num_sms();   // 8 CTAs of 256 threads per SM, grid-stride
   const long blocks = want < cap ? want : cap;
   if (params->math32)
-    k_head_output<float><<<(unsigned)blocks, 256, 0, s>>>(head, x_in, V, nh, *params, out);
+    ffno::launch(k_head_output<float>, (unsigned)blocks, 256, 0, s, head, x_in, V, nh, *params, out);
   else
-    k_head_output<double><<<(unsigned)blocks, 256, 0, s>>>(head, x_in, V, nh, *params, out);
+    ffno::launch(k_head_output<double>, (unsigned)blocks, 256, 0, s, head, x_in, V, nh, *params, out);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }

@@ -489,6 +489,7 @@ __device__ __forceinline__ void pipe_finish(const Pipe& p, uint32_t tmem_all, ui
 
 // Prologue: tensor memory (NCOLS columns per pipeline), barriers, the pipeline of this thread; NP pipelines per CTA.
 #define PIPE_PROLOGUE(NCOLS, NP)                                                         \
+  ffno::griddep_wait();                                                                  \
   __shared__ uint64_t bars[3];                                                           \
   __shared__ uint32_t tslot;                                                             \
   constexpr uint32_t NCOL = tmem_cols(NCOLS);                                            \
@@ -502,6 +503,7 @@ __device__ __forceinline__ void pipe_finish(const Pipe& p, uint32_t tmem_all, ui
   tc::tc_before_sync();                                                                  \
   __syncthreads();                                                                       \
   tc::tc_after_sync();                                                                   \
+  ffno::griddep_launch();                                                                \
   const int pid = tid / PT;                                                              \
   Pipe P{&bars[1 + pid], 0u, true, pid, tid % PT, tid & 31, (tid >> 5) & 3, (tid % PT) / 128, \
          tslot + (uint32_t)pid * NCOL, (uint32_t)(32 * ((tid >> 5) & 3)) << 16};          \
@@ -2224,7 +2226,7 @@ int launch_mix_tc96(const float* in, float* out, long F, long nb, long sf, long 
   const long items = F * ((nb + TM - 1) / TM);
   const long pairs = (items + 1) / 2;   // two pipelines a CTA
   const long grid = pairs < sms() ? pairs : sms();
-  k_mix_tc96<<<(unsigned)grid, CT, smem, s>>>(in, out, F, nb, sf, sb, s_im, static_cast<const uint8_t*>(wpack), g, U,
+  ffno::launch(k_mix_tc96, (unsigned)grid, CT, smem, s, in, out, F, nb, sf, sb, s_im, static_cast<const uint8_t*>(wpack), g, U,
                                               Vm, rank, err);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -2281,7 +2283,7 @@ int ffno_mlp2_fwd_tc(int mode, const float* in, const float* prev_pre, const flo
 #define L96(M)                                                                                                    \
   if (mode == M) {                                                                                              \
     if (!launch_prep(k_mlp2_tc96<M>, smem)) return FFNO_ELAUNCH;                                                \
-    k_mlp2_tc96<M><<<nparts, PT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w, dw, pre, partials, err); \
+    ffno::launch(k_mlp2_tc96<M>, nparts, PT, smem, s, in, prev_pre, prev_coefs, res, xout, V, w, dw, pre, partials, err); \
   }
     L96(0) L96(1) L96(2)
 #undef L96
@@ -2295,13 +2297,13 @@ int ffno_mlp2_fwd_tc(int mode, const float* in, const float* prev_pre, const flo
     const size_t smem = mat_bytes(2 * CC, CC) + mat_bytes(CC, 2 * CC) + 2 * tile_bytes(2 * CC);
     if (mode == 0) {
       if (!launch_prep(k_mlp2_tc<CC, 0>, smem)) return FFNO_ELAUNCH;
-      k_mlp2_tc<CC, 0><<<nparts, CT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w, dw, pre, partials, err);
+      ffno::launch(k_mlp2_tc<CC, 0>, nparts, CT, smem, s, in, prev_pre, prev_coefs, res, xout, V, w, dw, pre, partials, err);
     } else if (mode == 1) {
       if (!launch_prep(k_mlp2_tc<CC, 1>, smem)) return FFNO_ELAUNCH;
-      k_mlp2_tc<CC, 1><<<nparts, CT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w, dw, pre, partials, err);
+      ffno::launch(k_mlp2_tc<CC, 1>, nparts, CT, smem, s, in, prev_pre, prev_coefs, res, xout, V, w, dw, pre, partials, err);
     } else {
       if (!launch_prep(k_mlp2_tc<CC, 2>, smem)) return FFNO_ELAUNCH;
-      k_mlp2_tc<CC, 2><<<nparts, CT, smem, s>>>(in, prev_pre, prev_coefs, res, xout, V, w, dw, pre, partials, err);
+      ffno::launch(k_mlp2_tc<CC, 2>, nparts, CT, smem, s, in, prev_pre, prev_coefs, res, xout, V, w, dw, pre, partials, err);
     }
   })
   FFNO_CHECK_LAUNCH();
@@ -2317,14 +2319,14 @@ int ffno_gate_fwd_tc(const float* x, long V, int C, const void* wpack, const flo
     if (!aligned32(x)) return FFNO_EINVAL;   // rows are read 32 bytes a request
     const size_t smem = 2 * mat_bytes(C96, C96) + 2 * tile_bytes(C96);
     if (!launch_prep(k_gate_tc<C96>, smem)) return FFNO_ELAUNCH;
-    k_gate_tc<C96><<<grid_tc(V), CT, smem, s>>>(x, V, static_cast<const uint8_t*>(wpack), zp, z, out, err);
+    ffno::launch(k_gate_tc<C96>, grid_tc(V), CT, smem, s, x, V, static_cast<const uint8_t*>(wpack), zp, z, out, err);
     FFNO_CHECK_LAUNCH();
     return FFNO_OK;
   }
   TC_DISPATCH(C, {
     const size_t smem = 2 * mat_bytes(CC, CC) + 2 * tile_bytes(CC);
     if (!launch_prep(k_gate_tc<CC>, smem)) return FFNO_ELAUNCH;
-    k_gate_tc<CC><<<grid_tc(V), CT, smem, s>>>(x, V, static_cast<const uint8_t*>(wpack), zp, z, out, err);
+    ffno::launch(k_gate_tc<CC>, grid_tc(V), CT, smem, s, x, V, static_cast<const uint8_t*>(wpack), zp, z, out, err);
   })
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -2341,7 +2343,7 @@ int ffno_fuse1_tc(const float* x, const float* spec_pre, const float* spec_coefs
       return FFNO_EINVAL;
     const size_t smem = mat_bytes(C96, 3 * C96) + mat_bytes(2 * C96, C96) + tile_bytes(KS);
     if (!launch_prep(k_fuse1_tc96, smem)) return FFNO_ELAUNCH;
-    k_fuse1_tc96<<<grid_tc(V), PT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre, vert_coefs, V,
+    ffno::launch(k_fuse1_tc96, grid_tc(V), PT, smem, s, x, spec_pre, spec_coefs, vert_pre, vert_coefs, V,
                                              static_cast<const uint8_t*>(wpack), bias, gates, hg, err);
     FFNO_CHECK_LAUNCH();
     return FFNO_OK;
@@ -2351,7 +2353,7 @@ int ffno_fuse1_tc(const float* x, const float* spec_pre, const float* spec_coefs
   TC_DISPATCH(C, {
     const size_t smem = mat_bytes(CC, 3 * CC) + mat_bytes(2 * CC, CC) + 2 * tile_bytes(CC);
     if (!launch_prep(k_fuse1_tc<CC>, smem)) return FFNO_ELAUNCH;
-    k_fuse1_tc<CC><<<grid_tc(V), CT, smem, s>>>(x, spec_pre, spec_coefs, vert_pre, vert_coefs, V,
+    ffno::launch(k_fuse1_tc<CC>, grid_tc(V), CT, smem, s, x, spec_pre, spec_coefs, vert_pre, vert_coefs, V,
                                                static_cast<const uint8_t*>(wpack), bias, gates, hg, err);
   })
   FFNO_CHECK_LAUNCH();
@@ -2372,7 +2374,7 @@ int ffno_fuse2_tc(const float* spec_pre, const float* spec_coefs, const float* v
   TC_DISPATCH(C, {
     const size_t smem = mat_bytes(2 * CC, 2 * CC) + mat_bytes(CC, 2 * CC) + 2 * tile_bytes(2 * CC);
     if (!launch_prep(k_fuse2_tc<CC>, smem)) return FFNO_ELAUNCH;
-    k_fuse2_tc<CC><<<nparts, CT, smem, s>>>(spec_pre, spec_coefs, vert_pre, vert_coefs, gates, V,
+    ffno::launch(k_fuse2_tc<CC>, nparts, CT, smem, s, spec_pre, spec_coefs, vert_pre, vert_coefs, gates, V,
                                            static_cast<const uint8_t*>(wpack), dw, pre, partials, err);
   })
   FFNO_CHECK_LAUNCH();
@@ -2387,7 +2389,7 @@ int ffno_fuse_hidden_tc(const float* spec_pre, const float* spec_coefs, const fl
   if (!aligned32(spec_pre) || !aligned32(vert_pre) || !aligned32(gates) || !aligned32(hf)) return FFNO_EINVAL;
   const size_t smem = mat_bytes(2 * C96, 2 * C96) + tile_bytes(KS);
   if (!launch_prep(k_fuse_hidden_tc96, smem)) return FFNO_ELAUNCH;
-  k_fuse_hidden_tc96<<<grid_tc(V), PT, smem, (cudaStream_t)stream>>>(spec_pre, spec_coefs, vert_pre, vert_coefs,
+  ffno::launch(k_fuse_hidden_tc96, grid_tc(V), PT, smem, (cudaStream_t)stream, spec_pre, spec_coefs, vert_pre, vert_coefs,
                                                                      gates, V, static_cast<const uint8_t*>(wpack), hf,
                                                                      err);
   FFNO_CHECK_LAUNCH();
@@ -2405,7 +2407,7 @@ int ffno_fuse_out_tc(const float* spec_pre, const float* spec_coefs, const float
     return FFNO_EINVAL;
   const size_t smem = mat_bytes(C96, 2 * C96) + tile_bytes(KS);
   if (!launch_prep(k_fuse_out_tc96, smem)) return FFNO_ELAUNCH;
-  k_fuse_out_tc96<<<nparts, PT, smem, (cudaStream_t)stream>>>(spec_pre, spec_coefs, vert_pre, vert_coefs, gates, hf, V,
+  ffno::launch(k_fuse_out_tc96, nparts, PT, smem, (cudaStream_t)stream, spec_pre, spec_coefs, vert_pre, vert_coefs, gates, hf, V,
                                                               static_cast<const uint8_t*>(wpack), dw, pre, partials,
                                                               err);
   FFNO_CHECK_LAUNCH();
@@ -2419,7 +2421,7 @@ int ffno_fuse_bwd_h_tc(const float* fused_pre_bar, const float* hf, long V, int 
   if (!aligned32(fused_pre_bar) || !aligned32(hf) || !aligned32(hf_bar)) return FFNO_EINVAL;
   const size_t smem = mat_bytes(C96, 2 * C96) + tile_bytes(KS);
   if (!launch_prep(k_fuse_bwd_h_tc96, smem)) return FFNO_ELAUNCH;
-  k_fuse_bwd_h_tc96<<<grid_tc(V), PT, smem, (cudaStream_t)stream>>>(fused_pre_bar, hf, V,
+  ffno::launch(k_fuse_bwd_h_tc96, grid_tc(V), PT, smem, (cudaStream_t)stream, fused_pre_bar, hf, V,
                                                                     static_cast<const uint8_t*>(wpack), hf_bar, err);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -2437,7 +2439,7 @@ int ffno_fuse_bwd_q_tc(const float* spec_pre, const float* spec_coefs, const flo
     return FFNO_EINVAL;
   const size_t smem = mat_bytes(2 * C96, 2 * C96) + tile_bytes(KS);
   if (!launch_prep(k_fuse_bwd_q_tc96, smem)) return FFNO_ELAUNCH;
-  k_fuse_bwd_q_tc96<<<grid_tc(V), PT, smem, (cudaStream_t)stream>>>(spec_pre, spec_coefs, vert_pre, vert_coefs, gates,
+  ffno::launch(k_fuse_bwd_q_tc96, grid_tc(V), PT, smem, (cudaStream_t)stream, spec_pre, spec_coefs, vert_pre, vert_coefs, gates,
                                                                     fused_pre_bar, hf_bar, V,
                                                                     static_cast<const uint8_t*>(wpack), spec_bar,
                                                                     vert_bar, q, err);
@@ -2454,7 +2456,7 @@ int ffno_fuse_bwd_x_tc(const float* q, const float* hg, const float* base, long 
     return FFNO_EINVAL;
   const size_t smem = mat_bytes(C96, 3 * C96) + mat_bytes(2 * C96, C96) + tile_bytes(KS);
   if (!launch_prep(k_fuse_bwd_x_tc96, smem)) return FFNO_ELAUNCH;
-  k_fuse_bwd_x_tc96<<<grid_tc(V), PT, smem, (cudaStream_t)stream>>>(q, hg, base, V, static_cast<const uint8_t*>(wpack),
+  ffno::launch(k_fuse_bwd_x_tc96, grid_tc(V), PT, smem, (cudaStream_t)stream, q, hg, base, V, static_cast<const uint8_t*>(wpack),
                                                                     x_bar, spec_bar, vert_bar, err);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -2468,7 +2470,7 @@ int ffno_mlp2_bwd_tc(const float* a, const float* pre_bar, const float* base, lo
     if (!aligned32(a) || !aligned32(pre_bar) || !aligned32(a_bar) || (base && !aligned32(base))) return FFNO_EINVAL;
     const size_t smem = mat_bytes(2 * C96, C96) + mat_bytes(C96, 2 * C96) + tile_bytes(C96);
     if (!launch_prep(k_mlp2_bwd_tc96, smem)) return FFNO_ELAUNCH;
-    k_mlp2_bwd_tc96<<<grid_tc(V), PT, smem, s>>>(a, pre_bar, base, V, static_cast<const uint8_t*>(wpack), a_bar, err);
+    ffno::launch(k_mlp2_bwd_tc96, grid_tc(V), PT, smem, s, a, pre_bar, base, V, static_cast<const uint8_t*>(wpack), a_bar, err);
     FFNO_CHECK_LAUNCH();
     return FFNO_OK;
   }
@@ -2476,7 +2478,7 @@ int ffno_mlp2_bwd_tc(const float* a, const float* pre_bar, const float* base, lo
   TC_DISPATCH(C, {
     const size_t smem = 3 * mat_bytes(2 * CC, CC) + 2 * tile_bytes(2 * CC);
     if (!launch_prep(k_mlp2_bwd_tc<CC>, smem)) return FFNO_ELAUNCH;
-    k_mlp2_bwd_tc<CC><<<grid_tc(V), CT, smem, s>>>(a, pre_bar, base, V, static_cast<const uint8_t*>(wpack), a_bar,
+    ffno::launch(k_mlp2_bwd_tc<CC>, grid_tc(V), CT, smem, s, a, pre_bar, base, V, static_cast<const uint8_t*>(wpack), a_bar,
                                                   err);
   })
   FFNO_CHECK_LAUNCH();
@@ -2493,7 +2495,7 @@ int ffno_gate_bwd_tc(const float* x, const float* g_bar, const float* base, long
     if (!aligned32(x)) return FFNO_EINVAL;
     const size_t smem = 2 * mat_bytes(C96, C96) + 2 * tile_bytes(C96);   // one pipeline; pack [g1, g2]
     if (!launch_prep(k_gate_bwd_tc<C96, 1>, smem)) return FFNO_ELAUNCH;
-    k_gate_bwd_tc<C96, 1><<<grid_tc(V), PT, smem, s>>>(x, g_bar, base, V, static_cast<const uint8_t*>(wpack), zp,
+    ffno::launch(k_gate_bwd_tc<C96, 1>, grid_tc(V), PT, smem, s, x, g_bar, base, V, static_cast<const uint8_t*>(wpack), zp,
                                                        x_bar, z_bar, err);
     FFNO_CHECK_LAUNCH();
     return FFNO_OK;
@@ -2501,7 +2503,7 @@ int ffno_gate_bwd_tc(const float* x, const float* g_bar, const float* base, long
   TC_DISPATCH(C, {
     const size_t smem = 4 * mat_bytes(CC, CC) + 4 * tile_bytes(CC);
     if (!launch_prep(k_gate_bwd_tc<CC>, smem)) return FFNO_ELAUNCH;
-    k_gate_bwd_tc<CC><<<grid_tc(V), CT, smem, s>>>(x, g_bar, base, V, static_cast<const uint8_t*>(wpack), zp, x_bar,
+    ffno::launch(k_gate_bwd_tc<CC>, grid_tc(V), CT, smem, s, x, g_bar, base, V, static_cast<const uint8_t*>(wpack), zp, x_bar,
                                                   z_bar, err);
   })
   FFNO_CHECK_LAUNCH();
@@ -2521,7 +2523,7 @@ int ffno_fuse_bwd_a_tc(const float* spec_pre, const float* spec_coefs, const flo
   TC_DISPATCH(C, {
     const size_t smem = mat_bytes(2 * CC, 2 * CC) + mat_bytes(2 * CC, CC) + 2 * tile_bytes(2 * CC);
     if (!launch_prep(k_fuse_bwd_a_tc<CC>, smem)) return FFNO_ELAUNCH;
-    k_fuse_bwd_a_tc<CC><<<grid_tc(V), CT, smem, s>>>(spec_pre, spec_coefs, vert_pre, vert_coefs, gates, fused_pre_bar,
+    ffno::launch(k_fuse_bwd_a_tc<CC>, grid_tc(V), CT, smem, s, spec_pre, spec_coefs, vert_pre, vert_coefs, gates, fused_pre_bar,
                                                     V, static_cast<const uint8_t*>(wpack), hf_bar, err);
   })
   FFNO_CHECK_LAUNCH();
@@ -2546,7 +2548,7 @@ int ffno_fuse_bwd_b_tc(const float* spec_pre, const float* spec_coefs, const flo
     const size_t smem =
         mat_bytes(2 * CC, 2 * CC) + mat_bytes(CC, 2 * CC) + mat_bytes(3 * CC, CC) + 2 * tile_bytes(CC);
     if (!launch_prep(k_fuse_bwd_b_tc<CC>, smem)) return FFNO_ELAUNCH;
-    k_fuse_bwd_b_tc<CC><<<grid_tc(V), CT, smem, s>>>(spec_pre, spec_coefs, vert_pre, vert_coefs, gates, hg,
+    ffno::launch(k_fuse_bwd_b_tc<CC>, grid_tc(V), CT, smem, s, spec_pre, spec_coefs, vert_pre, vert_coefs, gates, hg,
                                                     fused_pre_bar, hf_bar, base, V,
                                                     static_cast<const uint8_t*>(wpack), x_bar, spec_bar, vert_bar,
                                                     err);
@@ -2578,19 +2580,19 @@ static bool head_ok(const ffno_head_params* hp, int nh, int nhp) {
       constexpr int NN = 16;                                                                 \
       if (params->math32) {                                                                  \
         if (!launch_prep(KERNEL<CC, NN, float>, SMEM)) return FFNO_ELAUNCH;                  \
-        KERNEL<CC, NN, float><<<grid_tc(V), CT, SMEM, s>>>(__VA_ARGS__);                     \
+        ffno::launch(KERNEL<CC, NN, float>, grid_tc(V), CT, SMEM, s, __VA_ARGS__);                     \
       } else {                                                                               \
         if (!launch_prep(KERNEL<CC, NN, double>, SMEM)) return FFNO_ELAUNCH;                 \
-        KERNEL<CC, NN, double><<<grid_tc(V), CT, SMEM, s>>>(__VA_ARGS__);                    \
+        ffno::launch(KERNEL<CC, NN, double>, grid_tc(V), CT, SMEM, s, __VA_ARGS__);                    \
       }                                                                                      \
     } else {                                                                                 \
       constexpr int NN = 32;                                                                 \
       if (params->math32) {                                                                  \
         if (!launch_prep(KERNEL<CC, NN, float>, SMEM)) return FFNO_ELAUNCH;                  \
-        KERNEL<CC, NN, float><<<grid_tc(V), CT, SMEM, s>>>(__VA_ARGS__);                     \
+        ffno::launch(KERNEL<CC, NN, float>, grid_tc(V), CT, SMEM, s, __VA_ARGS__);                     \
       } else {                                                                               \
         if (!launch_prep(KERNEL<CC, NN, double>, SMEM)) return FFNO_ELAUNCH;                 \
-        KERNEL<CC, NN, double><<<grid_tc(V), CT, SMEM, s>>>(__VA_ARGS__);                    \
+        ffno::launch(KERNEL<CC, NN, double>, grid_tc(V), CT, SMEM, s, __VA_ARGS__);                    \
       }                                                                                      \
     }                                                                                        \
   })
@@ -2599,18 +2601,18 @@ static bool head_ok(const ffno_head_params* hp, int nh, int nhp) {
   if (nhp == 16) {                                                                                  \
     if (params->math32) {                                                                           \
       if (!launch_prep(KERNEL<16, float>, SMEM)) return FFNO_ELAUNCH;                               \
-      KERNEL<16, float><<<grid_tc(V), PT, SMEM, s>>>(__VA_ARGS__);                                  \
+      ffno::launch(KERNEL<16, float>, grid_tc(V), PT, SMEM, s, __VA_ARGS__);                                  \
     } else {                                                                                        \
       if (!launch_prep(KERNEL<16, double>, SMEM)) return FFNO_ELAUNCH;                              \
-      KERNEL<16, double><<<grid_tc(V), PT, SMEM, s>>>(__VA_ARGS__);                                 \
+      ffno::launch(KERNEL<16, double>, grid_tc(V), PT, SMEM, s, __VA_ARGS__);                                 \
     }                                                                                               \
   } else {                                                                                          \
     if (params->math32) {                                                                           \
       if (!launch_prep(KERNEL<32, float>, SMEM)) return FFNO_ELAUNCH;                               \
-      KERNEL<32, float><<<grid_tc(V), PT, SMEM, s>>>(__VA_ARGS__);                                  \
+      ffno::launch(KERNEL<32, float>, grid_tc(V), PT, SMEM, s, __VA_ARGS__);                                  \
     } else {                                                                                        \
       if (!launch_prep(KERNEL<32, double>, SMEM)) return FFNO_ELAUNCH;                              \
-      KERNEL<32, double><<<grid_tc(V), PT, SMEM, s>>>(__VA_ARGS__);                                 \
+      ffno::launch(KERNEL<32, double>, grid_tc(V), PT, SMEM, s, __VA_ARGS__);                                 \
     }                                                                                               \
   }
 

@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     k_mlp2_bwd_ws(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_pb,
                   const float* __restrict__ base, long V, const uint8_t* __restrict__ wpack, float* __restrict__ abar,
                   int* __restrict__ err) {
+  griddep_wait();
   static_assert(C == 32 || C == 64, "widths 32 and 64");
   constexpr uint32_t B1 = mat_bytes(2 * C, C);   // each of w1 (2C x C), w2t (2C x C), w1t (C x 2C)
   constexpr uint32_t WB = 3 * B1;
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   if (threadIdx.x == 0) {
     tc::mbar_arrive_expect_tx(&bars.w, WB);
@@ -296,6 +298,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
                   const float* __restrict__ pc, float res, float* __restrict__ xout, long V,
                   const uint8_t* __restrict__ wpack, const float* __restrict__ dw, float* __restrict__ pre,
                   double* __restrict__ partials, int* __restrict__ err) {
+  griddep_wait();
   static_assert(C == 32 || C == 64, "widths 32 and 64");
   constexpr uint32_t B1 = mat_bytes(2 * C, C);   // w1 (2C x C); w2 (C x 2C) has the same size
   constexpr uint32_t WB = 2 * B1;
@@ -333,6 +336,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   if (threadIdx.x == 0) {
     tc::mbar_arrive_expect_tx(&wbar, WB);
@@ -583,6 +587,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     k_gate_fwd_ws(const __grid_constant__ CUtensorMap map_x, const float* __restrict__ x, long V,
                   const uint8_t* __restrict__ wpack, const float* __restrict__ zp, const float* __restrict__ z,
                   float* __restrict__ out, int* __restrict__ err) {
+  griddep_wait();
   static_assert(C == 32 || C == 64, "widths 32 and 64");
   constexpr uint32_t B1 = mat_bytes(C, C);       // each of g1, g2
   constexpr uint32_t WB = 2 * B1;
@@ -615,6 +620,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   if (threadIdx.x == 0) {
     tc::mbar_arrive_expect_tx(&wbar, WB);
@@ -816,6 +822,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
                const __grid_constant__ CUtensorMap map_vp, const float* __restrict__ sc, const float* __restrict__ vc,
                long V, const uint8_t* __restrict__ wpack, const float* __restrict__ bias, float* __restrict__ gates,
                float* __restrict__ hg, int* __restrict__ err) {
+  griddep_wait();
   static_assert(C == 32 || C == 64, "widths 32 and 64");
   constexpr uint32_t B1 = mat_bytes(C, 3 * C), B2 = mat_bytes(2 * C, C);
   constexpr uint32_t WB = B1 + B2;
@@ -860,6 +867,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   if (threadIdx.x == 0) {
     tc::mbar_arrive_expect_tx(&wbar, WB);
@@ -1077,6 +1085,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
                const __grid_constant__ CUtensorMap map_g, const float* __restrict__ sc, const float* __restrict__ vc,
                long V, const uint8_t* __restrict__ wpack, const float* __restrict__ dw, float* __restrict__ pre,
                double* __restrict__ partials, int* __restrict__ err) {
+  griddep_wait();
   static_assert(C == 32 || C == 64, "widths 32 and 64");
   constexpr uint32_t B1 = mat_bytes(2 * C, 2 * C), B2 = mat_bytes(C, 2 * C);
   constexpr uint32_t WB = B1 + B2;
@@ -1125,6 +1134,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   if (threadIdx.x == 0) {
     tc::mbar_arrive_expect_tx(&wbar, WB);
@@ -1397,6 +1407,7 @@ __global__ void __launch_bounds__(448, 1)
                   const float* __restrict__ base, long V, const uint8_t* __restrict__ wpack,
                   const float* __restrict__ zp, float* __restrict__ xbar, float* __restrict__ zbar,
                   int* __restrict__ err) {
+  griddep_wait();
   static_assert(C == 32 || C == 64, "widths 32 and 64");
   constexpr int GW_TMA = 0, GW_MMA = 1, GW_CVT = 2, GW_E13 = 6, GW_E24 = 10;
   constexpr uint32_t B1 = mat_bytes(C, C);       // each of g1, g2, g2t, g1t
@@ -1433,6 +1444,7 @@ __global__ void __launch_bounds__(448, 1)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   if (threadIdx.x == 0) {
     tc::mbar_arrive_expect_tx(&wbar, WB);
@@ -1726,7 +1738,7 @@ int launch_mlp2_bwd(const float* a, const float* pb, const float* base, long V, 
     return FFNO_ELAUNCH;
   const long nt = (V + TM - 1) / TM;
   const int grid = (int)(nt < sms() ? nt : sms());
-  k_mlp2_bwd_ws<C><<<grid, NTHREADS, smem, s>>>(ma, mp, base, V, static_cast<const uint8_t*>(wpack), abar, err);
+  ffno::launch(k_mlp2_bwd_ws<C>, grid, NTHREADS, smem, s, ma, mp, base, V, static_cast<const uint8_t*>(wpack), abar, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
 
@@ -1739,7 +1751,7 @@ int launch_mlp2_fwd(const float* in, const float* prev, const float* pc, float r
   if (MODE != 0 ? !row_map(&mp, prev, V, C) : !row_map(&mp, in, V, C)) return FFNO_EINVAL;
   const size_t smem = 1024 + 2 * (size_t)mat_bytes(2 * C, C) + 2 * (size_t)((MODE == 0 ? 1 : 2) * (C / 32) * BOX_BYTES);
   if (!ffno::smem_cap_ok(k_mlp2_fwd_ws<C, MODE>, smem)) return FFNO_ELAUNCH;
-  k_mlp2_fwd_ws<C, MODE><<<nparts, F_NTHREADS, smem, s>>>(mi, mp, pc, res, xout, V, static_cast<const uint8_t*>(wpack),
+  ffno::launch(k_mlp2_fwd_ws<C, MODE>, nparts, F_NTHREADS, smem, s, mi, mp, pc, res, xout, V, static_cast<const uint8_t*>(wpack),
                                                          dw, pre, partials, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
@@ -1754,7 +1766,7 @@ int launch_gate_fwd(const float* x, long V, const void* wpack, const float* zp, 
     return FFNO_ELAUNCH;
   const long nt = (V + TM - 1) / TM;
   const int grid = (int)(nt < sms() ? nt : sms());
-  k_gate_fwd_ws<C><<<grid, NTHREADS, smem, s>>>(mx, x, V, static_cast<const uint8_t*>(wpack), zp, z, out, err);
+  ffno::launch(k_gate_fwd_ws<C>, grid, NTHREADS, smem, s, mx, x, V, static_cast<const uint8_t*>(wpack), zp, z, out, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
 
@@ -1768,7 +1780,7 @@ int launch_gate_bwd(const float* x, const float* gbar, const float* base, long V
     return FFNO_ELAUNCH;
   const long nt = (V + TM - 1) / TM;
   const int grid = (int)(nt < sms() ? nt : sms());
-  k_gate_bwd_ws<C><<<grid, 448, smem, s>>>(mx, mg, base, V, static_cast<const uint8_t*>(wpack), zp, xbar, zbar, err);
+  ffno::launch(k_gate_bwd_ws<C>, grid, 448, smem, s, mx, mg, base, V, static_cast<const uint8_t*>(wpack), zp, xbar, zbar, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
 
@@ -1781,7 +1793,7 @@ int launch_fuse2(const float* sp, const float* sc, const float* vp, const float*
   const size_t smem = 1024 + (size_t)mat_bytes(2 * C, 2 * C) + mat_bytes(C, 2 * C) + 3 * (size_t)(2 * BOX_BYTES);
   if (!ffno::smem_cap_ok(k_fuse2_ws<C>, smem))
     return FFNO_ELAUNCH;
-  k_fuse2_ws<C><<<nparts, F_NTHREADS, smem, s>>>(ms, mv, mg, sc, vc, V, static_cast<const uint8_t*>(wpack), dw, pre,
+  ffno::launch(k_fuse2_ws<C>, nparts, F_NTHREADS, smem, s, ms, mv, mg, sc, vc, V, static_cast<const uint8_t*>(wpack), dw, pre,
                                                 partials, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
@@ -1796,7 +1808,7 @@ int launch_fuse1(const float* x, const float* sp, const float* sc, const float* 
     return FFNO_ELAUNCH;
   const long nt = (V + TM - 1) / TM;
   const int grid = (int)(nt < sms() ? nt : sms());
-  k_fuse1_ws<C><<<grid, F_NTHREADS, smem, s>>>(mx, ms, mv, sc, vc, V, static_cast<const uint8_t*>(wpack), bias, gates,
+  ffno::launch(k_fuse1_ws<C>, grid, F_NTHREADS, smem, s, mx, ms, mv, sc, vc, V, static_cast<const uint8_t*>(wpack), bias, gates,
                                               hg, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }

@@ -47,6 +47,7 @@ template <int MR, int NR, bool VEC>
 __global__ void __launch_bounds__(NT, MR * NR > 32 ? 2 : 3) k_xform(const float* __restrict__ T, const float* __restrict__ in,
                                                  float* __restrict__ out, ffno_xform_desc d, long ntn, long ntm,
                                                  int accumulate, long t_b, long ncols) {
+  griddep_sync();
   using R = XRows<MR>;
   constexpr int TN = 16 * NR, TPT = (R::TM * XK + NT - 1) / NT;   // table elements a thread moves per chunk
   __shared__ __align__(16) float ts[2][XK][R::LD];
@@ -197,7 +198,7 @@ int launch_xform(const float* T, const float* in, float* out, const ffno_xform_d
   const long ntn = (ncols + 16 * NR - 1) / (16 * NR), ntm = (d.M + 16 * MR - 1) / (16 * MR);
   const long blocks = ntn * ntm * (t_b ? d.nb : 1);
   if (blocks > 0x7fffffffL) return FFNO_EINVAL;
-  k_xform<MR, NR, VEC><<<(unsigned)blocks, NT, 0, s>>>(T, in, out, d, ntn, ntm, accumulate, t_b, ncols);
+  ffno::launch(k_xform<MR, NR, VEC>, (unsigned)blocks, NT, 0, s, T, in, out, d, ntn, ntm, accumulate, t_b, ncols);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -246,6 +247,7 @@ __global__ void __launch_bounds__(NT, C <= 32 ? 3 : 2) k_mix(const float* __rest
                                                long sf, long sb, long s_im, const float* __restrict__ wbig,
                                                const float* __restrict__ g, const float* __restrict__ U,
                                                const float* __restrict__ Vm, int rank, int al) {
+  griddep_sync();
   extern __shared__ __align__(16) float sm[];
   float* xs = sm;                               // [2C][64]
   g32::Ring ring(xs + 2 * C * BM, g32::KC * 2 * C, al);
@@ -366,6 +368,7 @@ constexpr int OT = 64;
 __global__ void __launch_bounds__(256) k_col_outer(const float* __restrict__ A, int Ra, const float* __restrict__ B,
                                                    int Rb, long ncol, int C, long rs, double* __restrict__ out,
                                                    int accumulate) {
+  griddep_sync();
   extern __shared__ float osm[];
   const int LD = C + 1;
   float* as = osm;             // [OT][C + 1]
@@ -419,7 +422,7 @@ int ffno_col_outer(const float* A, int Ra, const float* B, int Rb, long ncol, in
   if (!A || !B || !out || Ra < 1 || Rb < 1 || ncol < 1 || C < 1 || C > 512 || ncol > 0x7fffffffL) return FFNO_EINVAL;
   const size_t smem = (size_t)2 * OT * (C + 1) * sizeof(float);
   if (!ffno::smem_cap_ok(k_col_outer, smem)) return FFNO_ELAUNCH;
-  k_col_outer<<<(unsigned)ncol, 256, smem, (cudaStream_t)stream>>>(A, Ra, B, Rb, ncol, C, row_stride, out,
+  ffno::launch(k_col_outer, (unsigned)ncol, 256, smem, (cudaStream_t)stream, A, Ra, B, Rb, ncol, C, row_stride, out,
                                                                   accumulate);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -441,7 +444,7 @@ int ffno_spectral_mix(const float* in, float* out, long F, long nb, long sf, lon
   case CC: {                                                                                               \
     const size_t smem = mix_smem<CC>();                                                                    \
     if (!ffno::smem_cap_ok(k_mix<CC>, smem)) return FFNO_ELAUNCH;                                          \
-    k_mix<CC><<<(unsigned)blocks, NT, smem, s>>>(in, out, F, nb, sf, sb, s_im, wbig, g, U, Vm, rank, al);  \
+    ffno::launch(k_mix<CC>, (unsigned)blocks, NT, smem, s, in, out, F, nb, sf, sb, s_im, wbig, g, U, Vm, rank, al);  \
     break;                                                                                                 \
   }
     L(16) L(32) L(64) L(96)

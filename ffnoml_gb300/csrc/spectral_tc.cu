@@ -103,6 +103,7 @@ __device__ __forceinline__ void xf_fill_chunk(uint8_t* st, uint32_t hb, const fl
 __global__ void __launch_bounds__(2 * RT, 1)
     k_xform_rt(const uint8_t* __restrict__ tpack, int Mp, int Kp, const float* __restrict__ in, float* __restrict__ out,
                ffno_xform_desc d, int nbi, int nshift, long ntn, long items, int accumulate, int* __restrict__ err) {
+  griddep_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t TB = (uint32_t)Mp * Kp * 2;                 // one split half of the table
@@ -128,6 +129,7 @@ __global__ void __launch_bounds__(2 * RT, 1)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot + (uint32_t)pipe * 256u;
   const uint32_t lq = (uint32_t)(32 * q) << 16;
   bool ok = __syncthreads_and(tc::mbar_wait(&bar_t, 0)) != 0;
@@ -248,6 +250,7 @@ constexpr uint32_t SSB = 128u * XKC * 2;    // one split half of a data stage of
 __global__ void __launch_bounds__(RT, 2)
     k_xform_st(const uint8_t* __restrict__ tpack, int MT, int Kp, const float* __restrict__ in, float* __restrict__ out,
                ffno_xform_desc d, int nbi, int nshift, long ntn, long items, int accumulate, int* __restrict__ err) {
+  griddep_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t TSB = (uint32_t)MT * 128u * XKC * 2;        // one split half of a table stage
@@ -271,6 +274,7 @@ __global__ void __launch_bounds__(RT, 2)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   const uint32_t lq = (uint32_t)(32 * q) << 16;
   const int nch = (Kp + XKC - 1) / XKC;
@@ -423,6 +427,7 @@ __global__ void __launch_bounds__(XT, 1)
     k_mix_tc(const __grid_constant__ CUtensorMap tmap, float* __restrict__ out, long F, long nb, long sf, long sb,
              long s_im, const uint8_t* __restrict__ wpack, const float* __restrict__ g, const float* __restrict__ U,
              const float* __restrict__ Vm, int rank, MixGeom geo, int* __restrict__ err) {
+  griddep_wait();
   constexpr int K2 = 2 * C;
   constexpr int CB = C < 32 ? C : 32;       // channels per staging row (one box row)
   constexpr int NH = C / CB;                // boxes per item
@@ -464,6 +469,7 @@ __global__ void __launch_bounds__(XT, 1)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   const uint32_t lq = (uint32_t)(32 * q) << 16;
   const long nbt = (nb + 127) / 128, items = F * nbt;
@@ -704,6 +710,7 @@ __global__ void __launch_bounds__(OT, 1) k_outer_tc(const float* __restrict__ A,
                                                     const float* __restrict__ B, long ldb, int Mb, long N, int TI,
                                                     int NB, int NS, long cps, float* __restrict__ part, long so,
                                                     long si, long sj, int* __restrict__ err) {
+  griddep_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   __shared__ uint64_t bar[2];
@@ -722,6 +729,7 @@ __global__ void __launch_bounds__(OT, 1) k_outer_tc(const float* __restrict__ A,
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
+  griddep_launch();
   const uint32_t tmem = tslot;
   const long nchunks = (N + OKC - 1) / OKC;
   const long c0 = blockIdx.x * cps, c1 = c0 + cps < nchunks ? c0 + cps : nchunks;
@@ -824,6 +832,7 @@ constexpr int RD_EL = 32, RD_SEGS = 8;
 __global__ void __launch_bounds__(RD_EL* RD_SEGS) k_outer_tc_reduce(const float* __restrict__ part, long nsplit, long n,
                                                                     long cols, long ldo, double* __restrict__ out,
                                                                     int accumulate) {
+  griddep_sync();
   __shared__ double red[RD_SEGS][RD_EL];
   const int tx = threadIdx.x % RD_EL, sg = threadIdx.x / RD_EL;
   const long e = (long)blockIdx.x * RD_EL + tx;
@@ -884,7 +893,7 @@ int ffno_xform_tc(const void* tpack, const float* in, float* out, const ffno_xfo
   if (!ffno::smem_cap_ok(k_xform_st, smem))
     return FFNO_ELAUNCH;
   const long grid = items < 2L * sms() ? items : 2L * sms();   // two CTAs per SM
-  k_xform_st<<<(unsigned)grid, RT, smem, (cudaStream_t)stream>>>(static_cast<const uint8_t*>(tpack), MT, Kp, in, out,
+  ffno::launch(k_xform_st, (unsigned)grid, RT, smem, (cudaStream_t)stream, static_cast<const uint8_t*>(tpack), MT, Kp, in, out,
                                                                 d, nbi, nshift, ntn, items, accumulate, err);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -911,7 +920,7 @@ int ffno_xform_tcr(const void* tpack, int Mp, int Kp, const float* in, float* ou
     return FFNO_ELAUNCH;
   const long pairs = (items + 1) / 2;
   const long grid = pairs < sms() ? pairs : sms();
-  k_xform_rt<<<(unsigned)grid, 2 * RT, smem, (cudaStream_t)stream>>>(static_cast<const uint8_t*>(tpack), Mp, Kp, in,
+  ffno::launch(k_xform_rt, (unsigned)grid, 2 * RT, smem, (cudaStream_t)stream, static_cast<const uint8_t*>(tpack), Mp, Kp, in,
                                                                     out, d, nbi, nshift, ntn, items, accumulate, err);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
@@ -974,7 +983,7 @@ int ffno_spectral_mix_tc(const float* in, float* out, long F, long nb, long sf, 
   case CC: {                                                                                                      \
     if (!ffno::smem_cap_ok(k_mix_tc<CC>, smem)) \
       return FFNO_ELAUNCH;                                                                                        \
-    k_mix_tc<CC><<<(unsigned)grid, XT, smem, s>>>(map, out, F, nb, sf, sb, s_im, static_cast<const uint8_t*>(wpack), \
+    ffno::launch(k_mix_tc<CC>, (unsigned)grid, XT, smem, s, map, out, F, nb, sf, sb, s_im, static_cast<const uint8_t*>(wpack), \
                                                  g, U, Vm, rank, geo, err);                                       \
     break;                                                                                                        \
   }
@@ -1012,10 +1021,10 @@ int ffno_outer_tc_ld(const float* A, long lda, int Ma, const float* B, long ldb,
   const long n = (long)Ma * Mb;
   cudaStream_t s = (cudaStream_t)stream;
   if (trans)
-    k_outer_tc<<<nsplit, OT, smem, s>>>(B, ldb, Mb, A, lda, Ma, N, TI, NB, NS, cps, part, n, 1, Mb, err);
+    ffno::launch(k_outer_tc, nsplit, OT, smem, s, B, ldb, Mb, A, lda, Ma, N, TI, NB, NS, cps, part, n, 1, Mb, err);
   else
-    k_outer_tc<<<nsplit, OT, smem, s>>>(A, lda, Ma, B, ldb, Mb, N, TI, NB, NS, cps, part, n, Mb, 1, err);
-  k_outer_tc_reduce<<<(unsigned)((n + RD_EL - 1) / RD_EL), RD_EL * RD_SEGS, 0, s>>>(part, nsplit, n, Mb, ldo, out, accumulate);
+    ffno::launch(k_outer_tc, nsplit, OT, smem, s, A, lda, Ma, B, ldb, Mb, N, TI, NB, NS, cps, part, n, Mb, 1, err);
+  ffno::launch(k_outer_tc_reduce, (unsigned)((n + RD_EL - 1) / RD_EL), RD_EL * RD_SEGS, 0, s, part, nsplit, n, Mb, ldo, out, accumulate);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
