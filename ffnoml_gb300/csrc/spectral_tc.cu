@@ -43,8 +43,6 @@ __device__ __forceinline__ bool bounded(bool ok, int* err, int code) {
 // CTA take alternate items, each with two data stages (double-buffered against the MMAs), 256 tensor-memory columns
 // and its own mbarriers; the table is shared. Every wait is bounded.
 constexpr int RT = 256;                     // threads per pipeline
-constexpr int RKC = 64;                     // data rows k per chunk
-constexpr uint32_t RSB = 128u * RKC * 2;    // one split half of a data stage
 constexpr int RT_MAXK = 512;                // largest padded K of a resident table
 
 __device__ __forceinline__ void rt_sync(int pipe) { asm volatile("bar.sync %0, %1;" ::"r"(1 + pipe), "n"(RT) : "memory"); }
@@ -65,9 +63,7 @@ __device__ __forceinline__ bool rt_sync_and(int pipe, bool p) {
 // Row k0 + kr of piece u is kr = 8 (2u + (w >> 2)) + (lane & 7); the columns nf..nf+7 depend on the thread only.
 // NP pieces a thread: NP x 32 bytes in flight, the whole chunk of 16 NP rows per pipeline (NP = 4: the 64-row chunks
 // of k_xform_rt; NP = 2: the 32-row chunks of k_xform_st). hb: bytes of one split half of the stage.
-constexpr int XFB8 = 4;
-static_assert(XFB8 * RT * 8 == RKC * 128, "the pieces of a pipeline cover a whole chunk");
-static_assert(2 * RT * 8 == XKC * 128, "the pieces of a pipeline cover a whole streamed chunk");
+static_assert(2 * RT * 8 == 32 * 128, "the pieces of a pipeline cover a whole chunk");
 
 __device__ __forceinline__ int xf_fill_col(int ptid, int lane) { return 8 * (4 * ((ptid >> 5) & 3) + (lane >> 3)); }
 
@@ -100,27 +96,30 @@ __device__ __forceinline__ void xf_fill_chunk(uint8_t* st, uint32_t hb, const fl
   }
 }
 
-__global__ void __launch_bounds__(2 * RT, 1)
+template <int NPP, int KC>
+__global__ void __launch_bounds__(NPP * RT, 1)
     k_xform_rt(const uint8_t* __restrict__ tpack, int Mp, int Kp, const float* __restrict__ in, float* __restrict__ out,
                ffno_xform_desc d, int nbi, int nshift, long ntn, long items, int accumulate, int* __restrict__ err) {
   griddep_wait();
+  constexpr uint32_t RSB = 128u * KC * 2;    // one split half of a data stage
+  constexpr uint32_t PC = NPP == 2 ? 256u : NPP == 3 ? 160u : 128u;   // tensor-memory columns of a pipeline
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t TB = (uint32_t)Mp * Kp * 2;                 // one split half of the table
   uint8_t* sT = base;
   uint8_t* sD = base + ((2 * TB + 1023u) & ~1023u);          // [pipe][stage][hi | lo]
-  __shared__ uint64_t bar_t, bar_m[2][2];
+  __shared__ uint64_t bar_t, bar_m[NPP][2];
   __shared__ uint32_t tslot;
   __shared__ long row_in[RT_MAXK], row_out[256];   // element offsets of data row k and output row m
   const int tid = threadIdx.x, pipe = tid / RT, ptid = tid % RT, warp = tid >> 5, lane = tid & 31;
   const int q = warp & 3, half = ptid >> 7;
-  for (int k = tid; k < Kp; k += 2 * RT) row_in[k] = (long)(k / d.in_split) * d.in_hi + (long)(k % d.in_split) * d.in_lo;
-  for (int m = tid; m < Mp; m += 2 * RT)
+  for (int k = tid; k < Kp; k += NPP * RT) row_in[k] = (long)(k / d.in_split) * d.in_hi + (long)(k % d.in_split) * d.in_lo;
+  for (int m = tid; m < Mp; m += NPP * RT)
     row_out[m] = (long)(m / d.out_split) * d.out_hi + (long)(m % d.out_split) * d.out_lo;
   if (warp == 0) tc::tmem_alloc(&tslot, 512);
   if (tid == 0) {
     tc::mbar_init(&bar_t, 1);
-    for (int i = 0; i < 4; ++i) tc::mbar_init(&bar_m[i >> 1][i & 1], 1);
+    for (int i = 0; i < 2 * NPP; ++i) tc::mbar_init(&bar_m[i >> 1][i & 1], 1);
     tc::mbar_init_fence();
     tc::mbar_arrive_expect_tx(&bar_t, 2 * TB);
     for (uint32_t off = 0; off < 2 * TB; off += 32768u)
@@ -130,16 +129,16 @@ __global__ void __launch_bounds__(2 * RT, 1)
   __syncthreads();
   tc::tc_after_sync();
   griddep_launch();
-  const uint32_t tmem = tslot + (uint32_t)pipe * 256u;
+  const uint32_t tmem = tslot + (uint32_t)pipe * PC;
   const uint32_t lq = (uint32_t)(32 * q) << 16;
   bool ok = __syncthreads_and(tc::mbar_wait(&bar_t, 0)) != 0;
   if (!ok && tid == 0) atomicExch(err, 1);
-  const int nch = (Kp + RKC - 1) / RKC;
+  const int nch = (Kp + KC - 1) / KC;
   const uint32_t idesc = tc::idesc_bf16_ab(128, Mp, true, false);
   const uint32_t t_hi = tc::smem_u32(sT), t_lo = t_hi + TB;
   uint32_t g = 0;                                            // chunks issued by this pipeline
   const int n_ep = 32 * q + lane;                            // epilogue column of this thread
-  for (long it = 2L * blockIdx.x + pipe; ok && it < items; it += 2L * gridDim.x) {
+  for (long it = (long)NPP * blockIdx.x + pipe; ok && it < items; it += (long)NPP * gridDim.x) {
     long bfirst, n0;
     if (nbi > 1) {
       bfirst = it * nbi;
@@ -167,13 +166,13 @@ __global__ void __launch_bounds__(2 * RT, 1)
     const float* fsrc = in + foff;
     for (int ch = 0; ch < nch; ++ch, ++g) {
       const int s = (int)(g & 1u);
-      const int k0 = ch * RKC, kc = (Kp - k0) < RKC ? (Kp - k0) : RKC;
+      const int k0 = ch * KC, kc = (Kp - k0) < KC ? (Kp - k0) : KC;
       if (g >= 2) {
         const bool w = tc::mbar_wait(&bar_m[pipe][s], ((g - 2) >> 1) & 1u);
         if (!(ok = rt_sync_and(pipe, w))) break;
       }
       uint8_t* st = sD + (uint32_t)(pipe * 2 + s) * 2u * RSB;
-      xf_fill_chunk<XFB8>(st, RSB, fsrc, fv, row_in, d.K, k0, kc, ptid, lane, nf);
+      xf_fill_chunk<KC / 16>(st, RSB, fsrc, fv, row_in, d.K, k0, kc, ptid, lane, nf);
       tc::fence_async_smem();
       tc::tc_before_sync();
       rt_sync(pipe);
@@ -915,13 +914,18 @@ int ffno_xform_tcr(const void* tpack, int Mp, int Kp, const float* in, float* ou
   }
   const long ntn = (d.N + 127) / 128;
   const long items = nbi > 1 ? (d.nb + nbi - 1) / nbi : d.nb * ntn;
-  const size_t smem = 1024 + (((size_t)Mp * Kp * 4 + 1023) & ~(size_t)1023) + 4 * 2 * (size_t)RSB;
-  if (!ffno::smem_cap_ok(k_xform_rt, smem))
-    return FFNO_ELAUNCH;
-  const long pairs = (items + 1) / 2;
-  const long grid = pairs < sms() ? pairs : sms();
-  ffno::launch(k_xform_rt, (unsigned)grid, 2 * RT, smem, (cudaStream_t)stream, static_cast<const uint8_t*>(tpack), Mp, Kp, in,
-                                                                    out, d, nbi, nshift, ntn, items, accumulate, err);
+  auto go = [&](auto kernel, int npp, int kc) {
+    const size_t smem = 1024 + (((size_t)Mp * Kp * 4 + 1023) & ~(size_t)1023) + (size_t)npp * 2 * 2 * 128 * kc * 2;
+    if (!ffno::smem_cap_ok(kernel, smem)) return false;
+    const long groups = (items + npp - 1) / npp;
+    const long grid = groups < sms() ? groups : sms();
+    ffno::launch(kernel, (unsigned)grid, npp * RT, smem, (cudaStream_t)stream, static_cast<const uint8_t*>(tpack), Mp, Kp,
+                 in, out, d, nbi, nshift, ntn, items, accumulate, err);
+    return true;
+  };
+  const bool ok = Mp <= 128 ? go(k_xform_rt<4, 32>, 4, 32)
+                            : Mp <= 160 ? go(k_xform_rt<3, 32>, 3, 32) : go(k_xform_rt<2, 64>, 2, 64);
+  if (!ok) return FFNO_ELAUNCH;
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
