@@ -990,10 +990,10 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
           tc::split_pack(y[0], y[1], hi[2 * cc], lo[2 * cc]);
           tc::split_pack(y[2], y[3], hi[2 * cc + 1], lo[2 * cc + 1]);
         }
-        tc::mbar_arrive(&stg_empty[st]);
         const uint32_t A = tmem + lq + 32u * sl;
         tc::tmem_st16u(A, hi);
         tc::tmem_st16u(A + 16u, lo);
+        tc::mbar_arrive(&stg_empty[st]);   // after the stores: their operands prove that the loads have returned
         tc::tmem_wait_st();
         tc::tc_before_sync();
         tc::mbar_arrive(&sl_full[sl]);
@@ -1272,12 +1272,12 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
 #pragma unroll
           for (int e = 0; e < 4; ++e) b[4 * cc + e] *= gg[e];
         }
-        tc::mbar_arrive(&stg_empty[st]);
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) tc::split_pack(b[2 * e], b[2 * e + 1], hi[e], lo[e]);
         tc::tmem_st16u(tmem + lq + 32u * sl, hi);
         tc::tmem_st16u(tmem + lq + 32u * sl + 16u, lo);
+        tc::mbar_arrive(&stg_empty[st]);   // after the stores: their operands prove that the loads have returned
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {   // residual (B[c] + B[C + c]) / 2 in D2
           float rr[16];
