@@ -5,16 +5,20 @@
 // HBM reads, format conversion, tensor-core MMAs and the two epilogues of different tiles overlap:
 //   warp 0       TMA: FP32 tiles of a and pre_bar ([128 voxels][32 channels] boxes, 128-byte swizzle) into a
 //                two-stage shared-memory ring;
-//   warp 1       MMA issue (one thread): GEMM1 D1 = a W1^T and GEMM2 D2 = pre_bar W2, then GEMM3 D3 = G W1;
+//   warp 1       MMA issue (one thread): GEMM1 D1 = a W1^T and GEMM2 D2 = pre_bar W2, then GEMM3 D3 = G W1 of the tile
+//                before;
 //   warps 2-5    conversion: FP32 rows from the ring -> split BF16 (hi = bf16(x), lo = bf16(x - hi)) written straight
 //                into tensor memory, where they are the A operands of GEMM1/2 (lane = voxel);
 //   warps 6-13   epilogue 1: G = D2 * gelu'(D1), split and written back over D1 (per 16-feature chunk: 8 columns hi,
 //                8 columns lo), the A operand of GEMM3;
 //   warps 14-17  epilogue 2: a_bar = base + D3 to HBM.
-// Tensor memory (512 columns): two A stages of 128 columns [a hi | a lo | pre_bar hi | pre_bar lo] (D3 of the stage's
-// tile lands over its a half), D1 at 256, D2 at 384. Every wait is bounded; a time-out records a code in *err, the
-// role stops, the others run into their own bounded waits, and the CTA frees tensor memory only after the last MMA
-// commit and every issued TMA copy have been waited for.
+// Tensor memory (512 columns at C = 64): two operand slots of one 32-channel phase (16 columns hi, 16 lo), which GEMM1
+// and GEMM2 take as they fill, two D1 buffers (2C), D2 (2C) and D3 (C). A tile's chain is GEMM2 -> epilogue 1 -> the next
+// tile's GEMM2 (D2 is single); GEMM1 of the next tile, GEMM3 of this one and epilogue 2 run beside it. (With whole-tile
+// operand stages there is room for one D1 only, and GEMM1 waited for GEMM3 of the tile before: 2.4 M voxels, C = 64: 0.64
+// -> 0.54 ms in a VJP.) Every wait is bounded; a time-out records a code in *err, the role stops, the others run into their own
+// bounded waits, and the CTA frees tensor memory only after the last MMA commit and every issued TMA copy have been
+// waited for.
 #include "common.cuh"
 #include "tc.cuh"
 #include "ws.h"
@@ -33,12 +37,11 @@ constexpr int W_TMA = 0, W_MMA = 1, W_CVT = 2, W_E1 = 6, W_E2 = 14;
 // a thread.
 constexpr int F_NTHREADS = 22 * 32, F_E1 = 10, F_E2 = 18;
 constexpr uint32_t BOX_BYTES = TM * 32 * 4;   // one [128][32] FP32 box
-constexpr uint32_t D1 = 256, D2 = 384;        // accumulator columns
 
 __host__ __device__ constexpr uint32_t mat_bytes(int R, int K) { return (uint32_t)R * K * 2 * 2; }
 
 struct Bars {
-  uint64_t stg_full[2], stg_empty[2], a_full[2], a_empty[2], d3_full[2], d_full, g_full, w;
+  uint64_t stg_full[2], stg_empty[2], sl_full[2], sl_empty[2], d3_full, d3_free, d_full, g_full, w;
 };
 
 constexpr uint64_t WAIT_NS = 1000000000ull;   // one second: every legitimate wait here lasts microseconds
@@ -84,6 +87,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* ring = smem + WB;
+  constexpr int NPH = 2 * NB, NSL = 2;           // operand phases of a tile (a, then pre_bar); slots of one phase
+  constexpr uint32_t TD1 = 32 * NSL, TD2 = TD1 + 4 * C, TD3 = TD2 + 2 * C;
+  static_assert(TD3 + C <= 512, "tensor memory");
   __shared__ Bars bars;
   __shared__ uint32_t tslot;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -92,10 +98,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     for (int s = 0; s < 2; ++s) {
       tc::mbar_init(&bars.stg_full[s], 1);
       tc::mbar_init(&bars.stg_empty[s], 128);
-      tc::mbar_init(&bars.a_full[s], 128);
-      tc::mbar_init(&bars.a_empty[s], 128);
-      tc::mbar_init(&bars.d3_full[s], 1);
+      tc::mbar_init(&bars.sl_full[s], 128);
+      tc::mbar_init(&bars.sl_empty[s], 1);
     }
+    tc::mbar_init(&bars.d3_full, 1);
+    tc::mbar_init(&bars.d3_free, 128);
     tc::mbar_init(&bars.d_full, 1);
     tc::mbar_init(&bars.g_full, 256);
     tc::mbar_init(&bars.w, 1);
@@ -141,46 +148,52 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const uint32_t w1 = tc::smem_u32(smem), w2t = w1 + B1, w1t = w1 + 2 * B1, LO = B1 / 2;
     uint64_t* last = nullptr;   // the last commit's barrier and phase parity, waited for before exit
     uint32_t last_par = 0;
-    bool last_seen = true;
-    for (int i = 0; i < niter; ++i) {
-      const int s = i & 1;
-      const uint32_t n = (uint32_t)i >> 1;
-      if (!wait_or_flag(&bars.a_full[s], n & 1u, err, 4)) break;
-      if (i > 0) {   // GEMM3 of the previous tile has read G out of D1
-        if (!wait_or_flag(&bars.d3_full[(i - 1) & 1], ((uint32_t)(i - 1) >> 1) & 1u, err, 5)) break;
-        last_seen = true;
+    bool alive = true;
+    auto commit = [&](uint64_t* bar, uint32_t par) {
+      tc::mma_commit(bar);
+      last = bar;
+      last_par = par;
+    };
+    auto half = [&](int i, int ph0, uint32_t D, uint32_t w) {   // D = (operand of NB phases) x w^T, as the slots fill
+      for (int ph = ph0; ph < ph0 + NB; ++ph) {
+        const int u = i * NPH + ph, sl = u % NSL;
+        const uint32_t n = (uint32_t)(u / NSL) & 1u;
+        if (!wait_or_flag(&bars.sl_full[sl], n, err, 4)) return false;
+        tc::tc_after_sync();
+        const uint32_t A = tmem + 32u * sl;
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          const uint32_t k = (uint32_t)(2 * (ph - ph0) + kk);
+          mma3_ta(D, A + 8u * kk, A + 16u + 8u * kk, tc::kmajor_desc(w + 256u * k, 128u, C * 16u),
+                  tc::kmajor_desc(w + LO + 256u * k, 128u, C * 16u), i12, k > 0);
+        }
+        commit(&bars.sl_empty[sl], n);
       }
+      return true;
+    };
+    auto gemm3 = [&](int t) {   // D3 = G(t) W1, G in D1[t % 2]; epilogue 2 of tile t - 1 has read D3
+      if (t >= 1 && !wait_or_flag(&bars.d3_free, (uint32_t)(t - 1) & 1u, err, 5)) return false;
       tc::tc_after_sync();
-      const uint32_t A = tmem + (uint32_t)(128 * s);
+      const uint32_t g = tmem + TD1 + (uint32_t)(2 * C * (t & 1));
 #pragma unroll 1
-      for (int k = 0; k < C / 16; ++k) {
-        const uint32_t ah = A + 8u * k, al = A + C / 2 + 8u * k;
-        const uint32_t ph = A + C + 8u * k, pl = A + C + C / 2 + 8u * k;
-        const uint32_t bo = 256u * k;
-        mma3_ta(tmem + D1, ah, al, tc::kmajor_desc(w1 + bo, 128u, C * 16u), tc::kmajor_desc(w1 + LO + bo, 128u, C * 16u),
-                i12, k > 0);
-        mma3_ta(tmem + D2, ph, pl, tc::kmajor_desc(w2t + bo, 128u, C * 16u),
-                tc::kmajor_desc(w2t + LO + bo, 128u, C * 16u), i12, k > 0);
-      }
-      tc::mma_commit(&bars.d_full);
-      last = &bars.d_full;
-      last_par = (uint32_t)i & 1u;
-      last_seen = false;
-      if (!wait_or_flag(&bars.g_full, (uint32_t)i & 1u, err, 6)) break;
-      tc::tc_after_sync();
-#pragma unroll 1
-      for (int j = 0; j < 2 * C / 16; ++j) {
-        const uint32_t bo = 256u * j;
-        mma3_ta(tmem + (uint32_t)(128 * s), tmem + D1 + 16u * j, tmem + D1 + 16u * j + 8u,
-                tc::kmajor_desc(w1t + bo, 128u, 2 * C * 16u), tc::kmajor_desc(w1t + LO + bo, 128u, 2 * C * 16u), i3,
-                j > 0);
-      }
-      tc::mma_commit(&bars.d3_full[s]);
-      last = &bars.d3_full[s];
-      last_par = n & 1u;
-      last_seen = false;
+      for (int k = 0; k < 2 * C / 16; ++k)
+        mma3_ta(tmem + TD3, g + 16u * k, g + 16u * k + 8u, tc::kmajor_desc(w1t + 256u * k, 128u, 2 * C * 16u),
+                tc::kmajor_desc(w1t + LO + 256u * k, 128u, 2 * C * 16u), i3, k > 0);
+      commit(&bars.d3_full, (uint32_t)t & 1u);
+      return true;
+    };
+    for (int i = 0; i < niter && alive; ++i) {
+      // GEMM3 of tile i - 2 has read G out of D1[i % 2]
+      if (i >= 2 && !wait_or_flag(&bars.d3_full, (uint32_t)(i - 2) & 1u, err, 11)) break;
+      if (!half(i, 0, tmem + TD1 + (uint32_t)(2 * C * (i & 1)), w1)) break;
+      // epilogue 1 of tile i - 1 has read D2 and written G
+      if (i >= 1 && !wait_or_flag(&bars.g_full, (uint32_t)(i - 1) & 1u, err, 6)) break;
+      if (!half(i, NB, tmem + TD2, w2t)) break;
+      commit(&bars.d_full, (uint32_t)i & 1u);
+      if (i >= 1 && !gemm3(i - 1)) break;
+      if (i == niter - 1) alive = wait_or_flag(&bars.g_full, (uint32_t)i & 1u, err, 6) && gemm3(i);
     }
-    if (last && !last_seen) tc::mbar_wait_for(last, last_par, WAIT_NS);   // no MMA in flight when tensor memory is freed
+    if (last) tc::mbar_wait_for(last, last_par, WAIT_NS);   // no MMA in flight when tensor memory is freed
   } else if (ok && warp >= W_CVT && warp < W_E1) {
     const int q = warp & 3, r = 32 * q + lane;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
@@ -188,29 +201,32 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const int s = i & 1;
       const uint32_t n = (uint32_t)i >> 1;
       if (!warp_wait(&bars.stg_full[s], n & 1u, err, 7)) break;
-      if (!warp_wait(&bars.a_empty[s], (n & 1u) ^ 1u, err, 8)) break;
-      tc::tc_after_sync();
       const uint8_t* st = ring + s * SB;
-      const uint32_t A = tmem + lq + (uint32_t)(128 * s);
-#pragma unroll
-      for (int x = 0; x < 2; ++x)
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          const uint8_t* rowp = st + x * XB + b * BOX_BYTES + r * 128;
-          uint32_t hi[16], lo[16];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float4 v = *reinterpret_cast<const float4*>(rowp + ((c ^ (r & 7)) << 4));
-            tc::split_pack(v.x, v.y, hi[2 * c], lo[2 * c]);
-            tc::split_pack(v.z, v.w, hi[2 * c + 1], lo[2 * c + 1]);
-          }
-          tc::tmem_st16u(A + (uint32_t)(x * C + 16 * b), hi);
-          tc::tmem_st16u(A + (uint32_t)(x * C + C / 2 + 16 * b), lo);
+      bool alive = true;
+#pragma unroll 1
+      for (int ph = 0; ph < NPH; ++ph) {
+        const int u = i * NPH + ph, sl = u % NSL;
+        if (!warp_wait(&bars.sl_empty[sl], ((uint32_t)(u / NSL) & 1u) ^ 1u, err, 8)) {   // its MMAs have read the slot
+          alive = false;
+          break;
         }
-      tc::mbar_arrive(&bars.stg_empty[s]);
-      tc::tmem_wait_st();
-      tc::tc_before_sync();
-      tc::mbar_arrive(&bars.a_full[s]);
+        tc::tc_after_sync();
+        const uint8_t* rowp = st + ph * BOX_BYTES + r * 128;   // the boxes of a, then those of pre_bar
+        uint32_t hi[16], lo[16];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float4 v = *reinterpret_cast<const float4*>(rowp + ((c ^ (r & 7)) << 4));
+          tc::split_pack(v.x, v.y, hi[2 * c], lo[2 * c]);
+          tc::split_pack(v.z, v.w, hi[2 * c + 1], lo[2 * c + 1]);
+        }
+        tc::tmem_st16u(tmem + lq + 32u * sl, hi);
+        tc::tmem_st16u(tmem + lq + 32u * sl + 16u, lo);
+        tc::tmem_wait_st();
+        tc::tc_before_sync();
+        tc::mbar_arrive(&bars.sl_full[sl]);
+      }
+      if (!alive) break;
+      tc::mbar_arrive(&bars.stg_empty[s]);   // after the stores: their operands prove that the loads have returned
     }
   } else if (ok && warp >= W_E1 && warp < W_E2) {
     const int q = warp & 3, hf = (warp - W_E1) >> 2;
@@ -218,11 +234,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     for (int i = 0; i < niter; ++i) {
       if (!warp_wait(&bars.d_full, (uint32_t)i & 1u, err, 9)) break;
       tc::tc_after_sync();
+      const uint32_t D = tmem + lq + TD1 + (uint32_t)(2 * C * (i & 1));
 #pragma unroll 1
       for (int j = hf; j < 2 * C / 16; j += 2) {
         uint32_t h[16], gb[16];
-        tc::tmem_ld16u(tmem + lq + D1 + 16u * j, h);
-        tc::tmem_ld16u(tmem + lq + D2 + 16u * j, gb);
+        tc::tmem_ld16u(D + 16u * j, h);
+        tc::tmem_ld16u(tmem + lq + TD2 + 16u * j, gb);
         tc::tmem_wait_ld();
         uint32_t hi[8], lo[8];
 #pragma unroll
@@ -231,8 +248,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           mul_gelu_grad_tc2(__uint_as_float(h[2 * e]), __uint_as_float(h[2 * e + 1]), g0, g1);
           tc::split_pack(g0, g1, hi[e], lo[e]);
         }
-        tc::tmem_st8u(tmem + lq + D1 + 16u * j, hi);
-        tc::tmem_st8u(tmem + lq + D1 + 16u * j + 8u, lo);
+        tc::tmem_st8u(D + 16u * j, hi);
+        tc::tmem_st8u(D + 16u * j + 8u, lo);
       }
       tc::tmem_wait_st();
       tc::tc_before_sync();
@@ -242,8 +259,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int q = warp & 3, r = 32 * q + lane;
     const uint32_t lq = (uint32_t)(32 * q) << 16;
     for (int i = 0; i < niter; ++i) {
-      const int s = i & 1;
-      const uint32_t n = (uint32_t)i >> 1;
       const long v = tile_of(i) * TM + r;
       const bool live = v < V;
       float bv[C];
@@ -256,16 +271,16 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           for (int e = 0; e < 8; ++e) bv[c + e] = 0.f;
         }
       }
-      if (!warp_wait(&bars.d3_full[s], n & 1u, err, 10)) break;
+      if (!warp_wait(&bars.d3_full, (uint32_t)i & 1u, err, 10)) break;
       tc::tc_after_sync();
 #pragma unroll
       for (int k = 0; k < C / 16; ++k) {
         uint32_t d[16];
-        tc::tmem_ld16u(tmem + lq + (uint32_t)(128 * s + 16 * k), d);
+        tc::tmem_ld16u(tmem + lq + TD3 + 16u * k, d);
         tc::tmem_wait_ld();
-        if (k == C / 16 - 1) {   // the stage's tensor memory is free once D3 is in registers
+        if (k == C / 16 - 1) {   // D3 is free once its last columns are in registers
           tc::tc_before_sync();
-          tc::mbar_arrive(&bars.a_empty[s]);
+          tc::mbar_arrive(&bars.d3_free);
         }
         if (live) {
           float o[16];
