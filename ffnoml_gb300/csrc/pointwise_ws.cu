@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          const float4 v = *reinterpret_cast<const float4*>(rowp + ((c ^ (r & 7)) << 4));
+          const float4 v = tc::lds4(rowp + ((c ^ (r & 7)) << 4));
           tc::split_pack(v.x, v.y, hi[2 * c], lo[2 * c]);
           tc::split_pack(v.z, v.w, hi[2 * c + 1], lo[2 * c + 1]);
         }
@@ -457,9 +457,9 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
         for (int cc = 0; cc < 4; ++cc) {
           const int c = 4 * (bh & 1) + cc;
           const uint32_t o = (uint32_t)((c ^ (r & 7)) << 4);
-          float4 x = *reinterpret_cast<const float4*>(rin + o);
+          float4 x = tc::lds4(rin + o);
           if (MODE != 0) {
-            const float4 p = *reinterpret_cast<const float4*>(rin + XB + o);
+            const float4 p = tc::lds4(rin + XB + o);
             const int k = 32 * b + 4 * c;
             float y[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
           const int c = 4 * (bh & 1) + cc;
-          const float4 v = *reinterpret_cast<const float4*>(rin + ((c ^ (r & 7)) << 4));
+          const float4 v = tc::lds4(rin + ((c ^ (r & 7)) << 4));
           tc::split_pack(v.x, v.y, hi[2 * cc], lo[2 * cc]);
           tc::split_pack(v.z, v.w, hi[2 * cc + 1], lo[2 * cc + 1]);
         }
@@ -990,6 +990,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc) {
+          // (not tc::lds4: 1.34 ms with this, 1.41 with that, at 4.2 M voxels)
           const float4 p = *reinterpret_cast<const float4*>(rp + ((cc ^ (r & 7)) << 4));
           float y[4] = {p.x, p.y, p.z, p.w};
           if (t > 0) {
@@ -1274,8 +1275,8 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
 #pragma unroll
         for (int cc = 0; cc < 8; ++cc) {
           const uint32_t o = (uint32_t)((cc ^ (r & 7)) << 4);
-          const float4 p = *reinterpret_cast<const float4*>(rp + o);
-          const float4 g = *reinterpret_cast<const float4*>(rp + BOX_BYTES + o);
+          const float4 p = tc::lds4(rp + o);
+          const float4 g = tc::lds4(rp + BOX_BYTES + o);
           const float pp[4] = {p.x, p.y, p.z, p.w}, gg[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -1563,7 +1564,7 @@ __global__ void __launch_bounds__(448, 1)
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
           const int c = 4 * (bh & 1) + cc;
-          const float4 v = *reinterpret_cast<const float4*>(rin + ((c ^ (r & 7)) << 4));
+          const float4 v = tc::lds4(rin + ((c ^ (r & 7)) << 4));
           tc::split_pack(v.x, v.y, hi[2 * cc], lo[2 * cc]);
           tc::split_pack(v.z, v.w, hi[2 * cc + 1], lo[2 * cc + 1]);
         }
@@ -1667,8 +1668,8 @@ __global__ void __launch_bounds__(448, 1)
 #pragma unroll
           for (int cc = 0; cc < 4; ++cc) {
             const uint32_t off = (uint32_t)(((4 * (k & 1) + cc) ^ (r & 7)) << 4);
-            const float4 xv = *reinterpret_cast<const float4*>(rx + off);
-            const float4 gv = *reinterpret_cast<const float4*>(rx + XB + off);
+            const float4 xv = tc::lds4(rx + off);
+            const float4 gv = tc::lds4(rx + XB + off);
             const float xx[4] = {xv.x, xv.y, xv.z, xv.w}, gg[4] = {gv.x, gv.y, gv.z, gv.w};
             const float* bb = bv + 16 * k + 4 * cc;
             float qv[4];
