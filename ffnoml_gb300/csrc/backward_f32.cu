@@ -647,7 +647,8 @@ __global__ void __launch_bounds__(NT, 3) k_gate_bwd(const float* __restrict__ x,
 }
 
 // ------------------------------------------------------------------------------------------------ lift backward
-// x_in_bar[k][v] += sum_c pre_bar[v][c] w_lift[k][c]
+// x_in_bar[k][v] += sum_c pre_bar[v][c] w_lift[k][c]. The grid fills the SMs (seven or eight CTAs of 17-25 KB each): with
+// half of that, CTAs placed early piled up on half of the SMs (2.4 M voxels, C = 64: 588 us; full: 300).
 template <int C>
 __global__ void __launch_bounds__(NT) k_lift_bwd(const float* __restrict__ pb, int cin, long V,
                                                  const float* __restrict__ wl, float* __restrict__ xib) {
@@ -961,7 +962,7 @@ int ffno_gn_bwd_stats(int mode, const float* u, float r, const float* pre, const
   if (groups == GMAX && C <= 64 &&
       (reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(pre)) % 32 == 0) {   // 32-byte lanes
     switch (C) {
-#define L(CC) case CC: ffno::launch(k_gn_bwd_stats8<CC>, grid, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, V, partials, nparts); break;
+#define L(CC) case CC: ffno::launch_if(ffno::early_launch(V, CC), k_gn_bwd_stats8<CC>, grid, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, V, partials, nparts); break;
       L(16) L(32) L(64)
 #undef L
     }
@@ -998,7 +999,7 @@ int ffno_gn_bwd_apply(int mode, const float* u, float r, const float* pre, const
   const int cpg = C / groups;
   const int blocks = grid_of(V, 8 * 8, 4);
   switch (C) {
-#define L(CC) case CC: ffno::launch(k_gn_bwd_apply<CC>, blocks, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, sums, dw, V, pre_bar, w_bar, cpg, groups, eps); break;
+#define L(CC) case CC: ffno::launch_if(ffno::early_launch(V, CC), k_gn_bwd_apply<CC>, blocks, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, sums, dw, V, pre_bar, w_bar, cpg, groups, eps); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -1086,7 +1087,7 @@ int ffno_lift_bwd(const float* pre_bar, int cin, long V, int C, const float* w_l
   if (!pre_bar || !w_lift || !x_in_bar || !width_ok(C) || V < 1 || cin < 1 || cin > 8) return FFNO_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   switch (C) {
-#define L(CC) case CC: ffno::launch(k_lift_bwd<CC>, grid_of(V, BM, 4), NT, 0, s, pre_bar, cin, V, w_lift, x_in_bar); break;
+#define L(CC) case CC: ffno::launch(k_lift_bwd<CC>, grid_of(V, BM, CC <= 64 ? 8 : 7), NT, 0, s, pre_bar, cin, V, w_lift, x_in_bar); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
@@ -1152,7 +1153,7 @@ int ffno_outer(const float* A, long lda, int Ma, const float* B, long ldb, int M
   cudaStream_t s = (cudaStream_t)stream;
   ffno::launch(k_outer, (unsigned)((long)ti * tj * nsplit), NT, 0, s, A, lda, Ma, B, ldb, Mb, N, chunk, ti, tj, part);
   const long n = (long)Ma * Mb;
-  ffno::launch(k_outer_reduce, (unsigned)((n + OR_EL - 1) / OR_EL), OR_EL * OR_SEGS, 0, s, part, nsplit, n, out, accumulate);
+  ffno::launch_if(false, k_outer_reduce, (unsigned)((n + OR_EL - 1) / OR_EL), OR_EL * OR_SEGS, 0, s, part, nsplit, n, out, accumulate);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }
@@ -1206,7 +1207,7 @@ int ffno_outer_noalloc(const float* A, long lda, int Ma, const float* B, long ld
   cudaStream_t s = (cudaStream_t)stream;
   // every partial sum the reduction reads is written first by k_outer: nothing in the scratch has to start at zero
   ffno::launch(k_outer, (unsigned)((long)ti * tj * nsplit), NT, 0, s, A, lda, Ma, B, ldb, Mb, N, chunk, ti, tj, scratch);
-  ffno::launch(k_outer_reduce, (unsigned)((n + OR_EL - 1) / OR_EL), OR_EL * OR_SEGS, 0, s, scratch, nsplit, n, out, accumulate);
+  ffno::launch_if(false, k_outer_reduce, (unsigned)((n + OR_EL - 1) / OR_EL), OR_EL * OR_SEGS, 0, s, scratch, nsplit, n, out, accumulate);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;
 }

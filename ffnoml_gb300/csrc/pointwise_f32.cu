@@ -648,7 +648,11 @@ int ffno_gn_finalize(const double* partials, int nparts, int C, int groups, cons
                      float eps, float* coefs, double* gstats, ffno_stream_t stream) {
   if (!partials || !gamma || !beta || !coefs) return FFNO_EINVAL;
   if (nparts < 1 || C < 1 || groups < 1 || groups > GMAX || C % groups) return FFNO_EINVAL;
-  ffno::launch(k_gn_finalize, groups, FIN_NT, 0, (cudaStream_t)stream, partials, nparts, C, groups, gamma, beta, eps, coefs,
+  // more than half of an SM's shared memory, unused: the CTAs are FP64-bound, and placed together on the SM that frees up
+  // first they took up to 25 us (width 96) instead of 9
+  const size_t apart = 116 * 1024;
+  if (!ffno::smem_cap_ok(k_gn_finalize, apart)) return FFNO_ELAUNCH;
+  ffno::launch(k_gn_finalize, groups, FIN_NT, apart, (cudaStream_t)stream, partials, nparts, C, groups, gamma, beta, eps, coefs,
                                                              gstats);
   FFNO_CHECK_LAUNCH();
   return FFNO_OK;

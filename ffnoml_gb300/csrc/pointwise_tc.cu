@@ -2407,7 +2407,7 @@ int ffno_fuse_out_tc(const float* spec_pre, const float* spec_coefs, const float
     return FFNO_EINVAL;
   const size_t smem = mat_bytes(C96, 2 * C96) + tile_bytes(KS);
   if (!launch_prep(k_fuse_out_tc96, smem)) return FFNO_ELAUNCH;
-  ffno::launch(k_fuse_out_tc96, nparts, PT, smem, (cudaStream_t)stream, spec_pre, spec_coefs, vert_pre, vert_coefs, gates, hf, V,
+  ffno::launch_if(ffno::early_launch(V, 96), k_fuse_out_tc96, nparts, PT, smem, (cudaStream_t)stream, spec_pre, spec_coefs, vert_pre, vert_coefs, gates, hf, V,
                                                               static_cast<const uint8_t*>(wpack), dw, pre, partials,
                                                               err);
   FFNO_CHECK_LAUNCH();
@@ -2495,7 +2495,7 @@ int ffno_gate_bwd_tc(const float* x, const float* g_bar, const float* base, long
     if (!aligned32(x)) return FFNO_EINVAL;
     const size_t smem = 2 * mat_bytes(C96, C96) + 2 * tile_bytes(C96);   // one pipeline; pack [g1, g2]
     if (!launch_prep(k_gate_bwd_tc<C96, 1>, smem)) return FFNO_ELAUNCH;
-    ffno::launch(k_gate_bwd_tc<C96, 1>, grid_tc(V), PT, smem, s, x, g_bar, base, V, static_cast<const uint8_t*>(wpack), zp,
+    ffno::launch_if(ffno::early_launch(V, C), k_gate_bwd_tc<C96, 1>, grid_tc(V), PT, smem, s, x, g_bar, base, V, static_cast<const uint8_t*>(wpack), zp,
                                                        x_bar, z_bar, err);
     FFNO_CHECK_LAUNCH();
     return FFNO_OK;

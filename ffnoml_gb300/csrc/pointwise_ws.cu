@@ -1767,7 +1767,7 @@ int launch_mlp2_fwd(const float* in, const float* prev, const float* pc, float r
   if (MODE != 0 ? !row_map(&mp, prev, V, C) : !row_map(&mp, in, V, C)) return FFNO_EINVAL;
   const size_t smem = 1024 + 2 * (size_t)mat_bytes(2 * C, C) + 2 * (size_t)((MODE == 0 ? 1 : 2) * (C / 32) * BOX_BYTES);
   if (!ffno::smem_cap_ok(k_mlp2_fwd_ws<C, MODE>, smem)) return FFNO_ELAUNCH;
-  ffno::launch(k_mlp2_fwd_ws<C, MODE>, nparts, F_NTHREADS, smem, s, mi, mp, pc, res, xout, V, static_cast<const uint8_t*>(wpack),
+  ffno::launch_if(ffno::early_launch(V, C), k_mlp2_fwd_ws<C, MODE>, nparts, F_NTHREADS, smem, s, mi, mp, pc, res, xout, V, static_cast<const uint8_t*>(wpack),
                                                          dw, pre, partials, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
@@ -1782,7 +1782,7 @@ int launch_gate_fwd(const float* x, long V, const void* wpack, const float* zp, 
     return FFNO_ELAUNCH;
   const long nt = (V + TM - 1) / TM;
   const int grid = (int)(nt < sms() ? nt : sms());
-  ffno::launch(k_gate_fwd_ws<C>, grid, NTHREADS, smem, s, mx, x, V, static_cast<const uint8_t*>(wpack), zp, z, out, err);
+  ffno::launch_if(ffno::early_launch(V, C), k_gate_fwd_ws<C>, grid, NTHREADS, smem, s, mx, x, V, static_cast<const uint8_t*>(wpack), zp, z, out, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
 
@@ -1796,7 +1796,7 @@ int launch_gate_bwd(const float* x, const float* gbar, const float* base, long V
     return FFNO_ELAUNCH;
   const long nt = (V + TM - 1) / TM;
   const int grid = (int)(nt < sms() ? nt : sms());
-  ffno::launch(k_gate_bwd_ws<C>, grid, 448, smem, s, mx, mg, base, V, static_cast<const uint8_t*>(wpack), zp, xbar, zbar, err);
+  ffno::launch_if(ffno::early_launch(V, C), k_gate_bwd_ws<C>, grid, 448, smem, s, mx, mg, base, V, static_cast<const uint8_t*>(wpack), zp, xbar, zbar, err);
   return cudaGetLastError() == cudaSuccess ? FFNO_OK : FFNO_ELAUNCH;
 }
 
