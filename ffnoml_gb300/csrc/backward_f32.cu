@@ -173,46 +173,84 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats(int mode, const float* __r
   stats_partial_rows<C, VW>(d1, d2, active, q, cpg, groups, nparts, partials);
 }
 
-// The statistics for eight groups and C <= 64 (cpg = C / 8 channels a group): lanes of 8 channels (one 32-byte request
-// a lane and tensor), whose channels fall in NG = 8 / cpg groups, so the partials are kept per group (one double pair
-// at C = 64) instead of per channel slot. Same partials layout and fixed reduction order as k_gn_bwd_stats.
+// upstream() of two channels: (r u) * act'(y), the activation known at compile time
+template <int MODE>
+__device__ __forceinline__ uint64_t upstream2(float u0, float u1, float r, uint64_t y) {
+  float a0 = r * u0, a1 = r * u1, y0, y1;
+  upk2(y, y0, y1);
+  if constexpr (MODE == 1) a0 *= gelu_grad(y0), a1 *= gelu_grad(y1);
+  if constexpr (MODE == 2) mul_gelu_grad_tc2(y0, y1, a0, a1);
+  return pk2(a0, a1);
+}
+
+// Lanes of the eight-group kernels: a lane's VW channels lie in NG groups of CPG channels (every CPG is even, so a pair
+// of channels never straddles two), whose constants stay in registers.
 template <int C>
-__global__ void __launch_bounds__(256) k_gn_bwd_stats8(int mode, const float* __restrict__ u, float r,
+struct Gn8 : GnLanes<C, 8> {
+  static constexpr int VW = GnLanes<C, 8>::VW, CPG = C / GMAX, NG = VW > CPG ? VW / CPG : 1;
+  static_assert(C % GMAX == 0 && CPG % 2 == 0 && (VW % CPG == 0 || CPG % VW == 0), "groups");
+};
+
+// The statistics for eight groups: a lane reads 32 bytes of a row and tensor per request (16 at C = 96) and keeps packed
+// partials per group, with the activation fixed at compile time. Bound by instruction issue more than by HBM: two
+// channels an instruction and no branch on the mode inside the loop. Mean of a VJP's calls: 2.4 M voxels, C = 64 (1.2 GB):
+// 216 -> 206 us; 1.0 M, C = 96 (0.8 GB): 205 -> 178 us.
+// Same partials layout and fixed reduction order as k_gn_bwd_stats.
+template <int C, int MODE>
+__global__ void __launch_bounds__(256, 2) k_gn_bwd_stats8(const float* __restrict__ u, float r,
                                                        const float* __restrict__ pre, const float* __restrict__ gamma,
                                                        const float* __restrict__ beta,
                                                        const double* __restrict__ gst, long V,
                                                        double* __restrict__ partials, int nparts) {
   griddep_sync();
-  static_assert(C == 16 || C == 32 || C == 64, "eight groups of C / 8 channels");
-  using Ln = GnLanes<C, 8>;
-  constexpr int VW = 8, CPG = C / GMAX, NG = VW / CPG;
+  using Ln = Gn8<C>;
+  constexpr int VW = Ln::VW, CPG = Ln::CPG, NG = Ln::NG;
+  constexpr bool POW2 = (Ln::LPV & (Ln::LPV - 1)) == 0;
   __shared__ GnConst k;
-  __shared__ double red[8][GMAX][2];
+  __shared__ double red[8][POW2 ? GMAX : 32][2];
   load_gn_const(k, gst, nullptr, GMAX, 0.f);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane / Ln::LPV, q = lane % Ln::LPV;   // every lane is active: LPV divides 32
+  const int sub = lane / Ln::LPV, q = lane % Ln::LPV;
+  const bool active = sub < Ln::VPW;   // C = 96: 24 lanes of a warp
   const int c = VW * q, g0 = c / CPG;
-  float gm[VW], bt[VW];
+  uint64_t gm[VW / 2], bt[VW / 2], nmean[NG], rstd[NG];
 #pragma unroll
-  for (int j = 0; j < VW; ++j) {
-    gm[j] = __ldg(gamma + c + j);
-    bt[j] = __ldg(beta + c + j);
+  for (int j = 0; j < VW / 2; ++j) {
+    gm[j] = active ? pk2(__ldg(gamma + c + 2 * j), __ldg(gamma + c + 2 * j + 1)) : 0;
+    bt[j] = active ? pk2(__ldg(beta + c + 2 * j), __ldg(beta + c + 2 * j + 1)) : 0;
   }
-  double d1[NG], d2[NG];
-  float f1[NG], f2[NG];
 #pragma unroll
-  for (int l = 0; l < NG; ++l) d1[l] = d2[l] = 0.0, f1[l] = f2[l] = 0.f;
+  for (int l = 0; l < NG; ++l) {
+    nmean[l] = pk2(-k.mean[g0 + l], -k.mean[g0 + l]);
+    rstd[l] = pk2(k.rstd[g0 + l], k.rstd[g0 + l]);
+  }
+  const uint64_t one = pk2(1.f, 1.f);
+  double d1[NG], d2[NG];
+  uint64_t f1[NG], f2[NG];
+#pragma unroll
+  for (int l = 0; l < NG; ++l) d1[l] = d2[l] = 0.0, f1[l] = f2[l] = 0;
+  auto fold = [&] {
+#pragma unroll
+    for (int l = 0; l < NG; ++l) {
+      float a, b;
+      upk2(f1[l], a, b);
+      d1[l] += a + b;
+      upk2(f2[l], a, b);
+      d2[l] += a + b;
+      f1[l] = f2[l] = 0;
+    }
+  };
   const long step = (long)gridDim.x * 8 * Ln::VPW;
-  constexpr int UN = 2;   // voxels a thread loaded before any is used: 128 bytes in flight
+  constexpr int UN = 16 / VW;   // voxels a thread loaded before any is used: 128 bytes in flight
   int n = 0;
-  for (long v0 = ((long)blockIdx.x * 8 + warp) * Ln::VPW + sub; v0 < V; v0 += UN * step) {
+  for (long v0 = ((long)blockIdx.x * 8 + warp) * Ln::VPW + sub; active && v0 < V; v0 += UN * step) {
     float pu[UN][VW], pp[UN][VW];
 #pragma unroll
     for (int e = 0; e < UN; ++e) {
       const long v = v0 + e * step;
       if (v < V) {
-        ffno::tc::ld8(u + v * C + c, pu[e]);
-        ffno::tc::ld8(pre + v * C + c, pp[e]);
+        ldv<VW>(u + v * C + c, pu[e]);
+        ldv<VW>(pre + v * C + c, pp[e]);
       } else {
 #pragma unroll
         for (int j = 0; j < VW; ++j) pu[e][j] = pp[e][j] = 0.f;
@@ -222,48 +260,51 @@ __global__ void __launch_bounds__(256) k_gn_bwd_stats8(int mode, const float* __
     for (int e = 0; e < UN; ++e) {
       if (v0 + e * step >= V) break;
 #pragma unroll
-      for (int j = 0; j < VW; ++j) {
-        const int l = j / CPG, g = g0 + l;
-        const float xh = (pp[e][j] - k.mean[g]) * k.rstd[g];
-        const float gh = upstream(mode, pu[e][j], r, xh * gm[j] + bt[j]) * gm[j];
-        f1[l] += gh;
-        f2[l] += gh * xh;
+      for (int j = 0; j < VW / 2; ++j) {
+        const int l = NG == 1 ? 0 : 2 * j / CPG;
+        const uint64_t xh = mul2(fma2(pk2(pp[e][2 * j], pp[e][2 * j + 1]), one, nmean[l]), rstd[l]);
+        const uint64_t gh = mul2(upstream2<MODE>(pu[e][2 * j], pu[e][2 * j + 1], r, fma2(xh, gm[j], bt[j])), gm[j]);
+        f1[l] = fma2(gh, one, f1[l]);
+        f2[l] = fma2(gh, xh, f2[l]);
       }
     }
-    if (++n == 8) {   // float partials go to double every 16 voxels, as in k_gn_bwd_stats
-#pragma unroll
-      for (int l = 0; l < NG; ++l) {
-        d1[l] += f1[l];
-        d2[l] += f2[l];
-        f1[l] = f2[l] = 0.f;
-      }
+    if (++n == 16 / UN) {   // float partials go to double every 16 voxels, as in k_gn_bwd_stats
+      fold();
       n = 0;
     }
   }
+  fold();
+  // sum over the lanes of a group in a warp, then over the warps, in a fixed order
+  if constexpr (POW2) {
 #pragma unroll
-  for (int l = 0; l < NG; ++l) {
-    d1[l] += f1[l];
-    d2[l] += f2[l];
-  }
-  // lanes with the same q hold the same groups: sum over the VPW voxels of a warp, then over the warps, in a fixed order
+    for (int l = 0; l < NG; ++l) {
 #pragma unroll
-  for (int l = 0; l < NG; ++l) {
-#pragma unroll
-    for (int o = 16; o >= Ln::LPV; o >>= 1) {
-      d1[l] += __shfl_xor_sync(0xffffffffu, d1[l], o);
-      d2[l] += __shfl_xor_sync(0xffffffffu, d2[l], o);
+      for (int o = 16; o >= Ln::LPV; o >>= 1) {
+        d1[l] += __shfl_xor_sync(0xffffffffu, d1[l], o);
+        d2[l] += __shfl_xor_sync(0xffffffffu, d2[l], o);
+      }
+      if (sub == 0) {
+        red[warp][g0 + l][0] = d1[l];
+        red[warp][g0 + l][1] = d2[l];
+      }
     }
-    if (sub == 0) {
-      red[warp][g0 + l][0] = d1[l];
-      red[warp][g0 + l][1] = d2[l];
-    }
+  } else {
+    red[warp][lane][0] = d1[0];
+    red[warp][lane][1] = d2[0];
   }
   __syncthreads();
   if (threadIdx.x < 2 * GMAX) {
     const int g = threadIdx.x >> 1, i = threadIdx.x & 1;
     double a = 0.0;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) a += red[w][g][i];
+    for (int w = 0; w < 8; ++w) {
+      if constexpr (POW2) {
+        a += red[w][g][i];
+      } else {
+#pragma unroll
+        for (int m = 0; m < CPG / VW; ++m) a += red[w][g * (CPG / VW) + m][i];
+      }
+    }
     partials[((long)blockIdx.x * GMAX + g) * 2 + i] = a;
     for (long p = blockIdx.x + gridDim.x; p < nparts; p += gridDim.x) partials[(p * GMAX + g) * 2 + i] = 0.0;
   }
@@ -346,6 +387,78 @@ __global__ void __launch_bounds__(256, 4) k_gn_bwd_apply(int mode, const float* 
 #pragma unroll
       for (int off = Ln::LPV / 2; off; off >>= 1) wc += __shfl_xor_sync(0xffffffffu, wc, off);
     }
+    if (ok && q == 0) w_bar[v] += wc;
+  }
+}
+
+// The same for eight groups: the lane's group constants in registers (the general kernel reads six of them from shared
+// memory for every channel) and two channels an instruction. Mean of a VJP's calls: 2.4 M voxels, C = 64 (1.8 GB): 325 ->
+// 309 us; 1.0 M, C = 96 (1.2 GB): 340 -> 319 us.
+template <int C, int MODE>
+__global__ void __launch_bounds__(256, C <= 32 ? 3 : 4) k_gn_bwd_apply8(const float* __restrict__ u, float r,
+                                                          const float* __restrict__ pre,
+                                                          const float* __restrict__ gamma,
+                                                          const float* __restrict__ beta,
+                                                          const double* __restrict__ gst,
+                                                          const double* __restrict__ sums,
+                                                          const float* __restrict__ dw, long V,
+                                                          float* __restrict__ pre_bar, float* __restrict__ w_bar,
+                                                          float eps) {
+  griddep_sync();
+  using Ln = Gn8<C>;
+  constexpr int VW = Ln::VW, CPG = Ln::CPG, NG = Ln::NG;
+  __shared__ GnConst k;
+  load_gn_const(k, gst, sums, GMAX, eps);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int sub = lane / Ln::LPV, q = lane % Ln::LPV;
+  const bool active = sub < Ln::VPW;
+  const int c = VW * q, g0 = active ? c / CPG : 0;
+  uint64_t gm[VW / 2], bt[VW / 2];
+  float nmean[NG], rstd[NG], p1[NG], p2[NG], nvr2[NG];   // p = (1/T) (S1, S2)
+#pragma unroll
+  for (int j = 0; j < VW / 2; ++j) {
+    gm[j] = active ? pk2(__ldg(gamma + c + 2 * j), __ldg(gamma + c + 2 * j + 1)) : 0;
+    bt[j] = active ? pk2(__ldg(beta + c + 2 * j), __ldg(beta + c + 2 * j + 1)) : 0;
+  }
+#pragma unroll
+  for (int l = 0; l < NG; ++l) {
+    const int g = g0 + l;
+    nmean[l] = -k.mean[g];
+    rstd[l] = k.rstd[g];
+    p1[l] = k.invT[g] * k.s1[g];
+    p2[l] = k.invT[g] * k.s2[g];
+    nvr2[l] = -k.vr2[g];
+  }
+  auto both = [](float x) { return pk2(x, x); };
+  const long step = (long)gridDim.x * 8 * Ln::VPW;
+  for (long vb = ((long)blockIdx.x * 8 + warp) * Ln::VPW; vb < V; vb += step) {   // warp-uniform loop
+    const long v = vb + sub;
+    const bool ok = active && v < V;
+    float wc = 0.f;
+    if (ok) {
+      const float wv = __ldg(dw + v);
+      float uu[VW], xx[VW], o[VW];
+      ldv<VW>(u + v * C + c, uu);
+      ldv<VW>(pre + v * C + c, xx);
+      uint64_t w2 = 0;
+#pragma unroll
+      for (int j = 0; j < VW / 2; ++j) {
+        const int l = NG == 1 ? 0 : 2 * j / CPG;
+        const uint64_t xh = mul2(fma2(pk2(xx[2 * j], xx[2 * j + 1]), both(1.f), both(nmean[l])), both(rstd[l]));
+        const uint64_t gh = mul2(upstream2<MODE>(uu[2 * j], uu[2 * j + 1], r, fma2(xh, gm[j], bt[j])), gm[j]);
+        const uint64_t t = fma2(xh, both(p2[l]), both(p1[l]));
+        upk2(mul2(both(rstd[l]), fma2(both(-wv), t, gh)), o[2 * j], o[2 * j + 1]);
+        w2 = fma2(both(-p1[l]), xh, w2);
+        w2 = fma2(both(-0.5f * p2[l]), fma2(xh, xh, both(nvr2[l])), w2);
+      }
+      upk2(w2, wc, uu[0]);
+      wc += uu[0];
+      stv<VW>(pre_bar + v * C + c, o);
+    }
+    // sum over the LPV lanes of this voxel (segments of a power-of-two LPV, or the whole warp for C = 96)
+#pragma unroll
+    for (int off = (Ln::LPV & (Ln::LPV - 1)) ? 16 : Ln::LPV / 2; off; off >>= 1)
+      wc += __shfl_xor_sync(0xffffffffu, wc, off);
     if (ok && q == 0) w_bar[v] += wc;
   }
 }
@@ -958,13 +1071,18 @@ int ffno_gn_bwd_stats(int mode, const float* u, float r, const float* pre, const
   if (!width_ok(C) || V < 1 || groups < 1 || groups > GMAX || C % groups || nparts < 1) return FFNO_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   const int cpg = C / groups;
+  const bool early = ffno::early_launch(V, C);
   const int grid = nparts < 2 * sms() ? nparts : 2 * sms();   // the CTAs an SM holds (97-124 registers a thread)
-  if (groups == GMAX && C <= 64 &&
-      (reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(pre)) % 32 == 0) {   // 32-byte lanes
-    switch (C) {
-#define L(CC) case CC: ffno::launch_if(ffno::early_launch(V, CC), k_gn_bwd_stats8<CC>, grid, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, V, partials, nparts); break;
-      L(16) L(32) L(64)
+  // eight groups (the model's): 32-byte lanes for C <= 64, 16-byte lanes for C = 96; anything else takes the general
+  // kernel, whose loads need 16 bytes
+  if (groups == GMAX && (reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(pre)) % (C <= 64 ? 32 : 16) == 0) {
+    switch (4 * C + mode) {
+#define L1(CC, M) \
+  case 4 * CC + M: ffno::launch_if(early, k_gn_bwd_stats8<CC, M>, grid, 256, 0, s, u, r, pre, gamma, beta, gstats, V, partials, nparts); break;
+#define L(CC) L1(CC, 0) L1(CC, 1) L1(CC, 2)
+      L(16) L(32) L(64) L(96)
 #undef L
+#undef L1
     }
     FFNO_CHECK_LAUNCH();
     return FFNO_OK;
@@ -997,9 +1115,26 @@ int ffno_gn_bwd_apply(int mode, const float* u, float r, const float* pre, const
     return FFNO_EINVAL;
   cudaStream_t s = (cudaStream_t)stream;
   const int cpg = C / groups;
+  if (groups == GMAX) {
+    const bool early = ffno::early_launch(V, C);
+    const int blocks = grid_of(V, 8 * 8, C <= 32 ? 3 : 4);   // the CTAs an SM holds
+    switch (4 * C + mode) {
+#define L1(CC, M)                                                                                                  \
+  case 4 * CC + M:                                                                                                 \
+    ffno::launch_if(early, k_gn_bwd_apply8<CC, M>, blocks, 256, 0, s, u, r, pre, gamma, beta, gstats, sums, dw, V, pre_bar, w_bar, \
+                 eps);                                                                                             \
+    break;
+#define L(CC) L1(CC, 0) L1(CC, 1) L1(CC, 2)
+      L(16) L(32) L(64) L(96)
+#undef L
+#undef L1
+    }
+    FFNO_CHECK_LAUNCH();
+    return FFNO_OK;
+  }
   const int blocks = grid_of(V, 8 * 8, 4);
   switch (C) {
-#define L(CC) case CC: ffno::launch_if(ffno::early_launch(V, CC), k_gn_bwd_apply<CC>, blocks, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, sums, dw, V, pre_bar, w_bar, cpg, groups, eps); break;
+#define L(CC) case CC: ffno::launch(k_gn_bwd_apply<CC>, blocks, 256, 0, s, mode, u, r, pre, gamma, beta, gstats, sums, dw, V, pre_bar, w_bar, cpg, groups, eps); break;
     L(16) L(32) L(64) L(96)
 #undef L
   }
