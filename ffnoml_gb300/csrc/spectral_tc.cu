@@ -68,10 +68,9 @@ static_assert(2 * RT * 8 == 32 * 128, "the pieces of a pipeline cover a whole ch
 __device__ __forceinline__ int xf_fill_col(int ptid, int lane) { return 8 * (4 * ((ptid >> 5) & 3) + (lane >> 3)); }
 
 template <int NP>
-__device__ __forceinline__ void xf_fill_chunk(uint8_t* st, uint32_t hb, const float* fsrc, bool fv,
-                                              const long* row_in, int K, int k0, int kc, int ptid, int lane, int nf) {
+__device__ __forceinline__ void xf_load_chunk(float (&v)[NP][8], const float* fsrc, bool fv, const long* row_in, int K,
+                                              int k0, int kc, int ptid, int lane) {
   const int w = (ptid >> 5) & 7;
-  float v[NP][8];
 #pragma unroll
   for (int u = 0; u < NP; ++u) {   // every load of the chunk issued before any is converted
     const int kr = 8 * (2 * u + (w >> 2)) + (lane & 7);
@@ -83,6 +82,12 @@ __device__ __forceinline__ void xf_fill_chunk(uint8_t* st, uint32_t hb, const fl
       for (int i = 0; i < 8; ++i) v[u][i] = 0.f;
     }
   }
+}
+
+template <int NP>
+__device__ __forceinline__ void xf_store_chunk(const float (&v)[NP][8], uint8_t* st, uint32_t hb, int kc, int ptid,
+                                               int lane, int nf) {
+  const int w = (ptid >> 5) & 7;
 #pragma unroll
   for (int u = 0; u < NP; ++u) {
     const int kr = 8 * (2 * u + (w >> 2)) + (lane & 7);
@@ -94,6 +99,14 @@ __device__ __forceinline__ void xf_fill_chunk(uint8_t* st, uint32_t hb, const fl
     *reinterpret_cast<uint4*>(st + o) = make_uint4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<uint4*>(st + hb + o) = make_uint4(l[0], l[1], l[2], l[3]);
   }
+}
+
+template <int NP>
+__device__ __forceinline__ void xf_fill_chunk(uint8_t* st, uint32_t hb, const float* fsrc, bool fv,
+                                              const long* row_in, int K, int k0, int kc, int ptid, int lane, int nf) {
+  float v[NP][8];
+  xf_load_chunk<NP>(v, fsrc, fv, row_in, K, k0, kc, ptid, lane);
+  xf_store_chunk<NP>(v, st, hb, kc, ptid, lane, nf);
 }
 
 template <int NPP, int KC>
@@ -244,9 +257,12 @@ __global__ void __launch_bounds__(NPP * RT, 1)
 // The transposed transform GEMM of k_xform_rt for tables too large to keep resident (the H transforms, K = M = 2H):
 // per 32-row k-chunk the table slice [MT * 128][kc] (from the m-tile / k-chunk pack of ffno_xform_tc) arrives by
 // bulk copies into the stage next to the data chunk, both double-buffered against the MMAs. Chunks of 32 rows k keep
-// a CTA's stages near 100 KB, so that two CTAs of 256 threads share an SM (each with 256 tensor-memory columns).
+// a CTA's stages near 100 KB, so that two CTAs of 256 threads share an SM, each with 256 tensor-memory columns; three
+// with 67 KB and 128 columns where the table has at most 128 rows. Bound by the latency of the chunks (load, convert,
+// MMA, epilogue in turn within a CTA): each thread loads its part of the next chunk, also across items, before it waits
+// for the table and the MMAs of this one. 2.4 M voxels, C = 64: 363 -> 322 us; 1.0 M, C = 96: 377 -> 343; 4.2 M, C = 64: 614 -> 533 (4.0 TB/s).
 constexpr uint32_t SSB = 128u * XKC * 2;    // one split half of a data stage of k_xform_st
-__global__ void __launch_bounds__(RT, 2)
+__global__ void __launch_bounds__(RT, 3)
     k_xform_st(const uint8_t* __restrict__ tpack, int MT, int Kp, const float* __restrict__ in, float* __restrict__ out,
                ffno_xform_desc d, int nbi, int nshift, long ntn, long items, int accumulate, int* __restrict__ err) {
   griddep_wait();
@@ -262,7 +278,7 @@ __global__ void __launch_bounds__(RT, 2)
   const int Mp = MT * 128;
   for (int k = tid; k < Kp; k += RT) row_in[k] = (long)(k / d.in_split) * d.in_hi + (long)(k % d.in_split) * d.in_lo;
   for (int m = tid; m < Mp; m += RT) row_out[m] = (long)(m / d.out_split) * d.out_hi + (long)(m % d.out_split) * d.out_lo;
-  if (warp == 0) tc::tmem_alloc(&tslot, 256);
+  if (warp == 0) tc::tmem_alloc(&tslot, (uint32_t)Mp);
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&bar_t[i], 1);
@@ -282,8 +298,8 @@ __global__ void __launch_bounds__(RT, 2)
   bool ok = true;
   uint32_t g = 0;
   const int n_ep = 32 * q + lane;
-  for (long it = blockIdx.x; ok && it < items; it += gridDim.x) {
-    long bfirst, n0;
+  const int nf = xf_fill_col(tid, lane);
+  auto first = [&](long it, long& bfirst, long& n0) {   // an item's first outer index and column
     if (nbi > 1) {
       bfirst = it * nbi;
       n0 = 0;
@@ -291,22 +307,27 @@ __global__ void __launch_bounds__(RT, 2)
       bfirst = it / ntn;
       n0 = (it % ntn) * 128;
     }
-    const int nf = xf_fill_col(tid, lane);
-    long foff = 0;
-    bool fv;
-    {
-      long b, c;
-      if (nbi > 1) {
-        b = bfirst + (nf >> nshift);
-        c = nf & ((1 << nshift) - 1);
-      } else {
-        b = bfirst;
-        c = n0 + nf;
-      }
-      fv = b < d.nb && c < d.N;
-      if (fv) foff = (b / d.nb2) * d.in_b1 + (b % d.nb2) * d.in_b2 + c;
+  };
+  const float* fsrc = in;   // this thread's columns of the item whose chunks are being loaded
+  bool fv = false;
+  auto source = [&](long it) {
+    long b, c, n0;
+    first(it, b, n0);
+    if (nbi > 1) {
+      b += nf >> nshift;
+      c = nf & ((1 << nshift) - 1);
+    } else {
+      c = n0 + nf;
     }
-    const float* fsrc = in + foff;
+    fv = it < items && b < d.nb && c < d.N;
+    fsrc = fv ? in + (b / d.nb2) * d.in_b1 + (b % d.nb2) * d.in_b2 + c : in;
+  };
+  float v[2][8];   // the next chunk, loaded while the MMAs of this one run
+  source(blockIdx.x);
+  xf_load_chunk<2>(v, fsrc, fv, row_in, d.K, 0, Kp < XKC ? Kp : XKC, tid, lane);
+  for (long it = blockIdx.x; ok && it < items; it += gridDim.x) {
+    long bfirst, n0;
+    first(it, bfirst, n0);
     for (int ch = 0; ch < nch; ++ch, ++g) {
       const int s = (int)(g & 1u);
       const int k0 = ch * XKC, kc = (Kp - k0) < XKC ? (Kp - k0) : XKC;
@@ -325,7 +346,13 @@ __global__ void __launch_bounds__(RT, 2)
           tc::bulk_g2s(tt + (uint32_t)MT * part + mt * part, src + part, part, &bar_t[s]);
         }
       }
-      xf_fill_chunk<2>(st, SSB, fsrc, fv, row_in, d.K, k0, kc, tid, lane, nf);
+      xf_store_chunk<2>(v, st, SSB, kc, tid, lane, nf);
+      if (ch + 1 < nch) {
+        xf_load_chunk<2>(v, fsrc, fv, row_in, d.K, k0 + XKC, (Kp - k0 - XKC) < XKC ? (Kp - k0 - XKC) : XKC, tid, lane);
+      } else {
+        source(it + gridDim.x);
+        xf_load_chunk<2>(v, fsrc, fv, row_in, d.K, 0, Kp < XKC ? Kp : XKC, tid, lane);
+      }
       tc::fence_async_smem();
       const bool wt = tc::mbar_wait(&bar_t[s], (g >> 1) & 1u);
       tc::tc_before_sync();
@@ -367,15 +394,15 @@ __global__ void __launch_bounds__(RT, 2)
       if (nv) obase = (b / d.nb2) * d.out_b1 + (b % d.nb2) * d.out_b2 + c;
     }
     for (int jj = half; jj < Mp / 16; jj += 2) {
-      float v[16];
-      tc::tmem_ld16(tmem + lq + 16u * jj, v);
+      float o[16];
+      tc::tmem_ld16(tmem + lq + 16u * jj, o);
       if (nv) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const int m = 16 * jj + i;
           if (m < d.M) {
             float* p = out + obase + row_out[m];
-            *p = accumulate ? *p + v[i] : v[i];
+            *p = accumulate ? *p + o[i] : o[i];
           }
         }
       }
@@ -393,7 +420,7 @@ __global__ void __launch_bounds__(RT, 2)
   tc::tc_before_sync();
   __syncthreads();
   tc::tc_after_sync();
-  if (warp == 0) tc::tmem_free(tmem, 256);
+  if (warp == 0) tc::tmem_free(tmem, (uint32_t)Mp);
 }
 
 // ---------------------------------------------------------------------------------------------------- mixing
@@ -891,7 +918,8 @@ int ffno_xform_tc(const void* tpack, const float* in, float* out, const ffno_xfo
   const size_t smem = 1024 + 4 * (size_t)SSB + 2 * 2 * (size_t)MT * 128 * XKC * 2;
   if (!ffno::smem_cap_ok(k_xform_st, smem))
     return FFNO_ELAUNCH;
-  const long grid = items < 2L * sms() ? items : 2L * sms();   // two CTAs per SM
+  const long fit = (MT == 1 ? 3L : 2L) * sms();   // the CTAs that shared and tensor memory hold
+  const long grid = items < fit ? items : fit;
   ffno::launch(k_xform_st, (unsigned)grid, RT, smem, (cudaStream_t)stream, static_cast<const uint8_t*>(tpack), MT, Kp, in, out,
                                                                 d, nbi, nshift, ntn, items, accumulate, err);
   FFNO_CHECK_LAUNCH();
