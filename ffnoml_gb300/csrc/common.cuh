@@ -46,7 +46,6 @@ __device__ __forceinline__ Cdf cdf_tc(float x) {
   const float h = 0.5f * (p * t) * e;   // (1 - erf(u)) / 2
   return Cdf{x < 0.f ? h : 1.f - h, 0.39894228040143267794f * e};
 }
-__device__ __forceinline__ float gelu_tc(float x) { return x * cdf_tc(x).cdf; }
 __device__ __forceinline__ float gelu_grad_tc(float x) {
   const Cdf c = cdf_tc(x);
   return fmaf(x, c.pdf, c.cdf);
@@ -406,31 +405,6 @@ __device__ __forceinline__ void head_voxel_bwd(const ffno_head_params& hp, float
   }
 }
 
-// acc[i][j] = sum_k A[(ty + 16 i) * lda + k] * W[k * N + tx + 16 j] for i < RM rows per thread (a tile of 16 RM
-// rows); A in shared memory, W (row-major K x N) in global memory (read through L1; every CTA reads the same small
-// weight matrix).
-template <int K, int N, int RM = 4>
-__device__ __forceinline__ void tile_mm(const float* __restrict__ A, int lda, const float* __restrict__ W,
-                                        float (&acc)[RM][N / 16]) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-#pragma unroll
-  for (int i = 0; i < RM; ++i)
-#pragma unroll
-    for (int j = 0; j < N / 16; ++j) acc[i][j] = 0.f;
-#pragma unroll 4
-  for (int k = 0; k < K; ++k) {
-    float a[RM], b[N / 16];
-#pragma unroll
-    for (int i = 0; i < RM; ++i) a[i] = A[(ty + 16 * i) * lda + k];
-#pragma unroll
-    for (int j = 0; j < N / 16; ++j) b[j] = __ldg(W + k * N + tx + 16 * j);
-#pragma unroll
-    for (int i = 0; i < RM; ++i)
-#pragma unroll
-      for (int j = 0; j < N / 16; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-  }
-}
-
 // Copy rows v0 .. v0 + rows - 1 (C floats each, row-major, contiguous) into shared memory with row stride lds; rows at
 // or beyond V are zero.
 template <int C>
@@ -535,142 +509,6 @@ __device__ __forceinline__ void put_warp_stats(double (*acc)[3], const ShiftAcc&
     acc[lane >> 2][0] = a.w;
     acc[lane >> 2][1] = a.mean;
     acc[lane >> 2][2] = a.m2;
-  }
-}
-
-// Scratch (shared memory) for tile_group_stats: colsum [16][N], col [N], gmean [GMAX], gw (1)
-template <int N>
-struct StatsSmem {
-  float part[16 * N];
-  float col[N];
-  float gmean[GMAX];
-  float wsum;
-};
-
-// Accumulate the depth-weighted statistics of one tile's values val (rows ty + 16 i, columns tx + 16 j) into acc[g]
-// (held by thread g < groups). wr[i] is the weight of row i, zero for rows past the cube. Column c belongs to group
-// c / cpg. Deterministic: fixed summation order.
-template <int N, int RM = 4>
-__device__ __forceinline__ void tile_group_stats(const float (&val)[RM][N / 16], const float (&wr)[RM], int cpg,
-                                                 int groups, StatsSmem<N>& sm, GroupAcc& acc) {
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // tile weight: sum of the row weights (each row counted once: the threads with tx == 0 hold rows ty + 16 i)
-  if (tx == 0) {
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < RM; ++i) s += wr[i];
-    sm.part[ty] = s;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float s = 0.f;
-    for (int t = 0; t < 16; ++t) s += sm.part[t];
-    sm.wsum = s;
-  }
-  __syncthreads();
-  // pass 1: weighted sums
-#pragma unroll
-  for (int j = 0; j < N / 16; ++j) {
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < RM; ++i) s = fmaf(wr[i], val[i][j], s);
-    sm.part[ty * N + tx + 16 * j] = s;
-  }
-  __syncthreads();
-  for (int c = tid; c < N; c += NT) {
-    float s = 0.f;
-    for (int t = 0; t < 16; ++t) s += sm.part[t * N + c];
-    sm.col[c] = s;
-  }
-  __syncthreads();
-  if (tid < groups) {
-    float s = 0.f;
-    for (int c = tid * cpg; c < (tid + 1) * cpg; ++c) s += sm.col[c];
-    const float wt = sm.wsum * cpg;
-    sm.gmean[tid] = wt > 0.f ? s / wt : 0.f;
-  }
-  __syncthreads();
-  // pass 2: weighted squared deviations from the tile mean
-#pragma unroll
-  for (int j = 0; j < N / 16; ++j) {
-    const float m = sm.gmean[(tx + 16 * j) / cpg];
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < RM; ++i) {
-      const float d = val[i][j] - m;
-      s = fmaf(wr[i] * d, d, s);
-    }
-    sm.part[ty * N + tx + 16 * j] = s;
-  }
-  __syncthreads();
-  for (int c = tid; c < N; c += NT) {
-    float s = 0.f;
-    for (int t = 0; t < 16; ++t) s += sm.part[t * N + c];
-    sm.col[c] = s;
-  }
-  __syncthreads();
-  if (tid < groups) {
-    float s = 0.f;
-    for (int c = tid * cpg; c < (tid + 1) * cpg; ++c) s += sm.col[c];
-    chan_merge(acc, (double)sm.wsum * cpg, (double)sm.gmean[tid], (double)s);
-  }
-  __syncthreads();
-}
-
-// Per-group sums of two per-element quantities a, b of one tile (rows ty + 16 i, columns tx + 16 j), added in a fixed
-// order into the double accumulators s1, s2 held by thread g < groups. Used by the GroupNorm backward.
-template <int N, int RM = 4>
-__device__ __forceinline__ void tile_group_sums(const float (&a)[RM][N / 16], const float (&b)[RM][N / 16], int cpg,
-                                                int groups, float* part /* [16][N] */, float* col /* [2][N] */,
-                                                double& s1, double& s2) {
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-#pragma unroll
-  for (int j = 0; j < N / 16; ++j) {
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < RM; ++i) s += a[i][j];
-    part[ty * N + tx + 16 * j] = s;
-  }
-  __syncthreads();
-  for (int c = tid; c < N; c += NT) {
-    float s = 0.f;
-    for (int t = 0; t < 16; ++t) s += part[t * N + c];
-    col[c] = s;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < N / 16; ++j) {
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < RM; ++i) s += b[i][j];
-    part[ty * N + tx + 16 * j] = s;
-  }
-  __syncthreads();
-  for (int c = tid; c < N; c += NT) {
-    float s = 0.f;
-    for (int t = 0; t < 16; ++t) s += part[t * N + c];
-    col[N + c] = s;
-  }
-  __syncthreads();
-  if (tid < groups) {
-    float x = 0.f, y = 0.f;
-    for (int c = tid * cpg; c < (tid + 1) * cpg; ++c) {
-      x += col[c];
-      y += col[N + c];
-    }
-    s1 += (double)x;
-    s2 += (double)y;
-  }
-  __syncthreads();
-}
-
-__device__ __forceinline__ void write_partial(double* partials, int groups, const GroupAcc& acc) {
-  const int tid = threadIdx.x;
-  if (tid < groups) {
-    double* p = partials + ((long)blockIdx.x * groups + tid) * 3;
-    p[0] = acc.w;
-    p[1] = acc.mean;
-    p[2] = acc.m2;
   }
 }
 

@@ -2,7 +2,7 @@
 // 64 voxels by N output channels per CTA of 256 threads, operands in shared memory, FP32 FMAs in ascending k.
 //
 // What bounds it: the FP32 pipe (71 TFLOP/s measured for an outer-product loop in registers) once the operands arrive
-// in few enough instructions. A thread owns 4 consecutive voxels and N / 16 output channels, so one k step is one
+// in few enough instructions (f32x2: two FMAs an instruction). A thread owns 4 consecutive voxels and N / 16 output channels, so one k step is one
 // 16-byte read of the activations, one 8- or 16-byte read of the weights per 2-4 channels and 4 N / 16 FMAs: shared
 // memory moves 4-5 wavefronts per 32-48 FMAs of a warp. (The form before read every operand as one 4-byte word, the
 // weights from global memory: 12 loads per 32 FMAs, bound by the load unit at about 20 TFLOP/s.)

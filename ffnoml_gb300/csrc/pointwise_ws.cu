@@ -303,8 +303,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // (MODE 1: act = GELU, MODE 2: identity), and the depth-weighted GroupNorm partials of pre (one per CTA, its tiles
 // merged in order with Chan's update, so the statistics do not depend on timing). Roles as in the backward:
 //   warp 0 TMA ring of in [and prev]; warp 1 MMA: GEMM1 D1[t % 2] = x W1^T (N = 2C), and GEMM2 D2 = H W2^T (N = C)
-//   one tile behind, so that epilogue 1 of a tile overlaps GEMM1 of the next; warps 2-5 conversion with the residual
-//   prologue (xout); warps 6-13 epilogue 1: H = gelu(D1), split over D1; warps 14-17 epilogue 2: pre and statistics.
+//   one tile behind, so that epilogue 1 of a tile overlaps GEMM1 of the next; warps 2-9 conversion (two groups of four)
+//   with the residual prologue (xout); warps 10-17 epilogue 1: H = gelu(D1), split over D1; warps 18-21 epilogue 2: pre
+//   and statistics.
 // Tensor memory: four A stages of C columns from column 0 ([x hi | x lo], D2 of the stage's tile over them: a stage is
 // held from conversion to epilogue 2), D1 buffers at 256 and 384.
 template <int C, int MODE>
@@ -826,8 +827,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // The ffno_fuse1_tc contract: gates [V][2C] = sigmoid(gelu(A Wg1^T) Wg2^T + bias), A = [x, gelu(GN_s(spec_pre)),
 // gelu(GN_v(vert_pre))] (K = 3C), and hg [V][C] = A Wg1^T when hg is not NULL. Roles as in the forward MLP: warp 0 TMA,
 // 3 NB phases of 32 channels per tile (x, spec_pre, vert_pre boxes) through a four-stage ring; warp 1 MMA: GEMM1
-// D1[t % 2] = A Wg1^T (N = C), and GEMM2 D2 = H Wg2^T (N = 2C) one tile behind, over the tile's A stage; warps 2-5
-// conversion; warps 6-13 epilogue 1: hg to HBM, H = gelu(D1) split over D1; warps 14-17 epilogue 2: the gates.
+// D1[t % 2] = A Wg1^T (N = C), and GEMM2 D2 = H Wg2^T (N = 2C) one tile behind; warps 2-9 conversion
+// (two groups, alternate phases); warps 10-17 epilogue 1: hg to HBM, H = gelu(D1) split over D1; warps 18-21 epilogue
+// 2: the gates.
 // Tensor memory: four A slots of one phase (16 columns hi, 16 lo) at 0, two D1 buffers (C) behind them, two D2 buffers
 // (2C). GEMM1 takes each phase as its slot fills, so conversion, GEMM1, epilogue 1, GEMM2 and epilogue 2 of neighbouring
 // tiles overlap. 4.2 M voxels, C = 64: 1.34 ms (2.22 with a whole tile's operand per stage and one conversion group).
@@ -1089,12 +1091,12 @@ __global__ void __launch_bounds__(F_NTHREADS, 1)
 // pre = gelu(B Wf1^T) Wf2^T + (B[:, :C] + B[:, C:]) / 2, with the depth-weighted GroupNorm partials of pre.
 // Roles: warp 0 TMA: per tile 2 NB phases of 32 channels (spec_pre boxes, then vert_pre boxes), each a pre box and the
 // matching gates box, through a three-stage ring; warp 1 MMA: GEMM1 D1 = B Wf1^T (N = K = 2C) and, one tile behind,
-// GEMM2 D2 += H Wf2^T (N = C); warps 2-5 conversion: B split into the tile's A stage and the FP32 residual
-// (B[:, c] + B[:, C + c]) / 2 into its D2 buffer (GEMM2 accumulates onto it); warps 6-13 epilogue 1: H = gelu(D1),
-// split over D1; warps 14-17 epilogue 2: pre and its statistics, as in the forward MLP. Tensor memory: A slots
+// GEMM2 D2 += H Wf2^T (N = C); warps 2-9 conversion (two groups): B split into the phase's A slot and the
+// FP32 residual (B[:, c] + B[:, C + c]) / 2 into the tile's D2 buffer (GEMM2 accumulates onto it); warps 10-17 epilogue
+// 1: H = gelu(D1), split over D1; warps 18-21 epilogue 2: pre and its statistics, as in the forward MLP. Tensor memory: A slots
 // of one phase (32 columns each), two D1 buffers (2C), three D2 buffers (C). GEMM1 takes each phase as its slot fills; a
 // tile's residual needs its D2 buffer free, so with three of them conversion runs up to two tiles ahead of epilogue 2.
-// 4.2 M voxels, C = 64: 1.42 ms (1.95 with a whole tile's operand per stage, one D1 and one conversion group).
+// 4.2 M voxels, C = 64: 1.28 ms (1.95 with a whole tile's operand per stage, one D1 and one conversion group).
 template <int C>
 __global__ void __launch_bounds__(F_NTHREADS, 1)
     k_fuse2_ws(const __grid_constant__ CUtensorMap map_sp, const __grid_constant__ CUtensorMap map_vp,

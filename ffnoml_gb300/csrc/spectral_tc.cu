@@ -3,7 +3,7 @@
 //
 // Transform GEMM: out[b][m][n] = sum_k T[m][k] in[b][k][n], computed transposed, D^T [128 data columns][M] = X^T T^T,
 // so that tensor-memory lanes are data columns and the stores of a warp cover 32 consecutive columns of one output
-// row. Data chunks of 64 rows k are converted from FP32 HBM into split MN-major tiles (the columns are contiguous in
+// row. Data chunks of 32 or 64 rows k are converted from FP32 HBM into split MN-major tiles (the columns are contiguous in
 // HBM); the split table is either resident in shared memory (k_xform_rt, tables up to 80 KB: the W and height
 // transforms) or streamed per k-chunk next to the data (k_xform_st: the H transforms). Accumulators live in tensor
 // memory (<= 256 columns per pipeline).
@@ -36,12 +36,13 @@ __device__ __forceinline__ bool bounded(bool ok, int* err, int code) {
 
 // ------------------------------------------------------------------------------------------- resident table
 // The transform GEMM with the whole split table resident in shared memory, in the transposed orientation:
-// D^T [128 data columns n][M rows m] = X^T T^T, with X a chunk of 64 data rows k x 128 columns n (A operand, MN-major:
+// D^T [128 data columns n][M rows m] = X^T T^T, with X a chunk of 32 or 64 data rows k x 128 columns n (A operand, MN-major:
 // n contiguous, as in HBM) and T the table [Mp][Kp] (B operand, K-major). The tensor-memory lane is the data column
 // n, so the stores of one warp cover 32 consecutive columns of one output row. An item is 128 columns: one n-tile of
-// one batch, or 128 / N whole batches when N divides 128 (the W transforms, N = C). Two pipelines of 256 threads per
-// CTA take alternate items, each with two data stages (double-buffered against the MMAs), 256 tensor-memory columns
-// and its own mbarriers; the table is shared. Every wait is bounded.
+// one batch, or 128 / N whole batches when N divides 128 (the W transforms, N = C). Two to four pipelines of 256 threads
+// per CTA take alternate items, each with two data stages (double-buffered against the MMAs), its share of the tensor
+// memory and its own mbarriers; the table is shared. Bound by the latency of a chunk (loads, conversion, MMAs, epilogue
+// in turn within a pipeline), so more pipelines are better as long as accumulators and stages fit. Every wait is bounded.
 constexpr int RT = 256;                     // threads per pipeline
 constexpr int RT_MAXK = 512;                // largest padded K of a resident table
 
@@ -951,6 +952,10 @@ int ffno_xform_tcr(const void* tpack, int Mp, int Kp, const float* in, float* ou
                  in, out, d, nbi, nshift, ntn, items, accumulate, err);
     return true;
   };
+  // Pipelines an SM: four where the accumulators of four (128 columns each) fit tensor memory, three up to 160 rows,
+  // else two. Four / three need chunks of 32 rows for their stages; at two, chunks of 64. All resident-table
+  // transforms of a two-block forward of 4.2 M voxels, C = 64 (two of them above 160 rows, two of 129 to 160): 3.58 ms
+  // with two pipelines everywhere, 3.23 with this rule; of a VJP of 2.4 M voxels: 4.28 and 3.65 ms.
   const bool ok = Mp <= 128 ? go(k_xform_rt<4, 32>, 4, 32)
                             : Mp <= 160 ? go(k_xform_rt<3, 32>, 3, 32) : go(k_xform_rt<2, 64>, 2, 64);
   if (!ok) return FFNO_ELAUNCH;

@@ -16,7 +16,7 @@
  *  - GroupNorm coefficients `coefs` are [3][C] floats: per channel the group mean, gamma*rstd and beta; the
  *    normalised value is (x - coefs[0][c]) * coefs[1][c] + coefs[2][c].
  *  - GroupNorm partial statistics `partials` are [nparts][groups][3] doubles (total weight, mean, M2), one row per
- *    CTA of the producing kernel, which is launched with exactly nparts CTAs.
+ *    CTA of the producing kernel; a launch with fewer CTAs writes zero rows (no weight) for the rest.
  *  - Return value: FFNO_OK (0) or an error code; no call traps, aborts or throws.
  *  - Supported widths C: 16, 32, 64, 96.
  */
