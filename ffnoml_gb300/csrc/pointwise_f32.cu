@@ -648,9 +648,11 @@ int ffno_gn_finalize(const double* partials, int nparts, int C, int groups, cons
                      float eps, float* coefs, double* gstats, ffno_stream_t stream) {
   if (!partials || !gamma || !beta || !coefs) return FFNO_EINVAL;
   if (nparts < 1 || C < 1 || groups < 1 || groups > GMAX || C % groups) return FFNO_EINVAL;
-  // more than half of an SM's shared memory, unused: the CTAs are FP64-bound, and placed together on the SM that frees up
-  // first they took up to 25 us (width 96) instead of 9
-  const size_t apart = 116 * 1024;
+  // Above width 64: more than half of an SM's shared memory, unused. The CTAs are FP64-bound, and placed together on the
+  // SM that frees up first they took up to 25 us at width 96 instead of 9 (a forward of 296 k voxels 8.16 -> 8.07 ms).
+  // Narrower models lose by it (the SMs' shared memory is set up anew around each launch): width 32, 65 k voxels,
+  // 2.15 -> 2.21 ms.
+  const size_t apart = C > 64 ? 116 * 1024 : 0;
   if (!ffno::smem_cap_ok(k_gn_finalize, apart)) return FFNO_ELAUNCH;
   ffno::launch(k_gn_finalize, groups, FIN_NT, apart, (cudaStream_t)stream, partials, nparts, C, groups, gamma, beta, eps, coefs,
                                                              gstats);
