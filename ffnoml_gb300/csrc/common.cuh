@@ -310,7 +310,9 @@ struct HeadBase32 {
     const float pe = fmaf(dd, IL, fmaf(de, IH, fmaf(dd, IH, -p)));
     const float m = two_sum(hi, -mean, me);
     const float r = two_sum(m, p, se);
-    return __fadd_rn(r, __fadd_rn(se, __fadd_rn(__fadd_rn(me, lo), pe)));
+    // an infinite base or level: the plain sum is the answer (-inf for a density of zero or an empty level), and the
+    // error terms are inf - inf
+    return fabsf(r) <= 3.402823466e38f ? __fadd_rn(r, __fadd_rn(se, __fadd_rn(__fadd_rn(me, lo), pe))) : r;
   }
 };
 __device__ __forceinline__ HeadBase64 head_base(double b, double) { return HeadBase64(b); }
