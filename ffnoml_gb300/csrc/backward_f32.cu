@@ -797,9 +797,9 @@ __global__ void __launch_bounds__(NT, 2) k_head_bwd(const float* __restrict__ x,
                                                  float* __restrict__ xbar, float* __restrict__ xinbar, int al) {
   griddep_sync();
   extern __shared__ __align__(16) float sm[];
-  __shared__ double etab[EXP_TAB];
+  __shared__ double etab[HEAD_TAB];
   constexpr int LO = NHP + 1, N2 = 2 * C / 16;
-  if (kLte) fill_exp_table(etab);
+  if (kLte) fill_head_table(hp, etab);
   float* SA = sm;                    // [C][64] input, then [2C][64] hidden, then its gradient
   float* SG = SA + 2 * C * BM;       // [NHP][64] gradient of the head channels
   float* SO = SG + NHP * BM;         // [64][NHP + 1] head channels, then their gradient
@@ -880,8 +880,8 @@ __global__ void __launch_bounds__(256) k_head_output_bwd(const float* __restrict
                                                          const __grid_constant__ ffno_head_params hp,
                                                          float* __restrict__ hbar, float* __restrict__ xinbar) {
   griddep_sync();
-  __shared__ double etab[EXP_TAB];
-  fill_exp_table(etab);
+  __shared__ double etab[HEAD_TAB];
+  fill_head_table(hp, etab);
   __syncthreads();
   float o[FFNO_MAX_LEVELS + FFNO_MAX_SPECIES];
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < V; v += (long)gridDim.x * blockDim.x) {

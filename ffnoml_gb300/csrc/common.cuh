@@ -153,8 +153,30 @@ constexpr int EXP_TAB = 128;
 constexpr double LN2HI = 0.005415208637714386, LN2LO = 3.710410186743494e-09;
 constexpr double LG2HI = 0.002351796254515648, LG2LO = 5.866092051994237e-10;
 
-__device__ __forceinline__ void fill_exp_table(double* tab) {
+// The table of exponentials and, behind it, 1 if every constant of the head is an ordinary number: finite, and the
+// divisors (the bound of the totals, the scales std_Y) not zero either. Otherwise every voxel takes CUDA's functions and
+// divisions, whose infinities and NaN the functions below do not reproduce. One warp looks, once a CTA.
+constexpr int HEAD_TAB = EXP_TAB + 1;
+
+__device__ __forceinline__ void fill_head_table(const ffno_head_params& hp, double* tab) {
   for (int i = threadIdx.x; i < EXP_TAB; i += blockDim.x) tab[i] = exp2((double)i / EXP_TAB);
+  static_assert(FFNO_MAX_LEVELS <= 32, "a lane a level");
+  if (threadIdx.x < 32) {
+    auto divisor = [](float x) { return fabsf(x) >= 1.17549435e-38f && fabsf(x) <= 3.402823466e38f; };
+    int levels = 0;
+    for (int s = 0; s < hp.nspecies; ++s) levels += hp.levels[s];
+    bool ok = divisor(hp.total_bound);
+    if (threadIdx.x < levels && threadIdx.x < FFNO_MAX_LEVELS) {
+      const int g = threadIdx.x;
+      ok = ok && divisor(hp.std_y[g]) && isfinite(hp.log_g[g]) && isfinite(hp.ev[g]) && isfinite(hp.ndxi[g]) &&
+           isfinite(hp.dion[g]);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (threadIdx.x == 0) tab[EXP_TAB] = ok ? 1.0 : 0.0;
+  }
+}
+__device__ __forceinline__ bool head_ordinary(const double* tab) {
+  return __double2hiint(tab[EXP_TAB]) != 0;   // an integer comparison: not on the FP64 pipe
 }
 
 __device__ __forceinline__ double rcp64(double x) {
@@ -207,7 +229,7 @@ struct HeadMath;
 template <>
 struct HeadMath<double> {
   const double* tab;
-  bool fast;   // every head channel below 1e6 in size, 0.5 < log10 T < 15, |log10 ne| < 40
+  bool fast;   // ordinary constants, every head channel below 1e6 in size, 0.5 < log10 T < 15, |log10 ne| < 40
   __device__ __forceinline__ double exp_(double x) const { return fast ? exp_tab(tab, x) : exp(x); }
   __device__ __forceinline__ double log_(double x) const { return fast ? log_tab(tab, x) : log(x); }
   __device__ __forceinline__ double tanh_(double x) const { return fast ? tanh_tab(tab, x) : tanh(x); }
@@ -223,10 +245,11 @@ struct HeadMath<float> {
   __device__ __forceinline__ float inv_(float x) const { return 1.f / x; }
 };
 
-__device__ __forceinline__ bool head_fast(const ffno_head_params& hp, const float* o, int nh, const HeadInputs& in) {
+__device__ __forceinline__ bool head_fast(const ffno_head_params& hp, const double* tab, const float* o, int nh,
+                                          const HeadInputs& in) {
   const float lt = fmaf(in.lt, hp.std_x[hp.temperature_channel], hp.mean_x[hp.temperature_channel]);
   const float ln = fmaf(in.lne, hp.std_x[hp.ne_channel], hp.mean_x[hp.ne_channel]);
-  bool ok = lt > 0.5f && lt < 15.f && fabsf(ln) < 40.f;
+  bool ok = head_ordinary(tab) && lt > 0.5f && lt < 15.f && fabsf(ln) < 40.f;
   for (int c = 0; c < nh; ++c) ok = ok && fabsf(o[c]) < 1e6f;
   return ok;
 }
@@ -318,12 +341,12 @@ struct HeadBase32 {
 __device__ __forceinline__ HeadBase64 head_base(double b, double) { return HeadBase64(b); }
 __device__ __forceinline__ HeadBase32 head_base(double b, float) { return HeadBase32(b); }
 
-// Forward: out[g * V + v] = the normalised log10 population of level g. tab: fill_exp_table's.
+// Forward: out[g * V + v] = the normalised log10 population of level g. tab: fill_head_table's.
 template <typename T>
 __device__ __forceinline__ void head_voxel_fwd(const ffno_head_params& hp, const float* o, const HeadInputs& in,
                                                float* __restrict__ out, long V, long v, const double* tab) {
   HeadMath<T> hm{tab, false};
-  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, o, head_channels(hp), in);
+  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, tab, o, head_channels(hp), in);
   const Lte<T> e(hp, in, hm);
   // the total term and the assembly of log10 n (log10 rho - log10 m + s ~ 20, minus mean_Y) stay beyond FP32 for both
   // T: in FP32 their rounding (~1e-6 dex at that magnitude, and a few ulp of b for tanh) would move every level of
@@ -341,7 +364,8 @@ __device__ __forceinline__ void head_voxel_fwd(const ffno_head_params& hp, const
     const T lse = hm.log_(shifted_exp_sum(hm, logit, L, mx));
     const double tb = (double)hp.total_bound;
     const float u = o[hc + L];
-    const double th = fabsf(u) < 1e6f ? tanh_tab(tab, (double)u * rcp64(tb)) : tanh((double)u / tb);
+    const double th =
+        fabsf(u) < 1e6f && head_ordinary(tab) ? tanh_tab(tab, (double)u * rcp64(tb)) : tanh((double)u / tb);
     const auto base = head_base(lrho - (double)hp.log10_particle_mass[s] + tb * th, T(0));
     for (int i = 0; i < L; ++i) {
       const int g = lvl + i;
@@ -360,7 +384,7 @@ __device__ __forceinline__ void head_voxel_bwd(const ffno_head_params& hp, float
                                                const float* __restrict__ ybar, long V, long v,
                                                float* __restrict__ xinbar, const double* tab) {
   HeadMath<T> hm{tab, false};
-  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, o, head_channels(hp), in);
+  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, tab, o, head_channels(hp), in);
   const Lte<T> e(hp, in, hm);
   T gsum = 0, ltb = 0, lneb = 0;
   int hc = 0, lvl = 0;

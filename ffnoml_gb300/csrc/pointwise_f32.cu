@@ -529,9 +529,9 @@ __global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, con
                                              float* __restrict__ head_out, int al) {
   griddep_sync();
   extern __shared__ __align__(16) float sm[];
-  __shared__ double etab[EXP_TAB];
+  __shared__ double etab[HEAD_TAB];
   constexpr int LO = NHP + 1;
-  if (kLte) fill_exp_table(etab);
+  if (kLte) fill_head_table(hp, etab);
   float* as = sm;                    // [C][64] input, then [2C][64] hidden
   float* os = as + 2 * C * BM;       // [64][NHP + 1] head channels
   g32::Ring ring(os + BM * LO, g32::KC * 2 * C, al);
@@ -589,8 +589,8 @@ __global__ void __launch_bounds__(256) k_head_output(const float* __restrict__ h
                                                      long V, int nh, const __grid_constant__ ffno_head_params hp,
                                                      float* __restrict__ out) {
   griddep_sync();
-  __shared__ double etab[EXP_TAB];
-  fill_exp_table(etab);
+  __shared__ double etab[HEAD_TAB];
+  fill_head_table(hp, etab);
   __syncthreads();
   float o[FFNO_MAX_LEVELS + FFNO_MAX_SPECIES];
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < V; v += (long)gridDim.x * blockDim.x) {

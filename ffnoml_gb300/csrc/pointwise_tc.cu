@@ -1297,8 +1297,8 @@ __global__ void __launch_bounds__(CT, 1) k_head_tc(const float* __restrict__ x, 
                                                    float* __restrict__ out, float* __restrict__ head_out,
                                                    int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ double etab[EXP_TAB];
-  fill_exp_table(etab);
+  __shared__ double etab[HEAD_TAB];
+  fill_head_table(hp, etab);
   __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C), RB = head_region(C, NHP, false);
   constexpr int LO = NHP + 1;
@@ -1359,8 +1359,8 @@ __global__ void __launch_bounds__(CT, 1) k_head_bwd_tc(const float* __restrict__
                                                        float* __restrict__ xbar, float* __restrict__ xinbar,
                                                        int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ double etab[EXP_TAB];
-  if (sizeof(T) == 8) fill_exp_table(etab);
+  __shared__ double etab[HEAD_TAB];
+  if (sizeof(T) == 8) fill_head_table(hp, etab);
   __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C), RB = head_region(C, NHP, true);
   constexpr int LO = NHP + 1;
@@ -2140,8 +2140,8 @@ __global__ void __launch_bounds__(PT, 1) k_head_tc96(const float* __restrict__ x
                                                      int* __restrict__ err) {
   constexpr int C = C96;
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ double etab[EXP_TAB];
-  fill_exp_table(etab);
+  __shared__ double etab[HEAD_TAB];
+  fill_head_table(hp, etab);
   __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C);
   PIPE_PROLOGUE(2 * C + NHP, 1)
@@ -2218,8 +2218,8 @@ __global__ void __launch_bounds__(PT, 1) k_head_bwd_tc96(const float* __restrict
                                                          int* __restrict__ err) {
   constexpr int C = C96;
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ double etab[EXP_TAB];
-  if (sizeof(T) == 8) fill_exp_table(etab);
+  __shared__ double etab[HEAD_TAB];
+  if (sizeof(T) == 8) fill_head_table(hp, etab);
   __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C);
   constexpr uint32_t DO = 2 * C, D3 = 2 * C + NHP, D4 = 4 * C + NHP;
