@@ -377,7 +377,7 @@ __device__ __forceinline__ void load_oct(Oct<KW>& a, long v0, long V, int ptid, 
     const int e = ptid + u * PT, q = e >> 3;
     const long v = v0 + (q / KB) * 8 + (e & 7);
     if (v < V) {
-      tc::ld8_now(f(v, (q % KB) * 8), a[u]);
+      tc::ld8(f(v, (q % KB) * 8), a[u]);
     } else {
 #pragma unroll
       for (int i = 0; i < 8; ++i) a[u][i] = 0.f;
@@ -1116,7 +1116,7 @@ __global__ void __launch_bounds__(CT, 1) k_fuse_bwd_a_tc(const float* __restrict
       o[4] = s1.x * g[4], o[5] = s1.y * g[5], o[6] = s1.z * g[6], o[7] = s1.w * g[7];
     });
     float fr[FB / 2][8];   // F_bar, loaded while the first GEMM runs
-    load_tile8<C>(fr, v0, V, P.ptid, [&](long v, int k, float (&o)[8]) { tc::ld8_now(fb + v * C + k, o); });
+    load_tile8<C>(fr, v0, V, P.ptid, [&](long v, int k, float (&o)[8]) { tc::ld8(fb + v * C + k, o); });
     if (!pipe_gemms(P, err, Gemm{P.tmem, wf1, kop(Bt, 2 * C), 2 * C, false})) break;
     store_tile8<C>(Ft, fr, P.ptid);
     if (!pipe_gemms(P, err, Gemm{P.tmem + TM, wf2t, kop(Ft, C), C, false})) break;
@@ -1564,8 +1564,8 @@ __global__ void __launch_bounds__(PT, 1) k_mlp2_bwd_tc96(const float* __restrict
 #pragma unroll
       for (int i = 0; i < 16; ++i) bv[n][i] = 0.f;
       if (!base || v >= V) continue;
-      tc::ld8_now(base + v * C + 16 * (2 * n + P.half), bv[n]);
-      tc::ld8_now(base + v * C + 16 * (2 * n + P.half) + 8, bv[n] + 8);
+      tc::ld8(base + v * C + 16 * (2 * n + P.half), bv[n]);
+      tc::ld8(base + v * C + 16 * (2 * n + P.half) + 8, bv[n] + 8);
     }
     for (int h = 0; h < 2; ++h) {
 #pragma unroll 1

@@ -112,7 +112,8 @@ __device__ __forceinline__ float4 lds4(const void* p) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(smem_u32(p)));
+               : "r"(smem_u32(p))
+               : "memory");   // neither above the mbarrier wait of its stage nor below the arrival that releases it
   return v;
 }
 
@@ -316,16 +317,13 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
 
 // 32 contiguous bytes (8 floats) per thread in one request, p 32-byte aligned: when every thread of a warp reads its
 // own row (one voxel's channels), the warp asks for 32 sectors per request instead of 32 half sectors twice
+// Volatile with a clobber: to the compiler a plain asm is a function of the pointer, free to move above the wait that makes
+// the data valid (griddepcontrol.wait above all) and, issued ahead of a wait for MMAs, to sink to its use.
 __device__ __forceinline__ void ld8(const float* p, float* o) {
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
-      : "l"(p));
-}
-// ld8 that stays where it is written (a load issued ahead of a wait that the compiler must not sink to its use)
-__device__ __forceinline__ void ld8_now(const float* p, float* o) {
   asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
-               : "l"(p));
+               : "l"(p)
+               : "memory");
 }
 __device__ __forceinline__ void st8(float* p, const float* v) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
