@@ -283,7 +283,7 @@ def _weights_key(model):
     """Address and version of every parameter and buffer, in module order. Each call walks the modules as they are now
     (a replaced submodule, parameter or buffer changes the key): a plain walk over the registries, because this runs
     before the first launch of every call and Module.parameters() takes 2 ms of it on a model of 8 blocks (0.3 ms so)."""
-    items, stack = [], [model]
+    items, stack, seen = [], [model], {id(model)}
     while stack:
         m = stack.pop()
         for t in m._parameters.values():
@@ -292,7 +292,10 @@ def _weights_key(model):
         for t in m._buffers.values():
             if t is not None:
                 items.append((t.data_ptr(), t._version))
-        stack.extend(c for c in m._modules.values() if c is not None)
+        for c in m._modules.values():       # each module once: a submodule may hold the model that holds it
+            if c is not None and id(c) not in seen:
+                seen.add(id(c))
+                stack.append(c)
     return tuple(items)
 
 
