@@ -140,13 +140,13 @@ __device__ __forceinline__ HeadInputs head_inputs(const ffno_head_params& hp, co
 
 // FP64 elementary functions of the head. The FP64 pipe of this chip takes about two lanes a cycle and SM, so the head is
 // bound by the number of its FP64 operations: about 1100 a voxel of two six-level species with CUDA's exp, log, exp10,
-// tanh, division and square root, about 370 with these. Each is the textbook method, full double precision (a few
-// 2^-53) on the range that the caller checks; outside it the head takes CUDA's functions.
+// tanh, division and square root, about 370 with these. Each is the textbook method, to a few 2^-53 of the result (tanh:
+// of 1) on the range that the caller checks; outside it the head takes CUDA's functions.
 //   exp(x) = 2^(n / 128) e^r, n = round(128 x / ln 2), |r| <= ln 2 / 256: a table of 2^(i / 128) (filled once per CTA with
 //     exp2) and the Taylor polynomial of e^r - 1 to r^5 (remainder 5e-19);
 //   10^x the same with n = round(128 x log2 10);
 //   log(s), s near 1 .. 32: one Newton step y + e - e^2 / 2, e = s exp(-y) - 1, from FP32's y (e < 1e-6);
-//   tanh(x) = sign(x) (1 - q) / (1 + q), q = exp(-2 |x|);
+//   tanh(x) = sign(x) (1 - q) / (1 + q), q = exp(-2 |x|), to a few 2^-53 absolutely (1 - q cancels for small x);
 //   1 / x: two Newton-Raphson steps from the hardware's 20-bit reciprocal.
 constexpr int EXP_TAB = 128;
 // ln 2 / 128 and log10(2) / 128 in two parts, the first with 32 trailing zero bits (its products with n are exact)
@@ -155,7 +155,9 @@ constexpr double LG2HI = 0.002351796254515648, LG2LO = 5.866092051994237e-10;
 
 // The table of exponentials and, behind it, 1 if every constant of the head is an ordinary number: finite, and the
 // divisors (the bound of the totals, the scales std_Y) not zero either. Otherwise every voxel takes CUDA's functions and
-// divisions, whose infinities and NaN the functions below do not reproduce. One warp looks, once a CTA.
+// divisions, whose infinities and NaN the functions below do not reproduce. So it does for a bound above 1e6 (a model
+// whose totals are not to be bounded): b tanh(u / b) multiplies tanh_tab's absolute error by b, and up to 1e6 that stays
+// four digits below a float32 rounding of the output. One warp looks, once a CTA.
 constexpr int HEAD_TAB = EXP_TAB + 1;
 
 __device__ __forceinline__ void fill_head_table(const ffno_head_params& hp, double* tab) {
@@ -165,7 +167,7 @@ __device__ __forceinline__ void fill_head_table(const ffno_head_params& hp, doub
     auto divisor = [](float x) { return fabsf(x) >= 1.17549435e-38f && fabsf(x) <= 3.402823466e38f; };
     int levels = 0;
     for (int s = 0; s < hp.nspecies; ++s) levels += hp.levels[s];
-    bool ok = divisor(hp.total_bound);
+    bool ok = divisor(hp.total_bound) && fabsf(hp.total_bound) <= 1e6f;
     if (threadIdx.x < levels && threadIdx.x < FFNO_MAX_LEVELS) {
       const int g = threadIdx.x;
       ok = ok && divisor(hp.std_y[g]) && isfinite(hp.log_g[g]) && isfinite(hp.ev[g]) && isfinite(hp.ndxi[g]) &&

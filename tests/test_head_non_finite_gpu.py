@@ -1,7 +1,7 @@
-"""Non-finite values in the level-fraction head: what is infinite or not a number in the float64 oracle is so here too,
-with the same sign, and every other output keeps its accuracy (FP32 precision: one float32 rounding of the output and one
-of the oracle's own inputs, 2^-23; split-BF16 precision: FP32 level weights, 1e-5; both of the larger of the output and 1,
-the bounds of test_head_ranges_gpu.py)."""
+"""Non-finite values and unusual constants in the level-fraction head: what is infinite or not a number in the float64
+oracle is so here too, with the same sign, and every other output keeps its accuracy (FP32 precision: one float32 rounding
+of the output and one of the oracle's own inputs, 2^-23; split-BF16 precision: FP32 level weights, 1e-5; both of the
+larger of the output and 1, the bounds of test_head_ranges_gpu.py)."""
 import math
 
 import pytest
@@ -98,6 +98,22 @@ def test_total_of_zero_over_a_bound_of_zero(precision):
     ref = OracleFFNO3D(state, dict(model_config(CFG), total_bound=0.0), torch.float64).head(head.double(), x.double())
     assert bool(torch.isnan(ref[0, :6, 5]).all())
     assert torch.equal(torch.isnan(y), torch.isnan(ref))
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("bound", [1e-3, 1e5, 1e7, 1e14])
+def test_total_bounds_from_small_to_none(precision, bound):
+    """A large bound leaves the totals as they are: to the accuracy of the other outputs, not to that of the bound."""
+    from oracle.ffno_oracle import OracleFFNO3D
+    m = _model(precision)
+    m.total_bound = bound
+    head, x = _voxels()
+    y = m.head_output(head.cuda(), x.cuda()).double().cpu()
+    state = {k: v.double().cpu() for k, v in m.state_dict().items()}
+    ref = OracleFFNO3D(state, dict(model_config(CFG), total_bound=torch.tensor(bound).item()), torch.float64).head(
+        head.double(), x.double())
+    err = (y - ref).abs() / ref.abs().clamp_min(1.0)
+    assert err.max().item() <= (2.0 ** -23 if precision == "fp32" else 1e-5)
 
 
 def test_output_scale_of_zero():
