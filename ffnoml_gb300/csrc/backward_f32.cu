@@ -793,13 +793,13 @@ __global__ void __launch_bounds__(NT, 2) k_head_bwd(const float* __restrict__ x,
                                                  const float* __restrict__ ybar, long V, const float* __restrict__ p1,
                                                  const float* __restrict__ p2, const float* __restrict__ b2,
                                                  const float* __restrict__ p2t, const float* __restrict__ p1t,
-                                                 const __grid_constant__ ffno_head_params hp, int nh,
+                                                 const __grid_constant__ HeadParams hp, int nh,
                                                  float* __restrict__ xbar, float* __restrict__ xinbar, int al) {
   griddep_sync();
   extern __shared__ __align__(16) float sm[];
-  __shared__ double etab[HEAD_TAB];
+  __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1, N2 = 2 * C / 16;
-  if (kLte) fill_head_table(hp, etab);
+  if (kLte) fill_exp_table(etab);
   float* SA = sm;                    // [C][64] input, then [2C][64] hidden, then its gradient
   float* SG = SA + 2 * C * BM;       // [NHP][64] gradient of the head channels
   float* SO = SG + NHP * BM;         // [64][NHP + 1] head channels, then their gradient
@@ -877,11 +877,11 @@ __global__ void __launch_bounds__(NT, 2) k_head_bwd(const float* __restrict__ x,
 template <typename T>
 __global__ void __launch_bounds__(256) k_head_output_bwd(const float* __restrict__ head, const float* __restrict__ xin,
                                                          const float* __restrict__ ybar, long V, int nh,
-                                                         const __grid_constant__ ffno_head_params hp,
+                                                         const __grid_constant__ HeadParams hp,
                                                          float* __restrict__ hbar, float* __restrict__ xinbar) {
   griddep_sync();
-  __shared__ double etab[HEAD_TAB];
-  fill_head_table(hp, etab);
+  __shared__ double etab[EXP_TAB];
+  fill_exp_table(etab);
   __syncthreads();
   float o[FFNO_MAX_LEVELS + FFNO_MAX_SPECIES];
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < V; v += (long)gridDim.x * blockDim.x) {

@@ -1,12 +1,15 @@
-// Shared device helpers for the FFNO3D kernels: activations, the FP32 SIMT tile GEMM used by the pointwise (1x1x1
-// convolution) chains, and the deterministic depth-weighted GroupNorm statistics.
+// Shared helpers of the FFNO3D kernels: activations, the level-fraction head, the deterministic depth-weighted GroupNorm
+// statistics, launches.
 //
 // Activation layout: channels last, one row of C floats per voxel, voxel v = (d * H + h) * W + w of one cube.
-// A "tile" is BM = 64 consecutive voxels processed by one CTA of NT = 256 threads; thread (ty, tx) = (tid / 16,
-// tid % 16) owns rows ty + 16 i (i < 4) and columns tx + 16 j (j < N / 16) of every tile GEMM output.
+// A "tile" is BM = 64 consecutive voxels processed by one CTA of NT = 256 threads (the FP32 chains' tile GEMM and its
+// thread mapping: gemm_f32.cuh).
 #pragma once
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
+
+#include <cmath>
 
 #include "../../include/ffnoml_gb300.h"
 
@@ -127,7 +130,28 @@ constexpr double kLN_CCON = -36.113482555935598575;
 // level logits, then its total channel). The LTE math and the log-softmax run in T: double is the reference's FP64
 // (torch.log_softmax on float64 logits, :741); float is the split-BF16 path's FP32, where the sum of the max-shifted
 // exponentials (each in (0, 1]) is compensated (below), so that the level shares of a voxel add up to 1 within a few
-// FP32 roundings. The total term and the final sum of log10 n are FP64 in both.
+// FP32 roundings. The total term is FP64 in both; the final sum of log10 n is FP64 or two floats (HeadBase32).
+
+// What the head's kernels take: the caller's parameters and whether every constant among them is an ordinary number:
+// finite, the divisors (the bound of the totals, the scales std_Y) not zero either. Otherwise every voxel takes CUDA's
+// functions and divisions, whose infinities and NaN the table functions below do not reproduce. So it does for a bound
+// above 1e6 (a model whose totals are not to be bounded): b tanh(u / b) multiplies tanh_tab's absolute error by b, and
+// up to 1e6 that stays four digits below a float32 rounding of the output. The host looks, at the launch (a warp of
+// every CTA doing it took 3-9 us a launch).
+struct HeadParams : ffno_head_params {
+  int ordinary;
+  explicit HeadParams(const ffno_head_params& p) : ffno_head_params(p) {
+    auto divisor = [](float x, float most) { return fabsf(x) >= FLT_MIN && fabsf(x) <= most; };
+    int levels = 0;
+    for (int s = 0; s < nspecies && s < FFNO_MAX_SPECIES; ++s) levels += p.levels[s];
+    bool ok = divisor(total_bound, 1e6f);
+    for (int g = 0; g < levels && g < FFNO_MAX_LEVELS; ++g)
+      ok = ok && divisor(std_y[g], FLT_MAX) && std::isfinite(log_g[g]) && std::isfinite(ev[g]) &&
+           std::isfinite(ndxi[g]) && std::isfinite(dion[g]);
+    ordinary = ok;
+  }
+};
+
 struct HeadInputs {
   float lt, lne, lrho;   // log10 T, log10 ne (SI), log10 rho of the voxel (denormalised)
 };
@@ -142,8 +166,8 @@ __device__ __forceinline__ HeadInputs head_inputs(const ffno_head_params& hp, co
 // bound by the number of its FP64 operations: about 1100 a voxel of two six-level species with CUDA's exp, log, exp10,
 // tanh, division and square root, about 370 with these. Each is the textbook method, to a few 2^-53 of the result (tanh:
 // of 1) on the range that the caller checks; outside it the head takes CUDA's functions.
-//   exp(x) = 2^(n / 128) e^r, n = round(128 x / ln 2), |r| <= ln 2 / 256: a table of 2^(i / 128) (filled once per CTA with
-//     exp2) and the Taylor polynomial of e^r - 1 to r^5 (remainder 5e-19);
+//   exp(x) = 2^(n / 128) e^r, n = round(128 x / ln 2), |r| <= ln 2 / 256: a table of 2^(i / 128) (filled once per CTA
+//     with exp2) and the Taylor polynomial of e^r - 1 to r^5 (remainder 5e-19);
 //   10^x the same with n = round(128 x log2 10);
 //   log(s), s near 1 .. 32: one Newton step y + e - e^2 / 2, e = s exp(-y) - 1, from FP32's y (e < 1e-6);
 //   tanh(x) = sign(x) (1 - q) / (1 + q), q = exp(-2 |x|), to a few 2^-53 absolutely (1 - q cancels for small x);
@@ -153,32 +177,8 @@ constexpr int EXP_TAB = 128;
 constexpr double LN2HI = 0.005415208637714386, LN2LO = 3.710410186743494e-09;
 constexpr double LG2HI = 0.002351796254515648, LG2LO = 5.866092051994237e-10;
 
-// The table of exponentials and, behind it, 1 if every constant of the head is an ordinary number: finite, and the
-// divisors (the bound of the totals, the scales std_Y) not zero either. Otherwise every voxel takes CUDA's functions and
-// divisions, whose infinities and NaN the functions below do not reproduce. So it does for a bound above 1e6 (a model
-// whose totals are not to be bounded): b tanh(u / b) multiplies tanh_tab's absolute error by b, and up to 1e6 that stays
-// four digits below a float32 rounding of the output. One warp looks, once a CTA.
-constexpr int HEAD_TAB = EXP_TAB + 1;
-
-__device__ __forceinline__ void fill_head_table(const ffno_head_params& hp, double* tab) {
+__device__ __forceinline__ void fill_exp_table(double* tab) {
   for (int i = threadIdx.x; i < EXP_TAB; i += blockDim.x) tab[i] = exp2((double)i / EXP_TAB);
-  static_assert(FFNO_MAX_LEVELS <= 32, "a lane a level");
-  if (threadIdx.x < 32) {
-    auto divisor = [](float x) { return fabsf(x) >= 1.17549435e-38f && fabsf(x) <= 3.402823466e38f; };
-    int levels = 0;
-    for (int s = 0; s < hp.nspecies; ++s) levels += hp.levels[s];
-    bool ok = divisor(hp.total_bound) && fabsf(hp.total_bound) <= 1e6f;
-    if (threadIdx.x < levels && threadIdx.x < FFNO_MAX_LEVELS) {
-      const int g = threadIdx.x;
-      ok = ok && divisor(hp.std_y[g]) && isfinite(hp.log_g[g]) && isfinite(hp.ev[g]) && isfinite(hp.ndxi[g]) &&
-           isfinite(hp.dion[g]);
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (threadIdx.x == 0) tab[EXP_TAB] = ok ? 1.0 : 0.0;
-  }
-}
-__device__ __forceinline__ bool head_ordinary(const double* tab) {
-  return __double2hiint(tab[EXP_TAB]) != 0;   // an integer comparison: not on the FP64 pipe
 }
 
 __device__ __forceinline__ double rcp64(double x) {
@@ -247,11 +247,10 @@ struct HeadMath<float> {
   __device__ __forceinline__ float inv_(float x) const { return 1.f / x; }
 };
 
-__device__ __forceinline__ bool head_fast(const ffno_head_params& hp, const double* tab, const float* o, int nh,
-                                          const HeadInputs& in) {
+__device__ __forceinline__ bool head_fast(const HeadParams& hp, const float* o, int nh, const HeadInputs& in) {
   const float lt = fmaf(in.lt, hp.std_x[hp.temperature_channel], hp.mean_x[hp.temperature_channel]);
   const float ln = fmaf(in.lne, hp.std_x[hp.ne_channel], hp.mean_x[hp.ne_channel]);
-  bool ok = head_ordinary(tab) && lt > 0.5f && lt < 15.f && fabsf(ln) < 40.f;
+  bool ok = hp.ordinary && lt > 0.5f && lt < 15.f && fabsf(ln) < 40.f;
   for (int c = 0; c < nh; ++c) ok = ok && fabsf(o[c]) < 1e6f;
   return ok;
 }
@@ -318,7 +317,8 @@ struct HeadBase64 {
   }
 };
 // FP32 (the split-BF16 path): in pairs of floats (value and rounding error, 48 bits), by the error-free sum of Knuth and
-// the error-free product by fused multiply-add: 20 FP32 operations where the FP64 form has 6 at 1 / 64 of the rate.
+// the error-free product by fused multiply-add: 20 FP32 operations where the FP64 form has 6 at 1 / 64 of the rate. The
+// result, rounded to float, is the FP64 form's in all but 2 of 4 million random assemblies (log10 n of 5 to 40).
 __device__ __forceinline__ float two_sum(float a, float b, float& err) {
   const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
   err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
@@ -343,12 +343,12 @@ struct HeadBase32 {
 __device__ __forceinline__ HeadBase64 head_base(double b, double) { return HeadBase64(b); }
 __device__ __forceinline__ HeadBase32 head_base(double b, float) { return HeadBase32(b); }
 
-// Forward: out[g * V + v] = the normalised log10 population of level g. tab: fill_head_table's.
+// Forward: out[g * V + v] = the normalised log10 population of level g. tab: fill_exp_table's.
 template <typename T>
-__device__ __forceinline__ void head_voxel_fwd(const ffno_head_params& hp, const float* o, const HeadInputs& in,
+__device__ __forceinline__ void head_voxel_fwd(const HeadParams& hp, const float* o, const HeadInputs& in,
                                                float* __restrict__ out, long V, long v, const double* tab) {
   HeadMath<T> hm{tab, false};
-  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, tab, o, head_channels(hp), in);
+  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, o, head_channels(hp), in);
   const Lte<T> e(hp, in, hm);
   // the total term and the assembly of log10 n (log10 rho - log10 m + s ~ 20, minus mean_Y) stay beyond FP32 for both
   // T: in FP32 their rounding (~1e-6 dex at that magnitude, and a few ulp of b for tanh) would move every level of
@@ -367,7 +367,7 @@ __device__ __forceinline__ void head_voxel_fwd(const ffno_head_params& hp, const
     const double tb = (double)hp.total_bound;
     const float u = o[hc + L];
     const double th =
-        fabsf(u) < 1e6f && head_ordinary(tab) ? tanh_tab(tab, (double)u * rcp64(tb)) : tanh((double)u / tb);
+        hp.ordinary && fabsf(u) < 1e6f ? tanh_tab(tab, (double)u * rcp64(tb)) : tanh((double)u / tb);
     const auto base = head_base(lrho - (double)hp.log10_particle_mass[s] + tb * th, T(0));
     for (int i = 0; i < L; ++i) {
       const int g = lvl + i;
@@ -382,11 +382,11 @@ __device__ __forceinline__ void head_voxel_fwd(const ffno_head_params& hp, const
 // Backward: with ybar[g * V + v] the cotangent of the normalised output, overwrites o[0..nhp) with the gradient of the
 // head channels (zero past the last species) and writes x_in_bar[k * V + v] for every input channel k.
 template <typename T>
-__device__ __forceinline__ void head_voxel_bwd(const ffno_head_params& hp, float* o, int nhp, const HeadInputs& in,
+__device__ __forceinline__ void head_voxel_bwd(const HeadParams& hp, float* o, int nhp, const HeadInputs& in,
                                                const float* __restrict__ ybar, long V, long v,
                                                float* __restrict__ xinbar, const double* tab) {
   HeadMath<T> hm{tab, false};
-  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, tab, o, head_channels(hp), in);
+  if constexpr (sizeof(T) == 8) hm.fast = head_fast(hp, o, head_channels(hp), in);
   const Lte<T> e(hp, in, hm);
   T gsum = 0, ltb = 0, lneb = 0;
   int hc = 0, lvl = 0;

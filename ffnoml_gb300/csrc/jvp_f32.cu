@@ -353,13 +353,13 @@ template <int C, int NHP>
 __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* __restrict__ x, const float* __restrict__ xd,
                                                  const float* __restrict__ xin, const float* __restrict__ xind, long V,
                                                  const float* __restrict__ p1, const float* __restrict__ p2,
-                                                 const float* __restrict__ b2, ffno_head_params hp,
+                                                 const float* __restrict__ b2, HeadParams hp,
                                                  float* __restrict__ outd, int al) {
   griddep_sync();
   extern __shared__ __align__(16) float sm[];
-  __shared__ double etab[HEAD_TAB];
+  __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1, TAN = 2 * C * BM;
-  fill_head_table(hp, etab);
+  fill_exp_table(etab);
   float* as = sm;                 // [C][64] input, then [2C][64] hidden; their tangents TAN floats on
   float* os = as + 2 * TAN;       // [64][NHP + 1] head channels, then their tangents
   float* ods = os + BM * LO;
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(NT, C <= 64 ? 2 : 1) k_head_jvp(const float* _
         const float* od = ods + r * LO;
         const int tc = hp.temperature_channel, ec = hp.ne_channel, rc = hp.rho_channel;
         const HeadInputs in = head_inputs(hp, xin, V, v);
-        const HeadMath<double> hm{etab, head_fast(hp, etab, o, head_channels(hp), in)};
+        const HeadMath<double> hm{etab, head_fast(hp, o, head_channels(hp), in)};
         const Lte<double> le(hp, in, hm);
         const double dlt = (double)__ldg(xind + (long)tc * V + v) * (double)hp.std_x[tc];
         const double dlne = (double)__ldg(xind + (long)ec * V + v) * (double)hp.std_x[ec];

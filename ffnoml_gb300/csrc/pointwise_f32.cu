@@ -182,10 +182,11 @@ __global__ void __launch_bounds__(NT, 3) k_lift(const float* __restrict__ xin, i
 // One CTA per group, each thread a few partials: the group's mean is the weighted mean of the partials' means, and its
 // M2 the sum of the partials' M2 and of w (mean_p - mean)^2, so the loops hold no division (a serial Chan merge has two
 // dependent FP64 divisions per partial). Bound by latency: two passes over at most a few partials a thread, two
-// block-wide sums in a fixed tree (deterministic), one FP64 division. The groups take a CTA (an SM) each because the
-// FP64 rate of one SM (about two operations a cycle) would serialise eight groups of 304 partials. 304 partials,
-// 8 groups, C = 64: 22.0 us a launch with one warp per group and Chan merges -> 6.6 us (one SM: the groups' FP64 serialised; now a
-// chain of three block sums, a division and a square root).
+// block-wide sums in a fixed tree (deterministic), one FP64 division. The groups take a CTA each because the FP64 rate of
+// one SM (about two operations a cycle) would serialise eight groups of 304 partials; they spread over the SMs where the
+// device places them, and above width 64 the launch keeps them on different ones (ffno_gn_finalize has the figures).
+// 304 partials, 8 groups, C = 64: 22.0 us a launch in the form before (one CTA, a warp per group, Chan merges), 6.6 us in
+// this one (a chain of three block sums, a division and a square root).
 constexpr int FIN_NT = 128;
 
 __device__ __forceinline__ double block_sum(double v, double* red) {
@@ -525,13 +526,13 @@ template <int C, int NHP, typename T, bool kLte = true>
 __global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, const float* __restrict__ xin, long V,
                                              const float* __restrict__ p1, const float* __restrict__ p2,
                                              const float* __restrict__ b2, int nh,
-                                             const __grid_constant__ ffno_head_params hp, float* __restrict__ out,
+                                             const __grid_constant__ HeadParams hp, float* __restrict__ out,
                                              float* __restrict__ head_out, int al) {
   griddep_sync();
   extern __shared__ __align__(16) float sm[];
-  __shared__ double etab[HEAD_TAB];
+  __shared__ double etab[EXP_TAB];
   constexpr int LO = NHP + 1;
-  if (kLte) fill_head_table(hp, etab);
+  if (kLte) fill_exp_table(etab);
   float* as = sm;                    // [C][64] input, then [2C][64] hidden
   float* os = as + 2 * C * BM;       // [64][NHP + 1] head channels
   g32::Ring ring(os + BM * LO, g32::KC * 2 * C, al);
@@ -586,11 +587,11 @@ __global__ void __launch_bounds__(NT, 2) k_head(const float* __restrict__ x, con
 // written channels-first. Bound by HBM: (nh + 3 + levels) * 4 bytes a voxel.
 template <typename T>
 __global__ void __launch_bounds__(256) k_head_output(const float* __restrict__ head, const float* __restrict__ xin,
-                                                     long V, int nh, const __grid_constant__ ffno_head_params hp,
+                                                     long V, int nh, const __grid_constant__ HeadParams hp,
                                                      float* __restrict__ out) {
   griddep_sync();
-  __shared__ double etab[HEAD_TAB];
-  fill_head_table(hp, etab);
+  __shared__ double etab[EXP_TAB];
+  fill_exp_table(etab);
   __syncthreads();
   float o[FFNO_MAX_LEVELS + FFNO_MAX_SPECIES];
   for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < V; v += (long)gridDim.x * blockDim.x) {

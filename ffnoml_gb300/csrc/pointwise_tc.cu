@@ -1293,12 +1293,12 @@ __host__ __device__ constexpr uint32_t head_region(int C, int NHP, bool bwd) {
 template <int C, int NHP, typename T>
 __global__ void __launch_bounds__(CT, 1) k_head_tc(const float* __restrict__ x, const float* __restrict__ xin, long V,
                                                    const uint8_t* __restrict__ wpack, const float* __restrict__ b2,
-                                                   int nh, const __grid_constant__ ffno_head_params hp,
+                                                   int nh, const __grid_constant__ HeadParams hp,
                                                    float* __restrict__ out, float* __restrict__ head_out,
                                                    int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ double etab[HEAD_TAB];
-  fill_head_table(hp, etab);
+  __shared__ double etab[EXP_TAB];
+  fill_exp_table(etab);
   __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C), RB = head_region(C, NHP, false);
   constexpr int LO = NHP + 1;
@@ -1355,12 +1355,12 @@ template <int C, int NHP, typename T>
 __global__ void __launch_bounds__(CT, 1) k_head_bwd_tc(const float* __restrict__ x, const float* __restrict__ xin,
                                                        const float* __restrict__ ybar, long V,
                                                        const uint8_t* __restrict__ wpack, const float* __restrict__ b2,
-                                                       const __grid_constant__ ffno_head_params hp,
+                                                       const __grid_constant__ HeadParams hp,
                                                        float* __restrict__ xbar, float* __restrict__ xinbar,
                                                        int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ double etab[HEAD_TAB];
-  if (sizeof(T) == 8) fill_head_table(hp, etab);
+  __shared__ double etab[EXP_TAB];
+  if (sizeof(T) == 8) fill_exp_table(etab);
   __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C), RB = head_region(C, NHP, true);
   constexpr int LO = NHP + 1;
@@ -2135,13 +2135,13 @@ __global__ void __launch_bounds__(CT, 1) k_mix_tc96(const float* __restrict__ in
 template <int NHP, typename T>
 __global__ void __launch_bounds__(PT, 1) k_head_tc96(const float* __restrict__ x, const float* __restrict__ xin, long V,
                                                      const uint8_t* __restrict__ wpack, const float* __restrict__ b2,
-                                                     int nh, const __grid_constant__ ffno_head_params hp,
+                                                     int nh, const __grid_constant__ HeadParams hp,
                                                      float* __restrict__ out, float* __restrict__ head_out,
                                                      int* __restrict__ err) {
   constexpr int C = C96;
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ double etab[HEAD_TAB];
-  fill_head_table(hp, etab);
+  __shared__ double etab[EXP_TAB];
+  fill_exp_table(etab);
   __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C);
   PIPE_PROLOGUE(2 * C + NHP, 1)
@@ -2213,13 +2213,13 @@ __global__ void __launch_bounds__(PT, 1) k_head_bwd_tc96(const float* __restrict
                                                          const float* __restrict__ ybar, long V,
                                                          const uint8_t* __restrict__ wpack,
                                                          const float* __restrict__ b2,
-                                                         const __grid_constant__ ffno_head_params hp,
+                                                         const __grid_constant__ HeadParams hp,
                                                          float* __restrict__ xbar, float* __restrict__ xinbar,
                                                          int* __restrict__ err) {
   constexpr int C = C96;
   extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ double etab[HEAD_TAB];
-  if (sizeof(T) == 8) fill_head_table(hp, etab);
+  __shared__ double etab[EXP_TAB];
+  if (sizeof(T) == 8) fill_exp_table(etab);
   __syncthreads();
   constexpr uint32_t B1 = mat_bytes(2 * C, C), B2 = mat_bytes(NHP, 2 * C);
   constexpr uint32_t DO = 2 * C, D3 = 2 * C + NHP, D4 = 4 * C + NHP;
