@@ -283,19 +283,20 @@ def _weights_key(model):
     """Address and version of every parameter and buffer, in module order. Each call walks the modules as they are now
     (a replaced submodule, parameter or buffer changes the key): a plain walk over the registries, because this runs
     before the first launch of every call and Module.parameters() takes 2 ms of it on a model of 8 blocks (0.3 ms so)."""
-    items, stack, seen = [], [model], {id(model)}
+    items, stack, seen = [], [model], set()
     while stack:
         m = stack.pop()
+        if m._modules:                      # once each: a submodule may hold the model that holds it
+            if id(m) in seen:
+                continue
+            seen.add(id(m))
+            stack.extend(c for c in m._modules.values() if c is not None)
         for t in m._parameters.values():
             if t is not None:
                 items.append((t.data_ptr(), t._version))
         for t in m._buffers.values():
             if t is not None:
                 items.append((t.data_ptr(), t._version))
-        for c in m._modules.values():       # each module once: a submodule may hold the model that holds it
-            if c is not None and id(c) not in seen:
-                seen.add(id(c))
-                stack.append(c)
     return tuple(items)
 
 
@@ -1014,8 +1015,9 @@ class Executor:
     def backward(self, state, ybar, errs=None, heights=True):
         """Input VJP: ybar [B, L, D, H, W] -> (x_bar [B, Cin, D, H, W], z_bar [B, D, H, W]). errs: as in forward
         (the backward's flag and that of the forward that made the state). heights False: the caller takes no
-        gradient in the heights; z_bar is None and what only it needs (the height tables' gradient products and
-        their walk back to the columns, the z_proj and depth-weight terms) does not run."""
+        gradient in the heights; z_bar is None, and of what only it needs the height tables' gradient products,
+        their walk back to the columns, the z_proj term and the depth weights' own gradient do not run. (The gradient
+        in the depth weights, a per-voxel sum inside every GroupNorm backward, is still taken and then not used.)"""
         m = self.model
         x, z_scale, dx, dy = state["x"], state["z"], state["dx"], state["dy"]
         pk, geo, hgt, pln, pfr = self._setup(x, z_scale, dx, dy, state.get("geo"))
